@@ -90,13 +90,13 @@ typedef struct {
   int grad_accumulate;             // 1: add the weight gradient to what grad_home already holds
   int bank, no_self_push;          // cross-launch prefetch, see RtpLinearFwd
   const void* next_home; unsigned long long next_bytes; int next_kind;
-  // Optional row of M ones (bf16).  Where rtp_linear_bwd_folds_bias() says yes and dbias_full is null, the bias gradient
-  // is one more GEMM phase of the launch (ones[1, M] x dy[M, out], fp32 accumulation) and needs no column-sum kernel.
+  // Optional row of M ones (bf16).  Where rtp_linear_bwd_folds_bias() says yes and dbias_full is null, the launch makes the
+  // bias gradient itself (in fp32, beside the weight gradient) and needs no column-sum kernel.
   const void* ones;
 } RtpLinearBwd;
 int rtp_linear_bwd(const RtpRing* ring, const RtpLinearBwd* op, void* stream);
-// 1 if the launch described by `op` computes the bias gradient itself from op->ones (1-rank ring, tiles on single CTAs,
-// M a multiple of 8), 0 if the caller has to supply the column sums in dbias_full.
+// 1 if the launch described by `op` computes the bias gradient itself (1-rank ring, op->ones given, 16-byte aligned
+// operands), 0 if the caller has to supply the column sums in dbias_full.  Every other field must be as for the launch.
 int rtp_linear_bwd_folds_bias(const RtpRing* ring, const RtpLinearBwd* op);
 
 // Rotating experts (MoE): rank r owns n_local whole experts; x / y hold the dispatched tokens expert-major
@@ -124,6 +124,8 @@ typedef struct {
   const void* mask; long long ldmask; float mask_scale;   // optional activation backward applied to dx
 } RtpExpertBwd;
 int rtp_expert_bwd(const RtpRing* ring, const RtpExpertBwd* op, void* stream);
+// 1 if the launch makes the experts' bias gradients itself when dbias_full is null (1-rank ring, aligned operands).
+int rtp_expert_bwd_folds_bias(const RtpRing* ring, const RtpExpertBwd* op);
 int rtp_expert_fwd_emu(const RtpRing* rings, const RtpExpertFwd* ops, int world, void* stream);
 int rtp_expert_bwd_emu(const RtpRing* rings, const RtpExpertBwd* ops, int world, void* stream);
 

@@ -24,6 +24,7 @@
 #include <cstdlib>
 #include "api.h"
 #include "gemm_kernel.cuh"
+#include "gemm_local.h"
 #include "launch.h"
 #include "tmap.h"
 
@@ -489,13 +490,6 @@ int build_linear_fwd(const RtpRing& R, const RtpLinearFwd& op, RtpProgram& P) {
   return add_prefetch_pushes(R, P, op.next_home, op.next_bytes, 1 - op.bank, op.next_kind);
 }
 
-// Whether a backward launch computes its bias gradient as a GEMM phase of its own (see RtpLinearBwd::ones).  Needs the
-// pair decision of the launch to have been made (decide_pair).
-bool folds_bias(const RtpRing& R, const RtpLinearBwd& op) {
-  return R.world == 1 && !pair_mode() && op.M % 8 == 0 && op.out_features % 8 == 0 &&
-         (reinterpret_cast<uintptr_t>(op.ones) & 15) == 0;
-}
-
 int build_linear_bwd(const RtpRing& R, const RtpLinearBwd& op, RtpProgram& P) {
   // Backward on a ring of N ranks.  Rank r visits the shards in the order r-1, r-2, ..., r (step s handles shard
   // j = r-1-s; weights are pushed by their owners into weight slot s).  The weight gradient of shard j computed here
@@ -634,23 +628,6 @@ int build_linear_bwd(const RtpRing& R, const RtpLinearBwd& op, RtpProgram& P) {
       }
       set_vec_ok(ph);
     }
-  }
-  if (op.bias_off >= 0 && !op.dbias_full && op.ones && folds_bias(R, op)) {
-    // ---- bias gradient as a GEMM: db[1, out] = ones[1, M] dy[M, out].  One row of A is real, the rest of the 128-row
-    //      tile is zero fill; the few extra tiles ride in the grid beside the weight-gradient tiles.
-    if (make_map_k(&P.maps[4], op.ones, 1, op.M, op.M)) return -1;
-    if (make_map_mn3(&P.maps[5], op.dy, op.out_features, op.M, op.ldy, (op.out_features % 64 == 0) ? 2 : 0, &P.map3d[5]))
-      return -1;
-    RtpPhase& ph = P.phases[np++];
-    init_phase(ph);
-    ph.a_map = 4; ph.a_mn = 0;
-    ph.b_map = 5; ph.b_mn = 1;
-    ph.M = 1; ph.N = op.out_features; ph.K = op.M;
-    ph.bn = 128;
-    __nv_bfloat16* db = reinterpret_cast<__nv_bfloat16*>(op.grad_home) + op.bias_off;
-    ph.d = db; ph.ldd = op.out_features;
-    if (op.grad_accumulate) { ph.c = db; ph.ldc = op.out_features; }
-    set_vec_ok(ph);
   }
   // The weight-gradient phases need only local operands, so they all come first and cover the time the weight shards
   // are in flight; the input-gradient phases follow, own shard first, then the visiting shards in order of arrival.
@@ -1076,6 +1053,99 @@ int build_reduce_blocks(const RtpRing& R, const RtpReduceBlocks& op, RtpProgram&
   return 0;
 }
 
+// ------------------------------------------------------------------------------------------------
+// rings of one rank: the same layers as plain GEMM jobs (gemm_local.cu)
+// ------------------------------------------------------------------------------------------------
+int run_local(const rtp::LocalGemm* jobs, int n, unsigned long long* status, unsigned long long timeout_ns, void* stream) {
+  if (!status) return fail("status word required");
+  if (rtp::local_gemm(jobs, n, pair_policy(), status, timeout_ns ? timeout_ns : 2000000000ull, (cudaStream_t)stream))
+    return fail(rtp::local_gemm_error());
+  return 0;
+}
+int run_local(const RtpRing& R, const rtp::LocalGemm* jobs, int n, void* stream) {
+  if (!R.ws[0]) return fail("ring workspace required");
+  return run_local(jobs, n, &ws_flags(R.ws[0])->status.v, R.timeout_ns, stream);
+}
+bool all_ok(const rtp::LocalGemm* jobs, int n) {
+  for (int i = 0; i < n; ++i)
+    if (!rtp::local_gemm_ok(jobs[i])) return false;
+  return true;
+}
+// The jobs of a launch on a ring of one rank; 0: the launch is not one for the local kernels.  A timeline (g_trace) is
+// only written by the rotation kernel.
+int local_linear_fwd(const RtpRing& R, const RtpLinearFwd& op, rtp::LocalGemm* j) {
+  if (R.world != 1 || g_trace || op.shard_bytes % 16 || op.bank < 0 || op.bank >= RTP_NUM_WBANKS) return 0;
+  j[0] = rtp::LocalGemm{};
+  j[0].a = op.x; j[0].lda = op.ldx; j[0].b = op.home; j[0].ldb = op.in_features;
+  j[0].M = op.M; j[0].N = op.out_features; j[0].K = op.in_features;
+  j[0].d = op.y; j[0].ldd = op.ldy;
+  if (op.bias_off >= 0) j[0].bias = reinterpret_cast<const __nv_bfloat16*>(op.home) + op.bias_off;
+  j[0].act = op.act;
+  j[0].drop_p = op.drop_p; j[0].seed = op.seed; j[0].offset = op.offset; j[0].step_ptr = op.step_ptr;
+  return all_ok(j, 1) ? 1 : 0;
+}
+int local_linear_bwd(const RtpRing& R, const RtpLinearBwd& op, rtp::LocalGemm* j) {
+  if (R.world != 1 || g_trace || op.dbias_full || op.bank < 0 || op.bank >= RTP_NUM_WBANKS) return 0;
+  int n = 0;
+  rtp::LocalGemm& w = j[n++] = rtp::LocalGemm{};      // dW = dy^T x, bias gradient = column sums of dy
+  w.a = op.dy; w.lda = op.ldy; w.a_mn = 1; w.b = op.x; w.ldb = op.ldx; w.b_mn = 1;
+  w.M = op.out_features; w.N = op.in_features; w.K = op.M;
+  w.d = op.grad_home; w.ldd = op.in_features;
+  if (op.grad_accumulate) { w.c = op.grad_home; w.ldc = op.in_features; }
+  if (op.bias_off >= 0 && op.ones) {
+    w.bsum = reinterpret_cast<__nv_bfloat16*>(op.grad_home) + op.bias_off;
+    w.bsum_add = op.grad_accumulate;
+  }
+  if (op.dx) {
+    rtp::LocalGemm& d = j[n++] = rtp::LocalGemm{};    // dx = dy W
+    d.a = op.dy; d.lda = op.ldy; d.b = op.home; d.ldb = op.in_features; d.b_mn = 1;
+    d.M = op.M; d.N = op.in_features; d.K = op.out_features;
+    d.d = op.dx; d.ldd = op.lddx;
+    if (op.dx_accumulate) { d.c = op.dx; d.ldc = op.lddx; }
+    d.mask = op.mask; d.ldmask = op.ldmask; d.mask_scale = op.mask_scale;
+  }
+  return all_ok(j, n) ? n : 0;
+}
+int local_expert_fwd(const RtpRing& R, const RtpExpertFwd& op, rtp::LocalGemm* j) {
+  if (R.world != 1 || g_trace || op.n_local < 1 || op.n_local > rtp::kLocalMaxJobs) return 0;
+  for (int e = 0; e < op.n_local; ++e) {
+    const __nv_bfloat16* w = reinterpret_cast<const __nv_bfloat16*>(op.home) + e * op.expert_stride;
+    j[e] = rtp::LocalGemm{};
+    j[e].a = reinterpret_cast<const __nv_bfloat16*>(op.x) + (long long)e * op.cap * op.ldx; j[e].lda = op.ldx;
+    j[e].b = w; j[e].ldb = op.in_features;
+    j[e].M = op.cap; j[e].N = op.out_features; j[e].K = op.in_features;
+    j[e].d = reinterpret_cast<__nv_bfloat16*>(op.y) + (long long)e * op.cap * op.ldy; j[e].ldd = op.ldy;
+    if (op.bias_off >= 0) j[e].bias = w + op.bias_off;
+    j[e].act = op.act;
+  }
+  return all_ok(j, op.n_local) ? op.n_local : 0;
+}
+int local_expert_bwd(const RtpRing& R, const RtpExpertBwd& op, rtp::LocalGemm* j) {
+  if (R.world != 1 || g_trace || op.dbias_full || op.n_local < 1 || 2 * op.n_local > rtp::kLocalMaxJobs) return 0;
+  int n = 0;
+  for (int e = 0; e < op.n_local; ++e) {
+    const __nv_bfloat16* dy = reinterpret_cast<const __nv_bfloat16*>(op.dy) + (long long)e * op.cap * op.ldy;
+    __nv_bfloat16* g = reinterpret_cast<__nv_bfloat16*>(op.grad_home) + e * op.expert_stride;
+    rtp::LocalGemm& w = j[n++] = rtp::LocalGemm{};
+    w.a = dy; w.lda = op.ldy; w.a_mn = 1;
+    w.b = reinterpret_cast<const __nv_bfloat16*>(op.x) + (long long)e * op.cap * op.ldx; w.ldb = op.ldx; w.b_mn = 1;
+    w.M = op.out_features; w.N = op.in_features; w.K = op.cap;
+    w.d = g; w.ldd = op.in_features;
+    if (op.bias_off >= 0) w.bsum = g + op.bias_off;
+    if (!op.dx) continue;
+    rtp::LocalGemm& d = j[n++] = rtp::LocalGemm{};
+    d.a = dy; d.lda = op.ldy;
+    d.b = reinterpret_cast<const __nv_bfloat16*>(op.home) + e * op.expert_stride; d.ldb = op.in_features; d.b_mn = 1;
+    d.M = op.cap; d.N = op.in_features; d.K = op.out_features;
+    d.d = reinterpret_cast<__nv_bfloat16*>(op.dx) + (long long)e * op.cap * op.lddx; d.ldd = op.lddx;
+    if (op.mask) {
+      d.mask = reinterpret_cast<const __nv_bfloat16*>(op.mask) + (long long)e * op.cap * op.ldmask;
+      d.ldmask = op.ldmask; d.mask_scale = op.mask_scale;
+    }
+  }
+  return all_ok(j, n) ? n : 0;
+}
+
 template <int NEMU, class Op, class Builder>
 int run_emu(const RtpRing* rings, const Op* ops, Builder build, cudaStream_t stream) {
   decide_pair(0, 0, 0, false);   // emulated ranks share one cooperative launch without clusters
@@ -1369,6 +1439,15 @@ int rtp_gemm(const RtpGemmArgs* a, void* stream) {
   RtpProgram& P = params.prog[0];
   init_program(P);
   if (a->M <= 0 || a->N <= 0 || a->K <= 0) return fail("empty GEMM");
+  if (!a->num_ctas && !a->bn && !a->d_fp32 && !(a->c && a->c_fp32) && !g_trace) {
+    rtp::LocalGemm j = {};
+    j.a = a->a; j.lda = a->lda; j.a_mn = a->a_mn; j.b = a->b; j.ldb = a->ldb; j.b_mn = a->b_mn;
+    j.M = a->M; j.N = a->N; j.K = a->K;
+    j.d = a->d; j.ldd = a->ldd; j.c = a->c; j.ldc = a->ldc; j.bias = a->bias; j.act = a->act;
+    j.mask = a->mask; j.ldmask = a->ldmask; j.mask_scale = a->mask_scale;
+    j.drop_p = a->drop_p; j.seed = a->seed; j.offset = a->offset; j.step_ptr = a->step_ptr;
+    if (rtp::local_gemm_ok(j)) return run_local(&j, 1, a->status, 0, stream);
+  }
   if (a->a_mn ? make_map_mn3(&P.maps[0], a->a, a->M, a->K, a->lda, 2, &P.map3d[0]) : make_map_k(&P.maps[0], a->a, a->M, a->K, a->lda))
     return -1;
   const int ctas = a->num_ctas > 0 ? a->num_ctas : sm_count();
@@ -1443,6 +1522,8 @@ int rtp_gemm_batched(const RtpGemmBatched* a, void* stream) {
 }
 
 int rtp_linear_fwd(const RtpRing* ring, const RtpLinearFwd* op, void* stream) {
+  rtp::LocalGemm jobs[rtp::kLocalMaxJobs];
+  if (const int n = local_linear_fwd(*ring, *op, jobs)) return run_local(*ring, jobs, n, stream);
   static thread_local rtp::GemmParams<1> params;
   // CTA pairs by size, on any ring (the pair protocol is local to one GPU; checked against an fp32 oracle on real rings)
   decide_pair(op->M, ring->world > 1 && op->mode == 0 ? op->out_features / ring->world : op->out_features, ring->ctas);
@@ -1453,6 +1534,8 @@ int rtp_linear_fwd(const RtpRing* ring, const RtpLinearFwd* op, void* stream) {
   return launch<1>(params, ring->ctas, false, (cudaStream_t)stream, true);
 }
 int rtp_linear_bwd(const RtpRing* ring, const RtpLinearBwd* op, void* stream) {
+  rtp::LocalGemm jobs[rtp::kLocalMaxJobs];
+  if (const int n = local_linear_bwd(*ring, *op, jobs)) return run_local(*ring, jobs, n, stream);
   static thread_local rtp::GemmParams<1> params;
   // CTA pairs by the size of the input-gradient GEMM [M, in-per-shard], on any ring
   decide_pair(op->M, op->mode == 0 ? op->in_features : op->in_features / ring->world, ring->ctas);
@@ -1463,10 +1546,12 @@ int rtp_linear_bwd(const RtpRing* ring, const RtpLinearBwd* op, void* stream) {
   return launch<1>(params, ring->ctas, false, (cudaStream_t)stream, true);
 }
 int rtp_linear_bwd_folds_bias(const RtpRing* ring, const RtpLinearBwd* op) {
-  decide_pair(op->M, op->mode == 0 ? op->in_features : op->in_features / ring->world, ring->ctas);
-  return (op->bias_off >= 0 && op->ones && folds_bias(*ring, *op)) ? 1 : 0;
+  rtp::LocalGemm jobs[rtp::kLocalMaxJobs];
+  return op->bias_off >= 0 && op->ones && local_linear_bwd(*ring, *op, jobs) ? 1 : 0;
 }
 int rtp_expert_fwd(const RtpRing* ring, const RtpExpertFwd* op, void* stream) {
+  rtp::LocalGemm jobs[rtp::kLocalMaxJobs];
+  if (const int n = local_expert_fwd(*ring, *op, jobs)) return run_local(*ring, jobs, n, stream);
   static thread_local rtp::GemmParams<1> params;
   decide_pair(0, 0, ring->ctas);   // pairs only when forced
   if (build_expert_fwd(*ring, *op, params.prog[0])) return -1;
@@ -1474,7 +1559,13 @@ int rtp_expert_fwd(const RtpRing* ring, const RtpExpertFwd* op, void* stream) {
   params.ctas_per_rank = ring->ctas;
   return launch<1>(params, ring->ctas, false, (cudaStream_t)stream, true);
 }
+int rtp_expert_bwd_folds_bias(const RtpRing* ring, const RtpExpertBwd* op) {
+  rtp::LocalGemm jobs[rtp::kLocalMaxJobs];
+  return op->bias_off >= 0 && local_expert_bwd(*ring, *op, jobs) ? 1 : 0;
+}
 int rtp_expert_bwd(const RtpRing* ring, const RtpExpertBwd* op, void* stream) {
+  rtp::LocalGemm jobs[rtp::kLocalMaxJobs];
+  if (const int n = local_expert_bwd(*ring, *op, jobs)) return run_local(*ring, jobs, n, stream);
   static thread_local rtp::GemmParams<1> params;
   decide_pair(0, 0, ring->ctas);   // pairs only when forced
   if (build_expert_bwd(*ring, *op, params.prog[0])) return -1;

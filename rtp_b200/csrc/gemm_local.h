@@ -1,0 +1,37 @@
+// GEMMs of a ring of one rank: nothing is pushed, nothing is waited for, so a launch needs only a few jobs
+// D = epilogue(A * B^T (+ C)) that share one grid (see gemm_local.cu).  Host interface, used by gemm.cu.
+#pragma once
+#include <cuda.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace rtp {
+
+struct LocalGemm {
+  // operands (bf16), rows [M, K] or, with *_mn, stored [K, M]; likewise B with N
+  const void* a; long long lda; int a_mn;
+  const void* b; long long ldb; int b_mn;
+  int M, N, K;
+  // epilogue: (+ c) -> (+ bias) -> activation -> mask -> dropout, bf16 result
+  void* d; long long ldd;
+  const void* c; long long ldc;
+  const void* bias;
+  int act;
+  const void* mask; long long ldmask; float mask_scale;
+  float drop_p;
+  unsigned long long seed, offset;
+  const unsigned long long* step_ptr;
+  // column sums of A (a_mn = 1 only): bsum[m] (+)= sum_k A[m, k], in bf16
+  void* bsum; int bsum_add;
+};
+
+// Whether the local kernels take this job (16-byte aligned rows, N a multiple of 8).
+bool local_gemm_ok(const LocalGemm& g);
+// One launch for all jobs (1 .. kLocalMaxJobs), whose outputs are disjoint and whose inputs are no job's output.
+// `pair_policy`: 0 never on CTA pairs, 1 always, -1 by the cost model.
+constexpr int kLocalMaxJobs = 16;
+int local_gemm(const LocalGemm* jobs, int n, int pair_policy, unsigned long long* status, unsigned long long timeout_ns,
+               cudaStream_t stream);
+const char* local_gemm_error();
+
+}  // namespace rtp

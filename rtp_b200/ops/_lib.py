@@ -203,6 +203,7 @@ def lib():
         L.rtp_linear_fwd_emu.argtypes = [C.POINTER(Ring), C.POINTER(LinearFwd), C.c_int, C.c_void_p]
         L.rtp_linear_bwd_emu.argtypes = [C.POINTER(Ring), C.POINTER(LinearBwd), C.c_int, C.c_void_p]
         L.rtp_linear_bwd_folds_bias.argtypes = [C.POINTER(Ring), C.POINTER(LinearBwd)]
+        L.rtp_expert_bwd_folds_bias.argtypes = [C.POINTER(Ring), C.POINTER(ExpertBwd)]
         _lib = L
     return _lib
 

@@ -277,17 +277,16 @@ def linear_bwd_raw(eng, flat, layout_info, x2d, dy2d, row, in_f, out_f, need_dx=
     if dx is not None:
         op.dx, op.lddx = dx.data_ptr(), dx.stride(0)
     op.grad_home = gflat.data_ptr()
-    if has_bias:
-        # On a 1-rank ring the bias gradient is one more GEMM phase of the launch (a row of ones times dy); elsewhere
-        # the column sums of dy come from a kernel of their own.
-        op.ones = eng.ones_row(M).data_ptr()
-        if not _lib.lib().rtp_linear_bwd_folds_bias(C.byref(eng.ring), C.byref(op)):
-            op.ones = None
-            op.dbias_full = K.colsum(dy2d, dbias_buf).data_ptr()
     if mask is not None:
         op.mask, op.ldmask, op.mask_scale = mask.data_ptr(), mask.stride(0), mask_scale
     op.dx_accumulate = int(dx_accumulate)
     _set_prefetch(op, bank, pushed, next_flat, next_kind)
+    if has_bias:
+        # On a 1-rank ring the launch sums the columns of dy itself; elsewhere they come from a kernel of their own.
+        op.ones = eng.ones_row(M).data_ptr()
+        if not _lib.lib().rtp_linear_bwd_folds_bias(C.byref(eng.ring), C.byref(op)):
+            op.ones = None
+            op.dbias_full = K.colsum(dy2d, dbias_buf).data_ptr()
     _lib.check(_lib.lib().rtp_linear_bwd(C.byref(eng.ring), C.byref(op), _lib.stream_ptr()), "rtp_linear_bwd")
     return dx, gflat
 
@@ -897,11 +896,6 @@ class _FusedExpertLinearFn(torch.autograd.Function):
         need_dx = ctx.needs_input_grad[1]
         dx = torch.empty(E * cap, in_f, dtype=torch.bfloat16, device=dy.device) if need_dx else None
         gflat = torch.empty_like(flat)
-        dbias = None
-        if bias_off >= 0:
-            dbias = torch.empty(E, out_f, dtype=torch.float32, device=dy.device)
-            for g in range(E):
-                K.colsum(dy2[g * cap:(g + 1) * cap], dbias[g])
         op = _lib.ExpertBwd()
         op.cap, op.n_local, op.in_features, op.out_features = cap, L, in_f, out_f
         op.home, op.expert_stride, op.bias_off = flat.data_ptr(), stride, bias_off
@@ -910,7 +904,11 @@ class _FusedExpertLinearFn(torch.autograd.Function):
         if dx is not None:
             op.dx, op.lddx = dx.data_ptr(), in_f
         op.grad_home = gflat.data_ptr()
-        op.dbias_full = dbias.data_ptr() if dbias is not None else None
+        if bias_off >= 0 and not _lib.lib().rtp_expert_bwd_folds_bias(C.byref(ctx.eng.ring), C.byref(op)):
+            dbias = torch.empty(E, out_f, dtype=torch.float32, device=dy.device)
+            for g in range(E):
+                K.colsum(dy2[g * cap:(g + 1) * cap], dbias[g])
+            op.dbias_full = dbias.data_ptr()
         _lib.check(_lib.lib().rtp_expert_bwd(C.byref(ctx.eng.ring), C.byref(op), _lib.stream_ptr()), "rtp_expert_bwd")
         grads = [gflat[off:off + n].view(shape) for off, n, shape in places]
         return (None, dx.view(E, cap, in_f) if dx is not None else None, *grads)
