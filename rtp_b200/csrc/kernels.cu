@@ -347,6 +347,104 @@ __global__ void ce_kernel(__nv_bfloat16* logits, long long ld, const long long* 
   }
 }
 
+// The same with the row in registers: every logit is read once and every gradient written once.  A block of 512 threads
+// takes one row, NG 16-byte words a thread, all in flight at once; two blocks share an SM, so that one loads or stores
+// while the other computes.  The two exponentials a logit (16 a clock and SM) and the unpacking bound it, not memory:
+// 4096 x 32000 162 -> 126 us, 8192 x 50304 553 -> 540, 1024 x 8192 9.7 -> 9.1 against the kernel above, which reads a row
+// three times, twice from L2.  Tried and dropped: the row in shared memory, filled and drained by bulk copies (604 us at
+// 50304 logits); 1024 threads with half the words (642 us, one block per SM); unpacking anew in every pass instead of
+// letting the compiler spill what does not fit (720 us).
+constexpr int kCeThreads = 512;
+constexpr int kCeMaxV = 65536;
+template <int NG>
+__global__ void __launch_bounds__(kCeThreads, 2) ce_row_kernel(
+    const __nv_bfloat16* logits, long long ld, const long long* __restrict__ target, float* __restrict__ loss, int V,
+    float grad_scale, const float* __restrict__ scale_ptr, long long ignore_index, __nv_bfloat16* grad, long long ldg) {
+  __shared__ float red[32];
+  constexpr float kLog2e = 1.4426950408889634f;
+  const int row = blockIdx.x, tid = threadIdx.x, n = V >> 3;
+  const uint4* lp = reinterpret_cast<const uint4*>(logits + (size_t)row * ld);
+  const long long t = target[row];
+  const bool ignored = t == ignore_index || t < 0 || t >= V;
+  uint4 u[NG];
+  const uint32_t kNegInf2 = 0xff80ff80u;                 // two bf16 -inf: words beyond the row count for nothing
+#pragma unroll
+  for (int q = 0; q < NG; ++q) {
+    const int i = q * kCeThreads + tid;
+    u[q] = i < n ? __ldcs(lp + i) : make_uint4(kNegInf2, kNegInf2, kNegInf2, kNegInf2);
+  }
+  const float lt = (tid == 0 && !ignored) ? __bfloat162float(logits[(size_t)row * ld + t]) : 0.f;
+  if (scale_ptr) grad_scale *= __ldg(scale_ptr);
+  float mx = -INFINITY;
+#pragma unroll
+  for (int q = 0; q < NG; ++q) {
+    float v[8];
+    unpack8(u[q], v);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) mx = fmaxf(mx, v[k]);
+  }
+  mx = block_max(mx, red);
+  float se = 0.f;
+#pragma unroll
+  for (int q = 0; q < NG; ++q) {
+    if (q * kCeThreads + tid < n) {
+      float v[8];
+      unpack8(u[q], v);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) se += exp2f((v[k] - mx) * kLog2e);
+    }
+  }
+  se = block_sum(se, red);
+  if (tid == 0) loss[row] = ignored ? 0.f : mx + __logf(se) - lt;
+  if (!grad) return;
+  const float sc = grad_scale / se;
+  uint4* gp = reinterpret_cast<uint4*>(grad + (size_t)row * ldg);
+#pragma unroll
+  for (int q = 0; q < NG; ++q) {
+    const int i = q * kCeThreads + tid;
+    if (i < n) {
+      float v[8];
+      unpack8(u[q], v);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        v[k] = exp2f((v[k] - mx) * kLog2e) * sc;
+        if (i * 8 + k == (int)t) v[k] -= grad_scale;
+        if (ignored) v[k] = 0.f;
+      }
+      __stcs(gp + i, pack8(v));
+    }
+  }
+}
+
+// n = number of targets that count (at least one), for the mean: out[0] = n, out[1] = 1 / n.
+__global__ void ce_count_kernel(const long long* __restrict__ target, int M, long long ignore_index, float* out) {
+  __shared__ int total;
+  int c = 0;
+  for (int i = threadIdx.x; i < M; i += blockDim.x) c += target[i] != ignore_index;
+  c = __reduce_add_sync(0xffffffffu, c);
+  if (threadIdx.x == 0) total = 0;
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) atomicAdd(&total, c);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const float n = (float)max(total, 1);
+    out[0] = n;
+    out[1] = 1.f / n;
+  }
+}
+// g *= *scale, except by one: the usual gradient of a loss costs no pass over the logits' gradient.
+__global__ void scale_unless_one_kernel(__nv_bfloat16* g, const float* __restrict__ scale, long long n8) {
+  const float s = __ldg(scale);
+  if (s == 1.f) return;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n8; i += (long long)gridDim.x * blockDim.x) {
+    float v[8];
+    unpack8(reinterpret_cast<const uint4*>(g)[i], v);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] *= s;
+    reinterpret_cast<uint4*>(g)[i] = pack8(v);
+  }
+}
+
 // ------------------------------------------------------------------------------------------------
 // Embedding gather for one visiting table shard [V, Ds]: out[t, col_off + c] =
 //   dropout(table[ids[t], c] * scale + pe[t / tokens_per_pos, col_off + c])
@@ -1122,13 +1220,13 @@ __global__ void cast_f32_bf16_kernel(const float* in, __nv_bfloat16* out, long l
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i < n) out[i] = __float2bfloat16(in[i] * scale);
 }
-// sum of fp32 vector * scale -> out[0] (single block)
-__global__ void sum_kernel(const float* in, float* out, int n, float scale) {
+// sum of fp32 vector * scale (/ *divisor) -> out[0] (single block)
+__global__ void sum_kernel(const float* in, float* out, int n, float scale, const float* __restrict__ divisor) {
   __shared__ float red[32];
   float s = 0.f;
   for (int i = threadIdx.x; i < n; i += blockDim.x) s += in[i];
   s = block_sum(s, red);
-  if (threadIdx.x == 0) out[0] = s * scale;
+  if (threadIdx.x == 0) out[0] = divisor ? s * scale / *divisor : s * scale;
 }
 
 }  // namespace
@@ -1180,11 +1278,44 @@ int rtp_cross_entropy(void* logits, long long ld, const long long* target, float
 }
 int rtp_cross_entropy_to(void* logits, long long ld, const long long* target, float* loss, int M, int V, float grad_scale,
                          long long ignore_index, int write_grad, void* grad, long long ldg, void* stream) {
+  return rtp_cross_entropy_scaled(logits, ld, target, loss, M, V, grad_scale, nullptr, ignore_index, write_grad, grad, ldg, stream);
+}
+int rtp_cross_entropy_scaled(void* logits, long long ld, const long long* target, float* loss, int M, int V, float grad_scale,
+                             const float* scale_ptr, long long ignore_index, int write_grad, void* grad, long long ldg,
+                             void* stream) {
   if (V % 8 || ld % 8 || (grad && ldg % 8)) { k_err = "cross_entropy: V and the row pitches must be multiples of 8"; return -1; }
+  if (M > 0 && V > 0 && V <= kCeMaxV) {
+#define RTP_CE(NG)                                                                                                        \
+  ce_row_kernel<NG><<<M, kCeThreads, 0, (cudaStream_t)stream>>>(                                                          \
+      (const __nv_bfloat16*)logits, ld, target, loss, V, grad_scale, scale_ptr, ignore_index,                             \
+      (__nv_bfloat16*)(write_grad ? (grad ? grad : logits) : nullptr), grad ? ldg : ld)
+    const int ng = (V / 8 + kCeThreads - 1) / kCeThreads;
+    if (ng == 1) RTP_CE(1); else if (ng == 2) RTP_CE(2); else if (ng == 3) RTP_CE(3); else if (ng == 4) RTP_CE(4);
+    else if (ng <= 6) RTP_CE(6); else if (ng <= 8) RTP_CE(8); else if (ng <= 10) RTP_CE(10); else if (ng <= 13) RTP_CE(13);
+    else RTP_CE(16);
+#undef RTP_CE
+    LAUNCH_CHECK("cross_entropy");
+    return 0;
+  }
+  if (scale_ptr) { k_err = "cross_entropy: a device-side scale needs rows of at most 65536 logits"; return -1; }
   const int grid = M < 148 * 8 ? M : 148 * 8;
   ce_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>((__nv_bfloat16*)logits, ld, target, loss, M, V, grad_scale,
                                                     ignore_index, write_grad, (__nv_bfloat16*)grad, ldg);
   LAUNCH_CHECK("cross_entropy");
+  return 0;
+}
+int rtp_ce_count(const long long* target, int M, long long ignore_index, float* out2, void* stream) {
+  ce_count_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(target, M, ignore_index, out2);
+  LAUNCH_CHECK("ce_count");
+  return 0;
+}
+int rtp_scale_unless_one(void* g, const float* scale, long long n, void* stream) {
+  if (n % 8 || (reinterpret_cast<uintptr_t>(g) & 15)) { k_err = "scale: n must be a multiple of 8 and the buffer aligned"; return -1; }
+  if (n == 0) return 0;
+  const long long blocks = (n / 8 + 255) / 256;
+  scale_unless_one_kernel<<<(int)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, (cudaStream_t)stream>>>((__nv_bfloat16*)g, scale,
+                                                                                                     n / 8);
+  LAUNCH_CHECK("scale");
   return 0;
 }
 int rtp_embed_fwd(const void* table, const long long* ids, const void* pe, long long ld_pe, int tokens_per_pos,
@@ -1397,8 +1528,8 @@ int rtp_cast_f32_bf16(const float* in, void* out, long long n, float scale, void
   LAUNCH_CHECK("cast");
   return 0;
 }
-int rtp_sum_f32(const float* in, float* out, int n, float scale, void* stream) {
-  sum_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(in, out, n, scale);
+int rtp_sum_f32(const float* in, float* out, int n, float scale, const float* divisor, void* stream) {
+  sum_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(in, out, n, scale, divisor);
   LAUNCH_CHECK("sum");
   return 0;
 }

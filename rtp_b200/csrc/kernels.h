@@ -28,6 +28,14 @@ int rtp_cross_entropy(void* logits, long long ld, const long long* target, float
 // Same, but the gradient goes to `grad` (row pitch ldg) and the logits stay as they are; grad = null: in place.
 int rtp_cross_entropy_to(void* logits, long long ld, const long long* target, float* loss, int M, int V, float grad_scale,
                          long long ignore_index, int write_grad, void* grad, long long ldg, void* stream);
+// Same with a device-side factor of the gradient (scale_ptr, may be null; rows of at most 65536 logits).
+int rtp_cross_entropy_scaled(void* logits, long long ld, const long long* target, float* loss, int M, int V, float grad_scale,
+                             const float* scale_ptr, long long ignore_index, int write_grad, void* grad, long long ldg,
+                             void* stream);
+// out2[0] = max(1, number of targets other than ignore_index), out2[1] = its reciprocal
+int rtp_ce_count(const long long* target, int M, long long ignore_index, float* out2, void* stream);
+// bf16 g[n] *= *scale (n % 8 == 0, 16-byte aligned); nothing is read or written when *scale is one
+int rtp_scale_unless_one(void* g, const float* scale, long long n, void* stream);
 int rtp_embed_fwd(const void* table, const long long* ids, const void* pe, long long ld_pe, int tokens_per_pos,
                   void* out, long long ld_out, int col_off, int T, int Ds, int D, float scale, float drop_p,
                   unsigned long long seed, unsigned long long offset, const unsigned long long* step_ptr,
@@ -92,7 +100,8 @@ int rtp_moe_gather(const void* src, const int* slot, const float* scale, void* d
 int rtp_moe_rowdot(const void* a, const void* b, const int* slot, float* out, int S, int M, void* stream);
 int rtp_add(const void* a, const void* b, void* out, long long n, void* stream);
 int rtp_cast_f32_bf16(const float* in, void* out, long long n, float scale, void* stream);
-int rtp_sum_f32(const float* in, float* out, int n, float scale, void* stream);
+// out[0] = scale * sum(in) (/ *divisor when given)
+int rtp_sum_f32(const float* in, float* out, int n, float scale, const float* divisor, void* stream);
 
 #ifdef __cplusplus
 }

@@ -91,33 +91,48 @@ def rms_norm(x, weight, eps=1e-5):
 
 
 class _CrossEntropyFn(torch.autograd.Function):
-    """Mean token cross-entropy of bf16 logits.  The input is never modified: the softmax gradient, produced in the same
-    pass over the logits, goes to a buffer of its own, and only when the logits need a gradient."""
+    """Mean (or, with ``mean=False``, summed) token cross-entropy of bf16 logits.  The input is never modified: the softmax
+    gradient, produced in the same pass over the logits and already divided by the number of tokens, goes to a buffer of
+    its own, and only when the logits need a gradient.  ``backward`` multiplies it by the incoming gradient, which for a
+    loss that is differentiated itself is one and costs nothing."""
 
     @staticmethod
-    def forward(ctx, logits, target, ignore_index):
+    def forward(ctx, logits, target, ignore_index, mean):
         from . import kernels as K
         lg = logits.reshape(-1, logits.shape[-1])
         if lg.stride(1) != 1 or lg.stride(0) % 8:
             lg = lg.contiguous()
         t = target.reshape(-1)
-        n = (t != ignore_index).sum().clamp(min=1)
         grad = torch.empty(lg.shape, dtype=lg.dtype, device=lg.device) if ctx.needs_input_grad[0] else None
-        rows = K.cross_entropy_to(lg, t, grad, grad_scale=1.0, ignore_index=ignore_index)
-        ctx.save_for_backward(grad, n)
+        if K.cross_entropy_one_read(lg):
+            t = t.contiguous()
+            cnt = K.ce_count(t, ignore_index) if mean else None
+            rows = K.cross_entropy_to(lg, t, grad, scale=cnt[1:] if mean else None, ignore_index=ignore_index)
+            loss = K.sum_f32(rows, torch.empty((), dtype=torch.float32, device=lg.device), divisor=cnt)
+            ctx.save_for_backward(grad, None)
+        else:
+            rows = K.cross_entropy_to(lg, t, grad, grad_scale=1.0, ignore_index=ignore_index)
+            n = (t != ignore_index).sum().clamp(min=1) if mean else torch.ones((), device=lg.device)
+            loss = rows.sum() / n
+            ctx.save_for_backward(grad, n)
         ctx.shape = logits.shape
-        return rows.sum() / n
+        return loss
 
     @staticmethod
     def backward(ctx, g):
+        from . import kernels as K
         grad, n = ctx.saved_tensors
-        return grad.mul_((g / n).to(grad.dtype)).view(ctx.shape), None, None
+        if n is None:
+            grad = K.scale_unless_one_(grad, g.float().contiguous())
+        else:
+            grad = grad.mul_((g / n).to(grad.dtype))
+        return grad.view(ctx.shape), None, None, None
 
 
 def cross_entropy(logits, target, ignore_index=-100):
     """Mean token cross-entropy; the softmax gradient is produced in the same pass over the logits."""
     if use_kernels(logits) and logits.shape[-1] % 8 == 0:
-        return _CrossEntropyFn.apply(logits, target, ignore_index)
+        return _CrossEntropyFn.apply(logits, target, ignore_index, True)
     return F.cross_entropy(logits.reshape(-1, logits.shape[-1]).float(), target.reshape(-1), ignore_index=ignore_index)
 
 
@@ -239,7 +254,7 @@ class _ChunkedHeadLossFn(torch.autograd.Function):
                 # sum over the chunk's tokens; the division by the global count happens once, below
                 tc = t1d[r0:r1]
                 if use_kernels(logits) and logits.shape[-1] % 8 == 0:
-                    loss_c = cross_entropy(logits, tc, ignore_index) * (tc != ignore_index).sum().clamp(min=1)
+                    loss_c = _CrossEntropyFn.apply(logits, tc, ignore_index, False)
                 else:
                     loss_c = F.cross_entropy(logits.float(), tc, ignore_index=ignore_index, reduction="sum")
                 grads = torch.autograd.grad(loss_c, [hc] + list(params), allow_unused=True)

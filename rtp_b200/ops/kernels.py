@@ -23,7 +23,9 @@ def _L():
         L.rtp_kernels_last_error.restype = C.c_char_p
         L.rtp_norm_fwd.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, i, i, f, i, f, ull, ull, vp, vp]
         L.rtp_norm_bwd.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, f, ull, ull, vp, vp, vp]
-        L.rtp_cross_entropy.argtypes = [vp, ll, vp, vp, i, i, f, ll, i, vp]
+        L.rtp_cross_entropy_scaled.argtypes = [vp, ll, vp, vp, i, i, f, vp, ll, i, vp, ll, vp]
+        L.rtp_ce_count.argtypes = [vp, i, ll, vp, vp]
+        L.rtp_scale_unless_one.argtypes = [vp, vp, ll, vp]
         L.rtp_embed_fwd.argtypes = [vp, vp, vp, ll, i, vp, ll, i, i, i, i, f, f, ull, ull, vp, vp]
         L.rtp_embed_bwd.argtypes = [vp, vp, vp, ll, i, i, i, i, f, f, ull, ull, vp, vp]
         L.rtp_attn_small_fwd.argtypes = [vp, vp, i, i, i, i, i, f, f, ull, ull, vp, vp]
@@ -51,7 +53,7 @@ def _L():
         L.rtp_causal_softmax.argtypes = [vp, ll, i, f, vp]
         L.rtp_causal_softmax_bwd.argtypes = [vp, vp, ll, i, f, vp]
         L.rtp_cast_f32_bf16.argtypes = [vp, vp, ll, f, vp]
-        L.rtp_sum_f32.argtypes = [vp, vp, i, f, vp]
+        L.rtp_sum_f32.argtypes = [vp, vp, i, f, vp, vp]
         _declared = True
     return L
 
@@ -97,35 +99,51 @@ def norm_bwd(dy, h, gamma, mean, rstd, *, rms=False, has_beta=True, drop_p=0.0, 
     return dx, dsub, dgamma, dbeta
 
 
+def _cross_entropy(logits, target, loss, grad_scale, scale, ignore_index, write_grad, grad):
+    M, V = logits.shape
+    _check(_L().rtp_cross_entropy_scaled(_p(logits), logits.stride(0), _p(target), _p(loss), M, V, float(grad_scale), _p(scale),
+                                         int(ignore_index), int(write_grad), _p(grad),
+                                         grad.stride(0) if grad is not None else 0, _lib.stream_ptr()), "cross_entropy")
+    return loss
+
+
 def cross_entropy_(logits, target, *, grad_scale=1.0, ignore_index=-100, write_grad=True):
     """Per-row loss (fp32 [M]); overwrites ``logits`` with ``grad_scale * (softmax - onehot)``."""
-    M, V = logits.shape
-    loss = torch.empty(M, dtype=torch.float32, device=logits.device)
-    _check(_L().rtp_cross_entropy(_p(logits), logits.stride(0), _p(target), _p(loss), M, V, float(grad_scale),
-                                  int(ignore_index), int(write_grad), _lib.stream_ptr()), "cross_entropy")
-    return loss
+    loss = torch.empty(logits.shape[0], dtype=torch.float32, device=logits.device)
+    return _cross_entropy(logits, target, loss, grad_scale, None, ignore_index, write_grad, None)
 
 
 def cross_entropy_into(logits, target, loss, *, grad_scale=1.0, ignore_index=-100, write_grad=True):
     """Same as :func:`cross_entropy_` but writes the per-row loss into a caller-provided fp32 buffer."""
-    M, V = logits.shape
-    _check(_L().rtp_cross_entropy(_p(logits), logits.stride(0), _p(target), _p(loss), M, V, float(grad_scale),
-                                  int(ignore_index), int(write_grad), _lib.stream_ptr()), "cross_entropy")
-    return loss
+    return _cross_entropy(logits, target, loss, grad_scale, None, ignore_index, write_grad, None)
 
 
-def cross_entropy_to(logits, target, grad=None, *, grad_scale=1.0, ignore_index=-100):
+def cross_entropy_to(logits, target, grad=None, *, grad_scale=1.0, scale=None, ignore_index=-100):
     """Per-row loss (fp32 [M]) of bf16 ``logits`` [M, V], which are NOT modified; when ``grad`` (bf16 [M, V]) is given it
-    receives ``grad_scale * (softmax - onehot)``."""
+    receives ``grad_scale * scale * (softmax - onehot)``.  ``scale``: optional fp32 device scalar (rows that
+    :func:`cross_entropy_one_read` accepts)."""
+    loss = torch.empty(logits.shape[0], dtype=torch.float32, device=logits.device)
+    return _cross_entropy(logits, target, loss, grad_scale, scale, ignore_index, grad is not None, grad)
+
+
+def cross_entropy_one_read(logits):
+    """Whether the rows fit the kernel that keeps a row in registers (and takes a device-side gradient factor)."""
     M, V = logits.shape
-    loss = torch.empty(M, dtype=torch.float32, device=logits.device)
-    L = _L()
-    L.rtp_cross_entropy_to.argtypes = [C.c_void_p, C.c_longlong, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_float,
-                                       C.c_longlong, C.c_int, C.c_void_p, C.c_longlong, C.c_void_p]
-    _check(L.rtp_cross_entropy_to(_p(logits), logits.stride(0), _p(target), _p(loss), M, V, float(grad_scale),
-                                  int(ignore_index), int(grad is not None), _p(grad),
-                                  grad.stride(0) if grad is not None else 0, _lib.stream_ptr()), "cross_entropy")
-    return loss
+    return M > 0 and 0 < V <= 65536
+
+
+def ce_count(target, ignore_index=-100):
+    """fp32 [2]: the number of targets other than ``ignore_index`` (at least one) and its reciprocal."""
+    out = torch.empty(2, dtype=torch.float32, device=target.device)
+    _check(_L().rtp_ce_count(_p(target), target.numel(), int(ignore_index), _p(out), _lib.stream_ptr()), "ce_count")
+    return out
+
+
+def scale_unless_one_(g, scale):
+    """bf16 ``g`` *= the fp32 device scalar ``scale``; a factor of one costs no pass over ``g``."""
+    _check(_L().rtp_scale_unless_one(_p(g), _p(scale), g.numel(), _lib.stream_ptr()), "scale")
+    torch.autograd.graph.increment_version(g)
+    return g
 
 
 def embed_fwd(table, ids, out, col_off, *, D, scale=1.0, pe=None, tokens_per_pos=1, drop_p=0.0, seed=0, offset=0,
@@ -276,8 +294,8 @@ def cast_f32_bf16(src, dst, scale=1.0):
     return dst
 
 
-def sum_f32(src, out, scale=1.0):
-    _check(_L().rtp_sum_f32(_p(src), _p(out), src.numel(), float(scale), _lib.stream_ptr()), "sum")
+def sum_f32(src, out, scale=1.0, divisor=None):
+    _check(_L().rtp_sum_f32(_p(src), _p(out), src.numel(), float(scale), _p(divisor), _lib.stream_ptr()), "sum")
     return out
 
 

@@ -2,8 +2,8 @@
 that end inside a tile, contractions that end inside a k-block, one and many tiles per unit, every epilogue, the column
 sums beside the weight gradient, and several experts in one launch.
 
-Tolerance: a result is one bf16 rounding (relative 2^-9) of an fp32 sum whose terms are exact products; 2^-8 of the
-result plus 2^-18 of the sum of absolute products covers both."""
+Tolerance: a result is one bf16 rounding (2^-8 of the result) of an fp32 sum whose terms are exact products (2^-18 of the
+sum of absolute products)."""
 import pytest
 import torch
 
