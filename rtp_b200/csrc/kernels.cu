@@ -507,10 +507,16 @@ __global__ void embed_bwd_kernel(__nv_bfloat16* __restrict__ gtable, const long 
 }
 
 // ------------------------------------------------------------------------------------------------
-// Short-sequence attention (S <= 128, head_dim 64) on packed projections.
+// Short-sequence attention (S <= 128, head_dim 64) on packed projections, in fp32 throughout.
 // qkv: [T, 3*D] with T = S*B tokens (token = s*B + b). The projection comes out of a column-rotated
 // linear, so its columns are grouped per shard: shard j holds [q_j | k_j | v_j], each D/nshard wide.
 // out: [T, D], column = head*64 + d. One block per (batch, head).
+//
+// There are few blocks (batch x heads) and little work in each, so a block's latency is the kernel's time.  Products run
+// on register tiles (2 x 2 scores, 2 x 4 outputs a thread) fed by 16-byte shared-memory reads, 256 or 512 threads a block;
+// rows of 64 floats hold their 16-byte chunks swizzled by row % 8, so that eight rows read side by side touch different
+// banks.  One score per thread from rows of 65 floats, 128 threads: 13 x 12 blocks of S = 50 took 32 us forward and
+// 97 us backward, now 13 and 27 us.
 // ------------------------------------------------------------------------------------------------
 constexpr int kHd = 64;
 __device__ __forceinline__ int qkv_col(int head, int which, int D, int nshard, int heads) {
@@ -518,42 +524,82 @@ __device__ __forceinline__ int qkv_col(int head, int which, int D, int nshard, i
   const int j = head / hps, hl = head % hps;
   return j * (3 * (D / nshard)) + which * (D / nshard) + hl * kHd;
 }
+// 16-byte chunk c (0..15) of row r
+__device__ __forceinline__ float4& chunk_at(float* base, int r, int c) {
+  return reinterpret_cast<float4*>(base)[r * 16 + (c ^ (r & 7))];
+}
+__device__ __forceinline__ float dot4(const float4& a, const float4& b, float acc) {
+  acc = fmaf(a.x, b.x, acc); acc = fmaf(a.y, b.y, acc); acc = fmaf(a.z, b.z, acc);
+  return fmaf(a.w, b.w, acc);
+}
+__device__ __forceinline__ void axpy4(float s, const float4& v, float4& acc) {
+  acc.x = fmaf(s, v.x, acc.x); acc.y = fmaf(s, v.y, acc.y); acc.z = fmaf(s, v.z, acc.z); acc.w = fmaf(s, v.w, acc.w);
+}
+__device__ __forceinline__ void fill_rows(float* dst, const __nv_bfloat16* __restrict__ src, long long ld, int S, int B, int b,
+                                          int col, float scale) {
+  for (int i = threadIdx.x; i < S * 8; i += blockDim.x) {
+    const int s = i >> 3, c = i & 7;
+    float f[8];
+    unpack8(*reinterpret_cast<const uint4*>(src + (size_t)(s * B + b) * ld + col + c * 8), f);
+    chunk_at(dst, s, 2 * c) = make_float4(f[0] * scale, f[1] * scale, f[2] * scale, f[3] * scale);
+    chunk_at(dst, s, 2 * c + 1) = make_float4(f[4] * scale, f[5] * scale, f[6] * scale, f[7] * scale);
+  }
+}
+// out[r, c] = <a_r, b_c> for c <= r (causal) or all c, -inf / 0 elsewhere (`other`), on 2 x 2 tiles
+__device__ __forceinline__ void row_dots(float* a, float* b, float* out, int S, int causal, float other) {
+  const int nt = (S + 1) >> 1;
+  for (int i = threadIdx.x; i < nt * nt; i += blockDim.x) {
+    const int r0 = (i / nt) * 2, c0 = (i % nt) * 2;
+    const int r1 = min(r0 + 1, S - 1), c1 = min(c0 + 1, S - 1);
+    float d00 = 0.f, d01 = 0.f, d10 = 0.f, d11 = 0.f;
+    if (!causal || c0 <= r1) {
+#pragma unroll 8
+      for (int e = 0; e < 16; ++e) {
+        const float4 x0 = chunk_at(a, r0, e), x1 = chunk_at(a, r1, e), y0 = chunk_at(b, c0, e), y1 = chunk_at(b, c1, e);
+        d00 = dot4(x0, y0, d00); d01 = dot4(x0, y1, d01); d10 = dot4(x1, y0, d10); d11 = dot4(x1, y1, d11);
+      }
+    }
+    const int ld = S + 1;
+    out[r0 * ld + c0] = (!causal || c0 <= r0) ? d00 : other;
+    if (c0 + 1 < S) out[r0 * ld + c0 + 1] = (!causal || c0 + 1 <= r0) ? d01 : other;
+    if (r0 + 1 < S) {
+      out[(r0 + 1) * ld + c0] = (!causal || c0 <= r0 + 1) ? d10 : other;
+      if (c0 + 1 < S) out[(r0 + 1) * ld + c0 + 1] = (!causal || c0 + 1 <= r0 + 1) ? d11 : other;
+    }
+  }
+}
+// acc[u] = sum_c w(r0 + u, c) v_c[4 e .. 4 e + 3] over c in [lo, hi), w(r, c) = p[r * sr + c * sc]
+__device__ __forceinline__ void row_sums(const float* p, int sr, int sc, float* v, int r0, int r1, int e, int lo, int hi,
+                                         float4 (&acc)[2]) {
+  acc[0] = acc[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+  for (int c = lo; c < hi; ++c) {
+    const float4 x = chunk_at(v, c, e);
+    axpy4(p[r0 * sr + c * sc], x, acc[0]);
+    axpy4(p[r1 * sr + c * sc], x, acc[1]);
+  }
+}
+__device__ __forceinline__ void store4(__nv_bfloat16* dst, const float4& v, float s) {
+  *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16(v.x * s, v.y * s), pack_bf16(v.z * s, v.w * s));
+}
 
-__global__ void attn_small_fwd_kernel(const __nv_bfloat16* __restrict__ qkv, __nv_bfloat16* __restrict__ out, int S,
-                                      int B, int heads, int nshard, int causal, float sm_scale, uint32_t thresh,
+__global__ void __launch_bounds__(512) attn_small_fwd_kernel(const __nv_bfloat16* __restrict__ qkv, __nv_bfloat16* __restrict__ out,
+                                      int S, int B, int heads, int nshard, int causal, float sm_scale, uint32_t thresh,
                                       float drop_scale, uint64_t seed, uint64_t offset,
                                       const unsigned long long* __restrict__ step_ptr) {
-  extern __shared__ float smf[];
+  extern __shared__ __align__(16) float smf[];
   if (step_ptr) offset += __ldg(step_ptr) * 65536ull;
   const int D = heads * kHd;
   const int b = blockIdx.x / heads, h = blockIdx.x % heads;
-  float* q = smf;                 // [S][65]
-  float* k = q + S * 65;
-  float* v = k + S * 65;
-  float* p = v + S * 65;          // [S][S+1]
-  const int cq = qkv_col(h, 0, D, nshard, heads), ck = qkv_col(h, 1, D, nshard, heads), cv = qkv_col(h, 2, D, nshard, heads);
-  for (int i = threadIdx.x; i < S * 8; i += blockDim.x) {
-    const int s = i / 8, c = (i % 8) * 8;
-    const size_t rowp = (size_t)(s * B + b) * (3 * D);
-    float f[8];
-    unpack8(*reinterpret_cast<const uint4*>(qkv + rowp + cq + c), f);
-    for (int e = 0; e < 8; ++e) q[s * 65 + c + e] = f[e] * sm_scale;
-    unpack8(*reinterpret_cast<const uint4*>(qkv + rowp + ck + c), f);
-    for (int e = 0; e < 8; ++e) k[s * 65 + c + e] = f[e];
-    unpack8(*reinterpret_cast<const uint4*>(qkv + rowp + cv + c), f);
-    for (int e = 0; e < 8; ++e) v[s * 65 + c + e] = f[e];
-  }
+  float* q = smf;                 // [S][64], pre-scaled
+  float* k = q + S * kHd;
+  float* v = k + S * kHd;
+  float* p = v + S * kHd;         // [S][S+1]
+  fill_rows(q, qkv, 3 * D, S, B, b, qkv_col(h, 0, D, nshard, heads), sm_scale);
+  fill_rows(k, qkv, 3 * D, S, B, b, qkv_col(h, 1, D, nshard, heads), 1.f);
+  fill_rows(v, qkv, 3 * D, S, B, b, qkv_col(h, 2, D, nshard, heads), 1.f);
   __syncthreads();
-  for (int i = threadIdx.x; i < S * S; i += blockDim.x) {
-    const int r = i / S, c = i % S;
-    float acc = -INFINITY;
-    if (!causal || c <= r) {
-      acc = 0.f;
-#pragma unroll 16
-      for (int e = 0; e < kHd; ++e) acc += q[r * 65 + e] * k[c * 65 + e];
-    }
-    p[r * (S + 1) + c] = acc;
-  }
+  row_dots(q, k, p, S, causal, -INFINITY);
   __syncthreads();
   // softmax per row: one warp per row
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
@@ -579,58 +625,40 @@ __global__ void attn_small_fwd_kernel(const __nv_bfloat16* __restrict__ qkv, __n
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < S * kHd; i += blockDim.x) {
-    const int r = i / kHd, e = i % kHd;
-    float acc = 0.f;
-    const int lim = causal ? r + 1 : S;
-    for (int c = 0; c < lim; ++c) acc += p[r * (S + 1) + c] * v[c * 65 + e];
-    out[(size_t)(r * B + b) * D + h * kHd + e] = __float2bfloat16(acc);
+  const int nt = (S + 1) >> 1;
+  for (int i = threadIdx.x; i < nt * 16; i += blockDim.x) {
+    const int r0 = (i >> 4) * 2, e = i & 15, r1 = min(r0 + 1, S - 1);
+    float4 acc[2];
+    row_sums(p, S + 1, 1, v, r0, r1, e, 0, causal ? r0 + 1 : S, acc);
+    if (causal && r1 > r0) axpy4(p[r1 * (S + 1) + r1], chunk_at(v, r1, e), acc[1]);   // row r0 does not see key r1
+    __nv_bfloat16* o = out + h * kHd + 4 * e;
+    store4(o + (size_t)(r0 * B + b) * D, acc[0], 1.f);
+    if (r0 + 1 < S) store4(o + (size_t)(r1 * B + b) * D, acc[1], 1.f);
   }
 }
 
-__global__ void attn_small_bwd_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __restrict__ dout,
-                                      __nv_bfloat16* __restrict__ dqkv, int S, int B, int heads, int nshard,
-                                      int causal, float sm_scale, uint32_t thresh, float drop_scale, uint64_t seed,
-                                      uint64_t offset, const unsigned long long* __restrict__ step_ptr) {
-  extern __shared__ float smf[];
+__global__ void __launch_bounds__(512) attn_small_bwd_kernel(const __nv_bfloat16* __restrict__ qkv,
+                                      const __nv_bfloat16* __restrict__ dout, __nv_bfloat16* __restrict__ dqkv, int S, int B,
+                                      int heads, int nshard, int causal, float sm_scale, uint32_t thresh, float drop_scale,
+                                      uint64_t seed, uint64_t offset, const unsigned long long* __restrict__ step_ptr) {
+  extern __shared__ __align__(16) float smf[];
   if (step_ptr) offset += __ldg(step_ptr) * 65536ull;
   const int D = heads * kHd;
   const int b = blockIdx.x / heads, h = blockIdx.x % heads;
-  float* q = smf;                 // [S][65] (pre-scaled)
-  float* k = q + S * 65;
-  float* v = k + S * 65;
-  float* go = v + S * 65;         // dO
-  float* p = go + S * 65;         // [S][S+1] softmax probabilities (no dropout)
+  float* q = smf;                 // [S][64] (pre-scaled)
+  float* k = q + S * kHd;
+  float* v = k + S * kHd;
+  float* go = v + S * kHd;        // dO
+  float* p = go + S * kHd;        // [S][S+1] softmax probabilities (no dropout)
   float* ds = p + S * (S + 1);    // [S][S+1] dP then dS
   const int cq = qkv_col(h, 0, D, nshard, heads), ck = qkv_col(h, 1, D, nshard, heads), cv = qkv_col(h, 2, D, nshard, heads);
-  for (int i = threadIdx.x; i < S * 8; i += blockDim.x) {
-    const int s = i / 8, c = (i % 8) * 8;
-    const size_t rowp = (size_t)(s * B + b) * (3 * D);
-    float f[8];
-    unpack8(*reinterpret_cast<const uint4*>(qkv + rowp + cq + c), f);
-    for (int e = 0; e < 8; ++e) q[s * 65 + c + e] = f[e] * sm_scale;
-    unpack8(*reinterpret_cast<const uint4*>(qkv + rowp + ck + c), f);
-    for (int e = 0; e < 8; ++e) k[s * 65 + c + e] = f[e];
-    unpack8(*reinterpret_cast<const uint4*>(qkv + rowp + cv + c), f);
-    for (int e = 0; e < 8; ++e) v[s * 65 + c + e] = f[e];
-    unpack8(*reinterpret_cast<const uint4*>(dout + (size_t)(s * B + b) * D + h * kHd + c), f);
-    for (int e = 0; e < 8; ++e) go[s * 65 + c + e] = f[e];
-  }
+  fill_rows(q, qkv, 3 * D, S, B, b, cq, sm_scale);
+  fill_rows(k, qkv, 3 * D, S, B, b, ck, 1.f);
+  fill_rows(v, qkv, 3 * D, S, B, b, cv, 1.f);
+  fill_rows(go, dout, D, S, B, b, h * kHd, 1.f);
   __syncthreads();
-  for (int i = threadIdx.x; i < S * S; i += blockDim.x) {
-    const int r = i / S, c = i % S;
-    float acc = -INFINITY, dp = 0.f;
-    if (!causal || c <= r) {
-      acc = 0.f;
-#pragma unroll 16
-      for (int e = 0; e < kHd; ++e) {
-        acc += q[r * 65 + e] * k[c * 65 + e];
-        dp += go[r * 65 + e] * v[c * 65 + e];
-      }
-    }
-    p[r * (S + 1) + c] = acc;
-    ds[r * (S + 1) + c] = dp;   // dP of the dropped probabilities
-  }
+  row_dots(q, k, p, S, causal, -INFINITY);
+  row_dots(go, v, ds, S, causal, 0.f);                // dP of the dropped probabilities
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   for (int r = warp; r < S; r += nw) {
@@ -646,46 +674,46 @@ __global__ void attn_small_bwd_kernel(const __nv_bfloat16* __restrict__ qkv, con
     se = warp_sum(se);
     const float inv = 1.f / se;
     float dot = 0.f;
-    for (int c = lane; c < S; c += 32) {
+    uint32_t keep = 0;                                // bit j: element lane + 32 j survives (S <= 128)
+    for (int c = lane, j = 0; c < S; c += 32, ++j) {
       const float pv = p[r * (S + 1) + c] * inv;
       float m = 1.f;
       if (thresh) {
         const uint64_t e = ((uint64_t)blockIdx.x * S + r) * S + c;
-        m = dropout_keep(seed, offset, e, thresh) ? drop_scale : 0.f;
+        const bool kp = dropout_keep(seed, offset, e, thresh);
+        keep |= (kp ? 1u : 0u) << j;
+        m = kp ? drop_scale : 0.f;
       }
-      const float dpv = ds[r * (S + 1) + c] * m;  // gradient wrt the un-dropped probability
+      const float dpv = ds[r * (S + 1) + c] * m;      // gradient wrt the un-dropped probability
       p[r * (S + 1) + c] = pv;
       ds[r * (S + 1) + c] = dpv;
       dot += dpv * pv;
     }
     dot = warp_sum(dot);
-    for (int c = lane; c < S; c += 32) {
+    for (int c = lane, j = 0; c < S; c += 32, ++j) {
       const float pv = p[r * (S + 1) + c];
       const float dsv = pv * (ds[r * (S + 1) + c] - dot);
       // keep the dropped probability in p for dV
-      float m = 1.f;
-      if (thresh) {
-        const uint64_t e = ((uint64_t)blockIdx.x * S + r) * S + c;
-        m = dropout_keep(seed, offset, e, thresh) ? drop_scale : 0.f;
-      }
+      const float m = thresh ? (((keep >> j) & 1u) ? drop_scale : 0.f) : 1.f;
       p[r * (S + 1) + c] = pv * m;
       ds[r * (S + 1) + c] = dsv;
     }
   }
   __syncthreads();
   // dQ = dS K * scale ; dK = dS^T Q(pre-scaled) ; dV = Pd^T dO
-  for (int i = threadIdx.x; i < S * kHd; i += blockDim.x) {
-    const int r = i / kHd, e = i % kHd;
-    float dq = 0.f, dk = 0.f, dv = 0.f;
-    for (int c = 0; c < S; ++c) {
-      dq += ds[r * (S + 1) + c] * k[c * 65 + e];
-      dk += ds[c * (S + 1) + r] * q[c * 65 + e];
-      dv += p[c * (S + 1) + r] * go[c * 65 + e];
-    }
-    const size_t rowp = (size_t)(r * B + b) * (3 * D);
-    dqkv[rowp + cq + e] = __float2bfloat16(dq * sm_scale);
-    dqkv[rowp + ck + e] = __float2bfloat16(dk);
-    dqkv[rowp + cv + e] = __float2bfloat16(dv);
+  const int nt = (S + 1) >> 1, ld = S + 1;
+  for (int i = threadIdx.x; i < 3 * nt * 16; i += blockDim.x) {
+    const int which = i / (nt * 16), j = i - which * (nt * 16);
+    const int r0 = (j >> 4) * 2, e = j & 15, r1 = min(r0 + 1, S - 1);
+    float4 acc[2];
+    // entries above the diagonal are 0 with a causal mask: rows see the keys up to r1, keys the rows from r0 on
+    if (which == 0) row_sums(ds, ld, 1, k, r0, r1, e, 0, causal ? r1 + 1 : S, acc);
+    else if (which == 1) row_sums(ds, 1, ld, q, r0, r1, e, causal ? r0 : 0, S, acc);
+    else row_sums(p, 1, ld, go, r0, r1, e, causal ? r0 : 0, S, acc);
+    __nv_bfloat16* o = dqkv + (which == 0 ? cq : which == 1 ? ck : cv) + 4 * e;
+    const float sc = which == 0 ? sm_scale : 1.f;
+    store4(o + (size_t)(r0 * B + b) * (3 * D), acc[0], sc);
+    if (r0 + 1 < S) store4(o + (size_t)(r1 * B + b) * (3 * D), acc[1], sc);
   }
 }
 
@@ -1359,9 +1387,10 @@ int rtp_embed_bwd_blocks(void* gtable, const long long* ids, const void* dy, lon
 static int g_attn_tc = 1;
 void rtp_set_attn_tc(int on) { g_attn_tc = on ? 1 : 0; }
 static size_t attn_smem(int S, bool bwd) {
-  size_t f = (size_t)(bwd ? 4 : 3) * S * 65 + (size_t)(bwd ? 2 : 1) * S * (S + 1);
+  size_t f = (size_t)(bwd ? 4 : 3) * S * kHd + (size_t)(bwd ? 2 : 1) * S * (S + 1);
   return f * sizeof(float);
 }
+static int attn_threads(int S) { return S <= 40 ? 256 : 512; }   // a 2 x 2 tile of scores per thread and round
 int rtp_attn_small_fwd(const void* qkv, void* out, int S, int B, int heads, int nshard, int causal, float sm_scale,
                        float drop_p, unsigned long long seed, unsigned long long offset,
                        const unsigned long long* step_ptr, void* stream) {
@@ -1377,7 +1406,7 @@ int rtp_attn_small_fwd(const void* qkv, void* out, int S, int B, int heads, int 
     if (e != cudaSuccess) return kfail("attn fwd attr", e);
   }
   const float ds = drop_p > 0.f ? 1.f / (1.f - drop_p) : 1.f;
-  attn_small_fwd_kernel<<<B * heads, 128, smem, (cudaStream_t)stream>>>(
+  attn_small_fwd_kernel<<<B * heads, attn_threads(S), smem, (cudaStream_t)stream>>>(
       (const __nv_bfloat16*)qkv, (__nv_bfloat16*)out, S, B, heads, nshard, causal, sm_scale, host_thresh(drop_p), ds,
       seed, offset, step_ptr);
   LAUNCH_CHECK("attn_small_fwd");
@@ -1400,7 +1429,7 @@ int rtp_attn_small_bwd(const void* qkv, const void* dout, void* dqkv, int S, int
     if (e != cudaSuccess) return kfail("attn bwd attr", e);
   }
   const float ds = drop_p > 0.f ? 1.f / (1.f - drop_p) : 1.f;
-  attn_small_bwd_kernel<<<B * heads, 128, smem, (cudaStream_t)stream>>>(
+  attn_small_bwd_kernel<<<B * heads, attn_threads(S), smem, (cudaStream_t)stream>>>(
       (const __nv_bfloat16*)qkv, (const __nv_bfloat16*)dout, (__nv_bfloat16*)dqkv, S, B, heads, nshard, causal,
       sm_scale, host_thresh(drop_p), ds, seed, offset, step_ptr);
   LAUNCH_CHECK("attn_small_bwd");
