@@ -1,0 +1,44 @@
+"""LayerNorm / RMSNorm kernels against float64 at the widths where the number of threads per row changes, with row counts
+below, at and above what one pass of the grid takes.
+
+Tolerance: h is rounded to bf16 first, as the kernels do; y and dx are one rounding to bf16 (2^-8) of fp32 arithmetic
+whose error is 2^-16 of the largest term; dgamma / dbeta are fp32 sums over the rows (2^-16 of the sum of magnitudes)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+BF = torch.bfloat16
+
+
+@pytest.mark.parametrize("D", [8, 256, 264, 512, 520, 1024, 1032, 2048, 2056, 4104, 5120, 8192])
+@pytest.mark.parametrize("M", [1, 297, 2500])
+@pytest.mark.parametrize("rms,residual", [(False, True), (True, False)])
+def test_norm(D, M, rms, residual):
+    from rtp_b200.ops import kernels as K
+    g = torch.Generator(device="cuda").manual_seed(D + M)
+
+    def rnd(*s):
+        return torch.randn(*s, generator=g, device="cuda").to(BF)
+    x, dy, gamma, beta = rnd(M, D), rnd(M, D), rnd(D), rnd(D)
+    sub = rnd(M, D) if residual else None
+    y, h, mean, rstd = K.norm_fwd(x, sub, gamma, None if rms else beta, rms=rms)
+    href = (x.float() + sub.float()).to(BF) if residual else x
+    assert torch.equal(h, href)
+    hd = href.double().requires_grad_()
+    gd = gamma.double().requires_grad_()
+    mu = hd.mean(-1, keepdim=True) if not rms else 0.0
+    xh = (hd - mu) * torch.rsqrt((hd - mu).pow(2).mean(-1, keepdim=True) + 1e-5)
+    ref = xh * gd + (0.0 if rms else beta.double())
+
+    def close(a, r, mag, rel):
+        assert bool(((a.double() - r).abs() <= rel * r.abs() + 2.0 ** -16 * mag).all()), (a.double() - r).abs().max().item()
+    close(y, ref.detach(), ref.detach().abs().max(), 2.0 ** -8)
+    dx, dsub, dg, db = K.norm_bwd(dy, h, gamma, mean, rstd, rms=rms, has_beta=not rms, want_dsub=residual)
+    rx, rg = torch.autograd.grad(ref, (hd, gd), dy.double())
+    # dx cancels between its three terms: the fp32 error is relative to the largest of them
+    close(dx, rx, (dy.double() * gamma.double()).abs().amax() * rstd.double().max() * 4, 2.0 ** -8)
+    close(dg, rg, (dy.double() * xh.detach()).abs().sum(0), 0.0)
+    if not rms:
+        close(db, dy.double().sum(0), dy.double().abs().sum(0), 0.0)
+    if residual:
+        assert torch.equal(dsub, dx)
