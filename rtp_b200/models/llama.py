@@ -78,24 +78,20 @@ class LlamaBlock(nn.Module):
         self.gate_up = ColumnParallelLinear(cfg.d_model, 2 * cfg.d_ff, packed_parts=2, **kw)
         self.down = RowParallelLinear(cfg.d_ff, cfg.d_model, **kw)
 
-    def _split_packed(self, y, parts):
-        """Column blocks of a rotated packed projection are grouped per shard: [p0_j | p1_j | ...] for j = 0..N-1."""
-        B, S, W = y.shape
-        y = y.view(B, S, self.N, parts, W // (self.N * parts))
-        return [y[:, :, :, k].reshape(B, S, -1) for k in range(parts)]
-
     def forward(self, x, cos, sin):
         cfg = self.cfg
         B, S, D = x.shape
         hd = D // cfg.n_heads
-        q, k, v = self._split_packed(self.qkv(self.norm1(x)), 3)
-        q = apply_rope(q.view(B, S, cfg.n_heads, hd), cos, sin)
-        k = apply_rope(k.view(B, S, cfg.n_heads, hd), cos, sin)
-        v = v.view(B, S, cfg.n_heads, hd)
-        a = FO.causal_attention(q, k, v)                         # [B, S, H, hd]
-        x = x + self.proj(a.reshape(B, S, D))
-        g, u = self._split_packed(self.gate_up(self.norm2(x)), 2)
-        x = x + self.down(FO.swiglu(g, u))
+        qkv = self.qkv(self.norm1(x))
+        a = FO.rope_attention_packed(qkv, cos, sin, cfg.n_heads, self.N)
+        if a is None:
+            q, k, v = FO._split_packed(qkv, 3, self.N)
+            q = apply_rope(q.view(B, S, cfg.n_heads, hd), cos, sin)
+            k = apply_rope(k.view(B, S, cfg.n_heads, hd), cos, sin)
+            v = v.view(B, S, cfg.n_heads, hd)
+            a = FO.causal_attention(q, k, v).reshape(B, S, D)      # [B, S, H, hd]
+        x = x + self.proj(a)
+        x = x + self.down(FO.swiglu_packed(self.gate_up(self.norm2(x)), self.N))
         return x
 
 

@@ -152,24 +152,56 @@ def flash_attention(q, k, v, causal=False, attn_mask=None, key_padding_mask=None
                           sm_scale)
 
 
+def packed_fwd(qkv, B, S, H, nshard, seq_first=False, causal=False, attn_mask=None, key_padding_mask=None, drop_p=0.0, seed=0,
+               offset=0, step=None, keep=None):
+    """Forward launch on an aligned packed projection; returns (out, log-sum-exp).  Tensors made of the masks are appended to
+    ``keep``."""
+    T, W = qkv.shape
+    D = W // 3
+    hd = D // H
+    out = torch.empty(T, D, dtype=torch.bfloat16, device=qkv.device)
+    lse = torch.empty(B * H, S, dtype=torch.float32, device=qkv.device)
+    a = _lib.FlashArgs()
+    a.q, a.k, a.v = [_ref_packed(qkv, i, B, S, H, hd, nshard, seq_first, W) for i in range(3)]
+    a.o = _ref_packed(out, -1, B, S, H, hd, nshard, seq_first, D)
+    a.lse = lse.data_ptr()
+    _mask_args(a, attn_mask, key_padding_mask, [] if keep is None else keep)
+    _common(a, B, H, S, S, hd, causal, None, drop_p, seed, offset, step, qkv.device)
+    _check(_lib.lib().rtp_flash_fwd(C.byref(a), _lib.stream_ptr()), "rtp_flash_fwd")
+    return out, lse
+
+
+def packed_bwd(qkv, out, lse, dout, B, S, H, nshard, seq_first=False, causal=False, attn_mask=None, key_padding_mask=None,
+               drop_p=0.0, seed=0, offset=0, step=None):
+    """Backward launches; returns the gradient in the packed layout of ``qkv``."""
+    T, W = qkv.shape
+    D = W // 3
+    hd = D // H
+    if dout.stride(1) != 1 or dout.stride(0) % 8 or dout.data_ptr() % 16:
+        dout = dout.contiguous()
+    dqkv = torch.empty(T, W, dtype=torch.bfloat16, device=qkv.device)
+    delta = torch.empty_like(lse)
+    a = _lib.FlashArgs()
+    a.q, a.k, a.v = [_ref_packed(qkv, i, B, S, H, hd, nshard, seq_first, W) for i in range(3)]
+    a.dq, a.dk, a.dv = [_ref_packed(dqkv, i, B, S, H, hd, nshard, seq_first, W) for i in range(3)]
+    a.o = _ref_packed(out, -1, B, S, H, hd, nshard, seq_first, D)
+    a.dout = _ref_packed(dout, -1, B, S, H, hd, nshard, seq_first, D)
+    a.lse, a.delta = lse.data_ptr(), delta.data_ptr()
+    keep = []
+    _mask_args(a, attn_mask, key_padding_mask, keep)
+    _common(a, B, H, S, S, hd, causal, None, drop_p, seed, offset, step, qkv.device)
+    _check(_lib.lib().rtp_flash_bwd(C.byref(a), _lib.stream_ptr()), "rtp_flash_bwd")
+    return dqkv
+
+
 class _FlashPackedFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, qkv, B, S, H, nshard, seq_first, causal, attn_mask, key_padding_mask, drop_p, seed, offset, step):
-        T, W = qkv.shape
-        D = W // 3
-        hd = D // H
         if qkv.stride(1) != 1 or qkv.stride(0) % 8 or qkv.data_ptr() % 16:
             qkv = qkv.contiguous()
-        out = torch.empty(T, D, dtype=torch.bfloat16, device=qkv.device)
-        lse = torch.empty(B * H, S, dtype=torch.float32, device=qkv.device)
-        a = _lib.FlashArgs()
         keep = []
-        a.q, a.k, a.v = [_ref_packed(qkv, i, B, S, H, hd, nshard, seq_first, W) for i in range(3)]
-        a.o = _ref_packed(out, -1, B, S, H, hd, nshard, seq_first, D)
-        a.lse = lse.data_ptr()
-        _mask_args(a, attn_mask, key_padding_mask, keep)
-        _common(a, B, H, S, S, hd, causal, None, drop_p, seed, offset, step, qkv.device)
-        _check(_lib.lib().rtp_flash_fwd(C.byref(a), _lib.stream_ptr()), "rtp_flash_fwd")
+        out, lse = packed_fwd(qkv, B, S, H, nshard, seq_first, causal, attn_mask, key_padding_mask, drop_p, seed, offset, step,
+                              keep)
         ctx.save_for_backward(qkv, out, lse, *keep)
         ctx.cfg = (B, S, H, nshard, seq_first, causal, attn_mask is not None, key_padding_mask is not None, drop_p, seed,
                    offset, step)
@@ -179,26 +211,11 @@ class _FlashPackedFn(torch.autograd.Function):
     def backward(ctx, dout):
         qkv, out, lse, *keep = ctx.saved_tensors
         B, S, H, nshard, seq_first, causal, has_mask, has_kpm, drop_p, seed, offset, step = ctx.cfg
-        T, W = qkv.shape
-        D = W // 3
-        hd = D // H
-        if dout.stride(1) != 1 or dout.stride(0) % 8 or dout.data_ptr() % 16:
-            dout = dout.contiguous()
-        dqkv = torch.empty(T, W, dtype=torch.bfloat16, device=qkv.device)
-        delta = torch.empty_like(lse)
-        a = _lib.FlashArgs()
-        a.q, a.k, a.v = [_ref_packed(qkv, i, B, S, H, hd, nshard, seq_first, W) for i in range(3)]
-        a.dq, a.dk, a.dv = [_ref_packed(dqkv, i, B, S, H, hd, nshard, seq_first, W) for i in range(3)]
-        a.o = _ref_packed(out, -1, B, S, H, hd, nshard, seq_first, D)
-        a.dout = _ref_packed(dout, -1, B, S, H, hd, nshard, seq_first, D)
-        a.lse, a.delta = lse.data_ptr(), delta.data_ptr()
         it = iter(keep)
         m = next(it) if has_mask else None
         kp = next(it) if has_kpm else None
-        _mask_args(a, m, kp, [])
-        _common(a, B, H, S, S, hd, causal, None, drop_p, seed, offset, step, qkv.device)
-        _check(_lib.lib().rtp_flash_bwd(C.byref(a), _lib.stream_ptr()), "rtp_flash_bwd")
-        return (dqkv,) + (None,) * 12
+        return (packed_bwd(qkv, out, lse, dout, B, S, H, nshard, seq_first, causal, m, kp, drop_p, seed, offset, step),) + \
+            (None,) * 12
 
 
 def flash_attention_packed(qkv, B, S, H, nshard=1, seq_first=False, causal=False, attn_mask=None,

@@ -49,6 +49,9 @@ def recompute(kind: str, srcs):
     if kind == "swiglu":
         g, u = srcs
         return K.swiglu_fwd(g.reshape(-1, g.shape[-1]), u.reshape(-1, u.shape[-1])).view(g.shape)
+    if kind == "swiglu_packed":
+        y, nshard = srcs
+        return K.swiglu_packed(y.reshape(-1, y.shape[-1]), nshard).view(*y.shape[:-1], y.shape[-1] // 2)
     if kind == "norm":
         x, weight, bias, eps, rms = srcs
         y = K.norm_fwd(x.reshape(-1, x.shape[-1]), None, weight, bias, eps=eps, rms=rms, save_h=False)[0]
@@ -221,6 +224,72 @@ def swiglu(g, u):
         g, u = g.contiguous(), u.contiguous()
         return _tag(_SwigluFn.apply(g, u), "swiglu", g, u)
     return F.silu(g) * u
+
+
+class _SwigluPackedFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, y, nshard):
+        from . import kernels as K
+        y2 = y.reshape(-1, y.shape[-1]).contiguous()
+        ctx.save_for_backward(y2)
+        ctx.shape, ctx.nshard = y.shape, nshard
+        return K.swiglu_packed(y2, nshard).view(*y.shape[:-1], y.shape[-1] // 2)
+
+    @staticmethod
+    def backward(ctx, dy):
+        from . import kernels as K
+        (y2,) = ctx.saved_tensors
+        return K.swiglu_packed_bwd(y2, dy.reshape(y2.shape[0], -1).contiguous(), ctx.nshard).view(ctx.shape), None
+
+
+def _split_packed(y, parts, nshard):
+    """The ``parts`` projections of a rotated packed projection, whose columns are grouped per shard:
+    [p0_j | p1_j | ...] for j = 0..nshard-1."""
+    y = y.view(*y.shape[:-1], nshard, parts, y.shape[-1] // (nshard * parts))
+    return [y[..., k, :].reshape(*y.shape[:-3], -1) for k in range(parts)]
+
+
+def swiglu_packed(y, nshard=1):
+    """silu(g) * u of a rotated packed gate / up projection [..., 2 * F], read where it lies (no split copies)."""
+    if use_kernels(y) and y.shape[-1] % (16 * nshard) == 0 and y.is_contiguous() and y.data_ptr() % 16 == 0:
+        return _tag(_SwigluPackedFn.apply(y, nshard), "swiglu_packed", y, nshard)
+    return swiglu(*_split_packed(y, 2, nshard))
+
+
+class _RopeAttnPackedFn(torch.autograd.Function):
+    """Causal self-attention of a packed projection [B * S, 3 * D] with rotary embedding of q and k.  Forward makes one rotated
+    copy of the projection, which the flash kernels read in place; backward turns the q and k gradients back inside the
+    packed gradient that they wrote."""
+
+    @staticmethod
+    def forward(ctx, qkv, cos, sin, B, S, H, nshard):
+        from . import flash, kernels as K
+        hd = qkv.shape[1] // (3 * H)
+        rot = K.rope_packed(qkv, cos, sin, hd, nshard)
+        out, lse = flash.packed_fwd(rot, B, S, H, nshard, causal=True)
+        ctx.save_for_backward(rot, out, lse, cos, sin)
+        ctx.cfg = (B, S, H, nshard, hd)
+        return out
+
+    @staticmethod
+    def backward(ctx, dout):
+        from . import flash, kernels as K
+        rot, out, lse, cos, sin = ctx.saved_tensors
+        B, S, H, nshard, hd = ctx.cfg
+        dqkv = flash.packed_bwd(rot, out, lse, dout, B, S, H, nshard, causal=True)
+        return (K.rope_packed(dqkv, cos, sin, hd, nshard, out=dqkv, backward=True),) + (None,) * 6
+
+
+def rope_attention_packed(qkv, cos, sin, heads, nshard=1):
+    """Causal self-attention with rotary embedding on a rotated packed projection ``qkv`` [B, S, 3 * D] (its columns grouped
+    per shard) -> [B, S, D].  ``cos`` / ``sin``: [S, hd / 2]."""
+    B, S, W = qkv.shape
+    hd = W // (3 * heads)
+    small = hd == 64 and S <= 96             # the short-sequence kernels take those
+    if use_kernels(qkv) and hd in (64, 128) and not small and qkv.is_contiguous() and qkv.data_ptr() % 16 == 0:
+        c, s = cos.float().contiguous(), sin.float().contiguous()
+        return _RopeAttnPackedFn.apply(qkv.view(B * S, W), c, s, B, S, heads, nshard).view(B, S, W // 3)
+    return None
 
 
 # ---------------------------------------------------------------------------------------------------------------------

@@ -38,6 +38,7 @@ def _L():
         L.rtp_top2_gate_fwd.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, vp]
         L.rtp_top2_gate_bwd.argtypes = [vp, vp, vp, vp, vp, vp, vp, i, i, vp]
         L.rtp_rope.argtypes = [vp, vp, vp, vp, ll, i, i, i, i, i, vp]
+        L.rtp_rope_packed.argtypes = [vp, vp, vp, vp, ll, i, i, i, i, i, vp]
         L.rtp_im2col_last_error.restype = C.c_char_p
         L.rtp_im2col.argtypes = [vp, vp] + [i] * 13 + [vp]
         L.rtp_col2im.argtypes = [vp, vp] + [i] * 13 + [vp]
@@ -259,6 +260,26 @@ def swiglu_bwd(g, u, dy):
     return dg, du
 
 
+def swiglu_packed(y, nshard):
+    """silu(g) * u of a packed projection ``y`` [T, 2 * F] whose columns hold, for each of ``nshard`` shards, the gate and the
+    up block side by side -> [T, F]."""
+    T, W = y.shape
+    c = W // (2 * nshard)
+    out = torch.empty(T, W // 2, dtype=y.dtype, device=y.device)
+    _check(_L().rtp_swiglu_fwd(_p(y), y.data_ptr() + 2 * c, 2 * c, _p(out), T * nshard, c, _lib.stream_ptr()), "swiglu_fwd")
+    return out
+
+
+def swiglu_packed_bwd(y, dy, nshard):
+    """Gradient of :func:`swiglu_packed` in the packed layout of ``y``."""
+    T, W = y.shape
+    c = W // (2 * nshard)
+    dp = torch.empty_like(y)
+    _check(_L().rtp_swiglu_bwd(_p(y), y.data_ptr() + 2 * c, 2 * c, _p(dy), _p(dp), dp.data_ptr() + 2 * c, 2 * c, T * nshard, c,
+                               _lib.stream_ptr()), "swiglu_bwd")
+    return dp
+
+
 def moe_scatter(src, slot, scale, dst_rows):
     """dst[slot[s, k]] = scale[s, k] * src[s] (rows without a token stay zero). slot: int32 [S, 2], -1 = dropped."""
     S, M = src.shape
@@ -432,6 +453,16 @@ def rope(x, cos, sin, inner=1):
     """Rotary position embedding of bf16 `x` [..., H, hd] whose flattened leading dims are tokens; token t sits at
     position (t // inner) % S, with cos / sin of shape [S, hd / 2] (pairs (x[2i], x[2i+1]) rotate together)."""
     return _Rope.apply(x, cos, sin, inner)
+
+
+def rope_packed(qkv, cos, sin, hd, nshard, out=None, backward=False):
+    """Rotates the q and k blocks of a packed projection [T, 3 * D] (see ``ops.flash.flash_attention_packed``); token t sits
+    at position t % S, with fp32 cos / sin of shape [S, hd / 2].  ``out``: None for a new buffer, ``qkv`` for in place."""
+    T, W = qkv.shape
+    y = torch.empty_like(qkv) if out is None else out
+    _gate_check(_L().rtp_rope_packed(_p(qkv), _p(y), _p(cos), _p(sin), T, W // 3, hd, nshard, cos.shape[0], int(backward),
+                                     _lib.stream_ptr()), "rope_packed")
+    return y
 
 
 def _pair(v):
