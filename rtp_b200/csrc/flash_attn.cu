@@ -910,6 +910,23 @@ __global__ void __launch_bounds__(kThreads, 1) flash_dkv_kernel(const __grid_con
       const bool plain = keys_plain && !(M.causal && it < 2);
       const float4* lse4 = reinterpret_cast<const float4*>(sStat + st * 2 * kHalf + wg * 32);
       const float4* del4 = reinterpret_cast<const float4*>(sStat + st * 2 * kHalf + kHalf + wg * 32);
+      // Dropout bits.  One generator call covers four neighbouring keys, which sit in four neighbouring lanes: each lane
+      // calls it for every fourth query and the four exchange their nibbles (eight calls a thread instead of 32;
+      // 2 x 8 heads of 1024 x 1024, head_dim 64, causal: dK / dV 110 -> 43.3 us).
+      uint32_t kw[4] = {0u, 0u, 0u, 0u};                       // kw[e]: nibble g = keys of the quad, query 4 g + e
+      if constexpr (DRP) {
+        uint32_t mine = 0;
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+          const int q = min(qbase + 4 * g + (lane & 3), M.Sq - 1);
+          const unsigned long long idx = ((unsigned long long)bh * M.Sq + q) * (unsigned long long)M.Sk + (key & ~3);
+          const uint4 r = philox4x32(M.seed, offset, idx >> 2);
+          mine |= ((r.x >= M.thresh ? 1u : 0u) | (r.y >= M.thresh ? 2u : 0u) | (r.z >= M.thresh ? 4u : 0u) |
+                   (r.w >= M.thresh ? 8u : 0u)) << (4 * g);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) kw[e] = __shfl_sync(0xffffffffu, mine, (lane & ~3) + e) >> (lane & 3);
+      }
 #pragma unroll
       for (int g = 0; g < 8; ++g) {
         const float4 L4 = lse4[g], D4 = del4[g];
@@ -931,10 +948,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_dkv_kernel(const __grid_con
           }
           const float pr = ex2_approx(xs - lse_[e]);
           bool kp = true;
-          if constexpr (DRP) {
-            const unsigned long long idx = ((unsigned long long)bh * M.Sq + min(q, M.Sq - 1)) * (unsigned long long)M.Sk + key;
-            kp = dropout_keep(M.seed, offset, idx, M.thresh);
-          }
+          if constexpr (DRP) kp = (kw[e] >> (4 * g)) & 1u;
           const float d = kp ? dp[i] * M.drop_scale : 0.f;
           dp[i] = pr * (d - del_[e]);             // dS
           x[i] = kp ? pr * M.drop_scale : 0.f;    // dropped probability
