@@ -18,6 +18,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "launch.h"
 
 namespace {
 using namespace rtp;
@@ -230,6 +231,7 @@ __global__ void gate_bwd_kernel(const float* __restrict__ gates, const int* __re
 __global__ void rope_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y,
                             const float* __restrict__ cosv, const float* __restrict__ sinv, long long T, int H, int hd,
                             int S, int inner, float sin_sign) {
+  rtp::pdl_prologue();
   const int half = hd >> 1;
   const long long total = T * H * (half >> 2);   // 4 pairs (8 elements, 16 bytes) per item
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -260,6 +262,7 @@ __global__ void rope_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* 
 // zero-fills and additions of the slices' gradients.
 __global__ void rope_packed_kernel(const __nv_bfloat16* x, __nv_bfloat16* y, const float* __restrict__ cosv,
                                    const float* __restrict__ sinv, long long T, int D, int hd, int nshard, int S, float sin_sign) {
+  rtp::pdl_prologue();
   const int half = hd >> 1, blk = D / nshard;               // columns of one of a group's q / k / v blocks
   const int cols = x == y ? 2 * blk : 3 * blk;              // in place: only q and k of a group are touched
   const int per_group = cols >> 3, per_row = nshard * per_group;
@@ -329,7 +332,7 @@ int rtp_rope(const void* x, void* y, const float* cosv, const float* sinv, long 
   long long blocks = (total + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
   if (blocks < 1) return 0;
-  rope_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)x, (__nv_bfloat16*)y, cosv, sinv, T,
+  rtp::launch_k(rope_kernel, dim3((unsigned)blocks), dim3(256), 0, (cudaStream_t)stream, (const __nv_bfloat16*)x, (__nv_bfloat16*)y, cosv, sinv, T,
                                                                  H, hd, S, inner, backward ? -1.f : 1.f);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail("rope", e);
@@ -348,7 +351,7 @@ int rtp_rope_packed(const void* x, void* y, const float* cosv, const float* sinv
   long long blocks = (total + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
   if (blocks < 1) return 0;
-  rope_packed_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)x, (__nv_bfloat16*)y, cosv, sinv, T, D,
+  rtp::launch_k(rope_packed_kernel, dim3((unsigned)blocks), dim3(256), 0, (cudaStream_t)stream, (const __nv_bfloat16*)x, (__nv_bfloat16*)y, cosv, sinv, T, D,
                                                                         hd, nshard, S, backward ? -1.f : 1.f);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail("rope_packed", e);

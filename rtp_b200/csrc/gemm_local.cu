@@ -549,7 +549,7 @@ int launch_local(const Params<MAXJ>& P, cudaStream_t stream) {
   cfg.stream = stream;
   cudaLaunchAttribute at[2];
   int nat = 0;
-  if (pdl_enabled()) {
+  if (pdl_local()) {
     at[nat].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[nat].val.programmaticStreamSerializationAllowed = 1;
     ++nat;

@@ -108,13 +108,44 @@ __device__ __forceinline__ void block_sum_n(float (&v)[N], float* red, int turn)
     for (int i = 0; i < N; ++i) mine[w * N + i] = v[i];
   }
   __syncthreads();
+  // the warps' sums in the order of a butterfly: halves first
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    float t = mine[i];
+    float t[W];
 #pragma unroll
-    for (int k = 1; k < W; ++k) t += mine[k * N + i];
-    v[i] = t;
+    for (int k = 0; k < W; ++k) t[k] = mine[k * N + i];
+#pragma unroll
+    for (int o = W / 2; o > 0; o >>= 1)
+#pragma unroll
+      for (int k = 0; k < o; ++k) t[k] += t[k + o];
+    v[i] = t[0];
   }
+}
+
+// One sum over the block of NS values per thread, value i standing for the threads i T .. i T + T - 1 of a wider block.
+template <int T, int NS>
+__device__ __forceinline__ float row_sum(float (&v)[NS], float* red, int turn) {
+  if (NS == 1) {
+    block_sum_n<T, NS>(v, red, turn);
+    return v[0];
+  }
+  constexpr int W = T / 32;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  float* mine = red + turn * (W * NS);
+#pragma unroll
+  for (int i = 0; i < NS; ++i) {
+    v[i] = warp_sum(v[i]);
+    if (lane == 0) mine[i * W + w] = v[i];
+  }
+  __syncthreads();
+  float t[W * NS];
+#pragma unroll
+  for (int k = 0; k < W * NS; ++k) t[k] = mine[k];
+#pragma unroll
+  for (int o = W * NS / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int k = 0; k < o; ++k) t[k] += t[k + o];
+  return t[0];
 }
 
 template <int T, int NG>
@@ -123,7 +154,10 @@ __global__ void __launch_bounds__(T, T == 128 ? 7 : NG == 1 ? 4 : 2) norm_fwd_ke
     const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ h_out, __nv_bfloat16* __restrict__ y,
     float* __restrict__ mean_out, float* __restrict__ rstd_out, int M, int D, float eps, int rms, uint32_t thresh,
     float drop_scale, uint64_t seed, uint64_t offset, const unsigned long long* __restrict__ step_ptr) {
-  __shared__ float red[2 * (T / 32)];
+  pdl_prologue();
+  // 128 threads with two groups of columns each add up like 256 threads with one: the statistics have the same bits
+  constexpr int NS = T == 128 ? NG : 1;
+  __shared__ float red[2 * (T / 32) * NS];
   if (step_ptr) offset += __ldg(step_ptr) * 65536ull;
   const int c0 = threadIdx.x * 8;
   uint4 nx[NG], ns[NG], g[NG], bt[NG];
@@ -151,7 +185,9 @@ __global__ void __launch_bounds__(T, T == 128 ? 7 : NG == 1 ? 4 : 2) norm_fwd_ke
   for (int row = blockIdx.x; row < M; row += gridDim.x) {
     const size_t base = (size_t)row * D;
     float v[NG][8];
-    float s[1] = {0.f};
+    float s[NS];
+#pragma unroll
+    for (int i = 0; i < NS; ++i) s[i] = 0.f;
 #pragma unroll
     for (int q = 0; q < NG; ++q) {
       const int c = q * T * 8 + c0;
@@ -173,27 +209,27 @@ __global__ void __launch_bounds__(T, T == 128 ? 7 : NG == 1 ? 4 : 2) norm_fwd_ke
         unpack8(hp, v[q]);
         if (h_out) *reinterpret_cast<uint4*>(h_out + base + c) = hp;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) s[0] += v[q][i];
+        for (int i = 0; i < 8; ++i) s[q % NS] += v[q][i];
       }
     }
     if (row + (int)gridDim.x < M) fetch(row + gridDim.x);
     float mean = 0.f;
     if (!rms) {
-      block_sum_n<T, 1>(s, red, turn);
+      mean = row_sum<T, NS>(s, red, turn) / D;
       turn ^= 1;
-      mean = s[0] / D;
     }
-    float qq[1] = {0.f};
+    float qq[NS];
+#pragma unroll
+    for (int i = 0; i < NS; ++i) qq[i] = 0.f;
 #pragma unroll
     for (int q = 0; q < NG; ++q) {
       if (q * T * 8 + c0 < D) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) { const float d = v[q][i] - mean; qq[0] += d * d; }
+        for (int i = 0; i < 8; ++i) { const float d = v[q][i] - mean; qq[q % NS] += d * d; }
       }
     }
-    block_sum_n<T, 1>(qq, red, turn);
+    const float rstd = rsqrtf(row_sum<T, NS>(qq, red, turn) / D + eps);
     turn ^= 1;
-    const float rstd = rsqrtf(qq[0] / D + eps);
     if (threadIdx.x == 0) {
       if (mean_out) mean_out[row] = mean;
       rstd_out[row] = rstd;
@@ -227,6 +263,7 @@ __global__ void __launch_bounds__(256, 2) norm_bwd_kernel(
     __nv_bfloat16* __restrict__ dsub, float* __restrict__ dgamma, float* __restrict__ dbeta, int M, int D, int rms,
     uint32_t thresh, float drop_scale, uint64_t seed, uint64_t offset, const __nv_bfloat16* __restrict__ dres,
     const unsigned long long* __restrict__ step_ptr, int vec_atomics) {
+  pdl_prologue();
   constexpr int G = 256 / T;                   // row groups of the block
   __shared__ float red[2 * 8 * 2 * R];
   __shared__ float colsum[G > 1 ? 2 * 2048 : 1];
@@ -374,6 +411,7 @@ __global__ void __launch_bounds__(256, 2) norm_bwd_kernel(
 __global__ void ce_kernel(__nv_bfloat16* logits, long long ld, const long long* __restrict__ target,
                           float* __restrict__ loss, int M, int V, float grad_scale, long long ignore_index,
                           int write_grad, __nv_bfloat16* grad, long long ldg) {
+  pdl_prologue();
   __shared__ float red[32];
   for (int row = blockIdx.x; row < M; row += gridDim.x) {
     __nv_bfloat16* lp = logits + (size_t)row * ld;
@@ -424,14 +462,14 @@ __global__ void ce_kernel(__nv_bfloat16* logits, long long ld, const long long* 
 // three times, twice from L2.  Tried and dropped: the row in shared memory, filled and drained by bulk copies (604 us at
 // 50304 logits); 1024 threads with half the words (642 us, one block per SM); unpacking anew in every pass instead of
 // letting the compiler spill what does not fit (720 us).
-constexpr int kCeThreads = 512;
+// Up to 16384 logits 256 threads, which add up in the order of the kernel above.
 constexpr int kCeMaxV = 65536;
-template <int NG>
-__global__ void __launch_bounds__(kCeThreads, 2) ce_row_kernel(
+template <int kCeThreads, int NG>
+__global__ void __launch_bounds__(kCeThreads, kCeThreads == 512 ? 2 : 3) ce_row_kernel(
     const __nv_bfloat16* logits, long long ld, const long long* __restrict__ target, float* __restrict__ loss, int V,
     float grad_scale, const float* __restrict__ scale_ptr, long long ignore_index, __nv_bfloat16* grad, long long ldg) {
+  pdl_prologue();
   __shared__ float red[32];
-  constexpr float kLog2e = 1.4426950408889634f;
   const int row = blockIdx.x, tid = threadIdx.x, n = V >> 3;
   const uint4* lp = reinterpret_cast<const uint4*>(logits + (size_t)row * ld);
   const long long t = target[row];
@@ -461,13 +499,13 @@ __global__ void __launch_bounds__(kCeThreads, 2) ce_row_kernel(
       float v[8];
       unpack8(u[q], v);
 #pragma unroll
-      for (int k = 0; k < 8; ++k) se += exp2f((v[k] - mx) * kLog2e);
+      for (int k = 0; k < 8; ++k) se += __expf(v[k] - mx);
     }
   }
   se = block_sum(se, red);
   if (tid == 0) loss[row] = ignored ? 0.f : mx + __logf(se) - lt;
   if (!grad) return;
-  const float sc = grad_scale / se;
+  const float inv = 1.f / se;
   uint4* gp = reinterpret_cast<uint4*>(grad + (size_t)row * ldg);
 #pragma unroll
   for (int q = 0; q < NG; ++q) {
@@ -477,9 +515,9 @@ __global__ void __launch_bounds__(kCeThreads, 2) ce_row_kernel(
       unpack8(u[q], v);
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        v[k] = exp2f((v[k] - mx) * kLog2e) * sc;
-        if (i * 8 + k == (int)t) v[k] -= grad_scale;
-        if (ignored) v[k] = 0.f;
+        float p = __expf(v[k] - mx) * inv;
+        if (i * 8 + k == (int)t) p -= 1.f;
+        v[k] = ignored ? 0.f : p * grad_scale;
       }
       __stcs(gp + i, pack8(v));
     }
@@ -488,6 +526,7 @@ __global__ void __launch_bounds__(kCeThreads, 2) ce_row_kernel(
 
 // n = number of targets that count (at least one), for the mean: out[0] = n, out[1] = 1 / n.
 __global__ void ce_count_kernel(const long long* __restrict__ target, int M, long long ignore_index, float* out) {
+  pdl_prologue();
   __shared__ int total;
   int c = 0;
   for (int i = threadIdx.x; i < M; i += blockDim.x) c += target[i] != ignore_index;
@@ -524,6 +563,7 @@ __global__ void embed_fwd_kernel(const __nv_bfloat16* __restrict__ table, const 
                                  __nv_bfloat16* __restrict__ out, long long ld_out, int col_off, int T, int Ds, int D,
                                  float scale, uint32_t thresh, float drop_scale, uint64_t seed, uint64_t offset,
                                  const unsigned long long* __restrict__ step_ptr) {
+  pdl_prologue();
   if (step_ptr) offset += __ldg(step_ptr) * 65536ull;
   const int per_row = Ds / 8;
   const long long total = (long long)T * per_row;
@@ -555,6 +595,7 @@ __global__ void embed_bwd_kernel(__nv_bfloat16* __restrict__ gtable, const long 
                                  const __nv_bfloat16* __restrict__ dy, long long ld_dy, int col_off, int T, int Ds,
                                  int D, float scale, uint32_t thresh, float drop_scale, uint64_t seed, uint64_t offset,
                                  const unsigned long long* __restrict__ step_ptr, int blk_cols, int V) {
+  pdl_prologue();
   if (step_ptr) offset += __ldg(step_ptr) * 65536ull;
   const int per_row = Ds / 8;
   const long long total = (long long)T * per_row;
@@ -657,6 +698,7 @@ __global__ void __launch_bounds__(512) attn_small_fwd_kernel(const __nv_bfloat16
                                       int S, int B, int heads, int nshard, int causal, float sm_scale, uint32_t thresh,
                                       float drop_scale, uint64_t seed, uint64_t offset,
                                       const unsigned long long* __restrict__ step_ptr) {
+  pdl_prologue();
   extern __shared__ __align__(16) float smf[];
   if (step_ptr) offset += __ldg(step_ptr) * 65536ull;
   const int D = heads * kHd;
@@ -711,6 +753,7 @@ __global__ void __launch_bounds__(512) attn_small_bwd_kernel(const __nv_bfloat16
                                       const __nv_bfloat16* __restrict__ dout, __nv_bfloat16* __restrict__ dqkv, int S, int B,
                                       int heads, int nshard, int causal, float sm_scale, uint32_t thresh, float drop_scale,
                                       uint64_t seed, uint64_t offset, const unsigned long long* __restrict__ step_ptr) {
+  pdl_prologue();
   extern __shared__ __align__(16) float smf[];
   if (step_ptr) offset += __ldg(step_ptr) * 65536ull;
   const int D = heads * kHd;
@@ -812,6 +855,7 @@ __global__ void colsum_kernel(const __nv_bfloat16* __restrict__ x, long long ld,
 // block of the cluster adds them up through distributed shared memory and stores the result (no atomics, no zero-fill).
 __global__ void __launch_bounds__(256) colsum_vec_kernel(const __nv_bfloat16* __restrict__ x, long long ld, int M, int N,
                                                          float* __restrict__ out, int rows_per_block, int atomic) {
+  pdl_prologue();
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   __shared__ float red[32][65];
@@ -890,8 +934,8 @@ __device__ __forceinline__ void adam_element(float& p, float g, float& m, float&
   if (weight_decay != 0.f) {
     if (adamw) p = __fmul_rn(p, 1.f - decay); else g = __fmaf_rn(weight_decay, p, g);
   }
-  m = __fmaf_rn(beta1, m, __fmul_rn(1.f - beta1, g));
-  v = __fmaf_rn(beta2, v, __fmul_rn(__fmul_rn(1.f - beta2, g), g));
+  m = __fmaf_rn(1.f - beta1, g, __fmul_rn(beta1, m));
+  v = __fmaf_rn(__fmul_rn(1.f - beta2, g), g, __fmul_rn(beta2, v));
   p = __fsub_rn(p, __fdividef(__fmul_rn(step_size, m), __fmaf_rn(sqrtf(v), inv_sqrt_bc2, eps)));
 }
 struct AdamRegs {
@@ -1340,6 +1384,7 @@ __global__ void cast_f32_bf16_kernel(const float* in, __nv_bfloat16* out, long l
 }
 // sum of fp32 vector * scale (/ *divisor) -> out[0] (single block)
 __global__ void sum_kernel(const float* in, float* out, int n, float scale, const float* __restrict__ divisor) {
+  pdl_prologue();
   __shared__ float red[32];
   float s = 0.f;
   for (int i = threadIdx.x; i < n; i += blockDim.x) s += in[i];
@@ -1360,7 +1405,7 @@ int rtp_norm_fwd(const void* x, const void* sub, const void* gamma, const void* 
   const float ds = drop_p > 0.f ? 1.f / (1.f - drop_p) : 1.f;
   const bool drop = sub && drop_p > 0.f;
 #define RTP_NORM_FWD(T, NG, PER_SM)                                                                                   \
-  norm_fwd_kernel<T, NG><<<std::min(M, 148 * PER_SM), T, 0, (cudaStream_t)stream>>>(                                  \
+  rtp::launch_k(norm_fwd_kernel<T, NG>, dim3(std::min(M, 148 * PER_SM)), dim3(T), 0, (cudaStream_t)stream,                                  \
       (const __nv_bfloat16*)x, (const __nv_bfloat16*)sub, (const __nv_bfloat16*)gamma, (const __nv_bfloat16*)beta,    \
       (__nv_bfloat16*)h_out, (__nv_bfloat16*)y, mean, rstd, M, D, eps, rms, host_thresh(drop_p), ds, seed, offset,    \
       step_ptr)
@@ -1380,7 +1425,7 @@ int rtp_norm_bwd(const void* dy, const void* h, const void* gamma, const float* 
   const int vec_atomics = ((reinterpret_cast<uintptr_t>(dgamma) | reinterpret_cast<uintptr_t>(dbeta)) & 15) == 0;
   // few blocks: every block ends with one vector atomic per 4 columns of dgamma / dbeta
 #define RTP_NORM_BWD(T, NG, R)                                                                                        \
-  norm_bwd_kernel<T, NG, R><<<std::min((M + 256 / T * R - 1) / (256 / T * R), 296), 256, 0, (cudaStream_t)stream>>>(  \
+  rtp::launch_k(norm_bwd_kernel<T, NG, R>, dim3(std::min((M + 256 / T * R - 1) / (256 / T * R), 296)), dim3(256), 0, (cudaStream_t)stream,  \
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)h, (const __nv_bfloat16*)gamma, mean, rstd, (__nv_bfloat16*)dx, \
       (__nv_bfloat16*)dsub, dgamma, dbeta, M, D, rms, host_thresh(drop_p), ds, seed, offset,                          \
       (const __nv_bfloat16*)dres, step_ptr, vec_atomics)
@@ -1408,27 +1453,27 @@ int rtp_cross_entropy_scaled(void* logits, long long ld, const long long* target
                              void* stream) {
   if (V % 8 || ld % 8 || (grad && ldg % 8)) { k_err = "cross_entropy: V and the row pitches must be multiples of 8"; return -1; }
   if (M > 0 && V > 0 && V <= kCeMaxV) {
-#define RTP_CE(NG)                                                                                                        \
-  ce_row_kernel<NG><<<M, kCeThreads, 0, (cudaStream_t)stream>>>(                                                          \
+#define RTP_CE(T, NG)                                                                                                        \
+  rtp::launch_k(ce_row_kernel<T, NG>, dim3(M), dim3(T), 0, (cudaStream_t)stream,                                                          \
       (const __nv_bfloat16*)logits, ld, target, loss, V, grad_scale, scale_ptr, ignore_index,                             \
       (__nv_bfloat16*)(write_grad ? (grad ? grad : logits) : nullptr), grad ? ldg : ld)
-    const int ng = (V / 8 + kCeThreads - 1) / kCeThreads;
-    if (ng == 1) RTP_CE(1); else if (ng == 2) RTP_CE(2); else if (ng == 3) RTP_CE(3); else if (ng == 4) RTP_CE(4);
-    else if (ng <= 6) RTP_CE(6); else if (ng <= 8) RTP_CE(8); else if (ng <= 10) RTP_CE(10); else if (ng <= 13) RTP_CE(13);
-    else RTP_CE(16);
+    const int w = (V / 8 + 255) / 256;       // 16-byte words per thread of 256
+    if (w == 1) RTP_CE(256, 1); else if (w == 2) RTP_CE(256, 2); else if (w <= 4) RTP_CE(256, 4); else if (w == 5) RTP_CE(256, 5);
+    else if (w <= 8) RTP_CE(256, 8); else if (w <= 12) RTP_CE(512, 6); else if (w <= 16) RTP_CE(512, 8);
+    else if (w <= 20) RTP_CE(512, 10); else if (w <= 26) RTP_CE(512, 13); else RTP_CE(512, 16);
 #undef RTP_CE
     LAUNCH_CHECK("cross_entropy");
     return 0;
   }
   if (scale_ptr) { k_err = "cross_entropy: a device-side scale needs rows of at most 65536 logits"; return -1; }
   const int grid = M < 148 * 8 ? M : 148 * 8;
-  ce_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>((__nv_bfloat16*)logits, ld, target, loss, M, V, grad_scale,
+  rtp::launch_k(ce_kernel, dim3(grid), dim3(256), 0, (cudaStream_t)stream, (__nv_bfloat16*)logits, ld, target, loss, M, V, grad_scale,
                                                     ignore_index, write_grad, (__nv_bfloat16*)grad, ldg);
   LAUNCH_CHECK("cross_entropy");
   return 0;
 }
 int rtp_ce_count(const long long* target, int M, long long ignore_index, float* out2, void* stream) {
-  ce_count_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(target, M, ignore_index, out2);
+  rtp::launch_k(ce_count_kernel, dim3(1), dim3(1024), 0, (cudaStream_t)stream, target, M, ignore_index, out2);
   LAUNCH_CHECK("ce_count");
   return 0;
 }
@@ -1450,7 +1495,7 @@ int rtp_embed_fwd(const void* table, const long long* ids, const void* pe, long 
   int grid = (int)((total + 255) / 256);
   if (grid > 148 * 16) grid = 148 * 16;
   const float ds = drop_p > 0.f ? 1.f / (1.f - drop_p) : 1.f;
-  embed_fwd_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)table, ids, (const __nv_bfloat16*)pe,
+  rtp::launch_k(embed_fwd_kernel, dim3(grid), dim3(256), 0, (cudaStream_t)stream, (const __nv_bfloat16*)table, ids, (const __nv_bfloat16*)pe,
                                                            ld_pe, tokens_per_pos, (__nv_bfloat16*)out, ld_out, col_off,
                                                            T, Ds, D, scale, host_thresh(drop_p), ds, seed, offset,
                                                            step_ptr);
@@ -1473,7 +1518,7 @@ int rtp_embed_bwd_blocks(void* gtable, const long long* ids, const void* dy, lon
   int grid = (int)((total + 255) / 256);
   if (grid > 148 * 16) grid = 148 * 16;
   const float ds = drop_p > 0.f ? 1.f / (1.f - drop_p) : 1.f;
-  embed_bwd_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>((__nv_bfloat16*)gtable, ids, (const __nv_bfloat16*)dy, ld_dy,
+  rtp::launch_k(embed_bwd_kernel, dim3(grid), dim3(256), 0, (cudaStream_t)stream, (__nv_bfloat16*)gtable, ids, (const __nv_bfloat16*)dy, ld_dy,
                                                            col_off, T, Ds, D, scale, host_thresh(drop_p), ds, seed,
                                                            offset, step_ptr, blk_cols, V);
   LAUNCH_CHECK("embed_bwd");
@@ -1501,7 +1546,7 @@ int rtp_attn_small_fwd(const void* qkv, void* out, int S, int B, int heads, int 
     if (e != cudaSuccess) return kfail("attn fwd attr", e);
   }
   const float ds = drop_p > 0.f ? 1.f / (1.f - drop_p) : 1.f;
-  attn_small_fwd_kernel<<<B * heads, attn_threads(S), smem, (cudaStream_t)stream>>>(
+  rtp::launch_k(attn_small_fwd_kernel, dim3(B * heads), dim3(attn_threads(S)), smem, (cudaStream_t)stream,
       (const __nv_bfloat16*)qkv, (__nv_bfloat16*)out, S, B, heads, nshard, causal, sm_scale, host_thresh(drop_p), ds,
       seed, offset, step_ptr);
   LAUNCH_CHECK("attn_small_fwd");
@@ -1524,7 +1569,7 @@ int rtp_attn_small_bwd(const void* qkv, const void* dout, void* dqkv, int S, int
     if (e != cudaSuccess) return kfail("attn bwd attr", e);
   }
   const float ds = drop_p > 0.f ? 1.f / (1.f - drop_p) : 1.f;
-  attn_small_bwd_kernel<<<B * heads, attn_threads(S), smem, (cudaStream_t)stream>>>(
+  rtp::launch_k(attn_small_bwd_kernel, dim3(B * heads), dim3(attn_threads(S)), smem, (cudaStream_t)stream,
       (const __nv_bfloat16*)qkv, (const __nv_bfloat16*)dout, (__nv_bfloat16*)dqkv, S, B, heads, nshard, causal,
       sm_scale, host_thresh(drop_p), ds, seed, offset, step_ptr);
   LAUNCH_CHECK("attn_small_bwd");
@@ -1607,8 +1652,7 @@ int rtp_swiglu_bwd(const void* g, const void* u, long long ld, const void* dy, v
                    long long rows, int cols, void* stream) {
   if (cols % 8 || ld % 8 || ldo % 8) { k_err = "swiglu: cols and ld must be multiples of 8"; return -1; }
   const long long items = rows * (cols / 8);
-  swiglu_bwd_kernel<<<(unsigned)((items + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)g, (const __nv_bfloat16*)u, ld, (const __nv_bfloat16*)dy, (__nv_bfloat16*)dg, (__nv_bfloat16*)du, ldo, rows,
+  swiglu_bwd_kernel<<<(unsigned)((items + 255) / 256), 256, 0, (cudaStream_t)stream>>>(      (const __nv_bfloat16*)g, (const __nv_bfloat16*)u, ld, (const __nv_bfloat16*)dy, (__nv_bfloat16*)dg, (__nv_bfloat16*)du, ldo, rows,
       cols);
   LAUNCH_CHECK("swiglu_bwd");
   return 0;
@@ -1653,7 +1697,7 @@ int rtp_cast_f32_bf16(const float* in, void* out, long long n, float scale, void
   return 0;
 }
 int rtp_sum_f32(const float* in, float* out, int n, float scale, const float* divisor, void* stream) {
-  sum_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(in, out, n, scale, divisor);
+  rtp::launch_k(sum_kernel, dim3(1), dim3(1024), 0, (cudaStream_t)stream, in, out, n, scale, divisor);
   LAUNCH_CHECK("sum");
   return 0;
 }

@@ -5,16 +5,21 @@
 
 namespace rtp {
 
-// RTP_PDL=1 lets a kernel start while its predecessor drains (off by default: on the training step the kernels fill
-// the SMs' registers and shared memory, so a successor rarely finds room before its predecessor has left)
-inline bool pdl_enabled() {
-  static int on = -1;
-  if (on < 0) {
+// Programmatic dependent launch: a kernel may start, set itself up and wait (griddepcontrol.wait) while its predecessor in
+// the stream drains, which takes 0.7 to 1 us off a launch in a CUDA graph (README LM step 3682 -> 3594 us, the small LM 223 ->
+// 210).  Streaming kernels of very many blocks are launched without it: with Adam in it the step took 3790 us.  RTP_PDL unset: the kernels that work on this GPU
+// alone.  RTP_PDL=1: the rotation kernels too (on the training step of a ring they fill the SMs' registers and shared
+// memory, so a successor rarely finds room before its predecessor has left).  RTP_PDL=0: none.
+inline int pdl_env() {
+  static int v = -2;
+  if (v == -2) {
     const char* e = getenv("RTP_PDL");
-    on = (e && e[0] == '1') ? 1 : 0;
+    v = !e || !e[0] ? -1 : e[0] == '1' ? 1 : 0;
   }
-  return on == 1;
+  return v;
 }
+inline bool pdl_enabled() { return pdl_env() == 1; }      // rotation kernels
+inline bool pdl_local() { return pdl_env() != 0; }        // kernels that only touch this GPU
 
 // Raises the dynamic shared-memory limit of kernel `Kern` on the current device, once per (kernel, device): the
 // attribute belongs to the kernel on one device, so a process that drives several GPUs sets it on each.
@@ -40,7 +45,7 @@ cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t sme
   cfg.stream = stream;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+  at[0].val.programmaticStreamSerializationAllowed = pdl_local() ? 1 : 0;
   cfg.attrs = at;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
@@ -57,7 +62,7 @@ cudaError_t launch_kc(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t sm
   cfg.stream = stream;
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+  at[0].val.programmaticStreamSerializationAllowed = pdl_local() ? 1 : 0;
   at[1].id = cudaLaunchAttributeClusterDimension;
   at[1].val.clusterDim.x = cluster.x;
   at[1].val.clusterDim.y = cluster.y;
