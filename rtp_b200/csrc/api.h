@@ -93,11 +93,16 @@ typedef struct {
   // Optional row of M ones (bf16).  Where rtp_linear_bwd_folds_bias() says yes and dbias_full is null, the launch makes the
   // bias gradient itself (in fp32, beside the weight gradient) and needs no column-sum kernel.
   const void* ones;
+  // Optional workspace of at least rtp_linear_bwd_scratch() bytes, 16-byte aligned: the weight gradient's contraction may
+  // then be split over the SMs.  The launch's own: it must not be shared with work on another stream.
+  void* scratch; unsigned long long scratch_bytes;
 } RtpLinearBwd;
 int rtp_linear_bwd(const RtpRing* ring, const RtpLinearBwd* op, void* stream);
 // 1 if the launch described by `op` computes the bias gradient itself (1-rank ring, op->ones given, 16-byte aligned
 // operands), 0 if the caller has to supply the column sums in dbias_full.  Every other field must be as for the launch.
 int rtp_linear_bwd_folds_bias(const RtpRing* ring, const RtpLinearBwd* op);
+// Bytes of workspace with which the launch runs faster (0: none).  Every other field must be as for the launch.
+unsigned long long rtp_linear_bwd_scratch(const RtpRing* ring, const RtpLinearBwd* op);
 
 // Rotating experts (MoE): rank r owns n_local whole experts; x / y hold the dispatched tokens expert-major
 // ([world*n_local*cap, features], expert g = rows [g*cap, (g+1)*cap)).  One launch applies ONE linear of every

@@ -1106,6 +1106,40 @@ int local_linear_bwd(const RtpRing& R, const RtpLinearBwd& op, rtp::LocalGemm* j
   }
   return all_ok(j, n) ? n : 0;
 }
+// A weight gradient of a few tiles whose contraction runs over many tokens (a convolution's: [64, 288] over 36 864
+// positions) keeps a handful of SMs busy for hundreds of k-blocks.  Where its 128 x 128 tiles fill at most an eighth of the
+// SMs and each has 128 k-blocks or more, the contraction falls into eight slices that leave fp32 sums in a workspace.
+// Whole backward, cold L2, unsplit -> split: that convolution 187 -> 78 us (weights alone 165 -> 39), 512 x 512 over 36 864
+// 185 -> 84, 768 x 384 over 8 192 (18 tiles, the most that split) 50 -> 44.  Over 4 096 positions the launches that add up
+// the slices cost more than they save: [64, 288] 27.6 -> 29.7, 768 x 384 28.2 -> 36.9.
+constexpr int kWgradSlices = 8;
+long long part_stride(const rtp::LocalGemm& w) { return (long long)w.M * w.N + (w.bsum ? (w.M + 3) / 4 * 4 : 0); }
+bool splits_wgrad(const rtp::LocalGemm& w) {
+  const long long tiles = (long long)((w.M + 127) / 128) * ((w.N + 127) / 128);
+  return !w.c && !w.bsum_add && tiles * 8 <= sm_count() && w.K >= 128 * 64;
+}
+int run_split_bwd(const RtpRing& R, const RtpLinearBwd& op, const rtp::LocalGemm* j, int n, void* stream) {
+  rtp::LocalGemm all[rtp::kLocalMaxJobs];
+  const rtp::LocalGemm& w = j[0];
+  float* part = reinterpret_cast<float*>(op.scratch);
+  const long long stride = part_stride(w);
+  const int per = ((w.K + 63) / 64 + kWgradSlices - 1) / kWgradSlices * 64;      // k of a slice
+  int m = 0, slices = 0;
+  for (int k0 = 0; k0 < w.K; k0 += per, ++slices) {
+    rtp::LocalGemm& x = all[m++] = w;
+    x.a = reinterpret_cast<const __nv_bfloat16*>(w.a) + (long long)k0 * w.lda;
+    x.b = reinterpret_cast<const __nv_bfloat16*>(w.b) + (long long)k0 * w.ldb;
+    x.K = std::min(per, w.K - k0);
+    x.d = part + slices * stride; x.ldd = w.N; x.part = 1;
+    if (w.bsum) x.bsum = part + slices * stride + (long long)w.M * w.N;
+  }
+  for (int i = 1; i < n; ++i) all[m++] = j[i];
+  if (run_local(R, all, m, stream)) return -1;
+  if (rtp::local_reduce(part, slices, stride, w.d, (long long)w.M * w.N, (cudaStream_t)stream) ||
+      (w.bsum && rtp::local_reduce(part + (long long)w.M * w.N, slices, stride, w.bsum, w.M, (cudaStream_t)stream)))
+    return fail(rtp::local_gemm_error());
+  return 0;
+}
 int local_expert_fwd(const RtpRing& R, const RtpExpertFwd& op, rtp::LocalGemm* j) {
   if (R.world != 1 || g_trace || op.n_local < 1 || op.n_local > rtp::kLocalMaxJobs) return 0;
   for (int e = 0; e < op.n_local; ++e) {
@@ -1535,7 +1569,12 @@ int rtp_linear_fwd(const RtpRing* ring, const RtpLinearFwd* op, void* stream) {
 }
 int rtp_linear_bwd(const RtpRing* ring, const RtpLinearBwd* op, void* stream) {
   rtp::LocalGemm jobs[rtp::kLocalMaxJobs];
-  if (const int n = local_linear_bwd(*ring, *op, jobs)) return run_local(*ring, jobs, n, stream);
+  if (const int n = local_linear_bwd(*ring, *op, jobs)) {
+    if (op->scratch && splits_wgrad(jobs[0]) && (reinterpret_cast<uintptr_t>(op->scratch) & 15) == 0 &&
+        op->scratch_bytes >= (unsigned long long)(kWgradSlices * part_stride(jobs[0]) * 4))
+      return run_split_bwd(*ring, *op, jobs, n, stream);
+    return run_local(*ring, jobs, n, stream);
+  }
   static thread_local rtp::GemmParams<1> params;
   // CTA pairs by the size of the input-gradient GEMM [M, in-per-shard], on any ring
   decide_pair(op->M, op->mode == 0 ? op->in_features : op->in_features / ring->world, ring->ctas);
@@ -1544,6 +1583,11 @@ int rtp_linear_bwd(const RtpRing* ring, const RtpLinearBwd* op, void* stream) {
   if (!params.prog[0].status) return fail("ring workspace required");
   params.ctas_per_rank = ring->ctas;
   return launch<1>(params, ring->ctas, false, (cudaStream_t)stream, true);
+}
+unsigned long long rtp_linear_bwd_scratch(const RtpRing* ring, const RtpLinearBwd* op) {
+  rtp::LocalGemm jobs[rtp::kLocalMaxJobs];
+  if (!local_linear_bwd(*ring, *op, jobs) || !splits_wgrad(jobs[0])) return 0;
+  return (unsigned long long)(kWgradSlices * part_stride(jobs[0]) * 4);
 }
 int rtp_linear_bwd_folds_bias(const RtpRing* ring, const RtpLinearBwd* op) {
   rtp::LocalGemm jobs[rtp::kLocalMaxJobs];

@@ -56,6 +56,7 @@ struct alignas(64) Job {
   float mask_scale, drop_scale;
   uint32_t drop_thresh;
   int act;
+  int part;                                      // 1: fp32 results, bare sums
   int sum;                                       // 1: d[m] = sum_k A[m, k] (+ c[m]); B is the tile of ones, bn = 16
   unsigned long long seed, offset;
   const unsigned long long* step_ptr;
@@ -294,7 +295,7 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
       const Job& J = P.job[find_job(P, t)];
       int tm, tn;
       tile_pos(J, t - J.tile0, tm, tn);
-      const int M = J.M, N = J.N, bn = J.bn, act = J.act;
+      const int M = J.M, N = J.N, bn = J.bn, act = J.act, part = J.part;
       const int row0 = tm * TM + (int)crank * kTM + quad * 32, n0 = tn * bn;
       const __nv_bfloat16* c = reinterpret_cast<const __nv_bfloat16*>(J.c);
       const __nv_bfloat16* mask = reinterpret_cast<const __nv_bfloat16*>(J.mask);
@@ -315,7 +316,10 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
         tmem_ld_32x32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * 256), ra);    // column 0 of 16 equal ones
         tmem_ld_wait();
         const int m = row0 + lane;
-        if (m < M) d[m] = __float2bfloat16(__uint_as_float(ra[0]) + (c ? __bfloat162float(c[m]) : 0.f));
+        if (m < M) {
+          if (J.part) reinterpret_cast<float*>(J.d)[m] = __uint_as_float(ra[0]);
+          else d[m] = __float2bfloat16(__uint_as_float(ra[0]) + (c ? __bfloat162float(c[m]) : 0.f));
+        }
       }
       for (int ch = half; !J.sum && ch * 64 < bn; ch += 2) {
         const int col0 = n0 + ch * 64;
@@ -358,6 +362,17 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
           tmem_ld_32x32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * 256 + ch * 64 + hh * 32), ra);
           tmem_ld_wait();
           const int colh = col0 + hh * 32;
+          if (part) {        // a slice of a contraction: rows of 128 bytes per thread, a few tiles in all
+            if (row0 + lane < M) {
+              float* dp = reinterpret_cast<float*>(J.d) + (long long)(row0 + lane) * ldd + colh;
+#pragma unroll
+              for (int q = 0; q < 8; ++q)
+                if (colh + 4 * q < N)
+                  reinterpret_cast<float4*>(dp)[q] = make_float4(__uint_as_float(ra[4 * q]), __uint_as_float(ra[4 * q + 1]),
+                                                                 __uint_as_float(ra[4 * q + 2]), __uint_as_float(ra[4 * q + 3]));
+            }
+            continue;
+          }
           float v[32];
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(ra[i]);
@@ -412,6 +427,7 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
                 make_uint4(pack_bf16(v[8 * q], v[8 * q + 1]), pack_bf16(v[8 * q + 2], v[8 * q + 3]),
                            pack_bf16(v[8 * q + 4], v[8 * q + 5]), pack_bf16(v[8 * q + 6], v[8 * q + 7]));
         }
+        if (part) continue;
         __syncwarp();
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
@@ -446,6 +462,25 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
     tc_fence_after();
     if (PAIR) tmem_dealloc_pair(tmem_base, 512); else tmem_dealloc(tmem_base, 512);
   }
+}
+
+// Adds up the slices of a split contraction, four elements a thread, always in the same order.  A few hundred KB that are
+// still in L2: bound by its launch (a few us).
+__global__ void __launch_bounds__(256) local_reduce_kernel(const float* __restrict__ part, int n, long long stride,
+                                                           __nv_bfloat16* __restrict__ out, long long len) {
+  pdl_prologue();
+  const long long i = (blockIdx.x * 256ll + threadIdx.x) * 4;
+  if (i >= len) return;
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+  for (int k = 0; k < n; ++k) {
+    const float4 v = __ldcs(reinterpret_cast<const float4*>(part + k * stride + i));
+    s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+  }
+  const float r[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (i + k < len) out[i + k] = __float2bfloat16(r[k]);
 }
 
 // ------------------------------------------------------------------------------------------------------------- host
@@ -609,6 +644,7 @@ int run(const Item* it, int n, int pair_policy, unsigned long long* status, unsi
     const LocalGemm& x = *it[best_ord[q]].g;
     Job& J = P.job[q];
     J.sum = it[best_ord[q]].sum ? 1 : 0;
+    J.part = x.part;
     J.M = x.M; J.kblocks = (x.K + 63) / 64;
     J.tile0 = total;
     J.tiles_m = (x.M + tm - 1) / tm;
@@ -654,6 +690,13 @@ int run(const Item* it, int n, int pair_policy, unsigned long long* status, unsi
 
 }  // namespace
 
+int local_reduce(const float* part, int n, long long stride, void* out, long long len, cudaStream_t stream) {
+  if (len <= 0) return 0;
+  const cudaError_t e = launch_k(local_reduce_kernel, dim3((unsigned)((len + 1023) / 1024)), dim3(256), 0, stream, part, n, stride,
+                                 reinterpret_cast<__nv_bfloat16*>(out), len);
+  return e == cudaSuccess ? 0 : lfail(std::string("launch local_reduce_kernel: ") + cudaGetErrorString(e));
+}
+
 const char* local_gemm_error() { return l_err.c_str(); }
 
 bool local_gemm_ok(const LocalGemm& g) {
@@ -662,6 +705,7 @@ bool local_gemm_ok(const LocalGemm& g) {
   if (!al16(g.a) || !al16(g.b) || g.lda % 8 || g.ldb % 8) return false;
   if (!al16(g.d) || g.ldd % 8 || !al16(g.c) || !al16(g.mask) || !al16(g.bias)) return false;
   if ((g.c && g.ldc % 8) || (g.mask && g.ldmask % 8)) return false;
+  if (g.part && (g.c || g.bias || g.act || g.mask || g.drop_p > 0.f || g.bsum_add)) return false;
   return !g.bsum || g.a_mn;
 }
 

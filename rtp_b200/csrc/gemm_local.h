@@ -23,6 +23,9 @@ struct LocalGemm {
   const unsigned long long* step_ptr;
   // column sums of A (a_mn = 1 only): bsum[m] (+)= sum_k A[m, k], in bf16
   void* bsum; int bsum_add;
+  // 1: d and bsum are fp32 and receive the bare sums (no c, bias, activation, mask or dropout): one slice of a contraction
+  // that local_reduce adds up
+  int part;
 };
 
 // Whether the local kernels take this job (16-byte aligned rows, N a multiple of 8).
@@ -32,6 +35,8 @@ bool local_gemm_ok(const LocalGemm& g);
 constexpr int kLocalMaxJobs = 16;
 int local_gemm(const LocalGemm* jobs, int n, int pair_policy, unsigned long long* status, unsigned long long timeout_ns,
                cudaStream_t stream);
+// out[i] = bf16(sum over n parts of part[k * stride + i]), i < len (parts 16-byte aligned, stride a multiple of 4)
+int local_reduce(const float* part, int n, long long stride, void* out, long long len, cudaStream_t stream);
 const char* local_gemm_error();
 
 }  // namespace rtp

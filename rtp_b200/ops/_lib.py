@@ -80,6 +80,7 @@ class LinearBwd(C.Structure):
         ("bank", C.c_int), ("no_self_push", C.c_int),
         ("next_home", C.c_void_p), ("next_bytes", C.c_ulonglong), ("next_kind", C.c_int),
         ("ones", C.c_void_p),
+        ("scratch", C.c_void_p), ("scratch_bytes", C.c_ulonglong),
     ]
 
 
@@ -203,6 +204,8 @@ def lib():
         L.rtp_linear_fwd_emu.argtypes = [C.POINTER(Ring), C.POINTER(LinearFwd), C.c_int, C.c_void_p]
         L.rtp_linear_bwd_emu.argtypes = [C.POINTER(Ring), C.POINTER(LinearBwd), C.c_int, C.c_void_p]
         L.rtp_linear_bwd_folds_bias.argtypes = [C.POINTER(Ring), C.POINTER(LinearBwd)]
+        L.rtp_linear_bwd_scratch.argtypes = [C.POINTER(Ring), C.POINTER(LinearBwd)]
+        L.rtp_linear_bwd_scratch.restype = C.c_ulonglong
         L.rtp_expert_bwd_folds_bias.argtypes = [C.POINTER(Ring), C.POINTER(ExpertBwd)]
         _lib = L
     return _lib

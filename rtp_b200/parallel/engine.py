@@ -287,6 +287,12 @@ def linear_bwd_raw(eng, flat, layout_info, x2d, dy2d, row, in_f, out_f, need_dx=
         if not _lib.lib().rtp_linear_bwd_folds_bias(C.byref(eng.ring), C.byref(op)):
             op.ones = None
             op.dbias_full = K.colsum(dy2d, dbias_buf).data_ptr()
+    scratch = None
+    if M >= 8192:           # only a long contraction can want a workspace
+        need = _lib.lib().rtp_linear_bwd_scratch(C.byref(eng.ring), C.byref(op))
+        if need:
+            scratch = torch.empty(need, dtype=torch.uint8, device=x2d.device)
+            op.scratch, op.scratch_bytes = scratch.data_ptr(), need
     _lib.check(_lib.lib().rtp_linear_bwd(C.byref(eng.ring), C.byref(op), _lib.stream_ptr()), "rtp_linear_bwd")
     return dx, gflat
 

@@ -53,6 +53,19 @@ def test_linear(M, I, O):
     eng.check()
 
 
+@pytest.mark.parametrize("M,I,O", [(8191, 288, 64), (8192, 288, 64), (8200, 72, 8), (36864, 288, 64), (9001, 1032, 128)])
+def test_long_contraction(M, I, O):
+    """Weight gradients of few tiles: one slice of the contraction, eight, and eight with a short last one."""
+    E, eng, flat, info, off, rnd = _linear(M, I, O)
+    x, dy = rnd(M, I), rnd(M, O)
+    xd, dyd, w = x.double(), dy.double(), flat[:O * I].view(O, I).double()
+    dx, g = E.linear_bwd_raw(eng, flat, info, x, dy, False, I, O)
+    _close(dx, dyd @ w, dyd.abs() @ w.abs())
+    _close(g[:O * I].view(O, I), dyd.t() @ xd, dyd.abs().t() @ xd.abs())
+    _close(g[off:off + O], dyd.sum(0), dyd.abs().sum(0))
+    eng.check()
+
+
 def test_dropout_mask_of_the_general_kernel():
     """The same (seed, offset) drops the same elements as the rotation kernel, which a forced tile width selects."""
     from rtp_b200.ops import gemm as G
