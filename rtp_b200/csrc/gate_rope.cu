@@ -279,7 +279,8 @@ __global__ void rope_packed_kernel(const __nv_bfloat16* x, __nv_bfloat16* y, con
       sn.x *= sin_sign; sn.y *= sin_sign; sn.z *= sin_sign; sn.w *= sin_sign;
       auto turn = [](uint32_t w, float c0, float s0) {
         const float a = __uint_as_float(w << 16), b = __uint_as_float(w & 0xffff0000u);
-        const __nv_bfloat162 o = __floats2bfloat162_rn(a * c0 - b * s0, a * s0 + b * c0);
+        // contracted as rope_kernel is, so that both give the same bits
+        const __nv_bfloat162 o = __floats2bfloat162_rn(__fmaf_rn(a, c0, -__fmul_rn(b, s0)), __fmaf_rn(a, s0, __fmul_rn(b, c0)));
         return *reinterpret_cast<const uint32_t*>(&o);
       };
       raw = make_uint4(turn(raw.x, cs.x, sn.x), turn(raw.y, cs.y, sn.y), turn(raw.z, cs.z, sn.z), turn(raw.w, cs.w, sn.w));
