@@ -1492,8 +1492,8 @@ int rtp_embed_fwd(const void* table, const long long* ids, const void* pe, long 
                   void* stream) {
   if (Ds % 8 || col_off % 8 || ld_out % 8) { k_err = "embed: widths must be multiples of 8"; return -1; }
   const long long total = (long long)T * (Ds / 8);
-  int grid = (int)((total + 255) / 256);
-  if (grid > 148 * 16) grid = 148 * 16;
+  if (total <= 0) return 0;
+  int grid = (int)((total + 255) / 256 > 148 * 16 ? 148 * 16 : (total + 255) / 256);
   const float ds = drop_p > 0.f ? 1.f / (1.f - drop_p) : 1.f;
   rtp::launch_k(embed_fwd_kernel, dim3(grid), dim3(256), 0, (cudaStream_t)stream, (const __nv_bfloat16*)table, ids, (const __nv_bfloat16*)pe,
                                                            ld_pe, tokens_per_pos, (__nv_bfloat16*)out, ld_out, col_off,

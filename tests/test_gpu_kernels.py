@@ -265,3 +265,18 @@ def test_rotated_conv_on_gemm_kernels(cin, cout, k, stride, pad):
     _close(x.grad, xr.grad, 3e-2)
     _close(m.conv.weight.grad, w.grad, 3e-2)
     _close(m.conv.bias.grad, b.grad, 3e-2)
+
+
+@pytest.mark.parametrize("T,D", [(0, 64), (1, 8), (37, 72), (4096, 1032)])
+def test_plain_gather_gives_the_rotated_lookup(T, D):
+    from rtp_b200.ops import kernels as K
+    from rtp_b200.parallel import engine as E
+    from rtp_b200.parallel.context import get_context
+    torch.manual_seed(0)
+    table = torch.randn(100, D, device="cuda").to(BF)
+    ids = torch.randint(0, 100, (T,), device="cuda")
+    a, b = (torch.full((T, D), 7.0, device="cuda", dtype=BF) for _ in range(2))
+    K.embed_fwd(table, ids, a, 0, D=D)
+    if T:
+        E.embed_fwd_rot(E.get_engine(get_context()), table.view(-1), 100, D, ids, b, D, 1.0, None, 1, 0.0, 0, 0, None)
+    assert torch.equal(a, b) and torch.equal(a, table[ids])
