@@ -39,3 +39,21 @@ def test_both_paths_agree(moments, n, adamw):
     m, v = 0.9 * m + 0.1 * gr, 0.999 * v + 0.001 * gr * gr
     p = p - 1e-2 * 0.5 / (1 - 0.9 ** 3) * m / (v.sqrt() / (1 - 0.999 ** 3) ** 0.5 + 1e-8)
     assert bool(((out[0][0].double() - p).abs() <= 2.0 ** -8 * p.abs() + 1e-4).all())
+
+
+@pytest.mark.parametrize("device", ["cuda", "cpu"])
+def test_zero_grad_keeps_the_buffers(device):
+    from rtp_b200.optim import ShardedAdam
+    ps = [torch.nn.Parameter(torch.randn(n, 3, device=device, dtype=d))
+          for n in (1, 7, 70001) for d in (torch.bfloat16, torch.float32)]
+    opt = ShardedAdam(ps)
+    for i, p in enumerate(ps):
+        p.grad = torch.randn_like(p).t().contiguous().t() if i % 2 else torch.randn_like(p)
+    ps[1].grad = None
+    ps[2].grad = (torch.randn_like(ps[2]).requires_grad_() * 2)        # part of a graph: detached as well
+    ptrs = [None if p.grad is None else p.grad.data_ptr() for p in ps]
+    opt.zero_grad(set_to_none=False)
+    assert [None if p.grad is None else p.grad.data_ptr() for p in ps] == ptrs
+    assert all(p.grad is None or (not p.grad.requires_grad and not p.grad.any()) for p in ps)
+    opt.zero_grad()
+    assert all(p.grad is None for p in ps)
