@@ -103,7 +103,6 @@ __device__ __forceinline__ void setup(Ctl* ctl, int tid, int warp, int B, int he
                                       uint32_t tmem_cols) {
   constexpr int HPC = kRows / S_T;
   const int D = heads * kHd;
-  pdl_launch_dependents();
   if (tid < HPC) {
     const int bh = blockIdx.x * HPC + tid;
     const int ok = bh < n_bh;
@@ -127,6 +126,7 @@ __device__ __forceinline__ void setup(Ctl* ctl, int tid, int warp, int B, int he
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_launch_dependents();   // every CTA owns its TMEM columns first (see launch.h)
   pdl_wait();   // set-up touched shared memory and TMEM only; the loads below need the previous kernel's output
 }
 

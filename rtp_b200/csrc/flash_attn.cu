@@ -233,7 +233,6 @@ __device__ __forceinline__ uint4 pack8f(const float* v) {
 
 // Common set-up: barriers, TMEM, abort flag.  Returns the TMEM base.
 __device__ __forceinline__ uint32_t setup_cta(Ctl* ctl, const int* counts, int nbar, int warp, int lane) {
-  pdl_launch_dependents();
   if (warp == kProducerWarp) {
     if (lane < nbar) mbar_init(&ctl->bar[lane], counts[lane]);
     if (lane == 31) ctl->abort_flag = 0;
@@ -245,6 +244,7 @@ __device__ __forceinline__ uint32_t setup_cta(Ctl* ctl, const int* counts, int n
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_launch_dependents();      // every CTA owns its TMEM columns first (see launch.h)
   pdl_wait();
   return ctl->tmem_base;
 }

@@ -297,7 +297,6 @@ __global__ void __launch_bounds__(kNumThreads, 1) rtp_gemm_kernel(const __grid_c
   const bool tile_cta = cta < n_comp;
   const int GU = PAIR ? (n_comp >> 1) : n_comp;
 
-  pdl_launch_dependents();
 #define GEMM_STAMP(i) do { if (P.trace && cta == 0) P.trace[3 * 256 + 64 + (i)] = globaltimer_ns(); } while (0)
   if (threadIdx.x == 0) GEMM_STAMP(0);
   if (warp == 0) {
@@ -331,6 +330,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) rtp_gemm_kernel(const __grid_c
   tc_fence_after();
   const uint32_t tmem_base = ctl->tmem_base;
   // everything above touched only shared memory and TMEM; from here on the previous kernel of the stream must be complete
+  pdl_launch_dependents();           // every CTA owns its TMEM columns first (see launch.h)
   pdl_wait();
   // the previous launch has published its fill counts: one parallel read for all later wait targets (nothing waits
   // on a ring of one rank)

@@ -121,7 +121,6 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
   unsigned long long* status = P.status;
   const unsigned long long tmo = P.timeout_ns;
 
-  pdl_launch_dependents();
   if (warp == 2) {
     for (int j = lane; j < 2 * P.njobs; j += 32)
       if (!(j & 1) || !P.job[j >> 1].sum) prefetch_tmap(j & 1 ? &P.job[j >> 1].mb : &P.job[j >> 1].ma);
@@ -156,6 +155,7 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
   if (PAIR) cluster_sync_all();
   tc_fence_after();
   const uint32_t tmem_base = ctl->tmem_base;
+  pdl_launch_dependents();           // every CTA owns its TMEM columns first (see launch.h)
   pdl_wait();
 
   if (warp == 0) {

@@ -10,6 +10,9 @@ namespace rtp {
 // 210).  Streaming kernels of very many blocks are launched without it: with Adam in it the step took 3790 us.  RTP_PDL unset: the kernels that work on this GPU
 // alone.  RTP_PDL=1: the rotation kernels too (on the training step of a ring they fill the SMs' registers and shared
 // memory, so a successor rarely finds room before its predecessor has left).  RTP_PDL=0: none.
+// A kernel that uses TMEM gives its dependents leave to start (pdl_launch_dependents) only after its CTA has allocated its
+// columns.  A dependent's CTA on the same SM may hold columns while it waits for this kernel to complete; were a CTA of this
+// kernel still to allocate, both would wait for good.  So whoever waits for columns waits for kernels that all have theirs.
 inline int pdl_env() {
   static int v = -2;
   if (v == -2) {
