@@ -282,11 +282,13 @@ class _RopeAttnPackedFn(torch.autograd.Function):
 
 def rope_attention_packed(qkv, cos, sin, heads, nshard=1):
     """Causal self-attention with rotary embedding on a rotated packed projection ``qkv`` [B, S, 3 * D] (its columns grouped
-    per shard) -> [B, S, D].  ``cos`` / ``sin``: [S, hd / 2]."""
+    per shard) -> [B, S, D].  ``cos`` / ``sin``: [S, hd / 2].  None: not a case for these kernels (also where the shards' column
+    groups cut through heads)."""
     B, S, W = qkv.shape
     hd = W // (3 * heads)
     small = hd == 64 and S <= 96             # the short-sequence kernels take those
-    if use_kernels(qkv) and hd in (64, 128) and not small and qkv.is_contiguous() and qkv.data_ptr() % 16 == 0:
+    whole = heads % nshard == 0
+    if use_kernels(qkv) and hd in (64, 128) and whole and not small and qkv.is_contiguous() and qkv.data_ptr() % 16 == 0:
         c, s = cos.float().contiguous(), sin.float().contiguous()
         return _RopeAttnPackedFn.apply(qkv.view(B * S, W), c, s, B, S, heads, nshard).view(B, S, W // 3)
     return None
