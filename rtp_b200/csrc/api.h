@@ -90,15 +90,15 @@ typedef struct {
   int grad_accumulate;             // 1: add the weight gradient to what grad_home already holds
   int bank, no_self_push;          // cross-launch prefetch, see RtpLinearFwd
   const void* next_home; unsigned long long next_bytes; int next_kind;
-  // Optional row of M ones (bf16).  Where rtp_linear_bwd_folds_bias() says yes and dbias_full is null, the launch makes the
-  // bias gradient itself (in fp32, beside the weight gradient) and needs no column-sum kernel.
-  const void* ones;
+  // 1: where rtp_linear_bwd_folds_bias() says yes and dbias_full is null, the launch makes the bias gradient itself (in
+  // fp32, beside the weight gradient) and needs no column-sum kernel.
+  int fold_bias;
   // Optional workspace of at least rtp_linear_bwd_scratch() bytes, 16-byte aligned: the weight gradient's contraction may
   // then be split over the SMs.  The launch's own: it must not be shared with work on another stream.
   void* scratch; unsigned long long scratch_bytes;
 } RtpLinearBwd;
 int rtp_linear_bwd(const RtpRing* ring, const RtpLinearBwd* op, void* stream);
-// 1 if the launch described by `op` computes the bias gradient itself (1-rank ring, op->ones given, 16-byte aligned
+// 1 if the launch described by `op` computes the bias gradient itself (1-rank ring, op->fold_bias set, 16-byte aligned
 // operands), 0 if the caller has to supply the column sums in dbias_full.  Every other field must be as for the launch.
 int rtp_linear_bwd_folds_bias(const RtpRing* ring, const RtpLinearBwd* op);
 // Bytes of workspace with which the launch runs faster (0: none).  Every other field must be as for the launch.

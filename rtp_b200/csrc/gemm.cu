@@ -1092,7 +1092,7 @@ int local_linear_bwd(const RtpRing& R, const RtpLinearBwd& op, rtp::LocalGemm* j
   w.M = op.out_features; w.N = op.in_features; w.K = op.M;
   w.d = op.grad_home; w.ldd = op.in_features;
   if (op.grad_accumulate) { w.c = op.grad_home; w.ldc = op.in_features; }
-  if (op.bias_off >= 0 && op.ones) {
+  if (op.bias_off >= 0 && op.fold_bias) {
     w.bsum = reinterpret_cast<__nv_bfloat16*>(op.grad_home) + op.bias_off;
     w.bsum_add = op.grad_accumulate;
   }
@@ -1591,7 +1591,7 @@ unsigned long long rtp_linear_bwd_scratch(const RtpRing* ring, const RtpLinearBw
 }
 int rtp_linear_bwd_folds_bias(const RtpRing* ring, const RtpLinearBwd* op) {
   rtp::LocalGemm jobs[rtp::kLocalMaxJobs];
-  return op->bias_off >= 0 && op->ones && local_linear_bwd(*ring, *op, jobs) ? 1 : 0;
+  return op->bias_off >= 0 && op->fold_bias && local_linear_bwd(*ring, *op, jobs) ? 1 : 0;
 }
 int rtp_expert_fwd(const RtpRing* ring, const RtpExpertFwd* op, void* stream) {
   rtp::LocalGemm jobs[rtp::kLocalMaxJobs];

@@ -79,7 +79,7 @@ class LinearBwd(C.Structure):
         ("dx_accumulate", C.c_int), ("grad_accumulate", C.c_int),
         ("bank", C.c_int), ("no_self_push", C.c_int),
         ("next_home", C.c_void_p), ("next_bytes", C.c_ulonglong), ("next_kind", C.c_int),
-        ("ones", C.c_void_p),
+        ("fold_bias", C.c_int),
         ("scratch", C.c_void_p), ("scratch_bytes", C.c_ulonglong),
     ]
 

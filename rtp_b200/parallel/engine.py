@@ -142,18 +142,6 @@ class FusedEngine:
         if rc != 0:
             raise RuntimeError("rtp_ring_shift: " + _lib.lib().rtp_shift_last_error().decode())
 
-    def ones_row(self, n: int) -> torch.Tensor:
-        """A row of at least ``n`` bf16 ones (the A operand of the bias-gradient GEMM phase); grown on demand, and never
-        while a CUDA graph that captured the old row may still be replayed."""
-        row = getattr(self, "_ones", None)
-        if row is None or row.numel() < n:
-            if row is not None and torch.cuda.is_current_stream_capturing():
-                raise RuntimeError("ones row would have to grow during graph capture")
-            row = torch.ones(max(n, 32768), dtype=torch.bfloat16, device=self.device)
-            self._old_ones = getattr(self, "_old_ones", []) + ([self._ones] if getattr(self, "_ones", None) is not None else [])
-            self._ones = row
-        return row
-
     def counters(self):
         """(arrive, done, uses) lists of this rank's slot counters (synchronises the stream)."""
         L = _lib.lib()
@@ -283,9 +271,9 @@ def linear_bwd_raw(eng, flat, layout_info, x2d, dy2d, row, in_f, out_f, need_dx=
     _set_prefetch(op, bank, pushed, next_flat, next_kind)
     if has_bias:
         # On a 1-rank ring the launch sums the columns of dy itself; elsewhere they come from a kernel of their own.
-        op.ones = eng.ones_row(M).data_ptr()
+        op.fold_bias = 1
         if not _lib.lib().rtp_linear_bwd_folds_bias(C.byref(eng.ring), C.byref(op)):
-            op.ones = None
+            op.fold_bias = 0
             op.dbias_full = K.colsum(dy2d, dbias_buf).data_ptr()
     scratch = None
     if M >= 8192:           # only a long contraction can want a workspace

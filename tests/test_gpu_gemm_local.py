@@ -66,6 +66,22 @@ def test_long_contraction(M, I, O):
     eng.check()
 
 
+def test_long_batch_is_captured():
+    """The first backward of a biased linear over more rows than any before it may be one that a CUDA graph captures."""
+    E, eng, flat, info, off, rnd = _linear(40008, 72, 8)
+    x, dy = rnd(40008, 72), rnd(40008, 8)
+    E.linear_bwd_raw(eng, flat, info, x[:64], dy[:64], False, 72, 8)
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.graph(graph, stream=side):
+        _, g = E.linear_bwd_raw(eng, flat, info, x, dy, False, 72, 8)
+    graph.replay()
+    torch.cuda.synchronize()
+    _close(g[off:off + 8], dy.double().sum(0), dy.double().abs().sum(0))
+    _close(g[:8 * 72].view(8, 72), dy.double().t() @ x.double(), dy.double().abs().t() @ x.double().abs())
+    eng.check()
+
+
 def test_dropout_mask_of_the_general_kernel():
     """The same (seed, offset) drops the same elements as the rotation kernel, which a forced tile width selects."""
     from rtp_b200.ops import gemm as G
