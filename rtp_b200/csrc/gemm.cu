@@ -815,7 +815,11 @@ int build_expert_bwd(const RtpRing& R, const RtpExpertBwd& op, RtpProgram& P) {
   init_program(P);
   const int N = R.world, r = R.rank, L = op.n_local;
   if (N < 1 || N > RTP_MAX_WORLD || L < 1) return fail("world size out of range");
-  if (2 * N * L + 1 > RTP_MAX_PHASES || 3 + N * L > RTP_MAX_MAPS) return fail("too many experts for one launch");
+  // A capacity that is no whole number of k-blocks: the weight gradient's last block would run on into the next expert's
+  // tokens, so every expert gets maps of dy and x that end at its last token (the rest of the block is zero fill).
+  const bool ragged = op.cap % rtp::kBK != 0;
+  if (2 * N * L + 1 > RTP_MAX_PHASES || 3 + (ragged ? 3 : 1) * N * L > RTP_MAX_MAPS)
+    return fail("too many experts for one launch");
   if (N > 1 && op.shard_bytes > R.slot_bytes) return fail("shard larger than workspace slot");
   void* ws = R.ws[r];
   P.flags = ws ? ws_flags(ws) : nullptr;
@@ -823,7 +827,8 @@ int build_expert_bwd(const RtpRing& R, const RtpExpertBwd& op, RtpProgram& P) {
   P.status = ws ? &ws_flags(ws)->status.v : nullptr;
   P.timeout_ns = R.timeout_ns ? R.timeout_ns : 2000000000ull;
   const long long rows = (long long)N * L * op.cap;
-  // maps: 0 = dy (tokens are k), 1 = x (tokens are k), 2 = dy (out is k), 3.. = expert weights (home / slots)
+  // maps: 0 = dy (tokens are k), 1 = x (tokens are k), 2 = dy (out is k), 3.. = expert weights (home / slots), then, if
+  // ragged, dy and x of each expert (tokens are k)
   if (make_map_mn(&P.maps[0], op.dy, op.out_features, rows, op.ldy)) return -1;
   if (make_map_mn(&P.maps[1], op.x, op.in_features, rows, op.ldx)) return -1;
   if (op.dx && make_map_k(&P.maps[2], op.dy, rows, op.out_features, op.ldy)) return -1;
@@ -840,6 +845,15 @@ int build_expert_bwd(const RtpRing& R, const RtpExpertBwd& op, RtpProgram& P) {
         init_phase(ph);
         ph.a_map = 0; ph.a_mn = 1; ph.a_off_k = g * op.cap;
         ph.b_map = 1; ph.b_mn = 1; ph.b_off_k = g * op.cap;
+        if (ragged) {
+          ph.a_map = 3 + N * L + 2 * g; ph.a_off_k = 0;
+          ph.b_map = ph.a_map + 1; ph.b_off_k = 0;
+          const __nv_bfloat16* dy = reinterpret_cast<const __nv_bfloat16*>(op.dy) + (long long)g * op.cap * op.ldy;
+          const __nv_bfloat16* x = reinterpret_cast<const __nv_bfloat16*>(op.x) + (long long)g * op.cap * op.ldx;
+          if (make_map_mn(&P.maps[ph.a_map], dy, op.out_features, op.cap, op.ldy) ||
+              make_map_mn(&P.maps[ph.b_map], x, op.in_features, op.cap, op.ldx))
+            return -1;
+        }
         ph.M = op.out_features; ph.N = op.in_features; ph.K = op.cap;
         ph.bn = pick_bn(ph.M, ph.N, R.ctas);
         __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(gdst) + (long long)e * op.expert_stride;
@@ -1246,6 +1260,19 @@ void lint_copy(Lint& L, int rank, int p, char which, const RtpProgram& P, int ma
   }
 }
 
+// A contraction that ends inside a k-block: at least one operand's tensor has to end there, so that the rest of the block
+// is fill and adds nothing.
+void lint_tail(Lint& L, int rank, int p, const RtpProgram& P, const RtpPhase& ph, int a_map, long long a_k, int b_map,
+               long long b_k) {
+  if (ph.K % rtp::kBK == 0) return;
+  auto ends = [&](int map, bool mn_major, long long k) {
+    const rtp::HostTensorMap* h = host_map(&P.maps[map]);
+    return h && (long long)h->dims[mn_major ? 1 : 0] <= k + ph.K;
+  };
+  if (!ends(a_map, ph.a_mn != 0, a_k) && !ends(b_map, ph.b_mn != 0, b_k))
+    L.bad("rank " + lstr(rank) + " phase " + lstr(p) + ": the last k-block reads past the contraction's end in both operands");
+}
+
 struct LintRect {
   unsigned long long base;   // address of the tile's first element
   long long rows, cols, pitch;   // cols and pitch in bytes
@@ -1315,6 +1342,7 @@ void lint_program(Lint& L, const RtpRing& R, int rank, const RtpProgram& P, bool
             const long long a_k = ph.a_off_k + (nseg > 1 ? ph.seg_a_off_k[s] : 0);
             lint_copy(L, rank, p, 'A', P, a_map, ph.a_mn != 0, a_mn, a_k, half == 1);
             lint_copy(L, rank, p, 'B', P, nseg > 1 ? ph.seg_b_map[s] : b_map, ph.b_mn != 0, b_mn, ph.b_off_k, half == 1);
+            lint_tail(L, rank, p, P, ph, a_map, a_k, nseg > 1 ? ph.seg_b_map[s] : b_map, ph.b_off_k);
           }
           {
             const long long m0 = m0u + half * 128;

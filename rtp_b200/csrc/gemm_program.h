@@ -9,7 +9,7 @@
 #include <cuda.h>
 #include <stdint.h>
 
-#define RTP_MAX_MAPS 12
+#define RTP_MAX_MAPS 27      // backward of eight rotating experts: three maps of all tokens, then weight, dy and x of each
 #define RTP_MAX_PHASES 18
 #define RTP_MAX_PUSHES 16
 #define RTP_MAX_EMU_RANKS 4

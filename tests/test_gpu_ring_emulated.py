@@ -245,13 +245,13 @@ def test_serialised_mode_names_the_launch_whose_wait_ran_out():
         L.rtp_ws_destroy(w)
 
 
-@pytest.mark.parametrize("world,L", [(2, 2), (4, 1), (4, 2)])
-def test_rotating_experts_fwd_bwd(world, L):
+@pytest.mark.parametrize("world,L,cap", [(2, 2, 192), (4, 1, 192), (4, 2, 192), (2, 2, 40), (4, 2, 136)])
+def test_rotating_experts_fwd_bwd(world, L, cap):
     """One linear of every expert while the expert blocks rotate: tokens of expert g only ever meet weights of g."""
     from rtp_b200.ops import _lib, kernels as K
     lib = _lib.lib()
     torch.manual_seed(0)
-    cap, IN, OUT = 192, 256, 512
+    IN, OUT = 256, 512
     E = world * L
     G_ = (148 // world) & ~1
     blk_w = OUT * IN

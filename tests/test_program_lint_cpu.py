@@ -23,6 +23,15 @@ def test_expert_programs_are_clean(world, n_local):
         assert n == 0, (world, n_local, bwd, lines[:5])
 
 
+@pytest.mark.parametrize("world,n_local,cap", [(2, 1, 40), (2, 4, 8), (4, 2, 1000), (8, 1, 72)])
+def test_expert_contractions_end_with_the_expert(world, n_local, cap):
+    """The weight gradient of an expert sums over its own tokens: a capacity that is no whole number of k-blocks must not
+    reach into the rows of the next expert."""
+    for bwd in (False, True):
+        n, lines = lint.lint_experts(world, n_local, cap, 256, 512, backward=bwd)
+        assert n == 0, (world, n_local, cap, bwd, lines[:5])
+
+
 @pytest.mark.parametrize("inject,needle", [(1, "producers announce it"), (2, "not a multiple of 8 elements"),
                                            (3, "matching credit"), (4, "write the same bytes"),
                                            (5, "outside the slot")])
