@@ -542,35 +542,56 @@ constexpr int kTileFixed = 300;       // hand-over between two tiles of a unit
 struct Item { const LocalGemm* g; bool sum; };
 constexpr int kMaxItems = kLocalMaxJobs + kLocalMaxJobs / 2;
 
+// clocks of one tile of an item, and how many there are
+struct Tiles { long long cost, count; };
+Tiles tiles_of(const Item& x, const TileShape& s) {
+  const int tm = s.pair ? 256 : 128;
+  return Tiles{(long long)((x.g->K + 63) / 64) * (x.sum ? kSumClk : s.clk) + kTileFixed,
+               (long long)((x.g->M + tm - 1) / tm) * (x.sum ? 1 : (x.g->N + s.bn - 1) / s.bn)};
+}
 // Clocks of the longest unit of a launch in which job i uses tile shape sh[i]; `ord` sorts the jobs by falling tile cost.
+// A unit's load only changes where some job's first or last partial round ends, so one unit of each stretch between those
+// places is looked at, not every tile of every unit: a choice for a backward of 16 tiles or of 1 000 takes 1 us or less on
+// the host, where dealing out the tiles one by one took up to 12 us of an eager call (eager backward of 16384 x 256 -> 256
+// 31 us, 17 before there was a choice).
 long long makespan(const Item* it, int n, const TileShape* const* sh, int units, int* ord) {
-  const int tm = sh[0]->pair ? 256 : 128;
   long long cost[kMaxItems], count[kMaxItems];
   for (int i = 0; i < n; ++i) {
-    const LocalGemm& g = *it[i].g;
-    cost[i] = (long long)((g.K + 63) / 64) * (it[i].sum ? kSumClk : sh[i]->clk) + kTileFixed;
-    count[i] = (long long)((g.M + tm - 1) / tm) * (it[i].sum ? 1 : (g.N + sh[i]->bn - 1) / sh[i]->bn);
+    const Tiles t = tiles_of(it[i], *sh[i]);
+    cost[i] = t.cost; count[i] = t.count;
     ord[i] = i;
   }
   std::sort(ord, ord + n, [&](int a, int b) { return cost[a] != cost[b] ? cost[a] > cost[b] : a < b; });
-  long long load[256] = {0};
-  long long t = 0, total = 0, sum = 0, epi = 0;
+  long long first[kMaxItems + 1] = {0};          // of the jobs in order, and the end of the last
+  long long sum = 0, epi = 0;
   for (int q = 0; q < n; ++q) {
     const int i = ord[q];
-    total += count[i];
+    first[q + 1] = first[q] + count[i];
+    sum += count[i] * cost[i];
     if (!it[i].sum) epi = std::max(epi, (long long)sh[i]->epi);
   }
-  for (int q = 0; q < n; ++q) {
-    const int i = ord[q];
-    if (total > 8ll * units) { sum += count[i] * cost[i]; continue; }     // many rounds: the average is close enough
-    for (long long k = 0; k < count[i]; ++k, ++t) {
-      const int r = (int)(t / units), u = (int)(t % units);
-      load[(r & 1) ? units - 1 - u : u] += cost[i];
-    }
+  if (first[n] > 8ll * units) return sum / units + cost[ord[0]] / 2 + epi;     // many rounds: the average is close enough
+  // Of the first x tiles a unit takes one of every full round, and one of the last, partial round if the dealing has come
+  // to it (see unit_tile): the units below `turn` where that round runs upwards, those from it on where it runs back.
+  int rounds[kMaxItems + 1], turn[kMaxItems + 1];
+  for (int e = 0; e <= n; ++e) {
+    rounds[e] = (int)first[e] / units;
+    const int rem = (int)first[e] - rounds[e] * units;
+    turn[e] = rounds[e] & 1 ? units - rem : rem;
   }
-  if (total > 8ll * units) return sum / units + cost[ord[0]] / 2 + epi;
   long long best = 0;
-  for (int u = 0; u < units; ++u) best = std::max(best, load[u]);
+  for (int e = 0; e <= n; ++e) {
+    const int u = turn[e];                       // where a stretch of equal units begins
+    if (u == units) continue;
+    long long load = 0;
+    int before = 0;
+    for (int q = 0; q < n; ++q) {
+      const int upto = rounds[q + 1] + (rounds[q + 1] & 1 ? u >= turn[q + 1] : u < turn[q + 1]);
+      load += (upto - before) * cost[ord[q]];
+      before = upto;
+    }
+    best = std::max(best, load);
+  }
   return best + epi;
 }
 
@@ -600,13 +621,11 @@ int launch_local(const Params<MAXJ>& P, cudaStream_t stream) {
   return e == cudaSuccess ? 0 : lfail(std::string("launch local_gemm_kernel: ") + cudaGetErrorString(e));
 }
 
-template <int MAXJ>
-int run(const Item* it, int n, int pair_policy, unsigned long long* status, unsigned long long timeout_ns, cudaStream_t stream) {
-  // tile shapes: pairs or single CTAs for the launch, then the wide or the narrow tile for each job
-  const int n_sm = std::min(sms(), 256);
+// Tile shapes (pairs or single CTAs for the launch, then the wide or the narrow tile for each job) and the order of the
+// jobs.  Returns the clocks of the longest unit, -1: no shape for this device.
+long long choose(const Item* it, int n, int pair_policy, int n_sm, const TileShape** best_sh, int* best_ord) {
   const TileShape* sh[kMaxItems];
-  const TileShape* best_sh[kMaxItems];
-  int ord[kMaxItems], best_ord[kMaxItems];
+  int ord[kMaxItems];
   long long best = -1;
   for (int s = 0; s < 4; s += 2) {
     const TileShape *wide = &kShapes[s], *narrow = &kShapes[s + 1];
@@ -632,7 +651,15 @@ int run(const Item* it, int n, int pair_policy, unsigned long long* status, unsi
     std::fill(sh, sh + n, narrow);
     consider();
   }
-  if (best < 0) return lfail("no tile shape for this device");
+  return best;
+}
+
+template <int MAXJ>
+int run(const Item* it, int n, int pair_policy, unsigned long long* status, unsigned long long timeout_ns, cudaStream_t stream) {
+  const int n_sm = sms();
+  const TileShape* best_sh[kMaxItems];
+  int best_ord[kMaxItems];
+  if (choose(it, n, pair_policy, n_sm, best_sh, best_ord) < 0) return lfail("no tile shape for this device");
   const bool pair = best_sh[0]->pair;
 
   static thread_local Params<MAXJ> P;
@@ -688,6 +715,17 @@ int run(const Item* it, int n, int pair_policy, unsigned long long* status, unsi
   return pair ? launch_local<true, MAXJ>(P, stream) : launch_local<false, MAXJ>(P, stream);
 }
 
+int items_of(const LocalGemm* jobs, int n, Item* it) {
+  int m = 0;
+  for (int i = 0; i < n; ++i) it[m++] = Item{&jobs[i], false};
+  for (int i = 0; i < n; ++i)
+    if (jobs[i].bsum) {
+      if (m == kMaxItems) return -1;
+      it[m++] = Item{&jobs[i], true};
+    }
+  return m;
+}
+
 }  // namespace
 
 int local_reduce(const float* part, int n, long long stride, void* out, long long len, cudaStream_t stream) {
@@ -715,14 +753,37 @@ int local_gemm(const LocalGemm* jobs, int n, int pair_policy, unsigned long long
   for (int i = 0; i < n; ++i)
     if (!local_gemm_ok(jobs[i])) return lfail("local_gemm: operand not aligned to 16 bytes, or N not a multiple of 8");
   Item it[kMaxItems];
-  int m = 0;
-  for (int i = 0; i < n; ++i) it[m++] = Item{&jobs[i], false};
-  for (int i = 0; i < n; ++i)
-    if (jobs[i].bsum) {
-      if (m == kMaxItems) return lfail("local_gemm: too many column sums");
-      it[m++] = Item{&jobs[i], true};
-    }
+  const int m = items_of(jobs, n, it);
+  if (m < 0) return lfail("local_gemm: too many column sums");
   return m <= 3 ? run<3>(it, m, pair_policy, status, timeout_ns, stream) : run<kMaxItems>(it, m, pair_policy, status, timeout_ns, stream);
 }
 
 }  // namespace rtp
+
+// The choice that a launch of these jobs (4 numbers each: M, N, K, 1 = with the column sums of A) makes on a device of n_sm
+// SMs; host only.  out: clocks of the longest unit, units, the epilogue share of those clocks, then cost and number of the
+// tiles of each job and sum in the order in which they are dealt out.  Returns the number of those, -1: no such launch.
+extern "C" int rtp_lint_local_plan(int n_sm, int pair_policy, int n, const int* mnks, long long* out) {
+  using namespace rtp;
+  if (n < 1 || n > kLocalMaxJobs) return -1;
+  LocalGemm jobs[kLocalMaxJobs] = {};
+  for (int i = 0; i < n; ++i) {
+    jobs[i].M = mnks[4 * i]; jobs[i].N = mnks[4 * i + 1]; jobs[i].K = mnks[4 * i + 2];
+    jobs[i].bsum = mnks[4 * i + 3] ? &jobs[i] : nullptr;
+  }
+  Item it[kMaxItems];
+  const TileShape* sh[kMaxItems];
+  int ord[kMaxItems];
+  const int m = items_of(jobs, n, it);
+  if (m < 0 || (out[0] = choose(it, m, pair_policy, n_sm, sh, ord)) < 0) return -1;
+  const bool pair = sh[0]->pair;
+  out[1] = pair ? n_sm / 2 : n_sm;
+  out[2] = 0;
+  for (int q = 0; q < m; ++q) {
+    const int i = ord[q];
+    const Tiles t = tiles_of(it[i], *sh[i]);
+    if (!it[i].sum) out[2] = std::max(out[2], (long long)sh[i]->epi);
+    out[3 + 2 * q] = t.cost; out[4 + 2 * q] = t.count;
+  }
+  return m;
+}
