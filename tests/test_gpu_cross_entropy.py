@@ -11,7 +11,7 @@ import torch.nn.functional as F
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("V", [8, 1032, 8192, 12296, 32000, 50304, 65536, 65544])
+@pytest.mark.parametrize("V", [8, 1032, 8192, 12296, 16392, 20488, 32000, 36864, 50304, 65536, 65544])
 @pytest.mark.parametrize("M", [1, 150, 611])
 @pytest.mark.parametrize("factor", [1.0, 3.0])
 def test_loss_and_gradient(V, M, factor):
