@@ -45,3 +45,19 @@ def test_against_float64(S, p, causal):
     dqkv = K.attn_small_bwd(pack(q, k, v), pack(do), S, B, H, **kw).view(S, B, 3, H, 64).permute(2, 1, 3, 0, 4)
     for got, ref in zip(dqkv, grads):
         _close(got, ref)
+
+
+@pytest.mark.parametrize("S", [1, 4, 5, 12, 13])
+def test_bits_do_not_depend_on_the_number_of_blocks(S):
+    """Many blocks may run with fewer threads each; every sum keeps its order."""
+    from rtp_b200.ops import kernels as K
+    H, many, few = 2, 300, 3
+    g = torch.Generator(device="cuda").manual_seed(S)
+    qkv, do = (torch.randn(S, many, w * H * 64, generator=g, device="cuda").to(BF) for w in (3, 1))
+    for p in (0.0, 0.3):
+        def run(n):
+            x, y = qkv[:, :n].reshape(S * n, -1).contiguous(), do[:, :n].reshape(S * n, -1).contiguous()
+            kw = dict(causal=True, drop_p=p, seed=7, offset=2)
+            return [t.view(S, n, -1)[:, :few] for t in (K.attn_small_fwd(x, S, n, H, **kw), K.attn_small_bwd(x, y, S, n, H, **kw))]
+        for a, b in zip(run(many), run(few)):
+            assert torch.equal(a, b)
