@@ -88,10 +88,11 @@ uint32_t host_thresh(float p) {
 // global memory is touched exactly once per tensor.  Saves h (bf16) and the row statistics for backward.
 //
 // A block keeps the next row's words in flight while it reduces the current one, and a reduction is one barrier (its
-// scratch alternates).  D <= 2048 takes 128 threads a row (256 with dropout, whose generator is the longer part): seven
-// blocks fit on an SM, so that the 1024 rows of a small training step are one wave.  Microseconds
-// before and after: 650 x 768 with residual 4.0 -> 2.3, 8192 x 2048 21.5 -> 17, 4096 x 5120 (RMSNorm) 35 -> 17,
-// 3000 x 4096 23 -> 12; 1024 x 2048 with residual and dropout stays at 6.5.
+// scratch alternates).  D <= 1024 takes 128 threads a row: seven blocks fit on an SM, so that the 1024 rows of a small
+// training step are one wave.  Wider rows take 256; 128 threads with two groups of columns each were slower at every size
+// (RMSNorm of 256 x 2048 2.8 us, 256 threads 2.3; 8192 x 2048 19.3 and 17.1).  Microseconds before and after: 650 x 768
+// with residual 4.0 -> 2.3, 8192 x 2048 21.5 -> 17, 4096 x 5120 (RMSNorm) 35 -> 17, 3000 x 4096 23 -> 12; 1024 x 2048 with
+// residual and dropout stays at 6.2.
 // ------------------------------------------------------------------------------------------------
 // Sums N values of every thread over its group of T threads (the block is G groups): `red` holds 2 x G x T / 32 x N floats,
 // `turn` alternates between its halves.
@@ -122,32 +123,6 @@ __device__ __forceinline__ void block_sum_n(float (&v)[N], float* red, int turn)
   }
 }
 
-// One sum over the block of NS values per thread, value i standing for the threads i T .. i T + T - 1 of a wider block.
-template <int T, int NS>
-__device__ __forceinline__ float row_sum(float (&v)[NS], float* red, int turn) {
-  if (NS == 1) {
-    block_sum_n<T, NS>(v, red, turn);
-    return v[0];
-  }
-  constexpr int W = T / 32;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  float* mine = red + turn * (W * NS);
-#pragma unroll
-  for (int i = 0; i < NS; ++i) {
-    v[i] = warp_sum(v[i]);
-    if (lane == 0) mine[i * W + w] = v[i];
-  }
-  __syncthreads();
-  float t[W * NS];
-#pragma unroll
-  for (int k = 0; k < W * NS; ++k) t[k] = mine[k];
-#pragma unroll
-  for (int o = W * NS / 2; o > 0; o >>= 1)
-#pragma unroll
-    for (int k = 0; k < o; ++k) t[k] += t[k + o];
-  return t[0];
-}
-
 template <int T, int NG>
 __global__ void __launch_bounds__(T, T == 128 ? 7 : NG == 1 ? 4 : 2) norm_fwd_kernel(
     const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ sub, const __nv_bfloat16* __restrict__ gamma,
@@ -155,9 +130,7 @@ __global__ void __launch_bounds__(T, T == 128 ? 7 : NG == 1 ? 4 : 2) norm_fwd_ke
     float* __restrict__ mean_out, float* __restrict__ rstd_out, int M, int D, float eps, int rms, uint32_t thresh,
     float drop_scale, uint64_t seed, uint64_t offset, const unsigned long long* __restrict__ step_ptr) {
   pdl_prologue();
-  // 128 threads with two groups of columns each add up like 256 threads with one: the statistics have the same bits
-  constexpr int NS = T == 128 ? NG : 1;
-  __shared__ float red[2 * (T / 32) * NS];
+  __shared__ float red[2 * (T / 32)];
   if (step_ptr) offset += __ldg(step_ptr) * 65536ull;
   const int c0 = threadIdx.x * 8;
   uint4 nx[NG], ns[NG], g[NG], bt[NG];
@@ -185,9 +158,7 @@ __global__ void __launch_bounds__(T, T == 128 ? 7 : NG == 1 ? 4 : 2) norm_fwd_ke
   for (int row = blockIdx.x; row < M; row += gridDim.x) {
     const size_t base = (size_t)row * D;
     float v[NG][8];
-    float s[NS];
-#pragma unroll
-    for (int i = 0; i < NS; ++i) s[i] = 0.f;
+    float s[1] = {0.f};
 #pragma unroll
     for (int q = 0; q < NG; ++q) {
       const int c = q * T * 8 + c0;
@@ -209,26 +180,26 @@ __global__ void __launch_bounds__(T, T == 128 ? 7 : NG == 1 ? 4 : 2) norm_fwd_ke
         unpack8(hp, v[q]);
         if (h_out) *reinterpret_cast<uint4*>(h_out + base + c) = hp;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) s[q % NS] += v[q][i];
+        for (int i = 0; i < 8; ++i) s[0] += v[q][i];
       }
     }
     if (row + (int)gridDim.x < M) fetch(row + gridDim.x);
     float mean = 0.f;
     if (!rms) {
-      mean = row_sum<T, NS>(s, red, turn) / D;
+      block_sum_n<T, 1>(s, red, turn);
+      mean = s[0] / D;
       turn ^= 1;
     }
-    float qq[NS];
-#pragma unroll
-    for (int i = 0; i < NS; ++i) qq[i] = 0.f;
+    float qq[1] = {0.f};
 #pragma unroll
     for (int q = 0; q < NG; ++q) {
       if (q * T * 8 + c0 < D) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) { const float d = v[q][i] - mean; qq[q % NS] += d * d; }
+        for (int i = 0; i < 8; ++i) { const float d = v[q][i] - mean; qq[0] += d * d; }
       }
     }
-    const float rstd = rsqrtf(row_sum<T, NS>(qq, red, turn) / D + eps);
+    block_sum_n<T, 1>(qq, red, turn);
+    const float rstd = rsqrtf(qq[0] / D + eps);
     turn ^= 1;
     if (threadIdx.x == 0) {
       if (mean_out) mean_out[row] = mean;
@@ -1446,15 +1417,13 @@ int rtp_norm_fwd(const void* x, const void* sub, const void* gamma, const void* 
                  unsigned long long offset, const unsigned long long* step_ptr, void* stream) {
   if (D % 8 || D > 8192) { k_err = "norm: D must be a multiple of 8 and at most 8192"; return -1; }
   const float ds = drop_p > 0.f ? 1.f / (1.f - drop_p) : 1.f;
-  const bool drop = sub && drop_p > 0.f;
 #define RTP_NORM_FWD(T, NG, PER_SM)                                                                                   \
   rtp::launch_k(norm_fwd_kernel<T, NG>, dim3(std::min(M, 148 * PER_SM)), dim3(T), 0, (cudaStream_t)stream,                                  \
       (const __nv_bfloat16*)x, (const __nv_bfloat16*)sub, (const __nv_bfloat16*)gamma, (const __nv_bfloat16*)beta,    \
       (__nv_bfloat16*)h_out, (__nv_bfloat16*)y, mean, rstd, M, D, eps, rms, host_thresh(drop_p), ds, seed, offset,    \
       step_ptr)
-  if (D <= 1024) RTP_NORM_FWD(128, 1, 7); else if (D <= 2048 && !drop) RTP_NORM_FWD(128, 2, 7);
-  else if (D <= 2048) RTP_NORM_FWD(256, 1, 4); else if (D <= 4096) RTP_NORM_FWD(256, 2, 2);
-  else if (D <= 6144) RTP_NORM_FWD(256, 3, 2); else RTP_NORM_FWD(256, 4, 2);
+  if (D <= 1024) RTP_NORM_FWD(128, 1, 7); else if (D <= 2048) RTP_NORM_FWD(256, 1, 4);
+  else if (D <= 4096) RTP_NORM_FWD(256, 2, 2); else if (D <= 6144) RTP_NORM_FWD(256, 3, 2); else RTP_NORM_FWD(256, 4, 2);
 #undef RTP_NORM_FWD
   LAUNCH_CHECK("norm_fwd");
   return 0;
