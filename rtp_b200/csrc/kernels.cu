@@ -227,7 +227,10 @@ __global__ void __launch_bounds__(T, T == 128 ? 7 : NG == 1 ? 4 : 2) norm_fwd_ke
 // block works on 256 / T groups of R rows side by side, whose column sums it adds up before the atomics.
 // 256 x 256 6.6 -> 2.9 us, 650 x 768 8.1 -> 4.6, 1024 x 512 8.5 -> 4.8, 1024 x 2048 with dropout 11.0 -> 9.7,
 // 8192 x 2048 30.4 -> 28.7, 4096 x 5120 51 -> 34.
-template <int T, int NG, int R>
+// AHEAD: the next rows are fetched while the current ones are worked on.  It takes the registers of two more rows, so fewer
+// are in flight at once, and pays where a block has many rows: 16384 x 1536 with dropout, four rows 76.7 us, two and two
+// ahead 71.4; without dropout 60.2 and 48.5.
+template <int T, int NG, int R, bool AHEAD = false>
 __global__ void __launch_bounds__(256, 2) norm_bwd_kernel(
     const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restrict__ gamma,
     const float* __restrict__ mean_in, const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ dx,
@@ -250,29 +253,46 @@ __global__ void __launch_bounds__(256, 2) norm_bwd_kernel(
 #pragma unroll
     for (int i = 0; i < 8; ++i) { pg[q][i] = 0.f; pb[q][i] = 0.f; }
   }
-  int turn = 0;
-  for (int block0 = blockIdx.x * (G * R); block0 < M; block0 += gridDim.x * (G * R)) {
-    const int row0 = block0 + grp * R;
-    uint4 cd[R][NG], ch[R][NG];
-    float mean[R], rstd[R], s[2 * R];
+  uint4 nd[R][NG], nh[R][NG];
+  float nmean[R], nrstd[R];
+  auto fetch = [&](int row0) {
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int row = row0 + r;
-      mean[r] = rstd[r] = 0.f;
+      nmean[r] = nrstd[r] = 0.f;
       if (row < M) {
-        if (!rms) mean[r] = mean_in[row];
-        rstd[r] = rstd_in[row];
+        if (!rms) nmean[r] = mean_in[row];
+        nrstd[r] = rstd_in[row];
       }
 #pragma unroll
       for (int q = 0; q < NG; ++q) {
         const int c = (q * T + tid) * 8;
-        cd[r][q] = ch[r][q] = make_uint4(0u, 0u, 0u, 0u);
+        nd[r][q] = nh[r][q] = make_uint4(0u, 0u, 0u, 0u);
         if (c < D && row < M) {
-          cd[r][q] = __ldcs(reinterpret_cast<const uint4*>(dy + (size_t)row * D + c));
-          ch[r][q] = __ldcs(reinterpret_cast<const uint4*>(h + (size_t)row * D + c));
+          nd[r][q] = __ldcs(reinterpret_cast<const uint4*>(dy + (size_t)row * D + c));
+          nh[r][q] = __ldcs(reinterpret_cast<const uint4*>(h + (size_t)row * D + c));
         }
       }
     }
+  };
+  if (AHEAD) fetch(blockIdx.x * (G * R) + grp * R);
+  int turn = 0;
+  for (int block0 = blockIdx.x * (G * R); block0 < M; block0 += gridDim.x * (G * R)) {
+    const int row0 = block0 + grp * R;
+    if (!AHEAD) fetch(row0);
+    uint4 cd[R][NG], ch[R][NG];
+    float mean[R], rstd[R], s[2 * R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      mean[r] = nmean[r];
+      rstd[r] = nrstd[r];
+#pragma unroll
+      for (int q = 0; q < NG; ++q) {
+        cd[r][q] = nd[r][q];
+        ch[r][q] = nh[r][q];
+      }
+    }
+    if (AHEAD) fetch(row0 + gridDim.x * (G * R));
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       s[2 * r] = s[2 * r + 1] = 0.f;
@@ -1435,19 +1455,29 @@ int rtp_norm_bwd(const void* dy, const void* h, const void* gamma, const float* 
   if (D % 8 || D > 8192) { k_err = "norm: D must be a multiple of 8 and at most 8192"; return -1; }
   const float ds = drop_p > 0.f ? 1.f / (1.f - drop_p) : 1.f;
   const int vec_atomics = ((reinterpret_cast<uintptr_t>(dgamma) | reinterpret_cast<uintptr_t>(dbeta)) & 15) == 0;
-  // few blocks: every block ends with one vector atomic per 4 columns of dgamma / dbeta
-#define RTP_NORM_BWD(T, NG, R)                                                                                        \
-  rtp::launch_k(norm_bwd_kernel<T, NG, R>, dim3(std::min((M + 256 / T * R - 1) / (256 / T * R), 296)), dim3(256), 0, (cudaStream_t)stream,  \
+  // Few blocks: every block ends with one vector atomic per 4 columns of dgamma / dbeta.  Up to 1024 wide rows one block per
+  // SM (256 x 2048 256 blocks 10.3 us, 128 with two rows each 7.4; 1024 x 3072 256 blocks 18.3, 148 14.6), else two.
+  const int most = M <= 1024 && D > 1024 ? 148 : 296;
+#define RTP_NORM_BWD(T, NG, R, AHEAD)                                                                                 \
+  rtp::launch_k(norm_bwd_kernel<T, NG, R, AHEAD>, dim3(std::min((M + 256 / T * R - 1) / (256 / T * R), most)),         \
+      dim3(256), 0, (cudaStream_t)stream,                                                                             \
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)h, (const __nv_bfloat16*)gamma, mean, rstd, (__nv_bfloat16*)dx, \
       (__nv_bfloat16*)dsub, dgamma, dbeta, M, D, rms, host_thresh(drop_p), ds, seed, offset,                          \
       (const __nv_bfloat16*)dres, step_ptr, vec_atomics)
-  // rows in flight per group: no more than leave every SM a block or two
-  if (D <= 256) { if (M <= 2368) RTP_NORM_BWD(32, 1, 1); else RTP_NORM_BWD(32, 1, 4); }
-  else if (D <= 512) { if (M <= 1184) RTP_NORM_BWD(64, 1, 2); else RTP_NORM_BWD(64, 1, 4); }
-  else if (D <= 1024) { if (M <= 592) RTP_NORM_BWD(128, 1, 2); else RTP_NORM_BWD(128, 1, 4); }
-  else if (D <= 2048) {
-    if (M <= 296) RTP_NORM_BWD(256, 1, 1); else if (M <= 592) RTP_NORM_BWD(256, 1, 2); else RTP_NORM_BWD(256, 1, 4);
-  } else if (D <= 4096) RTP_NORM_BWD(256, 2, 2); else if (D <= 6144) RTP_NORM_BWD(256, 3, 1); else RTP_NORM_BWD(256, 4, 1);
+  // Rows in flight per group: no more than leave every SM a block or two, one where there are fewer rows than SMs
+  // (64 x 4096 with dropout, two rows 7.5 us, one 6.9).
+  if (D <= 256) { if (M <= 2368) RTP_NORM_BWD(32, 1, 1, false); else RTP_NORM_BWD(32, 1, 4, false); }
+  else if (D <= 512) {
+    if (M <= 148) RTP_NORM_BWD(64, 1, 1, false); else if (M <= 1184) RTP_NORM_BWD(64, 1, 2, false);
+    else RTP_NORM_BWD(64, 1, 4, false);
+  } else if (D <= 1024) {
+    if (M <= 148) RTP_NORM_BWD(128, 1, 1, false); else if (M <= 592) RTP_NORM_BWD(128, 1, 2, false);
+    else RTP_NORM_BWD(128, 1, 4, false);
+  } else if (D <= 2048) {
+    if (M <= 1024) RTP_NORM_BWD(256, 1, 2, false); else if (M < 4096) RTP_NORM_BWD(256, 1, 4, false);
+    else RTP_NORM_BWD(256, 1, 2, true);
+  } else if (D <= 4096) { if (M <= 148) RTP_NORM_BWD(256, 2, 1, false); else RTP_NORM_BWD(256, 2, 2, false); }
+  else if (D <= 6144) RTP_NORM_BWD(256, 3, 1, false); else RTP_NORM_BWD(256, 4, 1, false);
 #undef RTP_NORM_BWD
   LAUNCH_CHECK("norm_bwd");
   return 0;

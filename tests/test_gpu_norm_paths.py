@@ -11,7 +11,7 @@ BF = torch.bfloat16
 
 
 @pytest.mark.parametrize("D", [8, 256, 264, 512, 520, 1024, 1032, 2048, 2056, 4104, 5120, 8192])
-@pytest.mark.parametrize("M", [1, 297, 2500])
+@pytest.mark.parametrize("M", [1, 148, 297, 1025, 2500])
 @pytest.mark.parametrize("rms,residual", [(False, True), (True, False)])
 def test_norm(D, M, rms, residual):
     from rtp_b200.ops import kernels as K
@@ -42,3 +42,10 @@ def test_norm(D, M, rms, residual):
         close(db, dy.double().sum(0), dy.double().abs().sum(0), 0.0)
     if residual:
         assert torch.equal(dsub, dx)
+
+
+@pytest.mark.parametrize("M", [4096, 4098, 8001])
+@pytest.mark.parametrize("D", [1032, 1536, 2048])
+def test_many_wide_rows(M, D):
+    test_norm(D, M, False, True)
+    test_norm(D, M, True, False)
