@@ -533,21 +533,28 @@ int sms() {
 // {17.3, 14.5, 13.9, 21.1}, its backward {19.1, 23.3, 27.0, 37.8}, forward 1024 x 512 -> 512 {10.0, 8.2, 7.6, 7.2},
 // 8192 x 2048 -> 8192 {185, 252, 257, 454}.
 // A column-sum tile loads 16 KB per k-block and CTA.
+// `drain` is what bounds a tile of few k-blocks: the epilogue's warps empty one accumulator at a time, and a fifth of the
+// k-loop's clocks come on top (8192 x 8192 with K = 8 / 512, us: {72.8, 88.2, 84.6, 146} / {81, 96, 97, 155}); three fifths
+// of `epi` are left to add for the last one.  Without it the weight gradient of a few tokens fell into 64-wide tiles, each
+// as long as a 128-wide one: backward of 8 x 2048 -> 8192 70 to 82 us, now 47 (65 before there was a choice).
 constexpr int kSumClk = 330;
-struct TileShape { bool pair; int bn, clk, epi; };
-constexpr TileShape kShapes[4] = {{true, 256, 650, 4600}, {true, 128, 545, 1700}, {false, 128, 530, 700}, {false, 64, 480, 0}};
+struct TileShape { bool pair; int bn, clk, epi, drain; };
+constexpr TileShape kShapes[4] = {{true, 256, 650, 4600, 9400}, {true, 128, 545, 1700, 6000},
+                                  {false, 128, 530, 700, 5500}, {false, 64, 480, 0, 4750}};
 constexpr int kTileFixed = 300;       // hand-over between two tiles of a unit
 
 // a GEMM, or the column sums of its A
 struct Item { const LocalGemm* g; bool sum; };
 constexpr int kMaxItems = kLocalMaxJobs + kLocalMaxJobs / 2;
 
-// clocks of one tile of an item, and how many there are
-struct Tiles { long long cost, count; };
+// clocks of one tile of an item, how many there are, and what the last one's epilogue adds
+struct Tiles { long long cost, count, epi; };
 Tiles tiles_of(const Item& x, const TileShape& s) {
   const int tm = s.pair ? 256 : 128;
-  return Tiles{(long long)((x.g->K + 63) / 64) * (x.sum ? kSumClk : s.clk) + kTileFixed,
-               (long long)((x.g->M + tm - 1) / tm) * (x.sum ? 1 : (x.g->N + s.bn - 1) / s.bn)};
+  const long long k = (x.g->K + 63) / 64, rows = (x.g->M + tm - 1) / tm;
+  if (x.sum) return Tiles{k * kSumClk + kTileFixed, rows, 0};
+  const long long loop = k * s.clk + kTileFixed, drain = s.drain + loop / 5;
+  return Tiles{std::max(loop, drain), rows * ((x.g->N + s.bn - 1) / s.bn), loop >= drain ? s.epi : s.epi * 3 / 5};
 }
 // Clocks of the longest unit of a launch in which job i uses tile shape sh[i]; `ord` sorts the jobs by falling tile cost.
 // A unit's load only changes where some job's first or last partial round ends, so one unit of each stretch between those
@@ -555,20 +562,20 @@ Tiles tiles_of(const Item& x, const TileShape& s) {
 // the host, where dealing out the tiles one by one took up to 12 us of an eager call (eager backward of 16384 x 256 -> 256
 // 31 us, 17 before there was a choice).
 long long makespan(const Item* it, int n, const TileShape* const* sh, int units, int* ord) {
-  long long cost[kMaxItems], count[kMaxItems];
+  long long cost[kMaxItems], count[kMaxItems], epi = 0;
   for (int i = 0; i < n; ++i) {
     const Tiles t = tiles_of(it[i], *sh[i]);
     cost[i] = t.cost; count[i] = t.count;
+    epi = std::max(epi, t.epi);
     ord[i] = i;
   }
   std::sort(ord, ord + n, [&](int a, int b) { return cost[a] != cost[b] ? cost[a] > cost[b] : a < b; });
   long long first[kMaxItems + 1] = {0};          // of the jobs in order, and the end of the last
-  long long sum = 0, epi = 0;
+  long long sum = 0;
   for (int q = 0; q < n; ++q) {
     const int i = ord[q];
     first[q + 1] = first[q] + count[i];
     sum += count[i] * cost[i];
-    if (!it[i].sum) epi = std::max(epi, (long long)sh[i]->epi);
   }
   if (first[n] > 8ll * units) return sum / units + cost[ord[0]] / 2 + epi;     // many rounds: the average is close enough
   // Of the first x tiles a unit takes one of every full round, and one of the last, partial round if the dealing has come
@@ -782,7 +789,7 @@ extern "C" int rtp_lint_local_plan(int n_sm, int pair_policy, int n, const int* 
   for (int q = 0; q < m; ++q) {
     const int i = ord[q];
     const Tiles t = tiles_of(it[i], *sh[i]);
-    if (!it[i].sum) out[2] = std::max(out[2], (long long)sh[i]->epi);
+    out[2] = std::max(out[2], t.epi);
     out[3 + 2 * q] = t.cost; out[4 + 2 * q] = t.count;
   }
   return m;

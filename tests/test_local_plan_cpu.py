@@ -51,6 +51,15 @@ def test_estimate_is_the_longest_unit(policy):
     assert few > 50
 
 
+@pytest.mark.parametrize("tokens,i,o", [(1, 2048, 2048), (8, 2048, 8192), (100, 2048, 8192), (64, 4096, 4096)])
+def test_weight_gradients_of_few_tokens_take_wide_tiles(tokens, i, o):
+    """A tile of one or two k-blocks takes as long as its epilogue, which a narrower tile hardly shortens."""
+    f, args = plan(backward(tokens, i, o))
+    n = f(*args)
+    most = max(args[4][4 + 2 * q] for q in range(n))
+    assert most <= (o // 128) * (i // 128)
+
+
 def test_choice_is_as_quick_for_many_tiles():
     def took(jobs):
         f, args = plan(jobs)
