@@ -148,9 +148,11 @@ def scale_unless_one_(g, scale):
 
 
 def embed_fwd(table, ids, out, col_off, *, D, scale=1.0, pe=None, tokens_per_pos=1, drop_p=0.0, seed=0, offset=0,
-              step=None):
+              step=None, Ds=None):
+    """``Ds``: columns of a ``table`` that is given as the flat buffer it starts (default: its second dimension)."""
     T = ids.numel()
-    Ds = table.shape[1]
+    if Ds is None:
+        Ds = table.shape[1]
     _check(_L().rtp_embed_fwd(_p(table), _p(ids), _p(pe), pe.stride(0) if pe is not None else 0, tokens_per_pos,
                               _p(out), out.stride(0), col_off, T, Ds, D, float(scale), float(drop_p), seed, offset,
                               _p(step), _lib.stream_ptr()), "embed_fwd")

@@ -280,3 +280,17 @@ def test_plain_gather_gives_the_rotated_lookup(T, D):
     if T:
         E.embed_fwd_rot(E.get_engine(get_context()), table.view(-1), 100, D, ids, b, D, 1.0, None, 1, 0.0, 0, 0, None)
     assert torch.equal(a, b) and torch.equal(a, table[ids])
+
+
+@pytest.mark.parametrize("V,D", [(7, 24), (1001, 72)])
+def test_embedding_module_reads_its_flat_shard(V, D):
+    """The table of a rotated embedding is the start of a padded flat buffer."""
+    from rtp_b200.module.embedding import ParallelEmbedding
+    emb = ParallelEmbedding(V, D, device="cuda", dtype=torch.bfloat16)
+    ids = torch.randint(0, V, (3, 50), device="cuda")
+    ids[0, 0], ids[-1, -1] = 0, V - 1
+    y = emb(ids)
+    w = emb.embedding.weight
+    assert torch.equal(y.detach(), w.detach()[ids])
+    (g,) = torch.autograd.grad(y, w, torch.ones_like(y))
+    assert torch.equal(g.float(), torch.zeros(V, D, device="cuda").index_add_(0, ids.view(-1), torch.ones(150, D, device="cuda")))
