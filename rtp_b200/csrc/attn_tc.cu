@@ -537,12 +537,12 @@ int rtp_attn_tc_fwd(const void* qkv, void* out, int S, int B, int heads, int nsh
   const int grid = (n_bh + hpc - 1) / hpc;
   if (S == 32) {
     if (set_smem<attn_tc_fwd_kernel<32>>(kFwdSmem)) return -1;
-    rtp::launch_k(attn_tc_fwd_kernel<32>, dim3(grid), dim3(128), kFwdSmem, (cudaStream_t)stream, 
+    rtp::launch_k(attn_tc_fwd_kernel<32>, dim3(grid), dim3(128), kFwdSmem, (cudaStream_t)stream,
         (const __nv_bfloat16*)qkv, (__nv_bfloat16*)out, B, heads, nshard, causal, sm_scale, thresh_of(drop_p), ds, seed,
         offset, step_ptr, n_bh);
   } else {
     if (set_smem<attn_tc_fwd_kernel<64>>(kFwdSmem)) return -1;
-    rtp::launch_k(attn_tc_fwd_kernel<64>, dim3(grid), dim3(128), kFwdSmem, (cudaStream_t)stream, 
+    rtp::launch_k(attn_tc_fwd_kernel<64>, dim3(grid), dim3(128), kFwdSmem, (cudaStream_t)stream,
         (const __nv_bfloat16*)qkv, (__nv_bfloat16*)out, B, heads, nshard, causal, sm_scale, thresh_of(drop_p), ds, seed,
         offset, step_ptr, n_bh);
   }
@@ -561,12 +561,12 @@ int rtp_attn_tc_bwd(const void* qkv, const void* dout, void* dqkv, int S, int B,
   const int grid = (n_bh + hpc - 1) / hpc;
   if (S == 32) {
     if (set_smem<attn_tc_bwd_kernel<32>>(kBwdSmem)) return -1;
-    rtp::launch_k(attn_tc_bwd_kernel<32>, dim3(grid), dim3(128), kBwdSmem, (cudaStream_t)stream, 
+    rtp::launch_k(attn_tc_bwd_kernel<32>, dim3(grid), dim3(128), kBwdSmem, (cudaStream_t)stream,
         (const __nv_bfloat16*)qkv, (const __nv_bfloat16*)dout, (__nv_bfloat16*)dqkv, B, heads, nshard, causal, sm_scale,
         thresh_of(drop_p), ds, seed, offset, step_ptr, n_bh);
   } else {
     if (set_smem<attn_tc_bwd_kernel<64>>(kBwdSmem)) return -1;
-    rtp::launch_k(attn_tc_bwd_kernel<64>, dim3(grid), dim3(128), kBwdSmem, (cudaStream_t)stream, 
+    rtp::launch_k(attn_tc_bwd_kernel<64>, dim3(grid), dim3(128), kBwdSmem, (cudaStream_t)stream,
         (const __nv_bfloat16*)qkv, (const __nv_bfloat16*)dout, (__nv_bfloat16*)dqkv, B, heads, nshard, causal, sm_scale,
         thresh_of(drop_p), ds, seed, offset, step_ptr, n_bh);
   }

@@ -333,8 +333,8 @@ int rtp_rope(const void* x, void* y, const float* cosv, const float* sinv, long 
   long long blocks = (total + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
   if (blocks < 1) return 0;
-  rtp::launch_k(rope_kernel, dim3((unsigned)blocks), dim3(256), 0, (cudaStream_t)stream, (const __nv_bfloat16*)x, (__nv_bfloat16*)y, cosv, sinv, T,
-                                                                 H, hd, S, inner, backward ? -1.f : 1.f);
+  rtp::launch_k(rope_kernel, dim3((unsigned)blocks), dim3(256), 0, (cudaStream_t)stream, (const __nv_bfloat16*)x,
+                (__nv_bfloat16*)y, cosv, sinv, T, H, hd, S, inner, backward ? -1.f : 1.f);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail("rope", e);
   return 0;
@@ -352,8 +352,8 @@ int rtp_rope_packed(const void* x, void* y, const float* cosv, const float* sinv
   long long blocks = (total + 255) / 256;
   if (blocks > 148 * 16) blocks = 148 * 16;
   if (blocks < 1) return 0;
-  rtp::launch_k(rope_packed_kernel, dim3((unsigned)blocks), dim3(256), 0, (cudaStream_t)stream, (const __nv_bfloat16*)x, (__nv_bfloat16*)y, cosv, sinv, T, D,
-                                                                        hd, nshard, S, backward ? -1.f : 1.f);
+  rtp::launch_k(rope_packed_kernel, dim3((unsigned)blocks), dim3(256), 0, (cudaStream_t)stream, (const __nv_bfloat16*)x,
+                (__nv_bfloat16*)y, cosv, sinv, T, D, hd, nshard, S, backward ? -1.f : 1.f);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail("rope_packed", e);
   return 0;

@@ -40,7 +40,7 @@ constexpr int kPitch = 128;                      // staged row: 64 bf16, 16-byte
 constexpr int kEpiWarps = 8;
 constexpr int kStageOut = kEpiWarps * 32 * kPitch;
 constexpr int kThreads = 32 * (2 + kEpiWarps);
-constexpr int kOnes = 1024;                       // eight 128-byte rows of ones: a CTA's share of a pair's 16-wide tile
+constexpr int kOnes = 1024;                      // eight 128-byte rows of ones: a CTA's share of a pair's 16-wide tile
 constexpr int kSmem = 1024 + kArea + kStageOut + kOnes + 256;
 static_assert(kSmem <= 232448, "over the shared memory of a CTA");
 
@@ -762,7 +762,8 @@ int local_gemm(const LocalGemm* jobs, int n, int pair_policy, unsigned long long
   Item it[kMaxItems];
   const int m = items_of(jobs, n, it);
   if (m < 0) return lfail("local_gemm: too many column sums");
-  return m <= 3 ? run<3>(it, m, pair_policy, status, timeout_ns, stream) : run<kMaxItems>(it, m, pair_policy, status, timeout_ns, stream);
+  return m <= 3 ? run<3>(it, m, pair_policy, status, timeout_ns, stream)
+                : run<kMaxItems>(it, m, pair_policy, status, timeout_ns, stream);
 }
 
 }  // namespace rtp

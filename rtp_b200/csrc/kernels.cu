@@ -1438,7 +1438,7 @@ int rtp_norm_fwd(const void* x, const void* sub, const void* gamma, const void* 
   if (D % 8 || D > 8192) { k_err = "norm: D must be a multiple of 8 and at most 8192"; return -1; }
   const float ds = drop_p > 0.f ? 1.f / (1.f - drop_p) : 1.f;
 #define RTP_NORM_FWD(T, NG, PER_SM)                                                                                   \
-  rtp::launch_k(norm_fwd_kernel<T, NG>, dim3(std::min(M, 148 * PER_SM)), dim3(T), 0, (cudaStream_t)stream,                                  \
+  rtp::launch_k(norm_fwd_kernel<T, NG>, dim3(std::min(M, 148 * PER_SM)), dim3(T), 0, (cudaStream_t)stream,            \
       (const __nv_bfloat16*)x, (const __nv_bfloat16*)sub, (const __nv_bfloat16*)gamma, (const __nv_bfloat16*)beta,    \
       (__nv_bfloat16*)h_out, (__nv_bfloat16*)y, mean, rstd, M, D, eps, rms, host_thresh(drop_p), ds, seed, offset,    \
       step_ptr)
@@ -1482,14 +1482,6 @@ int rtp_norm_bwd(const void* dy, const void* h, const void* gamma, const float* 
   LAUNCH_CHECK("norm_bwd");
   return 0;
 }
-int rtp_cross_entropy(void* logits, long long ld, const long long* target, float* loss, int M, int V, float grad_scale,
-                      long long ignore_index, int write_grad, void* stream) {
-  return rtp_cross_entropy_to(logits, ld, target, loss, M, V, grad_scale, ignore_index, write_grad, nullptr, 0, stream);
-}
-int rtp_cross_entropy_to(void* logits, long long ld, const long long* target, float* loss, int M, int V, float grad_scale,
-                         long long ignore_index, int write_grad, void* grad, long long ldg, void* stream) {
-  return rtp_cross_entropy_scaled(logits, ld, target, loss, M, V, grad_scale, nullptr, ignore_index, write_grad, grad, ldg, stream);
-}
 int rtp_cross_entropy_scaled(void* logits, long long ld, const long long* target, float* loss, int M, int V, float grad_scale,
                              const float* scale_ptr, long long ignore_index, int write_grad, void* grad, long long ldg,
                              void* stream) {
@@ -1503,9 +1495,9 @@ int rtp_cross_entropy_scaled(void* logits, long long ld, const long long* target
     return 0;
   }
   if (M > 0 && V > 0 && V <= kCeMaxV) {
-#define RTP_CE(T, NG)                                                                                                        \
-  rtp::launch_k(ce_row_kernel<T, NG>, dim3(M), dim3(T), 0, (cudaStream_t)stream,                                                          \
-      (const __nv_bfloat16*)logits, ld, target, loss, V, grad_scale, scale_ptr, ignore_index,                             \
+#define RTP_CE(T, NG)                                                                                   \
+  rtp::launch_k(ce_row_kernel<T, NG>, dim3(M), dim3(T), 0, (cudaStream_t)stream,                        \
+      (const __nv_bfloat16*)logits, ld, target, loss, V, grad_scale, scale_ptr, ignore_index,           \
       (__nv_bfloat16*)(write_grad ? (grad ? grad : logits) : nullptr), grad ? ldg : ld)
     // As many 16-byte words a thread as the row needs, one kernel for each number: words that the row does not have cost
     // registers and spills.  Against numbers rounded up (to 1, 2, 4, 5, 8 and 6, 8, 10, 13, 16): 8192 x 5120 42.6 -> 36.6 us,
@@ -1525,8 +1517,8 @@ int rtp_cross_entropy_scaled(void* logits, long long ld, const long long* target
   }
   if (scale_ptr) { k_err = "cross_entropy: a device-side scale needs rows of at most 65536 logits"; return -1; }
   const int grid = M < 148 * 8 ? M : 148 * 8;
-  rtp::launch_k(ce_kernel, dim3(grid), dim3(256), 0, (cudaStream_t)stream, (__nv_bfloat16*)logits, ld, target, loss, M, V, grad_scale,
-                                                    ignore_index, write_grad, (__nv_bfloat16*)grad, ldg);
+  rtp::launch_k(ce_kernel, dim3(grid), dim3(256), 0, (cudaStream_t)stream, (__nv_bfloat16*)logits, ld, target, loss, M, V,
+                grad_scale, ignore_index, write_grad, (__nv_bfloat16*)grad, ldg);
   LAUNCH_CHECK("cross_entropy");
   return 0;
 }
@@ -1553,10 +1545,9 @@ int rtp_embed_fwd(const void* table, const long long* ids, const void* pe, long 
   if (total <= 0) return 0;
   int grid = (int)((total + 255) / 256 > 148 * 16 ? 148 * 16 : (total + 255) / 256);
   const float ds = drop_p > 0.f ? 1.f / (1.f - drop_p) : 1.f;
-  rtp::launch_k(embed_fwd_kernel, dim3(grid), dim3(256), 0, (cudaStream_t)stream, (const __nv_bfloat16*)table, ids, (const __nv_bfloat16*)pe,
-                                                           ld_pe, tokens_per_pos, (__nv_bfloat16*)out, ld_out, col_off,
-                                                           T, Ds, D, scale, host_thresh(drop_p), ds, seed, offset,
-                                                           step_ptr);
+  rtp::launch_k(embed_fwd_kernel, dim3(grid), dim3(256), 0, (cudaStream_t)stream, (const __nv_bfloat16*)table, ids,
+                (const __nv_bfloat16*)pe, ld_pe, tokens_per_pos, (__nv_bfloat16*)out, ld_out, col_off, T, Ds, D, scale,
+                host_thresh(drop_p), ds, seed, offset, step_ptr);
   LAUNCH_CHECK("embed_fwd");
   return 0;
 }
@@ -1576,9 +1567,9 @@ int rtp_embed_bwd_blocks(void* gtable, const long long* ids, const void* dy, lon
   int grid = (int)((total + 255) / 256);
   if (grid > 148 * 16) grid = 148 * 16;
   const float ds = drop_p > 0.f ? 1.f / (1.f - drop_p) : 1.f;
-  rtp::launch_k(embed_bwd_kernel, dim3(grid), dim3(256), 0, (cudaStream_t)stream, (__nv_bfloat16*)gtable, ids, (const __nv_bfloat16*)dy, ld_dy,
-                                                           col_off, T, Ds, D, scale, host_thresh(drop_p), ds, seed,
-                                                           offset, step_ptr, blk_cols, V);
+  rtp::launch_k(embed_bwd_kernel, dim3(grid), dim3(256), 0, (cudaStream_t)stream, (__nv_bfloat16*)gtable, ids,
+                (const __nv_bfloat16*)dy, ld_dy, col_off, T, Ds, D, scale, host_thresh(drop_p), ds, seed, offset, step_ptr,
+                blk_cols, V);
   LAUNCH_CHECK("embed_bwd");
   return 0;
 }
@@ -1716,7 +1707,8 @@ int rtp_swiglu_bwd(const void* g, const void* u, long long ld, const void* dy, v
                    long long rows, int cols, void* stream) {
   if (cols % 8 || ld % 8 || ldo % 8) { k_err = "swiglu: cols and ld must be multiples of 8"; return -1; }
   const long long items = rows * (cols / 8);
-  swiglu_bwd_kernel<<<(unsigned)((items + 255) / 256), 256, 0, (cudaStream_t)stream>>>(      (const __nv_bfloat16*)g, (const __nv_bfloat16*)u, ld, (const __nv_bfloat16*)dy, (__nv_bfloat16*)dg, (__nv_bfloat16*)du, ldo, rows,
+  swiglu_bwd_kernel<<<(unsigned)((items + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+      (const __nv_bfloat16*)g, (const __nv_bfloat16*)u, ld, (const __nv_bfloat16*)dy, (__nv_bfloat16*)dg, (__nv_bfloat16*)du, ldo, rows,
       cols);
   LAUNCH_CHECK("swiglu_bwd");
   return 0;

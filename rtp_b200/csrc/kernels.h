@@ -23,12 +23,9 @@ int rtp_norm_bwd(const void* dy, const void* h, const void* gamma, const float* 
                  void* dsub, float* dgamma, float* dbeta, int M, int D, int rms, float drop_p,
                  unsigned long long seed, unsigned long long offset, const void* dres,
                  const unsigned long long* step_ptr, void* stream);
-int rtp_cross_entropy(void* logits, long long ld, const long long* target, float* loss, int M, int V, float grad_scale,
-                      long long ignore_index, int write_grad, void* stream);
-// Same, but the gradient goes to `grad` (row pitch ldg) and the logits stay as they are; grad = null: in place.
-int rtp_cross_entropy_to(void* logits, long long ld, const long long* target, float* loss, int M, int V, float grad_scale,
-                         long long ignore_index, int write_grad, void* grad, long long ldg, void* stream);
-// Same with a device-side factor of the gradient (scale_ptr, may be null; rows of at most 65536 logits).
+// Loss per row of logits (pitch ld) and, with write_grad, the gradient of grad_scale * (*scale_ptr) * sum of the losses: into
+// `grad` (pitch ldg), the logits stay as they are, or over the logits (grad = null).  scale_ptr: a factor on the device, may
+// be null (rows of at most 65536 logits).
 int rtp_cross_entropy_scaled(void* logits, long long ld, const long long* target, float* loss, int M, int V, float grad_scale,
                              const float* scale_ptr, long long ignore_index, int write_grad, void* grad, long long ldg,
                              void* stream);

@@ -6,10 +6,14 @@
 namespace rtp {
 
 // Programmatic dependent launch: a kernel may start, set itself up and wait (griddepcontrol.wait) while its predecessor in
-// the stream drains, which takes 0.7 to 1 us off a launch in a CUDA graph (README LM step 3682 -> 3594 us, the small LM 223 ->
-// 210).  Streaming kernels of very many blocks are launched without it: with Adam in it the step took 3790 us.  RTP_PDL unset: the kernels that work on this GPU
-// alone.  RTP_PDL=1: the rotation kernels too (on the training step of a ring they fill the SMs' registers and shared
-// memory, so a successor rarely finds room before its predecessor has left).  RTP_PDL=0: none.
+// the stream drains, which takes 0.5 to 1 us off a launch in a CUDA graph: step of the small LM 225 -> 210 us, of the small
+// GPT 995 -> 966, of the README LM 3 657 -> 3 637; steps of many milliseconds stay as they are.  Who is launched with it:
+// everything but the streaming kernels (Adam, activations, casts), whose blocks fill the SMs and then only wait: with Adam
+// in it the README step took 0.2 ms longer.  Cross-entropy and attention have as many blocks and lose nothing by it (loss and
+// gradient of 8192 x 50304 462 us both ways, of 1024 x 8192 13.7 -> 12.5; short launches gain).
+// RTP_PDL unset: the kernels that work on this GPU alone.  RTP_PDL=1: the rotation kernels too (on the training step of a
+// ring they fill the SMs' registers and shared memory, so a successor rarely finds room before its predecessor has left).
+// RTP_PDL=0: none.
 // A kernel that uses TMEM gives its dependents leave to start (pdl_launch_dependents) only after its CTA has allocated its
 // columns.  A dependent's CTA on the same SM may hold columns while it waits for this kernel to complete; were a CTA of this
 // kernel still to allocate, both would wait for good.  So whoever waits for columns waits for kernels that all have theirs.
