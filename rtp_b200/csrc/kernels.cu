@@ -402,7 +402,6 @@ __global__ void __launch_bounds__(256, 2) norm_bwd_kernel(
 __global__ void ce_kernel(__nv_bfloat16* logits, long long ld, const long long* __restrict__ target,
                           float* __restrict__ loss, int M, int V, float grad_scale, long long ignore_index,
                           int write_grad, __nv_bfloat16* grad, long long ldg) {
-  pdl_prologue();
   __shared__ float red[32];
   for (int row = blockIdx.x; row < M; row += gridDim.x) {
     __nv_bfloat16* lp = logits + (size_t)row * ld;
@@ -446,13 +445,12 @@ __global__ void ce_kernel(__nv_bfloat16* logits, long long ld, const long long* 
   }
 }
 
-// The same with the row in registers: every logit is read once and every gradient written once.  A block of 512 threads
-// takes one row, NG 16-byte words a thread, all in flight at once; two blocks share an SM, so that one loads or stores
-// while the other computes.  The two exponentials a logit (16 a clock and SM) and the unpacking bound it, not memory:
-// 4096 x 32000 162 -> 126 us, 8192 x 50304 553 -> 540, 1024 x 8192 9.7 -> 9.1 against the kernel above, which reads a row
-// three times, twice from L2.  Tried and dropped: the row in shared memory, filled and drained by bulk copies (604 us at
-// 50304 logits); 1024 threads with half the words (642 us, one block per SM); unpacking anew in every pass instead of
-// letting the compiler spill what does not fit (720 us).
+// The same with the row in registers, for up to 32768 logits: every logit is read once and every gradient written once.  A
+// block takes one row, NG 16-byte words a thread, all in flight at once; two (512 threads) or three blocks share an SM, so
+// that one loads or stores while the other computes.  The two exponentials a logit (16 a clock and SM) and the unpacking
+// bound it, not memory: 4096 x 32000 166 -> 114 us, 1024 x 8192 10.4 -> 7.2 against the kernel above, which reads a row three
+// times.  Tried and dropped: the row in shared memory, filled and drained by bulk copies; 1024 threads with half the words
+// (one block per SM).
 // Up to 16384 logits 256 threads, which add up in the order of the kernel above.
 constexpr int kCeMaxV = 65536;
 template <int kCeThreads, int NG>
@@ -515,13 +513,15 @@ __global__ void __launch_bounds__(kCeThreads, kCeThreads == 512 ? 2 : 3) ce_row_
   }
 }
 
-// The loss alone of rows wider than 16384 logits: two reads, the second from L2, so that no word stays in registers and
-// four blocks share an SM.  Threads and order of the sums are those of ce_row_kernel, so is every bit.  A row held in
-// registers leaves two blocks an SM with nothing to store between their loads: 1024 x 57344 52 us, here 26; 8192 x 50304
-// 280 and 136.
-__global__ void __launch_bounds__(512, 4) ce_loss_kernel(const __nv_bfloat16* logits, long long ld,
-                                                         const long long* __restrict__ target, float* __restrict__ loss, int V,
-                                                         long long ignore_index) {
+// The same sums in the same order (so the same bits), with the row read again for each pass instead of held: the second and
+// third reads come from L2, little lives in registers and four blocks of 512 threads (eight of 256) share an SM.  A held row
+// leaves two blocks an SM that wait for memory and then compute, and above 32768 logits it spills.  us, held / read again:
+// loss and gradient of 8192 x 50304 451 / 296, 1024 x 40960 49 / 40, 64 x 65536 21.6 / 9.3, 8192 x 20480 140 / 138, 300 x
+// 20480 8.1 / 10.6; loss alone of 8192 x 50304 280 / 136, 1024 x 57344 52 / 26, 2048 x 9216 10.6 / 8.7.
+template <int T, bool GRAD>
+__global__ void __launch_bounds__(T, 2048 / T) ce_stream_kernel(
+    const __nv_bfloat16* logits, long long ld, const long long* __restrict__ target, float* __restrict__ loss, int V,
+    float grad_scale, const float* __restrict__ scale_ptr, long long ignore_index, __nv_bfloat16* grad, long long ldg) {
   pdl_prologue();
   __shared__ float red[32];
   const int row = blockIdx.x, tid = threadIdx.x, n = V >> 3;
@@ -531,7 +531,7 @@ __global__ void __launch_bounds__(512, 4) ce_loss_kernel(const __nv_bfloat16* lo
   const float lt = (tid == 0 && !ignored) ? __bfloat162float(logits[(size_t)row * ld + t]) : 0.f;
   float mx = -INFINITY;
 #pragma unroll 4
-  for (int i = tid; i < n; i += 512) {
+  for (int i = tid; i < n; i += T) {
     float v[8];
     unpack8(lp[i], v);
 #pragma unroll
@@ -540,7 +540,7 @@ __global__ void __launch_bounds__(512, 4) ce_loss_kernel(const __nv_bfloat16* lo
   mx = block_max(mx, red);
   float se = 0.f;
 #pragma unroll 4
-  for (int i = tid; i < n; i += 512) {
+  for (int i = tid; i < n; i += T) {
     float v[8];
     unpack8(lp[i], v);
 #pragma unroll
@@ -548,6 +548,22 @@ __global__ void __launch_bounds__(512, 4) ce_loss_kernel(const __nv_bfloat16* lo
   }
   se = block_sum(se, red);
   if (tid == 0) loss[row] = ignored ? 0.f : mx + __logf(se) - lt;
+  if (!GRAD) return;
+  if (scale_ptr) grad_scale *= __ldg(scale_ptr);
+  const float inv = 1.f / se;
+  uint4* gp = reinterpret_cast<uint4*>(grad + (size_t)row * ldg);
+#pragma unroll 4
+  for (int i = tid; i < n; i += T) {
+    float v[8];
+    unpack8(lp[i], v);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      float p = __expf(v[k] - mx) * inv;
+      if (i * 8 + k == (int)t) p -= 1.f;
+      v[k] = ignored ? 0.f : p * grad_scale;
+    }
+    __stcs(gp + i, pack8(v));
+  }
 }
 
 // n = number of targets that count (at least one), for the mean: out[0] = n, out[1] = 1 / n.
@@ -1486,39 +1502,37 @@ int rtp_cross_entropy_scaled(void* logits, long long ld, const long long* target
                              const float* scale_ptr, long long ignore_index, int write_grad, void* grad, long long ldg,
                              void* stream) {
   if (V % 8 || ld % 8 || (grad && ldg % 8)) { k_err = "cross_entropy: V and the row pitches must be multiples of 8"; return -1; }
-  // Loss alone: a register-held row only pays where a few rows leave the SMs idle (256 x 24576 4.4 us, two reads 5.8;
-  // 512 x 24576 7.4 and 7.3, 2048 x 20480 20.0 and 18.1, 64 x 40960 7.2 and 4.8).
-  if (!write_grad && M > 0 && V > 16384 && V <= kCeMaxV && (V > 32768 || M >= 512)) {
-    rtp::launch_k(ce_loss_kernel, dim3(M), dim3(512), 0, (cudaStream_t)stream, (const __nv_bfloat16*)logits, ld, target, loss, V,
-                  ignore_index);
-    LAUNCH_CHECK("cross_entropy");
-    return 0;
-  }
   if (M > 0 && V > 0 && V <= kCeMaxV) {
-#define RTP_CE(T, NG)                                                                                   \
-  rtp::launch_k(ce_row_kernel<T, NG>, dim3(M), dim3(T), 0, (cudaStream_t)stream,                        \
-      (const __nv_bfloat16*)logits, ld, target, loss, V, grad_scale, scale_ptr, ignore_index,           \
-      (__nv_bfloat16*)(write_grad ? (grad ? grad : logits) : nullptr), grad ? ldg : ld)
+    __nv_bfloat16* out = (__nv_bfloat16*)(write_grad ? (grad ? grad : logits) : nullptr);
+    const long long ldo = grad ? ldg : ld;
+#define RTP_CE(KERNEL, T, X)                                                                                         \
+  rtp::launch_k(KERNEL<T, X>, dim3(M), dim3(T), 0, (cudaStream_t)stream, (const __nv_bfloat16*)logits, ld, target,   \
+                loss, V, grad_scale, scale_ptr, ignore_index, out, ldo)
+#define RTP_CE_HELD(T, WORDS) RTP_CE(ce_row_kernel, T, WORDS)
+    // Held rows pay where a block has at most eight words a thread to hold, and for the loss alone only where a few rows
+    // leave the SMs idle (256 x 24576 4.4 us, read again 5.8; 512 x 24576 7.4 and 7.3; 2048 x 8192 8.1 and 7.9).
     // As many 16-byte words a thread as the row needs, one kernel for each number: words that the row does not have cost
-    // registers and spills.  Against numbers rounded up (to 1, 2, 4, 5, 8 and 6, 8, 10, 13, 16): 8192 x 5120 42.6 -> 36.6 us,
-    // 12288 89.8 -> 83.1, 36864 300 -> 267, 57344 628 -> 543.
-    switch (V <= 16384 ? (V + 2047) / 2048 : 4 + (V + 4095) / 4096) {
-      case 1: RTP_CE(256, 1); break; case 2: RTP_CE(256, 2); break; case 3: RTP_CE(256, 3); break;
-      case 4: RTP_CE(256, 4); break; case 5: RTP_CE(256, 5); break; case 6: RTP_CE(256, 6); break;
-      case 7: RTP_CE(256, 7); break; case 8: RTP_CE(256, 8); break;
-      case 9: RTP_CE(512, 5); break; case 10: RTP_CE(512, 6); break; case 11: RTP_CE(512, 7); break;
-      case 12: RTP_CE(512, 8); break; case 13: RTP_CE(512, 9); break; case 14: RTP_CE(512, 10); break;
-      case 15: RTP_CE(512, 11); break; case 16: RTP_CE(512, 12); break; case 17: RTP_CE(512, 13); break;
-      case 18: RTP_CE(512, 14); break; case 19: RTP_CE(512, 15); break; default: RTP_CE(512, 16); break;
+    // registers.  Against numbers rounded up to a few: 8192 x 5120 42.6 -> 36.6 us, 12288 89.8 -> 83.1.
+    if (V > 32768) { if (out) RTP_CE(ce_stream_kernel, 512, true); else RTP_CE(ce_stream_kernel, 512, false); }
+    else if (!out && V > 16384 && M >= 512) RTP_CE(ce_stream_kernel, 512, false);
+    else if (!out && V > 8192 && V <= 16384 && M >= 2048) RTP_CE(ce_stream_kernel, 256, false);
+    else switch (V <= 16384 ? (V + 2047) / 2048 : 4 + (V + 4095) / 4096) {
+      case 1: RTP_CE_HELD(256, 1); break; case 2: RTP_CE_HELD(256, 2); break; case 3: RTP_CE_HELD(256, 3); break;
+      case 4: RTP_CE_HELD(256, 4); break; case 5: RTP_CE_HELD(256, 5); break; case 6: RTP_CE_HELD(256, 6); break;
+      case 7: RTP_CE_HELD(256, 7); break; case 8: RTP_CE_HELD(256, 8); break;
+      case 9: RTP_CE_HELD(512, 5); break; case 10: RTP_CE_HELD(512, 6); break; case 11: RTP_CE_HELD(512, 7); break;
+      default: RTP_CE_HELD(512, 8); break;
     }
+#undef RTP_CE_HELD
 #undef RTP_CE
     LAUNCH_CHECK("cross_entropy");
     return 0;
   }
   if (scale_ptr) { k_err = "cross_entropy: a device-side scale needs rows of at most 65536 logits"; return -1; }
+  // without dependent launch: 512 x 100352 103 us, with it 119 (its blocks wait where others of the same kernel run)
   const int grid = M < 148 * 8 ? M : 148 * 8;
-  rtp::launch_k(ce_kernel, dim3(grid), dim3(256), 0, (cudaStream_t)stream, (__nv_bfloat16*)logits, ld, target, loss, M, V,
-                grad_scale, ignore_index, write_grad, (__nv_bfloat16*)grad, ldg);
+  ce_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>((__nv_bfloat16*)logits, ld, target, loss, M, V, grad_scale, ignore_index,
+                                                    write_grad, (__nv_bfloat16*)grad, ldg);
   LAUNCH_CHECK("cross_entropy");
   return 0;
 }

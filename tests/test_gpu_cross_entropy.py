@@ -40,9 +40,11 @@ def test_loss_and_gradient(V, M, factor):
         assert FO.cross_entropy(lg, t).item() == loss.item()
 
 
-@pytest.mark.parametrize("M,V", [(511, 16392), (512, 16392), (512, 20472), (3, 32776), (513, 50304), (64, 65536)])
+@pytest.mark.parametrize("M,V", [(511, 16392), (512, 16392), (512, 20472), (3, 32776), (513, 50304), (64, 65536), (2047, 8200),
+                                 (2048, 8192), (2048, 8200), (2048, 16384)])
 def test_loss_alone_has_the_same_bits(M, V):
-    """Losses without a gradient may come from a kernel of their own: row by row the same bits, whatever was ignored or masked."""
+    """Losses without a gradient may come from another kernel: row by row the same bits, whatever was ignored or masked; and
+    a gradient that overwrites the logits is the one that goes to a buffer of its own."""
     from rtp_b200.ops import kernels as K
     g = torch.Generator(device="cuda").manual_seed(M + V)
     lg = (3 * torch.randn(M, V, generator=g, device="cuda")).to(torch.bfloat16)
@@ -50,7 +52,10 @@ def test_loss_alone_has_the_same_bits(M, V):
     t = torch.randint(0, V, (M,), generator=g, device="cuda")
     t[0], t[1], t[2] = 0, -100, V + 3          # one of the few finite logits, ignored, out of range
     alone = K.cross_entropy_to(lg, t, None)
-    assert torch.equal(alone, K.cross_entropy_to(lg, t, torch.empty_like(lg)))
+    grad, over = torch.empty_like(lg), lg.clone()
+    assert torch.equal(alone, K.cross_entropy_to(lg, t, grad, grad_scale=0.5))
+    assert torch.equal(alone, K.cross_entropy_(over, t, grad_scale=0.5)) and torch.equal(grad, over)
+    assert not grad[1].any() and not grad[2].any()
     ref = F.cross_entropy(lg[3:].double(), t[3:], reduction="none") if M > 3 else None
     if ref is not None:
         assert bool(((alone[3:].double() - ref).abs() <= 2.0 ** -16 * (1 + ref.abs())).all())
