@@ -48,6 +48,7 @@ struct alignas(64) Job {
   CUtensorMap ma, mb;
   int M, N, bn, kblocks;
   int tile0, tiles_m, tiles_n;                   // first tile of the job in the launch's tile order
+  int group;                                     // tile rows of a group (see tile_pos)
   unsigned char a_mn, b_mn, a3, b3;              // a3 / b3: the MN-major map is 3-D {64 mn, k, mn / 64}
   void* d; long long ldd;
   const void* c; long long ldc;
@@ -83,13 +84,13 @@ static_assert(sizeof(Ctrl) <= 256, "control block");
 __device__ __forceinline__ int unit_tile(int round, int unit, int units) {
   return round * units + ((round & 1) ? units - 1 - unit : unit);
 }
-// Tile position inside a job: groups of eight tile rows, column by column, so that the tiles in flight share operands.
+// Tile position inside a job: groups of tile rows, column by column, so that the tiles in flight share operands.
 __device__ __forceinline__ void tile_pos(const Job& j, int lt, int& tm, int& tn) {
-  const int per = 8 * j.tiles_n;
+  const int per = j.group * j.tiles_n;
   const int g = lt / per, r = lt - g * per;
-  const int rows = min(8, j.tiles_m - g * 8);
+  const int rows = min(j.group, j.tiles_m - g * j.group);
   tn = r / rows;
-  tm = g * 8 + (r - tn * rows);
+  tm = g * j.group + (r - tn * rows);
 }
 template <int MAXJ>
 __device__ __forceinline__ int find_job(const Params<MAXJ>& P, int t) {
@@ -682,6 +683,7 @@ int run(const Item* it, int n, int pair_policy, unsigned long long* status, unsi
     J.M = x.M; J.kblocks = (x.K + 63) / 64;
     J.tile0 = total;
     J.tiles_m = (x.M + tm - 1) / tm;
+    J.group = 8;
     J.a_mn = (unsigned char)x.a_mn;
     if (operand_map(&J.ma, &J.a3, x.a, x.M, x.K, x.lda, x.a_mn, 128)) return -1;
     if (J.sum) {
@@ -698,6 +700,10 @@ int run(const Item* it, int n, int pair_policy, unsigned long long* status, unsi
     if (operand_map(&J.mb, &J.b3, x.b, x.N, x.K, x.ldb, x.b_mn, rows_b)) return -1;
     J.b_mn = (unsigned char)x.b_mn;
     J.N = x.N; J.tiles_n = (x.N + J.bn - 1) / J.bn;
+    // Every group reads all of B again, so a wide output takes 16 rows a group while their part of A still stays in L2 beside
+    // it: forward 4096 x 2048 -> 50304 563 -> 546 us, 8192 rows 1147 -> 1103.  Not for a tall one (weight gradient of 50304 x
+    // 2048 over 4096 1238 -> 1298 us) nor a long contraction (8192^3 724 -> 740).
+    if (J.tiles_n >= J.tiles_m && 16ll * tm * x.K * 2 <= (32ll << 20)) J.group = 16;
     total += J.tiles_m * J.tiles_n;
     J.d = x.d; J.ldd = x.ldd; J.c = x.c; J.ldc = x.ldc; J.bias = x.bias; J.act = x.act;
     J.mask = x.mask; J.ldmask = x.ldmask; J.mask_scale = x.mask_scale;

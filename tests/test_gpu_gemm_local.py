@@ -35,7 +35,7 @@ def _linear(M, I, O, seed=0):
 
 
 @pytest.mark.parametrize("M,I,O", [(1, 64, 8), (8, 8, 8), (127, 72, 136), (129, 200, 264), (257, 520, 120), (650, 768, 3080),
-                                   (1000, 1032, 520), (2500, 2048, 1160)])
+                                   (1000, 1032, 520), (2500, 2048, 1160), (2200, 136, 4104), (4500, 72, 8200)])
 def test_linear(M, I, O):
     E, eng, flat, info, off, rnd = _linear(M, I, O)
     x, dy, c, mask = rnd(M, I), rnd(M, O), rnd(M, I), rnd(M, I)
