@@ -104,6 +104,37 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   }
 }
 
+// Same, without the suspended wait of try_wait: a single thread that feeds the tensor cores sees the phase 200 to 400 clocks
+// earlier.  Not for whole warps, whose polling would take issue slots from the others.
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ bool mbar_spin(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag,
+                                          unsigned long long* status, unsigned long long timeout_ns) {
+  if (mbar_test_wait(bar, parity)) return true;
+  unsigned long long t0 = globaltimer_ns();
+  uint32_t it = 0;
+  while (true) {
+    if (mbar_test_wait(bar, parity)) return true;
+    if ((++it & 0xfff) == 0) {
+      if (*abort_flag) return false;
+      if (globaltimer_ns() - t0 > timeout_ns) {
+        *abort_flag = 1;
+        atomicCAS(status, (unsigned long long)ST_OK, (unsigned long long)ST_TIMEOUT_MBAR);
+        return false;
+      }
+    }
+  }
+}
+
 // Variants on 32-bit shared-memory addresses for the hot loops: the common case (barrier already complete) is one
 // try_wait; the bounded spin lives out of line so the loop body stays small.
 __device__ __forceinline__ bool mbar_try_wait_s(uint32_t bar, uint32_t parity) {
@@ -212,6 +243,16 @@ __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a_desc, uint
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// The same with A in TMEM: row i in lane i, two consecutive bf16 of the contraction in each 32-bit column (K-major).
+__device__ __forceinline__ void umma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+                                             uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 // Arrives on the mbarrier once every UMMA issued so far by this thread has completed.
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
@@ -277,6 +318,37 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
                ::"r"(smem_u32(bar)), "h"(mask)
                : "memory");
 }
+
+// Cluster launch control: a running CTA asks for a CTA of its grid that has not started, whose launch is then cancelled and
+// whose work it takes on.  The answer (16 bytes) lands in shared memory and completes on an mbarrier; after a "no" a CTA may
+// not ask again.
+__device__ __forceinline__ void clc_try_cancel(void* answer, uint64_t* bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+               ::"r"(smem_u32(answer)), "r"(smem_u32(bar))
+               : "memory");
+}
+// blockIdx.x of the cancelled CTA, -1: there was none left
+__device__ __forceinline__ int clc_answer(const void* answer) {
+  uint32_t yes, x;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b128 h;\n\t"
+      "ld.shared.b128 h, [%2];\n\t"
+      "mov.u32 %1, 0;\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, h;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(yes), "=r"(x)
+      : "r"(smem_u32(answer))
+      : "memory");
+  return yes ? (int)x : -1;
+}
+
+// Registers of the executing warpgroup (all four of its warps): a kernel's groups may hold no more together than it was
+// launched with.
+template <int N>
+__device__ __forceinline__ void reg_dealloc() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void reg_alloc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 
 // 32 lanes x 32 consecutive 32-bit columns: thread t of the warp gets lane (base_lane + t).
 __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t (&r)[32]) {

@@ -1,26 +1,30 @@
-// Flash attention on tcgen05 tensor cores: forward, dQ and dK/dV kernels (see flash_attn.h for the interface).
+// Flash attention on tcgen05 tensor cores: forward, delta and backward kernels (see flash_attn.h for the interface).
 //
-// One CTA = 128 query rows (forward, dQ) or 128 keys (dK/dV) of one (batch, head).  Ten warps:
-//   warps 0-7  "row" threads, two per row of the tile: thread (t, h) reads TMEM lane t and owns the key columns
-//              [64 h, 64 h + 64) of the 128-key block (warps w and w + 4 may both access lanes 32 (w % 4) ..).  The online
-//              softmax of a row (forward) and the dS algebra (backward) run in registers without shuffles; the two
-//              threads of a row exchange one partial maximum per block through shared memory (forward only).
+// A CTA works on 128-row tiles of one (batch, head) at a time.  Twelve warps:
+//   warps 0-7  "row" threads: thread = TMEM lane = row of a tile (forward: all 128 columns of a block; backward: 64).  The online
+//              softmax of a row (forward) and the dS algebra (backward) run in registers without shuffles.
 //   warp 8     TMA producer: Q / K / V / dO tiles, 128 rows x 64 columns per copy, 128-byte swizzle, local memory only.
 //   warp 9     UMMA issuer (one elected thread).
+//   warp 10    asks for the next piece of work (one elected thread); warp 11 is there for its registers.
 //
-// Forward, per block of 128 keys:  S = Q K^T (TMEM, double-buffered)  ->  row threads: scale, masks, running max,
-// P = exp2(S - m) as bf16 into a shared tile  ->  O += P V with O resident in TMEM.  O is rescaled in TMEM only when a
-// row's maximum has grown by more than 2^8 since the last rescale (the sum l carries the same offset, so the final
-// O / l is exact); most blocks skip the rescale.  Output: O / l and the row's log-sum-exp (log2 units).
+// Forward, per block of 128 keys:  S = Q K^T (TMEM)  ->  row threads: scale, masks, running max, P = exp2(S - m) as bf16 back into
+// TMEM  ->  O += P V with O resident in TMEM.  O is rescaled in TMEM only when a row's maximum has grown by more than 2^8
+// since the last rescale (the sum l carries the same offset, so the final O / l is exact); most blocks skip the rescale.
+// Output: O / l and the row's log-sum-exp (log2 units).
 //
-// Backward recomputes P from Q, K and the saved log-sum-exp; nothing of size S x S touches global memory.
-//   dQ kernel   (CTA = query block): delta = rowsum(dO * O);  per key block: S, dP = dO V^T -> dS = P (dP - delta)
-//               -> dQ += dS K.
-//   dK/dV kernel (CTA = key block): per query block: S, dP -> P, dS tiles -> dV += P^T dO, dK += dS^T Q.  The P / dS
-//               tiles are written row-per-thread once and read by the UMMA as MN-major A operands (= transposed).
-// Each kernel is compiled in six variants (no mask, key padding only, additive mask; dropout yes or no): the mask and
-// Philox code unrolled over a row's registers is several times larger than the plain softmax and, when merely branched
-// over, slowed the row threads down through instruction fetch alone.
+// Backward recomputes P from Q, K and the saved log-sum-exp; nothing of size S x S touches global memory.  delta = rowsum(dO * O)
+// comes from a kernel of its own, dQ of a block of queries and dK / dV of a block of keys are pieces of work of one launch.
+//
+// What it gives (us, before: one row tile a CTA with two threads a row, P and dS through shared memory, dQ and dK / dV in
+// launches of their own; now), forward and backward: 1 x 16 heads of 8192 x 8192 x 128 causal 338 -> 242 and 1 134 -> 805,
+// 4 x 16 of 2048 causal 126 -> 90 and 400 -> 285, 8 x 20 of 512 x 2048 x 64 121 -> 90 and 433 -> 250, 4 x 8 of 256 x 256 x 64
+// 8.3 -> 10 and 19 -> 13.  Per 128 x 128 block at head_dim 128 (SM clocks): forward 1 700 (tensor work 1 024, exponentials
+// 1 024), dK / dV 3 100 (tensor work 2 048), dQ 2 080 (1 536).  The forward is bound by the exponentials and the hand-overs
+// between row threads and issuer, dK / dV by the chain P -> dV -> S of the next block (TMEM has no room for a second S).
+//
+// Each kernel is compiled in variants (no mask, key padding only, additive mask; dropout yes or no; more work than SMs or not):
+// the mask and Philox code unrolled over a row's registers is several times larger than the plain softmax and, when merely
+// branched over, slowed the row threads down through instruction fetch alone.
 // Every mbarrier wait is bounded; on expiry the CTA records a status code, drains its copies and UMMAs, frees its TMEM
 // and returns.
 #include <cuda.h>
@@ -29,7 +33,9 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <string>
+#include <type_traits>
 
 #include "common.cuh"
 #include "flash_attn.h"
@@ -41,9 +47,12 @@ using namespace rtp;
 
 constexpr int kBlk = 128;              // rows of Q per CTA = keys per block
 constexpr int kSub = 16384;            // one [128 x 64] bf16 sub-tile with 128-byte rows
-constexpr int kThreads = 320;
-constexpr int kRowThreads = 256;
-constexpr int kProducerWarp = 8, kMmaWarp = 9;
+constexpr int kThreads = 384;          // two warpgroups of row threads, one of producer, issuer and two idle warps
+// A row thread holds 128 scores: of the 168 registers a thread that 384 threads are launched with, the third warpgroup
+// hands most to the other two.
+constexpr int kRowRegs = 208, kAuxRegs = 88;
+static_assert(2 * kRowRegs + kAuxRegs <= 3 * 168, "more registers than the launch has");
+constexpr int kProducerWarp = 8, kMmaWarp = 9, kSchedWarp = 10;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kRescaleGap = 8.f;     // rescale O when a row maximum grew by more than 2^8
 
@@ -71,12 +80,13 @@ struct MaskArgs {
 
 struct alignas(64) FlashParams {
   CUtensorMap mq, mk, mv, mdo;         // 3-D maps {columns, dim1, dim2}; *_seq1 tells which of dim1 / dim2 is the sequence
-  CUtensorMap mq64, mdo64, mk64, mv64; // the same tensors with boxes of 64 rows (backward kernels)
   int q_seq1, k_seq1, v_seq1, do_seq1;
   DRef q, k, v, o, dout, dq, dk, dv;
   float* lse;
   float* delta;
   int B, H;
+  int group;                           // (batch, head) pairs whose CTAs run side by side (see head_group)
+  int split;                           // forward: one row tile a CTA, its key blocks dealt to the two warpgroups
   MaskArgs m;
   unsigned long long* status;
   unsigned long long timeout_ns;
@@ -84,19 +94,12 @@ struct alignas(64) FlashParams {
 };
 
 struct Ctl {
-  uint64_t bar[24];
+  uint64_t bar[28];
+  uint4 next;                          // the scheduler's answer: the work that follows (see schedule)
   uint32_t tmem_base;
   uint32_t abort_flag;
 };
-// Exchange area of the two threads of a row (forward): per block one partial row maximum each way, double-buffered by
-// block parity.  The two warps that share 32 rows meet at an mbarrier of their own (64 arrivals per exchange).
-struct Xchg {
-  float val[2][2][128];
-};
 
-__device__ __forceinline__ uint32_t sw128(int row, int chunk) {
-  return (uint32_t)row * 128u + (uint32_t)((chunk ^ (row & 7)) << 4);
-}
 __device__ __forceinline__ void tmem_ld32f(uint32_t taddr, float* r) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -121,6 +124,53 @@ __device__ __forceinline__ void tmem_st32f(uint32_t taddr, const float* r) {
       : "memory");
 }
 
+// 16 columns of this thread's lane: 32 bf16 of a TMEM A operand
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+
+// 4 x 4 transpose of 16-byte chunks among four neighbouring lanes: lane i of four has chunks 0..3 of its row and leaves with
+// chunk i of the four rows.
+__device__ __forceinline__ uint4 sel4(bool a, const uint4& x, const uint4& y) {
+  return make_uint4(a ? x.x : y.x, a ? x.y : y.y, a ? x.z : y.z, a ? x.w : y.w);
+}
+__device__ __forceinline__ uint4 shfl4(const uint4& v, int d) {
+  return make_uint4(__shfl_xor_sync(0xffffffffu, v.x, d), __shfl_xor_sync(0xffffffffu, v.y, d), __shfl_xor_sync(0xffffffffu, v.z, d),
+                    __shfl_xor_sync(0xffffffffu, v.w, d));
+}
+__device__ __forceinline__ void transpose4(uint4 (&v)[4], int lane) {
+#pragma unroll
+  for (int d = 1; d < 4; d *= 2) {
+    const bool up = lane & d;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (k & d) continue;
+      const uint4 got = shfl4(sel4(up, v[k], v[k + d]), d);      // what the partner needs of this pair goes to it
+      if (up) v[k] = got; else v[k + d] = got;
+    }
+  }
+}
+// 32 columns of a warp's 32 rows to global memory as bf16: four lanes write 64 consecutive bytes of a row.  One row a thread, 16
+// bytes at a time, the 32 lanes of each store touched 32 lines (with it 288 -> 280 us, backward of 4 x 16 heads of 2048 x 128).  `rows` of the warp's rows are there; dst: row 0.
+__device__ __forceinline__ void store_rows32(__nv_bfloat16* dst, long long pitch, int rows, const float* o, int lane) {
+  uint4 v[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    v[k] = make_uint4(pack_bf16(o[8 * k], o[8 * k + 1]), pack_bf16(o[8 * k + 2], o[8 * k + 3]), pack_bf16(o[8 * k + 4], o[8 * k + 5]),
+                      pack_bf16(o[8 * k + 6], o[8 * k + 7]));
+  transpose4(v, lane);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int r = (lane & ~3) + k;
+    if (r < rows) *reinterpret_cast<uint4*>(dst + r * pitch + (lane & 3) * 8) = v[k];
+  }
+}
+
 // Loads one [128 rows x 64 * SUB columns] tile of a (batch, head) into SUB swizzled sub-tiles.
 template <int SUB>
 __device__ __forceinline__ void load_tile(uint32_t dst, const CUtensorMap* map, int seq1, int col, int b, int s0,
@@ -130,21 +180,6 @@ __device__ __forceinline__ void load_tile(uint32_t dst, const CUtensorMap* map, 
   for (int u = 0; u < SUB; ++u) {
     if (seq1) tma_load_3d_s(dst + u * kSub, m, col + u * 64, s0, b, bar);
     else tma_load_3d_s(dst + u * kSub, m, col + u * 64, b, s0, bar);
-  }
-}
-
-// The backward kernels walk the other sequence in sub-blocks of 64 rows, three stages deep.
-constexpr int kHalf = 64;                 // rows per sub-block
-constexpr int kHalfTile = kHalf * 128;    // one [64 x 64] bf16 sub-tile with 128-byte rows
-constexpr int kBwdStages = 3;
-template <int SUB>
-__device__ __forceinline__ void load_tile64(uint32_t dst, const CUtensorMap* map, int seq1, int col, int b, int s0,
-                                            uint32_t bar) {
-  const unsigned long long m = reinterpret_cast<unsigned long long>(map);
-#pragma unroll
-  for (int u = 0; u < SUB; ++u) {
-    if (seq1) tma_load_3d_s(dst + u * kHalfTile, m, col + u * 64, s0, b, bar);
-    else tma_load_3d_s(dst + u * kHalfTile, m, col + u * 64, b, s0, bar);
   }
 }
 
@@ -227,9 +262,6 @@ __device__ __forceinline__ uint32_t keep_bits(const MaskArgs& m, unsigned long l
   }
   return bits;
 }
-__device__ __forceinline__ uint4 pack8f(const float* v) {
-  return make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
-}
 
 // Common set-up: barriers, TMEM, abort flag.  Returns the TMEM base.
 __device__ __forceinline__ uint32_t setup_cta(Ctl* ctl, const int* counts, int nbar, int warp, int lane) {
@@ -256,35 +288,108 @@ __device__ __forceinline__ void teardown_cta(uint32_t tmem, int warp) {
     tmem_dealloc(tmem, 512);
   }
 }
-// Publishes `v` to the other thread of the row and returns the partner's value; `n` counts the exchanges of this row
-// group from 0.  The arrive releases the value, the (bounded) wait acquires the partner's.
-__device__ __forceinline__ float xchg_row(Xchg* x, uint64_t* xbar, int wg, int rt, uint32_t n, float v,
-                                          volatile uint32_t* abort_flag, unsigned long long* status,
-                                          unsigned long long timeout_ns, bool& ok) {
-  x->val[n & 1][wg][rt] = v;
-  mbar_arrive(xbar);
-  if (!mbar_wait(xbar, n & 1u, abort_flag, status, timeout_ns)) { ok = false; return v; }
-  return x->val[n & 1][wg ^ 1][rt];
-}
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// Two fp32 operations in one instruction (each rounded as the single one is).
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
+      "fma.rn.ftz.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.ftz.f32x2 x, x, y;\n\t"
+      "mov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmul.rn.ftz.f32x2 x, x, y;\n\t"
+      "mov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+// 2^x of two numbers on the multiply-add pipes, x >= -126 or taken as that: 2^round(x) rides in as an exponent, the rest is a
+// polynomial of degree 6 in [-1/2, 1/2] (least maximum relative error, by Remez exchange).  Relative error up to 1.1e-7 in
+// fp32, not above ex2.approx; twice its instructions, but the special-function unit has only four lanes an SM quarter.
+__device__ __forceinline__ float2 ex2_poly2(float2 t) {
+  const float2 magic = make_float2(12582912.f, 12582912.f);       // 1.5 * 2^23: rounds to integers, which stay in the low bits
+  t.x = fmaxf(t.x, -126.f);
+  t.y = fmaxf(t.y, -126.f);
+  const float2 r = add2(t, magic);
+  const float2 n = add2(r, make_float2(-12582912.f, -12582912.f));
+  const float2 f = fma2(n, make_float2(-1.f, -1.f), t);
+  float2 p = make_float2(1.3652998313773423e-4f, 1.3652998313773423e-4f);
+  p = fma2(p, f, make_float2(1.3320884900167584e-3f, 1.3320884900167584e-3f));
+  p = fma2(p, f, make_float2(9.6239959821105e-3f, 9.6239959821105e-3f));
+  p = fma2(p, f, make_float2(5.550621822476387e-2f, 5.550621822476387e-2f));
+  p = fma2(p, f, make_float2(0.24022623896598816f, 0.24022623896598816f));
+  p = fma2(p, f, make_float2(0.6931469440460205f, 0.6931469440460205f));
+  p = fma2(p, f, make_float2(1.f, 1.f));
+  return make_float2(__int_as_float(__float_as_int(p.x) + (__float_as_int(r.x) << 23)),
+                     __int_as_float(__float_as_int(p.y) + (__float_as_int(r.y) << 23)));
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
 __device__ __forceinline__ float max64(const float* s) {
   float m0 = s[0], m1 = s[1], m2 = s[2], m3 = s[3];
 #pragma unroll
-  for (int i = 4; i < 64; i += 4) {
-    m0 = fmaxf(m0, s[i]); m1 = fmaxf(m1, s[i + 1]); m2 = fmaxf(m2, s[i + 2]); m3 = fmaxf(m3, s[i + 3]);
+  for (int i = 4; i < 60; i += 8) {
+    m0 = max3(m0, s[i], s[i + 1]); m1 = max3(m1, s[i + 2], s[i + 3]);
+    m2 = max3(m2, s[i + 4], s[i + 5]); m3 = max3(m3, s[i + 6], s[i + 7]);
   }
-  return fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
+  return fmaxf(max3(max3(m0, m1, m2), m3, s[60]), max3(s[61], s[62], s[63]));
+}
+// The CTAs are persistent: when a role is done with one piece of work it goes on with the next, so that copies and products of
+// the next run under the end of the last, and TMEM and barriers are set up once.  A CTA's first work is its own blockIdx.x; from
+// then on one thread asks for a CTA that has not started yet (the longest are numbered first).  It asks when every role has begun
+// the current piece and the producer has copied all of it, no earlier: asked for at the beginning of the piece before, work was
+// tied to CTAs that were not the first to be free (16 heads of 8192 x 8192, head_dim 128, causal: forward 292 us, 249 without
+// persistence).  A launch that fits the SMs at once has nothing to ask for (MORE = false)
+// and is better off without the instruction: with it in the kernel, dependent launch around it no longer overlaps (32 heads of
+// 256 x 256, head_dim 64: backward 10.3 -> 13.5 us).
+__device__ __forceinline__ void schedule(Ctl* ctl, uint64_t* full, uint64_t* taken, volatile uint32_t* abort_flag,
+                                         unsigned long long* status, unsigned long long tmo) {
+  for (uint32_t n = 0;; ++n) {
+    if (!mbar_wait(taken, n & 1u, abort_flag, status, tmo)) return;
+    fence_proxy_async_smem();          // all roles have read the last answer: the next may be written over it
+    mbar_arrive_expect_tx(full, 16);
+    clc_try_cancel(&ctl->next, full);
+    if (!mbar_wait(full, n & 1u, abort_flag, status, tmo)) {
+      const unsigned long long t0 = globaltimer_ns();            // the answer lands (bounded) before the CTA may exit
+      while (!mbar_try_wait(full, n & 1u))
+        if (globaltimer_ns() - t0 > 2000000ull) break;
+      return;
+    }
+    if (clc_answer(&ctl->next) < 0) return;
+  }
+}
+// For every role, by all lanes of a warp or by one thread: the n-th next piece of work, -1: none, or a wait ran out.  The role
+// arrives on `taken` once for each piece, the first included.
+__device__ __forceinline__ int next_work(Ctl* ctl, uint64_t* full, uint32_t n, bool whole_warp, volatile uint32_t* abort_flag,
+                                         unsigned long long* status, unsigned long long tmo) {
+  uint32_t good = mbar_wait(full, n & 1u, abort_flag, status, tmo) ? 1u : 0u;
+  if (whole_warp) good = __all_sync(0xffffffffu, good);
+  if (!good) return -1;
+  const int w = clc_answer(&ctl->next);
+  if (whole_warp) __syncwarp();
+  return w;
 }
 // After an abort: wait (bounded) for the copies this thread has issued, so that none lands in a dead CTA.
-__device__ __forceinline__ void drain_loads(uint64_t* const* bars, const uint32_t* parity, const bool* issued, int n) {
-  for (int i = 0; i < n; ++i) {
-    if (!issued[i]) continue;
+__device__ __forceinline__ void drain_loads(uint64_t* bars, uint32_t used, uint32_t parity) {
+  for (int i = 0; i < 32; ++i) {
+    if (!((used >> i) & 1u)) continue;
     const unsigned long long t0 = globaltimer_ns();
-    while (!mbar_try_wait(bars[i], parity[i])) {
+    while (!mbar_try_wait(&bars[i], (parity >> i) & 1u)) {
       if (globaltimer_ns() - t0 > 2000000ull) break;
     }
   }
@@ -297,709 +402,808 @@ __device__ __forceinline__ void drain_mma(uint64_t* bar) {
   }
 }
 
-// =====================================================================================================  forward
-// barriers
-enum { F_QFULL = 0, F_KFULL = 1, F_KEMPTY = 3, F_VFULL = 5, F_VEMPTY = 7, F_SFULL = 9, F_SEMPTY = 11, F_PFULL = 13,
-       F_PVDONE = 14, F_DRAIN = 15, F_XCHG = 16 /* .. 19: one per group of 32 rows */ };
+// bf16 of 32 values into 16 columns of this thread's lane
+__device__ __forceinline__ void store_bf16x32(uint32_t taddr, const float* v) {
+  uint32_t pk[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) pk[i] = pack_bf16(v[2 * i], v[2 * i + 1]);
+  tmem_st16(taddr, pk);
+}
+// A warp's part of P or dS is in TMEM: one arrival for it.
+__device__ __forceinline__ void publish_rows(uint64_t* bar, int lane) {
+  tmem_st_wait();
+  tc_fence_before();
+  __syncwarp();
+  if (lane == 0) mbar_arrive(bar);
+}
+// Waits of all lanes of a warp; false for all if one ran out.
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, unsigned long long* status,
+                                          unsigned long long tmo) {
+  const uint32_t good = mbar_spin(bar, parity, abort_flag, status, tmo) ? 1u : 0u;
+  return __all_sync(0xffffffffu, good);
+}
+// D[128 x 128] = A B^T of two [128 x HD] K-major tiles
+template <int HD>
+__device__ __forceinline__ void umma_tiles(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc) {
+#pragma unroll
+  for (int u = 0; u < HD / 64; ++u)
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk)
+      umma_bf16(d, make_smem_desc(a + u * kSub + kk * 32, 16, 1024), make_smem_desc(b + u * kSub + kk * 32, 16, 1024), idesc,
+                (u | kk) ? 1u : 0u);
+}
+// D[128 x HD] += A B: A the two halves of a [128 x 128] bf16 operand in TMEM, 64 columns apart, B a [128 x HD] tile read MN-major
+__device__ __forceinline__ void umma_rows(uint32_t d, uint32_t a_tmem, uint32_t b, uint32_t idesc, bool add) {
+#pragma unroll
+  for (int kk = 0; kk < 8; ++kk)
+    umma_bf16_ts(d, a_tmem + (kk >> 2) * 64 + (kk & 3) * 8, make_smem_desc(b + kk * 2048, kSub, 1024), idesc,
+                 (add || kk > 0) ? 1u : 0u);
+}
 
-template <int HD, int MSK, bool DRP>
+// =====================================================================================================  forward
+// Two row tiles a CTA, one warpgroup each (thread = row), so that the softmax of one tile runs under the products of the
+// other: per 128 x 128 block the tensor cores need 1 024 clocks at head_dim 128 and the exponentials 1 024 (16 a clock),
+// and with both tiles in flight neither waits for the other's chain S -> softmax -> P V.  P goes back into the tile's own S
+// columns as bf16 and is the TMEM operand of P V: through shared memory (a 32 KB tile written, then read at the rate of the
+// UMMA itself) and with one tile a CTA the block took 2 750 clocks, now 1 700.  One exponential in four goes through the
+// multiply-add pipes (ex2_poly2): 266 -> 246 us at 16 heads of 8192 x 8192 x 128.  The UMMAs of a CTA run in the order of their issue, so
+// S(i + 1) of a tile may follow P V(i) into the same columns, and S(i + 1) complete means O is complete up to i.
+// `split`: both tiles are the SAME 128 queries and take turns at the key blocks (tile t: blocks t, t + 2, ..); the two partial
+// results are merged at the end.  Taken where the launch has too few row tiles to fill the SMs twice (see rtp_flash_fwd).
+// barriers
+enum { F_QFULL = 0 /* 2 tiles */, F_QEMPTY = 2 /* 2 */, F_KFULL = 4 /* 2 stages */, F_KEMPTY = 6, F_VFULL = 8, F_VEMPTY = 10,
+       F_SFULL = 12 /* 2 tiles */, F_PFULL = 14 /* 2 */, F_PTAIL = 16 /* 2 */, F_OFULL = 18 /* 2 */, F_WFULL = 20, F_TAKEN = 21,
+       F_DRAIN = 22 };
+
+// What blockIdx.x stands for: row tiles g0 (and g0 + 1) of a (batch, head), with n0 and n1 steps; nload key blocks in all.
+struct FwdWork {
+  int g0, bh, n0, n1, nload;
+};
+__device__ __forceinline__ FwdWork fwd_work(const FlashParams& p, int blk) {
+  const int nqb = (p.m.Sq + kBlk - 1) / kBlk, nkb = (p.m.Sk + kBlk - 1) / kBlk, BH = p.B * p.H;
+  const int per = p.split ? 1 : 2;                                  // row tiles of a piece of work
+  // heaviest (last) query blocks of a group of heads first
+  const int nt = (nqb + per - 1) / per, grp = blk / (p.group * nt) * p.group;
+  const int in_grp = blk - grp * nt, heads = min(p.group, BH - grp);
+  FwdWork w;
+  w.g0 = (nt - 1 - in_grp / heads) * per;
+  w.bh = grp + in_grp % heads;
+  const int nb0 = p.m.causal ? min(nkb, w.g0 + 1) : nkb;            // key blocks of the first tile, of the second
+  const int nb1 = w.g0 + 1 >= nqb ? 0 : p.m.causal ? min(nkb, w.g0 + 2) : nkb;
+  w.n0 = p.split ? (nb0 + 1) >> 1 : nb0;
+  w.n1 = p.split ? nb0 >> 1 : nb1;
+  w.nload = p.split ? nb0 : max(nb0, nb1);
+  return w;
+}
+
+template <int HD, int MSK, bool DRP, bool MORE>
 __global__ void __launch_bounds__(kThreads, 1) flash_fwd_kernel(const __grid_constant__ FlashParams p) {
   constexpr int SUB = HD / 64;
   constexpr int TILE = SUB * kSub;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sQ = sm;
-  uint8_t* sK = sQ + TILE;            // 2 stages
+  uint8_t* sQ = sm;                   // 2 tiles (split: the first serves both)
+  uint8_t* sK = sQ + 2 * TILE;        // 2 stages
   uint8_t* sV = sK + 2 * TILE;        // 2 stages
-  uint8_t* sP = sV + 2 * TILE;        // [128 x 128] bf16: two sub-tiles
-  Ctl* ctl = reinterpret_cast<Ctl*>(sP + 2 * kSub);
-  Xchg* xc = reinterpret_cast<Xchg*>(sP + 2 * kSub + 256);
+  Ctl* ctl = reinterpret_cast<Ctl*>(sV + 2 * TILE);
+  float* sX = reinterpret_cast<float*>(sV + 2 * TILE + 256);        // split: {maximum, sum} of each row and tile
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const MaskArgs& M = p.m;
-  const int nqb = (M.Sq + kBlk - 1) / kBlk;
-  const int BH = p.B * p.H;
-  // heaviest (last) query blocks first
-  const int qb = nqb - 1 - (int)(blockIdx.x / BH);
-  const int bh = (int)(blockIdx.x % BH);
-  const int b = bh / p.H, h = bh % p.H;
-  const int q0 = qb * kBlk;
-  int nkb = (M.Sk + kBlk - 1) / kBlk;
-  if (M.causal) nkb = min(nkb, qb + 1);
+  const bool split = p.split;                                       // one wave: no CTA has a second piece of work
 
-  // counts by barrier index: Q/K/V full and empty 1 each, S full 1, S empty 8 (one per row warp), P full 256, drain 1,
-  // row exchange 64 (two warps)
-  const int counts[20] = {1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 8, 8, kRowThreads, 1, 1, 64, 64, 64, 64};
-  const uint32_t tmem = setup_cta(ctl, counts, 20, warp, lane);
+  // counts by barrier index: copies and commits 1 each, P (its first three quarters, its last) 4: one per row warp of the tile,
+  // next work 1 and 10 (producer, issuer, eight row warps)
+  const int counts[23] = {1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 4, 4, 4, 4, 1, 1, 1, 10, 1};
+  const uint32_t tmem = setup_cta(ctl, counts, 23, warp, lane);
   volatile uint32_t* abort_flag = &ctl->abort_flag;
   unsigned long long* status = p.status;
   const unsigned long long tmo = p.timeout_ns;
   uint64_t* bar = ctl->bar;
+  auto following = [&](uint32_t n, bool whole_warp) {
+    return MORE ? next_work(ctl, &bar[F_WFULL], n, whole_warp, abort_flag, status, tmo) : -1;
+  };
 
+  if (warp >= kProducerWarp) {
+  reg_dealloc<kAuxRegs>();
   if (warp == kProducerWarp) {
     // ---------------------------------------------------------------------------------- TMA producer
     if (elect_one()) {
-      const int cq = head_col(p.q, h), ck = head_col(p.k, h), cv = head_col(p.v, h);
       bool ok = true;
-      uint64_t* dbar[5]; uint32_t dpar[5]; bool dis[5] = {false, false, false, false, false};
-      mbar_arrive_expect_tx(&bar[F_QFULL], TILE);
-      load_tile<SUB>(smem_u32(sQ), &p.mq, p.q_seq1, cq, b, q0, smem_u32(&bar[F_QFULL]));
-      dbar[0] = &bar[F_QFULL]; dpar[0] = 0; dis[0] = true;
-      for (int j = 0; j < nkb && ok; ++j) {
-        const int st = j & 1;
-        const uint32_t ph = (uint32_t)(j >> 1) & 1u;
-        if (!mbar_wait(&bar[F_KEMPTY + st], ph ^ 1u, abort_flag, status, tmo)) { ok = false; break; }
-        mbar_arrive_expect_tx(&bar[F_KFULL + st], TILE);
-        load_tile<SUB>(smem_u32(sK + st * TILE), &p.mk, p.k_seq1, ck, b, j * kBlk, smem_u32(&bar[F_KFULL + st]));
-        dbar[1 + st] = &bar[F_KFULL + st]; dpar[1 + st] = ph; dis[1 + st] = true;
-        if (!mbar_wait(&bar[F_VEMPTY + st], ph ^ 1u, abort_flag, status, tmo)) { ok = false; break; }
-        mbar_arrive_expect_tx(&bar[F_VFULL + st], TILE);
-        load_tile<SUB>(smem_u32(sV + st * TILE), &p.mv, p.v_seq1, cv, b, j * kBlk, smem_u32(&bar[F_VFULL + st]));
-        dbar[3 + st] = &bar[F_VFULL + st]; dpar[3 + st] = ph; dis[3 + st] = true;
+      uint32_t used = 0, par = 0, nkv = 0, nq[2] = {0, 0};          // barriers with copies, parity of their last
+      auto load = [&](int full, uint32_t ph, uint8_t* dst, const CUtensorMap* map, int seq1, int col, int b, int s0) {
+        mbar_arrive_expect_tx(&bar[full], TILE);
+        load_tile<SUB>(smem_u32(dst), map, seq1, col, b, s0, smem_u32(&bar[full]));
+        used |= 1u << full;
+        par = (par & ~(1u << full)) | (ph << full);
+      };
+      auto wait = [&](int i, uint32_t ph) { return mbar_wait(&bar[i], ph, abort_flag, status, tmo); };
+      uint32_t n = 0;
+      for (int blk = (int)blockIdx.x; blk >= 0 && ok; blk = following(n++, false)) {
+        const FwdWork w = fwd_work(p, blk);
+        const int b = w.bh / p.H, h = w.bh % p.H;
+        const int cq = head_col(p.q, h), ck = head_col(p.k, h), cv = head_col(p.v, h);
+        auto load_q = [&](int t) {
+          const uint32_t ph = nq[t]++ & 1u;
+          if (!wait(F_QEMPTY + t, ph ^ 1u)) return false;
+          load(F_QFULL + t, ph, sQ + t * TILE, &p.mq, p.q_seq1, cq, b, (w.g0 + t) * kBlk);
+          return true;
+        };
+        ok = load_q(0);
+        for (int j = 0; j < w.nload && ok; ++j, ++nkv) {
+          const int st = nkv & 1;
+          const uint32_t ph = (nkv >> 1) & 1u;
+          if (!wait(F_KEMPTY + st, ph ^ 1u)) { ok = false; break; }
+          load(F_KFULL + st, ph, sK + st * TILE, &p.mk, p.k_seq1, ck, b, j * kBlk);
+          if (j == 0 && !split && w.n1 > 0 && !load_q(1)) { ok = false; break; }
+          if (!wait(F_VEMPTY + st, ph ^ 1u)) { ok = false; break; }
+          load(F_VFULL + st, ph, sV + st * TILE, &p.mv, p.v_seq1, cv, b, j * kBlk);
+        }
+        if (!ok) break;
+        mbar_arrive(&bar[F_TAKEN]);
       }
-      if (!ok || *abort_flag) drain_loads(dbar, dpar, dis, 5);
+      if (!ok || *abort_flag) drain_loads(bar, used, par);
     }
   } else if (warp == kMmaWarp) {
     // ---------------------------------------------------------------------------------- UMMA issuer
     if (elect_one()) {
       const uint32_t id_s = make_idesc_bf16(128, 128, 0, 0), id_o = make_idesc_bf16(128, HD, 0, 1);
-      const uint32_t aQ = smem_u32(sQ), aK = smem_u32(sK), aV = smem_u32(sV), aP = smem_u32(sP);
+      const uint32_t aQ = smem_u32(sQ), aK = smem_u32(sK), aV = smem_u32(sV);
       bool ok = true, issued = false;
-      auto issue_s = [&](int j) {
-        const uint32_t kb = aK + (j & 1) * TILE, d = tmem + (uint32_t)((j & 1) * 128);
-#pragma unroll
-        for (int u = 0; u < SUB; ++u)
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            umma_bf16(d, make_smem_desc(aQ + u * kSub + kk * 32, 16, 1024), make_smem_desc(kb + u * kSub + kk * 32, 16, 1024),
-                      id_s, (u | kk) ? 1u : 0u);
-        umma_commit(&bar[F_KEMPTY + (j & 1)]);
-        umma_commit(&bar[F_SFULL + (j & 1)]);
-      };
-      ok = mbar_wait(&bar[F_QFULL], 0, abort_flag, status, tmo);
-      if (ok && nkb > 0) ok = mbar_wait(&bar[F_KFULL], 0, abort_flag, status, tmo);
-      if (ok && nkb > 0) { tc_fence_after(); issue_s(0); issued = true; }
-      for (int j = 0; j < nkb && ok; ++j) {
-        if (j + 1 < nkb) {
-          const int n = j + 1, st = n & 1;
-          const uint32_t ph = (uint32_t)(n >> 1) & 1u;
-          if (!mbar_wait(&bar[F_KFULL + st], ph, abort_flag, status, tmo)) { ok = false; break; }
-          if (!mbar_wait(&bar[F_SEMPTY + st], ph ^ 1u, abort_flag, status, tmo)) { ok = false; break; }
-          tc_fence_after();
-          issue_s(n);
-        }
-        const int st = j & 1;
-        long long* tm = (p.trace && blockIdx.x == 0 && j < 16) ? p.trace + 256 + j * 8 : nullptr;
-        if (tm) tm[0] = clock64();                       // S of the next block issued
-        if (!mbar_wait(&bar[F_VFULL + st], (uint32_t)(j >> 1) & 1u, abort_flag, status, tmo)) { ok = false; break; }
-        if (tm) tm[1] = clock64();                       // V landed
-        if (!mbar_wait(&bar[F_PFULL], (uint32_t)j & 1u, abort_flag, status, tmo)) { ok = false; break; }
-        if (tm) tm[2] = clock64();                       // P written
+      auto wait = [&](int i, uint32_t ph) { return mbar_spin(&bar[i], ph, abort_flag, status, tmo); };
+      // S of tile t against the c-th block since the start, once that is there; `last`: no other tile needs the block
+      auto issue_s = [&](int t, uint32_t c, bool last, bool q_done) {
+        if (!wait(F_KFULL + (c & 1), (c >> 1) & 1u)) return false;
         tc_fence_after();
-        const uint32_t vb = aV + st * TILE;
+        umma_tiles<HD>(tmem + (uint32_t)(t * 128), aQ + (split ? 0 : t * TILE), aK + (c & 1) * TILE, id_s);
+        if (last) umma_commit(&bar[F_KEMPTY + (c & 1)]);
+        if (q_done) umma_commit(&bar[F_QEMPTY + t]);
+        umma_commit(&bar[F_SFULL + t]);
+        issued = true;
+        return true;
+      };
+      uint32_t n = 0, kv0 = 0, np[2] = {0, 0}, nq[2] = {0, 0};      // blocks before this work, P tiles and Q tiles so far
+      for (int blk = (int)blockIdx.x; blk >= 0 && ok; blk = following(n++, false)) {
+        const FwdWork w = fwd_work(p, blk);
+        const int n0 = w.n0, n1 = w.n1;
+        mbar_arrive(&bar[F_TAKEN]);
+        ok = wait(F_QFULL, nq[0]++ & 1u) && issue_s(0, kv0, split || n1 == 0, !split && n0 == 1);
+        if (ok && n1 > 0) {
+          if (!split) ok = wait(F_QFULL + 1, nq[1]++ & 1u);
+          ok = ok && issue_s(1, kv0 + (split ? 1 : 0), true, !split && n1 == 1);
+        }
+        const int nmax = max(n0, n1);
+        for (int i = 0; i < nmax && ok; ++i) {
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          umma_bf16(tmem + 256, make_smem_desc(aP + (kk >> 2) * kSub + (kk & 3) * 32, 16, 1024),
-                    make_smem_desc(vb + kk * 2048, kSub, 1024), id_o, (j > 0 || kk > 0) ? 1u : 0u);
-        umma_commit(&bar[F_VEMPTY + st]);
-        umma_commit(&bar[F_PVDONE]);
-        if (tm) tm[3] = clock64();                       // P V issued
+          for (int t = 0; t < 2; ++t) {
+            const int nt = t ? n1 : n0;
+            if (!ok || i >= nt) continue;
+            const uint32_t c = kv0 + (split ? 2 * i + t : i);
+            const int st = c & 1;
+            // the block's second tile releases it; a tile that is done no longer counts
+            const bool last = split || t == 1 || i >= n1;
+            const uint32_t pp = np[t]++ & 1u;
+            if (!wait(F_VFULL + st, (c >> 1) & 1u) || !wait(F_PFULL + t, pp)) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t vb = aV + st * TILE, pt = tmem + (uint32_t)(t * 128), d = tmem + (uint32_t)(256 + t * HD);
+#pragma unroll
+            for (int kk = 0; kk < 6; ++kk)
+              umma_bf16_ts(d, pt + kk * 8, make_smem_desc(vb + kk * 2048, kSub, 1024), id_o, (i > 0 || kk > 0) ? 1u : 0u);
+            if (!wait(F_PTAIL + t, pp)) { ok = false; break; }
+            tc_fence_after();
+#pragma unroll
+            for (int kk = 6; kk < 8; ++kk)
+              umma_bf16_ts(d, pt + kk * 8, make_smem_desc(vb + kk * 2048, kSub, 1024), id_o, 1u);
+            if (last) umma_commit(&bar[F_VEMPTY + st]);
+            if (i + 1 < nt) ok = issue_s(t, split ? c + 2 : c + 1, split || t == 1 || i + 1 >= n1, !split && i + 2 == nt);
+            else umma_commit(&bar[F_OFULL + t]);
+          }
+        }
+        kv0 += w.nload;
+        if (!ok) break;
       }
-      if (!ok && issued) drain_mma(&bar[F_DRAIN]);
+      if ((!ok || *abort_flag) && issued) drain_mma(&bar[F_DRAIN]);
     }
+  } else if (warp == kSchedWarp) {
+    if (MORE && elect_one()) schedule(ctl, &bar[F_WFULL], &bar[F_TAKEN], abort_flag, status, tmo);
+  }
   } else {
+    reg_alloc<kRowRegs>();
     // ---------------------------------------------------------------------------------- row threads
-    const int wg = warp >> 2, rt = tid & 127;          // column half and row of this thread
-    const int row = q0 + rt;
+    const int t = warp >> 2, rt = tid & 127;           // tile and row of this thread
     const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    const uint32_t aS = lane_addr + (uint32_t)(t * 128), aO = lane_addr + (uint32_t)(256 + t * HD);
     const unsigned long long offset = M.offset + (M.step_ptr ? __ldg(M.step_ptr) * 65536ull : 0ull);
-    constexpr int OC = HD / 64;                        // 32-column chunks of O per thread
-    float m_used = -INFINITY, l = 0.f;                  // l: this thread's half of the row sum
     bool ok = true;
-    // stamps of two row warps of CTA 0: [warp 0 | warp 4][block < 16][event < 8]
+    uint32_t ns = 0, no = 0, n = 0;                    // S tiles, O tiles, pieces of work so far
+    // stamps of the two tiles' first warps of CTA 0: [warp 0 | warp 4][step < 16][event < 8]
     long long* tr = (p.trace && blockIdx.x == 0 && lane == 0 && (warp & 3) == 0) ? p.trace + (warp >> 2) * 128 : nullptr;
-    for (int j = 0; j < nkb; ++j) {
-      const int buf = j & 1;
-      if (tr && j < 16) tr[j * 8 + 0] = clock64();
-      const int col0 = j * kBlk + wg * 64;
-      const uint32_t dead[2] = {dead_keys<MSK>(M, b, col0, lane), dead_keys<MSK>(M, b, col0 + 32, lane)};
-      uint32_t good = mbar_wait(&bar[F_SFULL + buf], (uint32_t)(j >> 1) & 1u, abort_flag, status, tmo) ? 1u : 0u;
+    for (int blk = (int)blockIdx.x; blk >= 0; blk = following(n++, true)) {
+    const FwdWork w = fwd_work(p, blk);
+    if (lane == 0) mbar_arrive(&bar[F_TAKEN]);
+    const int bh = w.bh, b = bh / p.H, h = bh % p.H, n1 = w.n1;
+    const int nt = t ? n1 : w.n0, gt = w.g0 + (split ? 0 : t);
+    const int row = gt * kBlk + rt;
+    float m_used = -INFINITY, l = 0.f;
+    for (int i = 0; i < nt; ++i, ++ns) {
+      const int c = split ? 2 * i + t : i, col0 = c * kBlk;
+      if (tr && ns < 16) tr[ns * 8 + 0] = clock64();
+      uint32_t dead[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) dead[q] = dead_keys<MSK>(M, b, col0 + 32 * q, lane);
+      const uint32_t good = mbar_wait(&bar[F_SFULL + t], ns & 1u, abort_flag, status, tmo) ? 1u : 0u;
       if (!__all_sync(0xffffffffu, good)) { ok = false; break; }
       tc_fence_after();
-      if (tr && j < 16) tr[j * 8 + 1] = clock64();
-      float s[64];
-#pragma unroll
-      for (int c = 0; c < 2; ++c) tmem_ld32f(lane_addr + (uint32_t)(buf * 128 + wg * 64 + c * 32), s + 32 * c);
-      tmem_ld_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bar[F_SEMPTY + buf]);
-      if (tr && j < 16) tr[j * 8 + 2] = clock64();
-      const bool plain = MSK == 0 && !(M.causal && j == qb) && (j * kBlk + kBlk <= M.Sk);
-      // a block that only needs the scale keeps the raw scores: the scale rides in the exponent's multiply-add
+      if (tr && ns < 16) tr[ns * 8 + 1] = clock64();
+      // A block that needs more than the scale is put right in TMEM first, 32 columns at a time, so that the loop below is one
+      // for all blocks; one that only needs the scale keeps the raw scores: the scale rides in the exponent's multiply-add.
+      const bool plain = MSK != 2 && !(dead[0] | dead[1] | dead[2] | dead[3]) && !(M.causal && c == gt) && (col0 + kBlk <= M.Sk);
       if (!plain) {
-#pragma unroll
-        for (int c = 0; c < 2; ++c) score_chunk<32, MSK>(s + 32 * c, row, col0 + 32 * c, dead[c], M, false);
+#pragma unroll 1
+        for (int q = 0; q < 4; ++q) {
+          float x[32];
+          tmem_ld32f(aS + (uint32_t)(q * 32), x);
+          tmem_ld_wait();
+          score_chunk<32, MSK>(x, row, col0 + 32 * q, q == 0 ? dead[0] : q == 1 ? dead[1] : q == 2 ? dead[2] : dead[3], M, false);
+          tmem_st32f(aS + (uint32_t)(q * 32), x);
+        }
+        tmem_st_wait();
       }
+      float s[128];
+      tmem_ld32f(aS, s);
+      tmem_ld32f(aS + 32, s + 32);
+      tmem_ld_wait();
+      tmem_ld32f(aS + 64, s + 64);
+      tmem_ld32f(aS + 96, s + 96);
       float mx = max64(s);
+      tmem_ld_wait();
+      mx = fmaxf(mx, max64(s + 64));
       if (plain) mx *= M.scale_log2;      // the scale is positive: the maximum commutes with it
-      // both threads of the row must scale with the same reference: exchange the partial maxima
-      bool xok = true;
-      mx = fmaxf(mx, xchg_row(xc, &bar[F_XCHG + (warp & 3)], wg, rt, (uint32_t)j, mx, abort_flag, status, tmo, xok));
-      if (!__all_sync(0xffffffffu, xok ? 1u : 0u)) { ok = false; break; }
-      if (tr && j < 16) tr[j * 8 + 3] = clock64();
       const float cand = fmaxf(m_used, mx);
       const bool need = cand > m_used + kRescaleGap;
       const float m_new = need ? cand : m_used;
       const float mref = (m_new == -INFINITY) ? 0.f : m_new;
       const float mul = plain ? M.scale_log2 : 1.f;
-      if (j > 0) {
-        // P V of the previous block must be complete before the P tile is overwritten and before O is rescaled (it was
-        // issued a whole block ago: this wait is almost always over at once)
-        good = mbar_wait(&bar[F_PVDONE], (uint32_t)(j - 1) & 1u, abort_flag, status, tmo) ? 1u : 0u;
-        if (!__all_sync(0xffffffffu, good)) { ok = false; break; }
-        tc_fence_after();
-        if (__any_sync(0xffffffffu, need)) {
-          const float alpha = need ? ex2_approx(m_used - cand) : 1.f;
+      if (i > 0 && __any_sync(0xffffffffu, need)) {
+        // the S that was waited for came after the P V of the tile's previous step: O is complete up to there
+        const float alpha = need ? ex2_approx(m_used - cand) : 1.f;
 #pragma unroll
-          for (int c = 0; c < OC; ++c) {
-            float o[32];
-            tmem_ld32f(lane_addr + (uint32_t)(256 + (wg * OC + c) * 32), o);
-            tmem_ld_wait();
+        for (int q = 0; q < HD / 32; ++q) {
+          float o[32];
+          tmem_ld32f(aO + (uint32_t)(q * 32), o);
+          tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] *= alpha;
-            tmem_st32f(lane_addr + (uint32_t)(256 + (wg * OC + c) * 32), o);
+          for (int e = 0; e < 32; ++e) o[e] *= alpha;
+          tmem_st32f(aO + (uint32_t)(q * 32), o);
+        }
+        l *= alpha;
+      }
+      float2 ra = make_float2(0.f, 0.f), rb = ra;
+      const float2 mul2 = make_float2(mul, mul), ref2 = make_float2(-mref, -mref);
+      // some: one exponential in four by polynomial (blocks without masked scores, which have to become 0)
+      auto exponentials = [&](auto some) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        float* e = s + 32 * q;
+        uint32_t pk[16];
+        [[maybe_unused]] uint32_t keep = 0xffffffffu;
+        if constexpr (DRP) keep = keep_bits<32>(M, offset, bh, min(row, M.Sq - 1), col0 + 32 * q);
+#pragma unroll
+        for (int k = 0; k < 32; k += 4) {
+          float2 x = fma2(make_float2(e[k], e[k + 1]), mul2, ref2), y = fma2(make_float2(e[k + 2], e[k + 3]), mul2, ref2);
+          x = make_float2(ex2_approx(x.x), ex2_approx(x.y));
+          if (decltype(some)::value && (k & 4)) y = ex2_poly2(y);
+          else y = make_float2(ex2_approx(y.x), ex2_approx(y.y));
+          ra = add2(ra, x);
+          rb = add2(rb, y);
+          if constexpr (DRP) {
+            x.x = ((keep >> k) & 1u) ? x.x * M.drop_scale : 0.f;
+            x.y = ((keep >> (k + 1)) & 1u) ? x.y * M.drop_scale : 0.f;
+            y.x = ((keep >> (k + 2)) & 1u) ? y.x * M.drop_scale : 0.f;
+            y.y = ((keep >> (k + 3)) & 1u) ? y.y * M.drop_scale : 0.f;
           }
+          pk[k / 2] = pack_bf16(x.x, x.y);
+          pk[k / 2 + 1] = pack_bf16(y.x, y.y);
+        }
+        tmem_st16(aS + (uint32_t)(q * 16), pk);
+        if (q >= 2) {          // three quarters of P: their products run under the exponentials of the last
           tmem_st_wait();
-          l *= alpha;
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bar[(q == 2 ? F_PFULL : F_PTAIL) + t]);
         }
       }
-      if (tr && j < 16) tr[j * 8 + 4] = clock64();
-      // exponentials and the stores of P, eight columns at a time: the stores of one group issue while the special-
-      // function unit works on the next (the 64 ex2 of a thread are what bounds this loop)
-      float r0 = 0.f, r1 = 0.f, r2 = 0.f, r3 = 0.f;
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        float* e = s + 8 * c;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) e[i] = ex2_approx(fmaf(e[i], mul, -mref));
-        r0 += e[0] + e[4]; r1 += e[1] + e[5]; r2 += e[2] + e[6]; r3 += e[3] + e[7];
-        if constexpr (DRP) {
-          const uint32_t keep = keep_bits<8>(M, offset, bh, min(row, M.Sq - 1), col0 + 8 * c);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) e[i] = ((keep >> i) & 1u) ? e[i] * M.drop_scale : 0.f;
-        }
-        *reinterpret_cast<uint4*>(sP + wg * kSub + sw128(rt, c)) = pack8f(e);
-      }
+      };
+      if (!DRP && plain) exponentials(std::true_type{}); else exponentials(std::false_type{});
       m_used = m_new;
-      l += (r0 + r1) + (r2 + r3);
-      if (tr && j < 16) tr[j * 8 + 5] = clock64();
-      if (tr && j < 16) tr[j * 8 + 6] = clock64();
-      fence_proxy_async_smem();
-      tc_fence_before();
-      mbar_arrive(&bar[F_PFULL]);
-      if (tr && j < 16) tr[j * 8 + 7] = clock64();
+      l += (ra.x + ra.y) + (rb.x + rb.y);
+      if (tr && ns < 16) tr[ns * 8 + 2] = clock64();
     }
-    if (ok && nkb > 0) {
-      uint32_t good = mbar_wait(&bar[F_PVDONE], (uint32_t)(nkb - 1) & 1u, abort_flag, status, tmo) ? 1u : 0u;
+    if (ok && nt > 0) {
+      const uint32_t good = mbar_wait(&bar[F_OFULL + t], no++ & 1u, abort_flag, status, tmo) ? 1u : 0u;
       if (!__all_sync(0xffffffffu, good)) ok = false;
     }
-    if (ok) {
-      bool xok = true;
-      const float l_all = l + xchg_row(xc, &bar[F_XCHG + (warp & 3)], wg, rt, (uint32_t)nkb, l, abort_flag, status, tmo, xok);
-      if (!__all_sync(0xffffffffu, xok ? 1u : 0u)) ok = false;
+    tc_fence_after();
+    const bool merge = split && n1 > 0;
+    constexpr int OC = HD / 64;                        // 32-column chunks of half a row
+    float a_own = 1.f, a_other = 0.f;
+    if (merge) {
+      // Each thread of a row finishes half of its columns: it hands the other half, its maximum and its sum to the other
+      // tile's thread.  The products have read K (every S was issued before the last P V), so its stages hold the floats.
+      float* xo = reinterpret_cast<float*>(sK) + t * (HD / 2) * 128;
       if (ok) {
-        tc_fence_after();
-        const float inv = l_all > 0.f ? 1.f / l_all : 0.f;
-        __nv_bfloat16* dst = row < M.Sq ? row_ptr(p.o, b, row, h) : nullptr;
 #pragma unroll
-        for (int c = 0; c < OC; ++c) {
-          const int cc = wg * OC + c;
+        for (int q = 0; q < OC; ++q) {
           float o[32];
-          if (nkb > 0) {
-            tmem_ld32f(lane_addr + (uint32_t)(256 + cc * 32), o);
-            tmem_ld_wait();
+          tmem_ld32f(aO + (uint32_t)((t ^ 1) * (HD / 2) + q * 32), o);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 32; ++e) xo[(q * 32 + e) * 128 + rt] = o[e];
+        }
+        sX[t * 256 + rt] = m_used;
+        sX[t * 256 + 128 + rt] = l;
+      }
+      asm volatile("bar.sync 1, 256;" ::: "memory");   // all row threads come here, whether their waits ran out or not
+      const float m_o = sX[(t ^ 1) * 256 + rt], l_o = sX[(t ^ 1) * 256 + 128 + rt];
+      const float m_all = fmaxf(m_used, m_o);
+      a_own = m_used == -INFINITY ? 0.f : ex2_approx(m_used - m_all);
+      a_other = m_o == -INFINITY ? 0.f : ex2_approx(m_o - m_all);
+      l = l * a_own + l_o * a_other;
+      m_used = m_all;
+    }
+    if (ok && nt > 0) {
+      const float inv = l > 0.f ? 1.f / l : 0.f;
+      const float* xi = reinterpret_cast<const float*>(sK) + (t ^ 1) * (HD / 2) * 128;
+      const int r0 = gt * kBlk + (warp & 3) * 32;      // the warp's first row
+      __nv_bfloat16* dst = row_ptr(p.o, b, r0, h);
+      const int c0 = merge ? t * OC : 0, c1 = merge ? c0 + OC : 2 * OC;
+      for (int q = c0; q < c1; ++q) {
+        float o[32];
+        tmem_ld32f(aO + (uint32_t)(q * 32), o);
+        tmem_ld_wait();
+        if (merge) {
+#pragma unroll
+          for (int e = 0; e < 32; ++e) o[e] = o[e] * a_own + xi[((q - c0) * 32 + e) * 128 + rt] * a_other;
+        }
+#pragma unroll
+        for (int e = 0; e < 32; ++e) o[e] *= inv;
+        store_rows32(dst + q * 32, p.o.ss, M.Sq - r0, o, lane);
+      }
+      if (row < M.Sq && p.lse && !(merge && t)) {
+        const float mref = (m_used == -INFINITY) ? 0.f : m_used;
+        p.lse[(long long)bh * M.Sq + row] = l > 0.f ? mref + log2f(l) : INFINITY;
+      }
+      tc_fence_before();               // O has been read before the next P is announced
+    }
+    if (!ok) break;
+    }
+  }
+  teardown_cta(tmem, warp);
+}
+
+// =====================================================================================================  backward
+// delta[b, h, q] = rowsum(dO * O), HD / 8 lanes a row.  Reads both once (8192 tokens x 16 heads of 128: 67 MB), apart from the
+// launch below so that its two kinds of CTAs need nothing of each other.
+template <int HD>
+__global__ void __launch_bounds__(256) flash_delta_kernel(DRef o, DRef g, float* __restrict__ delta, int Sq, int H, long long rows) {
+  pdl_prologue();
+  constexpr int LPR = HD / 8;
+  const long long r = (blockIdx.x * 256ll + threadIdx.x) / LPR;
+  const int c = threadIdx.x % LPR;
+  float s = 0.f;
+  const long long bs = r / H;                                // rows in memory order: (batch, position, head)
+  const int h = (int)(r % H), b = (int)(bs / Sq), q = (int)(bs % Sq);
+  if (r < rows) {
+    const uint4 x = __ldg(reinterpret_cast<const uint4*>(row_ptr(o, b, q, h)) + c);
+    const uint4 y = __ldg(reinterpret_cast<const uint4*>(row_ptr(g, b, q, h)) + c);
+    s = bf16_lo(x.x) * bf16_lo(y.x) + bf16_hi(x.x) * bf16_hi(y.x) + bf16_lo(x.y) * bf16_lo(y.y) + bf16_hi(x.y) * bf16_hi(y.y) +
+        bf16_lo(x.z) * bf16_lo(y.z) + bf16_hi(x.z) * bf16_hi(y.z) + bf16_lo(x.w) * bf16_lo(y.w) + bf16_hi(x.w) * bf16_hi(y.w);
+  }
+#pragma unroll
+  for (int d = LPR / 2; d; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+  if (r < rows && c == 0) delta[((long long)b * H + h) * Sq + q] = s;
+}
+
+// Two kinds of work share one launch, the heaviest of each kind first: together they fill the SMs where either alone would
+// leave some idle, and neither has a tail of its own.  The row threads (two a row, 64 of the 128 columns each) make P and then
+// dS of a block; the products of one run under the other: while the rows work on dS(i) the tensor cores do dV(i) and S(i + 1),
+// while they work on P(i + 1) dK(i) and dP(i + 1).  P and dS go back into the TMEM columns of S and dP as bf16 A operands: in
+// shared memory, 64 columns a step, a block took 4 800 clocks in each of the two kernels there were, now 2 080 (dQ) and 3 100.
+//
+// dK / dV of 128 keys (rows of every product are KEYS), queries walked in blocks of 128, two stages of Q and dO:
+//   S^T = K Q^T, dP^T = V dO^T  ->  P^T, dS^T  ->  dV += P^T dO, dK += dS^T Q
+// dQ of 128 queries, keys walked in blocks of 128, three stages of K (dQ(i) still reads one while S(i + 2) needs another) and two of
+// V, S double-buffered:
+//   S = Q K^T, dP = dO V^T  ->  dS = P (dP - delta)  ->  dQ += dS K
+//
+// Shared memory is seven tiles, each with a "full" and an "empty" barrier of its own, whatever it holds: what follows is copied
+// into a tile as soon as its last product is done, also across pieces of work.
+//   dK / dV:  0 K   1 V   2, 3 Q   4, 5 dO            dQ:  0 Q   1 dO   2, 3, 4 K   5, 6 V
+// TMEM: S 0, dP 128; dK / dV: dV 256, dK 256 + HD; dQ: dQ 256, second S 384.
+// Barriers: tile t full t, empty 7 + t; the statistics of a block of queries (-log-sum-exp, -delta: the producer warp) beside
+// its Q tile; accumulators complete, and read out.
+enum { B_FULL = 0, B_EMPTY = 7, B_STAT = 14 /* 2 */, B_SFULL = 16 /* 2 */, B_PFULL = 18, B_DPFULL = 19, B_DSFULL = 20, B_ACC = 21,
+       B_ACCREAD = 22, B_WFULL = 23, B_TAKEN = 24, B_DRAIN = 25 };
+
+// What blockIdx.x stands for: the key block kb, or (kb < 0) the query block qb, of a (batch, head).
+struct BwdWork {
+  int kb, qb, bh;
+};
+__device__ __forceinline__ BwdWork bwd_work(const FlashParams& p, int blk) {
+  const int nq = (p.m.Sq + kBlk - 1) / kBlk, nk = (p.m.Sk + kBlk - 1) / kBlk, BH = p.B * p.H, both = min(nq, nk);
+  // a group of heads: levels of a key block and a query block of each, the longest first (causal: first keys, last queries), then
+  // what one kind has more
+  const int grp = blk / (p.group * (nq + nk)) * p.group, heads = min(p.group, BH - grp);
+  const int r = blk - grp * (nq + nk), level = r / (2 * heads);
+  BwdWork w = {-1, -1, grp + r % heads};
+  if (level < both) { if (r % (2 * heads) < heads) w.kb = level; else w.qb = nq - 1 - level; }
+  else {
+    const int i = (r - 2 * heads * both) / heads;
+    if (nk > nq) w.kb = both + i; else w.qb = nq - 1 - both - i;
+  }
+  return w;
+}
+
+constexpr int kBwdSlack = 768;          // all that a CTA's shared memory leaves for the alignment of the tiles (its base has it)
+
+template <int HD, int MSK, bool DRP, bool MORE>
+__global__ void __launch_bounds__(kThreads, 1) flash_bwd_kernel(const __grid_constant__ FlashParams p) {
+  constexpr int TILE = (HD / 64) * kSub;
+  extern __shared__ __align__(1024) uint8_t smem_tiles[];
+  uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_tiles) + 1023) & ~uintptr_t(1023));
+  if (sm - smem_tiles > kBwdSlack) {
+    if (threadIdx.x == 0) atomicCAS(p.status, (unsigned long long)ST_OK, (unsigned long long)ST_BAD_ARGUMENT);
+    return;
+  }
+  Ctl* ctl = reinterpret_cast<Ctl*>(sm + 7 * TILE);
+  float* sStat = reinterpret_cast<float*>(sm + 7 * TILE + 256);     // two stages of 128 x -log-sum-exp, 128 x -delta
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const MaskArgs& M = p.m;
+  const int nqb = (M.Sq + kBlk - 1) / kBlk, nkb = (M.Sk + kBlk - 1) / kBlk;
+  // counts by barrier index: copies and commits 1; statistics 32 (lanes); P and dS, accumulators read 8 (one per row warp); next work
+  // 1 and 10 (producer, issuer, eight row warps)
+  const int counts[26] = {1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 32, 32, 1, 1, 8, 1, 8, 1, 8, 1, 10, 1};
+  const uint32_t tmem = setup_cta(ctl, counts, 26, warp, lane);
+  volatile uint32_t* abort_flag = &ctl->abort_flag;
+  unsigned long long* status = p.status;
+  const unsigned long long tmo = p.timeout_ns;
+  uint64_t* bar = ctl->bar;
+  const uint32_t tS = tmem, tP = tmem + 128, tAcc = tmem + 256;
+  auto following = [&](uint32_t n, bool whole_warp) {
+    return MORE ? next_work(ctl, &bar[B_WFULL], n, whole_warp, abort_flag, status, tmo) : -1;
+  };
+
+  if (warp >= kProducerWarp) {
+  reg_dealloc<kAuxRegs>();
+  if (warp == kProducerWarp) {
+    // ---------------------------------------------------------------------------------- TMA producer
+    // the whole warp goes through the work: lane 0 issues the copies, every lane fetches the statistics of four queries
+    bool ok = true;
+    uint32_t uses = 0, copied = 0, n = 0;               // per tile: parity of its next use; copies issued
+    auto load = [&](int t, const CUtensorMap* map, int seq1, int col, int b, int s0) {
+      const uint32_t ph = (uses >> t) & 1u;
+      if (!warp_wait(&bar[B_EMPTY + t], ph ^ 1u, abort_flag, status, tmo)) return false;
+      if (lane == 0) {
+        mbar_arrive_expect_tx(&bar[B_FULL + t], TILE);
+        load_tile<HD / 64>(smem_u32(sm + t * TILE), map, seq1, col, b, s0, smem_u32(&bar[B_FULL + t]));
+      }
+      uses ^= 1u << t;
+      copied |= 1u << t;
+      return true;
+    };
+    for (int blk = (int)blockIdx.x; blk >= 0 && ok; blk = following(n++, true)) {
+      const BwdWork w = bwd_work(p, blk);
+      const int b = w.bh / p.H, h = w.bh % p.H;
+      const int cq = head_col(p.q, h), ck = head_col(p.k, h), cv = head_col(p.v, h), cg = head_col(p.dout, h);
+      if (w.kb >= 0) {
+        const long long base = (long long)w.bh * M.Sq;
+        const int i0 = M.causal ? w.kb : 0;
+        ok = load(0, &p.mk, p.k_seq1, ck, b, w.kb * kBlk);
+        for (int i = i0; i < nqb && ok; ++i) {
+          const int st = (i - i0) & 1, q0 = i * kBlk;
+          ok = load(2 + st, &p.mq, p.q_seq1, cq, b, q0);
+          if (!ok) break;
+          if (i == i0) ok = load(1, &p.mv, p.v_seq1, cv, b, w.kb * kBlk);
+          ok = ok && load(4 + st, &p.mdo, p.do_seq1, cg, b, q0);
+          float* stat = sStat + st * 2 * kBlk;          // free with its Q tile: dK read that after the rows had read these
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int q = q0 + e * 32 + lane;
+            stat[e * 32 + lane] = q < M.Sq ? -__ldg(p.lse + base + q) : -INFINITY;
+            stat[kBlk + e * 32 + lane] = q < M.Sq ? -__ldg(p.delta + base + q) : 0.f;
+          }
+          mbar_arrive(&bar[B_STAT + st]);
+        }
+      } else {
+        const int nb = M.causal ? min(nkb, w.qb + 1) : nkb;
+        ok = load(0, &p.mq, p.q_seq1, cq, b, w.qb * kBlk);
+        for (int j = 0; j < nb && ok; ++j) {
+          ok = load(2 + j % 3, &p.mk, p.k_seq1, ck, b, j * kBlk);
+          if (ok && j == 0) ok = load(1, &p.mdo, p.do_seq1, cg, b, w.qb * kBlk);
+          ok = ok && load(5 + (j & 1), &p.mv, p.v_seq1, cv, b, j * kBlk);
+        }
+      }
+      if (!ok) break;
+      if (lane == 0) mbar_arrive(&bar[B_TAKEN]);
+    }
+    if (lane == 0 && (!ok || *abort_flag)) drain_loads(bar + B_FULL, copied, ~uses);
+  } else if (warp == kMmaWarp) {
+    // ---------------------------------------------------------------------------------- UMMA issuer
+    if (elect_one()) {
+      const uint32_t id_s = make_idesc_bf16(128, 128, 0, 0), id_t = make_idesc_bf16(128, HD, 0, 1);
+      const uint32_t a0 = smem_u32(sm);
+      bool ok = true, issued = false;
+      uint32_t uses = 0, np = 0, nds = 0, n = 0;        // per tile: parity of its next use; P, dS and pieces of work so far
+      auto wait = [&](int i, uint32_t ph) { return mbar_spin(&bar[i], ph, abort_flag, status, tmo); };
+      auto tile = [&](int t) {
+        const bool got = wait(B_FULL + t, (uses >> t) & 1u);
+        uses ^= 1u << t;
+        return got;
+      };
+      auto at = [&](int t) { return a0 + (uint32_t)(t * TILE); };
+      auto done_with = [&](int t) { umma_commit(&bar[B_EMPTY + t]); };
+      // S or dP = tile a x tile b, the second of which has to be waited for; tiles that are read for the last time are released
+      auto product = [&](uint32_t d, int a, int bt, int sig, bool last_a, bool last_b) {
+        if (!tile(bt)) return false;
+        tc_fence_after();
+        umma_tiles<HD>(d, at(a), at(bt), id_s);
+        if (last_a) done_with(a);
+        if (last_b) done_with(bt);
+        umma_commit(&bar[sig]);
+        issued = true;
+        return true;
+      };
+      for (int blk = (int)blockIdx.x; blk >= 0 && ok; blk = following(n++, false)) {
+        const BwdWork w = bwd_work(p, blk);
+        mbar_arrive(&bar[B_TAKEN]);
+        const uint32_t read = (n & 1u) ^ 1u;            // the accumulators of the work before have been read out
+        if (w.kb >= 0) {
+          const int nit = nqb - (M.causal ? w.kb : 0);
+          ok = tile(0) && product(tS, 0, 2, B_SFULL, nit == 1, false) && tile(1) && product(tP, 1, 4, B_DPFULL, nit == 1, false) &&
+               wait(B_ACCREAD, read);
+          for (int it = 0; it < nit && ok; ++it) {
+            const int st = it & 1, ot = st ^ 1;
+            const bool more = it + 1 < nit, end = it + 2 == nit;
+            if (!wait(B_PFULL, np++ & 1u)) { ok = false; break; }
+            tc_fence_after();
+            umma_rows(tAcc, tS, at(4 + st), id_t, it > 0);
+            done_with(4 + st);
+            if (more && !product(tS, 0, 2 + ot, B_SFULL, end, false)) { ok = false; break; }
+            if (!wait(B_DSFULL, nds++ & 1u)) { ok = false; break; }
+            tc_fence_after();
+            umma_rows(tAcc + HD, tP, at(2 + st), id_t, it > 0);
+            done_with(2 + st);
+            if (more) ok = product(tP, 1, 4 + ot, B_DPFULL, end, false);
+            else umma_commit(&bar[B_ACC]);
+          }
+        } else {
+          const int nb = M.causal ? min(nkb, w.qb + 1) : nkb;
+          auto issue_s = [&](int j) {
+            return product(j & 1 ? tmem + 384 : tS, 0, 2 + j % 3, B_SFULL + (j & 1), j + 1 == nb, false);
+          };
+          auto issue_dp = [&](int j) { return product(tP, 1, 5 + (j & 1), B_DPFULL, j + 1 == nb, true); };
+          ok = tile(0) && issue_s(0) && tile(1) && issue_dp(0) && wait(B_ACCREAD, read) && (nb < 2 || issue_s(1));
+          for (int j = 0; j < nb && ok; ++j) {
+            if (!wait(B_DSFULL, nds++ & 1u)) { ok = false; break; }
+            tc_fence_after();
+            umma_rows(tAcc, tP, at(2 + j % 3), id_t, j > 0);
+            done_with(2 + j % 3);
+            if (j + 1 == nb) umma_commit(&bar[B_ACC]);
+            else ok = issue_dp(j + 1) && (j + 2 >= nb || issue_s(j + 2));
+          }
+        }
+        if (!ok) break;
+      }
+      if ((!ok || *abort_flag) && issued) drain_mma(&bar[B_DRAIN]);
+    }
+  } else if (warp == kSchedWarp) {
+    if (MORE && elect_one()) schedule(ctl, &bar[B_WFULL], &bar[B_TAKEN], abort_flag, status, tmo);
+  }
+  } else {
+    reg_alloc<kRowRegs>();
+    // ---------------------------------------------------------------------------------- row threads
+    const int wg = warp >> 2, rt = (warp & 3) * 32 + lane;       // column half and row of this thread
+    const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
+    const uint32_t aP = tP + lane_off + (uint32_t)(wg * 64);
+    const unsigned long long offset = M.offset + (M.step_ptr ? __ldg(M.step_ptr) * 65536ull : 0ull);
+    const float2 sc = make_float2(M.scale_log2, M.scale_log2);
+    bool ok = true;
+    uint32_t n = 0, ns = 0, ndp = 0, nst = 0;                    // pieces of work, S per buffer (bits), dP, statistics per stage (bits)
+    auto wait = [&](int i, uint32_t ph) { return warp_wait(&bar[i], ph, abort_flag, status, tmo); };
+    long long* tr = (p.trace && blockIdx.x == 0 && lane == 0 && (warp & 3) == 0) ? p.trace + (warp >> 2) * 128 : nullptr;
+    for (int blk = (int)blockIdx.x; blk >= 0 && ok; blk = following(n++, true)) {
+      const BwdWork w = bwd_work(p, blk);
+      if (lane == 0) mbar_arrive(&bar[B_TAKEN]);
+      const int bh = w.bh, b = bh / p.H, h = bh % p.H;
+      if (w.kb >= 0) {
+        const int k0 = w.kb * kBlk, i0 = M.causal ? w.kb : 0, nit = nqb - i0;
+        const uint32_t aS = tS + lane_off + (uint32_t)(wg * 64);
+        const int key = k0 + rt;
+        bool key_dead = key >= M.Sk;
+        if constexpr (MSK != 0) key_dead = key_dead || (M.kpm && __ldg(M.kpm + (long long)b * M.kpm_ld + key));
+        const bool keys_plain = MSK != 2 && !__any_sync(0xffffffffu, key_dead);
+        for (int it = 0; it < nit; ++it) {
+          const int st = it & 1;
+          const int qbase = (i0 + it) * kBlk + wg * 64;          // first query of this thread
+          const float* nlse = sStat + st * 2 * kBlk + wg * 64;
+          const float* ndel = nlse + kBlk;
+          // Dropout bits.  One generator call covers four neighbouring keys, which sit in four neighbouring lanes: each lane
+          // calls it for every fourth query and the four exchange their nibbles.
+          uint32_t kw[2][4] = {};                                // kw[c][e]: nibble g = keys of the quad, query 32 c + 4 g + e
+          if constexpr (DRP) {
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+              uint32_t mine = 0;
+#pragma unroll
+              for (int g = 0; g < 8; ++g) {
+                const int q = min(qbase + 32 * c + 4 * g + (lane & 3), M.Sq - 1);
+                const unsigned long long idx = ((unsigned long long)bh * M.Sq + q) * (unsigned long long)M.Sk + (key & ~3);
+                const uint4 r = philox4x32(M.seed, offset, idx >> 2);
+                mine |= ((r.x >= M.thresh ? 1u : 0u) | (r.y >= M.thresh ? 2u : 0u) | (r.z >= M.thresh ? 4u : 0u) |
+                         (r.w >= M.thresh ? 8u : 0u)) << (4 * g);
+              }
+#pragma unroll
+              for (int e = 0; e < 4; ++e) kw[c][e] = __shfl_sync(0xffffffffu, mine, (lane & ~3) + e) >> (lane & 3);
+            }
+          }
+          if (tr && it < 16) tr[it * 8] = clock64();
+          if (!wait(B_STAT + st, (nst >> st) & 1u)) { ok = false; break; }
+          nst ^= 1u << st;
+          float nl[64];                                          // read before S is there: the tensor cores keep shared memory busy
+#pragma unroll
+          for (int i = 0; i < 64; i += 4) *reinterpret_cast<float4*>(nl + i) = *reinterpret_cast<const float4*>(nlse + i);
+          if (!wait(B_SFULL, ns & 1u)) { ok = false; break; }
+          ns ^= 1u;
+          tc_fence_after();
+          if (tr && it < 16) tr[it * 8 + 1] = clock64();
+          float x[64];
+          tmem_ld32f(aS, x);
+          tmem_ld32f(aS + 32, x + 32);
+          tmem_ld_wait();
+          if (keys_plain && !(M.causal && it == 0)) {            // the diagonal crosses a causal key block's first query block
+#pragma unroll
+            for (int i = 0; i < 64; i += 2) {
+              const float2 u = fma2(make_float2(x[i], x[i + 1]), sc, make_float2(nl[i], nl[i + 1]));
+              x[i] = u.x; x[i + 1] = u.y;
+            }
           } else {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = 0.f;
-          }
-#pragma unroll
-          for (int i = 0; i < 32; ++i) o[i] *= inv;
-          if (dst) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) *reinterpret_cast<uint4*>(dst + cc * 32 + q * 8) = pack8f(o + 8 * q);
-          }
-        }
-        if (wg == 0 && row < M.Sq && p.lse) {
-          const float mref = (m_used == -INFINITY) ? 0.f : m_used;
-          p.lse[(long long)bh * M.Sq + row] = l_all > 0.f ? mref + log2f(l_all) : INFINITY;
-        }
-      }
-    }
-  }
-  teardown_cta(tmem, warp);
-}
-
-// =====================================================================================================  dQ
-// CTA = 128 queries of one (batch, head); the keys are walked in sub-blocks of 64, three stages of K / V deep:
-//   S = Q K^T and dP = dO V^T      [128 queries x 64 keys] each, in TMEM, double-buffered
-//   row threads (TMEM lane = query, two threads per query with 32 keys each): dS = P (dP - delta) as bf16 into a
-//                                  [128 x 64] K-major shared tile
-//   dQ += dS K                     contraction over the 64 keys; B = the K stage read MN-major
-// The products of sub-block i+1 run while the row threads work on sub-block i.
-enum { Q_QFULL = 0, Q_KVFULL = 1 /* 3 stages */, Q_KVEMPTY = 4 /* 3 stages */, Q_SDPFULL = 7 /* 2 */, Q_SDPEMPTY = 9 /* 2 */,
-       Q_DSFULL = 11, Q_DSEMPTY = 12, Q_DONE = 13, Q_DRAIN = 14 };
-
-template <int HD, int MSK, bool DRP>
-__global__ void __launch_bounds__(kThreads, 1) flash_dq_kernel(const __grid_constant__ FlashParams p) {
-  constexpr int SUB = HD / 64;
-  constexpr int TILE = SUB * kSub;          // Q or dO: 128 rows
-  constexpr int KT = SUB * kHalfTile;       // one stage of K or V: 64 rows
-  constexpr int NS = kBwdStages;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sQ = sm;
-  uint8_t* sG = sQ + TILE;            // dO
-  uint8_t* sK = sG + TILE;            // NS stages
-  uint8_t* sV = sK + NS * KT;         // NS stages
-  uint8_t* sS = sV + NS * KT;         // dS [128 queries x 64 keys] bf16
-  Ctl* ctl = reinterpret_cast<Ctl*>(sS + kSub);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const MaskArgs& M = p.m;
-  const int nqb = (M.Sq + kBlk - 1) / kBlk;
-  const int BH = p.B * p.H;
-  const int qb = nqb - 1 - (int)(blockIdx.x / BH);
-  const int bh = (int)(blockIdx.x % BH);
-  const int b = bh / p.H, h = bh % p.H;
-  const int q0 = qb * kBlk;
-  int nsb = (M.Sk + kHalf - 1) / kHalf;                 // key sub-blocks
-  if (M.causal) nsb = min(nsb, 2 * (qb + 1));
-  // counts by barrier index: Q/dO full 1; K/V stage full and empty 1; S/dP full 1, S/dP empty 8 (one per row warp);
-  // dS full 256; the rest 1
-  const int counts[15] = {1, 1, 1, 1, 1, 1, 1, 1, 1, 8, 8, kRowThreads, 1, 1, 1};
-  const uint32_t tmem = setup_cta(ctl, counts, 15, warp, lane);
-  volatile uint32_t* abort_flag = &ctl->abort_flag;
-  unsigned long long* status = p.status;
-  const unsigned long long tmo = p.timeout_ns;
-  uint64_t* bar = ctl->bar;
-
-  if (warp == kProducerWarp) {
-    if (elect_one()) {
-      const int cq = head_col(p.q, h), ck = head_col(p.k, h), cv = head_col(p.v, h), cg = head_col(p.dout, h);
-      bool ok = true;
-      uint64_t* dbar[1 + NS]; uint32_t dpar[1 + NS]; bool dis[1 + NS];
-      for (int i = 0; i < 1 + NS; ++i) dis[i] = false;
-      mbar_arrive_expect_tx(&bar[Q_QFULL], 2 * TILE);
-      load_tile<SUB>(smem_u32(sQ), &p.mq, p.q_seq1, cq, b, q0, smem_u32(&bar[Q_QFULL]));
-      load_tile<SUB>(smem_u32(sG), &p.mdo, p.do_seq1, cg, b, q0, smem_u32(&bar[Q_QFULL]));
-      dbar[0] = &bar[Q_QFULL]; dpar[0] = 0; dis[0] = true;
-      for (int j = 0; j < nsb && ok; ++j) {
-        const int st = j % NS;
-        const uint32_t ph = (uint32_t)(j / NS) & 1u;
-        if (!mbar_wait(&bar[Q_KVEMPTY + st], ph ^ 1u, abort_flag, status, tmo)) { ok = false; break; }
-        mbar_arrive_expect_tx(&bar[Q_KVFULL + st], 2 * KT);
-        load_tile64<SUB>(smem_u32(sK + st * KT), &p.mk64, p.k_seq1, ck, b, j * kHalf, smem_u32(&bar[Q_KVFULL + st]));
-        load_tile64<SUB>(smem_u32(sV + st * KT), &p.mv64, p.v_seq1, cv, b, j * kHalf, smem_u32(&bar[Q_KVFULL + st]));
-        dbar[1 + st] = &bar[Q_KVFULL + st]; dpar[1 + st] = ph; dis[1 + st] = true;
-      }
-      if (!ok || *abort_flag) drain_loads(dbar, dpar, dis, 1 + NS);
-    }
-  } else if (warp == kMmaWarp) {
-    if (elect_one()) {
-      const uint32_t id_s = make_idesc_bf16(128, kHalf, 0, 0), id_q = make_idesc_bf16(128, HD, 0, 1);
-      const uint32_t aQ = smem_u32(sQ), aG = smem_u32(sG), aK = smem_u32(sK), aV = smem_u32(sV), aS = smem_u32(sS);
-      bool ok = mbar_wait(&bar[Q_QFULL], 0, abort_flag, status, tmo);
-      bool issued = false;
-      // S = Q K^T (columns 0..63 of the buffer), dP = dO V^T (columns 64..127)
-      auto issue_sdp = [&](int n) {
-        const uint32_t ks = aK + (n % NS) * KT, vs = aV + (n % NS) * KT, d = tmem + (uint32_t)((n & 1) * 128);
-#pragma unroll
-        for (int u = 0; u < SUB; ++u)
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            umma_bf16(d, make_smem_desc(aQ + u * kSub + kk * 32, 16, 1024), make_smem_desc(ks + u * kHalfTile + kk * 32, 16, 1024),
-                      id_s, (u | kk) ? 1u : 0u);
-#pragma unroll
-        for (int u = 0; u < SUB; ++u)
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            umma_bf16(d + 64, make_smem_desc(aG + u * kSub + kk * 32, 16, 1024),
-                      make_smem_desc(vs + u * kHalfTile + kk * 32, 16, 1024), id_s, (u | kk) ? 1u : 0u);
-        umma_commit(&bar[Q_SDPFULL + (n & 1)]);
-      };
-      if (ok && nsb > 0) ok = mbar_wait(&bar[Q_KVFULL], 0, abort_flag, status, tmo);
-      if (ok && nsb > 0) { tc_fence_after(); issue_sdp(0); issued = true; }
-      for (int j = 0; j < nsb && ok; ++j) {
-        if (j + 1 < nsb) {
-          const int n = j + 1;
-          if (!mbar_wait(&bar[Q_KVFULL + n % NS], (uint32_t)(n / NS) & 1u, abort_flag, status, tmo)) { ok = false; break; }
-          if (!mbar_wait(&bar[Q_SDPEMPTY + (n & 1)], ((uint32_t)(n >> 1) & 1u) ^ 1u, abort_flag, status, tmo)) { ok = false; break; }
-          tc_fence_after();
-          issue_sdp(n);
-        }
-        if (!mbar_wait(&bar[Q_DSFULL], (uint32_t)j & 1u, abort_flag, status, tmo)) { ok = false; break; }
-        tc_fence_after();
-        // dQ += dS K   (A = dS, K-major over the 64 keys; B = the K stage read MN-major)
-        const uint32_t ks = aK + (j % NS) * KT;
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-          umma_bf16(tmem + 256, make_smem_desc(aS + kk * 32, 16, 1024), make_smem_desc(ks + kk * 2048, kHalfTile, 1024), id_q,
-                    (j > 0 || kk > 0) ? 1u : 0u);
-        umma_commit(&bar[Q_KVEMPTY + j % NS]);
-        umma_commit(&bar[Q_DSEMPTY]);
-        if (j == nsb - 1) umma_commit(&bar[Q_DONE]);
-      }
-      if (!ok && issued) drain_mma(&bar[Q_DRAIN]);
-    }
-  } else {
-    const int wg = warp >> 2, rt = tid & 127;          // key half and query row of this thread
-    const int row = q0 + rt;
-    const bool live = row < M.Sq;
-    const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    const unsigned long long offset = M.offset + (M.step_ptr ? __ldg(M.step_ptr) * 65536ull : 0ull);
-    // delta = rowsum(dO * O), kept for the dK / dV kernel as well (both threads of a row compute it, one stores it)
-    float delta = 0.f, lse2 = INFINITY;
-    if (live) {
-      const uint4* op = reinterpret_cast<const uint4*>(row_ptr(p.o, b, row, h));
-      const uint4* gp = reinterpret_cast<const uint4*>(row_ptr(p.dout, b, row, h));
-#pragma unroll
-      for (int c = 0; c < HD / 8; ++c) {
-        const uint4 a = __ldg(op + c), g = __ldg(gp + c);
-        delta += bf16_lo(a.x) * bf16_lo(g.x) + bf16_hi(a.x) * bf16_hi(g.x) + bf16_lo(a.y) * bf16_lo(g.y) +
-                 bf16_hi(a.y) * bf16_hi(g.y) + bf16_lo(a.z) * bf16_lo(g.z) + bf16_hi(a.z) * bf16_hi(g.z) +
-                 bf16_lo(a.w) * bf16_lo(g.w) + bf16_hi(a.w) * bf16_hi(g.w);
-      }
-      if (wg == 0) p.delta[(long long)bh * M.Sq + row] = delta;
-      lse2 = p.lse[(long long)bh * M.Sq + row];
-    }
-    bool ok = true;
-    for (int j = 0; j < nsb; ++j) {
-      const int buf = j & 1;
-      const int col0 = j * kHalf + wg * 32;
-      const uint32_t dead = dead_keys<MSK>(M, b, col0, lane);
-      uint32_t good = mbar_wait(&bar[Q_SDPFULL + buf], (uint32_t)(j >> 1) & 1u, abort_flag, status, tmo) ? 1u : 0u;
-      if (!__all_sync(0xffffffffu, good)) { ok = false; break; }
-      tc_fence_after();
-      float x[32], dp[32];
-      tmem_ld32f(lane_addr + (uint32_t)(buf * 128 + wg * 32), x);
-      tmem_ld32f(lane_addr + (uint32_t)(buf * 128 + 64 + wg * 32), dp);
-      tmem_ld_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bar[Q_SDPEMPTY + buf]);
-      // the diagonal crosses the last two sub-blocks of a causal query block
-      const bool plain = MSK == 0 && !(M.causal && j >= 2 * qb) && (j * kHalf + kHalf <= M.Sk);
-      score_chunk<32, MSK>(x, row, col0, dead, M, plain);
-      uint32_t keep = 0xffffffffu;
-      if constexpr (DRP) keep = keep_bits<32>(M, offset, bh, min(row, M.Sq - 1), col0);
-#pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const float pr = ex2_approx(x[i] - lse2);
-        const float d = ((keep >> i) & 1u) ? dp[i] * M.drop_scale : 0.f;
-        x[i] = pr * (d - delta);
-      }
-      if (j > 0) {
-        // the product of the previous sub-block must have read the dS tile
-        good = mbar_wait(&bar[Q_DSEMPTY], (uint32_t)(j - 1) & 1u, abort_flag, status, tmo) ? 1u : 0u;
-        if (!__all_sync(0xffffffffu, good)) { ok = false; break; }
-      }
-#pragma unroll
-      for (int c = 0; c < 4; ++c) *reinterpret_cast<uint4*>(sS + sw128(rt, wg * 4 + c)) = pack8f(x + 8 * c);
-      fence_proxy_async_smem();
-      tc_fence_before();
-      mbar_arrive(&bar[Q_DSFULL]);
-    }
-    if (ok && nsb > 0) {
-      uint32_t good = mbar_wait(&bar[Q_DONE], 0, abort_flag, status, tmo) ? 1u : 0u;
-      if (!__all_sync(0xffffffffu, good)) ok = false;
-    }
-    if (ok) {
-      tc_fence_after();
-      __nv_bfloat16* dst = live ? row_ptr(p.dq, b, row, h) : nullptr;
-#pragma unroll
-      for (int cc = 0; cc < HD / 64; ++cc) {
-        const int c = wg * (HD / 64) + cc;
-        float o[32];
-        if (nsb > 0) {
-          tmem_ld32f(lane_addr + (uint32_t)(256 + c * 32), o);
-          tmem_ld_wait();
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) o[i] = 0.f;
-        }
-#pragma unroll
-        for (int i = 0; i < 32; ++i) o[i] *= M.sm_scale;
-        if (dst) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) *reinterpret_cast<uint4*>(dst + c * 32 + q * 8) = pack8f(o + 8 * q);
-        }
-      }
-    }
-  }
-  teardown_cta(tmem, warp);
-}
-
-// =====================================================================================================  dK / dV
-// CTA = 128 keys of one (batch, head).  The rows of every product are KEYS (transposed formulation), and the queries are
-// walked in sub-blocks of 64:
-//   S^T = K Q^T and dP^T = V dO^T            [128 keys x 64 queries] each, in TMEM, double-buffered
-//   row threads (TMEM lane = key, two threads per key with 32 queries each): P^T and dS^T as bf16 into two
-//                                            [128 x 64] K-major shared tiles
-//   dV += P^T dO,  dK += dS^T Q              contraction over the 64 queries; B = the dO / Q stage read MN-major
-// With 64-query stages three of them fit beside K and V also at head_dim 128, and the double-buffered S^T / dP^T let the
-// products of sub-block i+1 run while the row threads work on sub-block i.  The per-query statistics (log-sum-exp and
-// delta) of a stage are put into shared memory by the producer warp and read as broadcasts.
-enum { K_KVFULL = 0, K_QGFULL = 1 /* 3 stages */, K_QGEMPTY = 4 /* 3 stages */, K_SDPFULL = 7 /* 2 */, K_SDPEMPTY = 9 /* 2 */,
-       K_DSFULL = 11, K_DSEMPTY = 12, K_DONE = 13, K_DRAIN = 14 };
-
-template <int HD, int MSK, bool DRP>
-__global__ void __launch_bounds__(kThreads, 1) flash_dkv_kernel(const __grid_constant__ FlashParams p) {
-  constexpr int SUB = HD / 64;
-  constexpr int TILE = SUB * kSub;          // K or V: 128 rows
-  constexpr int QT = SUB * kHalfTile;       // one stage of Q or dO: 64 rows
-  constexpr int NS = kBwdStages;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sK = sm;
-  uint8_t* sV = sK + TILE;
-  uint8_t* sQ = sV + TILE;            // NS stages
-  uint8_t* sG = sQ + NS * QT;         // NS stages (dO)
-  uint8_t* sP = sG + NS * QT;         // dropped probabilities, transposed: [keys][64 queries]
-  uint8_t* sS = sP + kSub;            // dS transposed
-  Ctl* ctl = reinterpret_cast<Ctl*>(sS + kSub);
-  float* sStat = reinterpret_cast<float*>(sS + kSub + 256);   // per stage: 64 log-sum-exp values, 64 deltas
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const MaskArgs& M = p.m;
-  const int nsub = (M.Sq + kHalf - 1) / kHalf;
-  const int BH = p.B * p.H;
-  // with a causal mask the first key blocks see the most query blocks: they go first
-  const int kb = (int)(blockIdx.x / BH);
-  const int bh = (int)(blockIdx.x % BH);
-  const int b = bh / p.H, h = bh % p.H;
-  const int k0 = kb * kBlk;
-  const int s_begin = M.causal ? k0 / kHalf : 0;
-  const int nit = max(nsub - s_begin, 0);
-  // counts by barrier index: K/V full 1; stage full 33 (the copy's issuer + 32 lanes that wrote the statistics); stage
-  // empty 1; S/dP full 1, S/dP empty 8 (one per row warp); dS full 256; the rest 1
-  const int counts[15] = {1, 33, 33, 33, 1, 1, 1, 1, 1, 8, 8, kRowThreads, 1, 1, 1};
-  const uint32_t tmem = setup_cta(ctl, counts, 15, warp, lane);
-  volatile uint32_t* abort_flag = &ctl->abort_flag;
-  unsigned long long* status = p.status;
-  const unsigned long long tmo = p.timeout_ns;
-  uint64_t* bar = ctl->bar;
-
-  if (warp == kProducerWarp) {
-    // the whole warp walks the stages: lane 0 issues the copies, every lane fetches the statistics of two queries
-    const int cq = head_col(p.q, h), ck = head_col(p.k, h), cv = head_col(p.v, h), cg = head_col(p.dout, h);
-    bool ok = true;
-    uint64_t* dbar[1 + NS]; uint32_t dpar[1 + NS]; bool dis[1 + NS];
-    for (int i = 0; i < 1 + NS; ++i) dis[i] = false;
-    if (lane == 0) {
-      mbar_arrive_expect_tx(&bar[K_KVFULL], 2 * TILE);
-      load_tile<SUB>(smem_u32(sK), &p.mk, p.k_seq1, ck, b, k0, smem_u32(&bar[K_KVFULL]));
-      load_tile<SUB>(smem_u32(sV), &p.mv, p.v_seq1, cv, b, k0, smem_u32(&bar[K_KVFULL]));
-      dbar[0] = &bar[K_KVFULL]; dpar[0] = 0; dis[0] = true;
-    }
-    for (int it = 0; it < nit; ++it) {
-      const int st = it % NS;
-      const uint32_t ph = (uint32_t)(it / NS) & 1u;
-      const uint32_t good = mbar_wait(&bar[K_QGEMPTY + st], ph ^ 1u, abort_flag, status, tmo) ? 1u : 0u;
-      if (!__all_sync(0xffffffffu, good)) { ok = false; break; }
-      const int q0 = (s_begin + it) * kHalf;
-      if (lane == 0) {
-        mbar_arrive_expect_tx(&bar[K_QGFULL + st], 2 * QT);
-        load_tile64<SUB>(smem_u32(sQ + st * QT), &p.mq64, p.q_seq1, cq, b, q0, smem_u32(&bar[K_QGFULL + st]));
-        load_tile64<SUB>(smem_u32(sG + st * QT), &p.mdo64, p.do_seq1, cg, b, q0, smem_u32(&bar[K_QGFULL + st]));
-        dbar[1 + st] = &bar[K_QGFULL + st]; dpar[1 + st] = ph; dis[1 + st] = true;
-      }
-      float2 ls = make_float2(INFINITY, INFINITY), dl = make_float2(0.f, 0.f);
-      const int q = q0 + 2 * lane;
-      const long long base = (long long)bh * M.Sq;
-      if (q < M.Sq) { ls.x = __ldg(p.lse + base + q); dl.x = __ldg(p.delta + base + q); }
-      if (q + 1 < M.Sq) { ls.y = __ldg(p.lse + base + q + 1); dl.y = __ldg(p.delta + base + q + 1); }
-      float* stat = sStat + st * 2 * kHalf;
-      *reinterpret_cast<float2*>(stat + 2 * lane) = ls;
-      *reinterpret_cast<float2*>(stat + kHalf + 2 * lane) = dl;
-      mbar_arrive(&bar[K_QGFULL + st]);
-    }
-    if (lane == 0 && (!ok || *abort_flag)) drain_loads(dbar, dpar, dis, 1 + NS);
-  } else if (warp == kMmaWarp) {
-    if (elect_one()) {
-      const uint32_t id_s = make_idesc_bf16(128, kHalf, 0, 0), id_t = make_idesc_bf16(128, HD, 0, 1);
-      const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), aQ = smem_u32(sQ), aG = smem_u32(sG);
-      const uint32_t aP = smem_u32(sP), aS = smem_u32(sS);
-      bool ok = mbar_wait(&bar[K_KVFULL], 0, abort_flag, status, tmo);
-      bool issued = false;
-      // S^T = K Q^T (columns 0..63 of the buffer), dP^T = V dO^T (columns 64..127): rows = keys
-      auto issue_sdp = [&](int n) {
-        const uint32_t qs = aQ + (n % NS) * QT, gs = aG + (n % NS) * QT, d = tmem + (uint32_t)((n & 1) * 128);
-#pragma unroll
-        for (int u = 0; u < SUB; ++u)
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            umma_bf16(d, make_smem_desc(aK + u * kSub + kk * 32, 16, 1024), make_smem_desc(qs + u * kHalfTile + kk * 32, 16, 1024),
-                      id_s, (u | kk) ? 1u : 0u);
-#pragma unroll
-        for (int u = 0; u < SUB; ++u)
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            umma_bf16(d + 64, make_smem_desc(aV + u * kSub + kk * 32, 16, 1024),
-                      make_smem_desc(gs + u * kHalfTile + kk * 32, 16, 1024), id_s, (u | kk) ? 1u : 0u);
-        umma_commit(&bar[K_SDPFULL + (n & 1)]);
-      };
-      if (ok && nit > 0) ok = mbar_wait(&bar[K_QGFULL], 0, abort_flag, status, tmo);
-      if (ok && nit > 0) { tc_fence_after(); issue_sdp(0); issued = true; }
-      for (int it = 0; it < nit && ok; ++it) {
-        if (it + 1 < nit) {
-          const int n = it + 1;
-          if (!mbar_wait(&bar[K_QGFULL + n % NS], (uint32_t)(n / NS) & 1u, abort_flag, status, tmo)) { ok = false; break; }
-          if (!mbar_wait(&bar[K_SDPEMPTY + (n & 1)], ((uint32_t)(n >> 1) & 1u) ^ 1u, abort_flag, status, tmo)) { ok = false; break; }
-          tc_fence_after();
-          issue_sdp(n);
-        }
-        long long* tm = (p.trace && blockIdx.x == 0 && it < 16) ? p.trace + 256 + it * 8 : nullptr;
-        if (tm) tm[0] = clock64();                       // S / dP of the next sub-block issued
-        if (!mbar_wait(&bar[K_DSFULL], (uint32_t)it & 1u, abort_flag, status, tmo)) { ok = false; break; }
-        if (tm) tm[1] = clock64();                       // dS written
-        tc_fence_after();
-        const uint32_t qs = aQ + (it % NS) * QT, gs = aG + (it % NS) * QT;
-        // dV += P^T dO, dK += dS^T Q: A = the transposed tiles (K-major over the 64 queries), B = the stage, MN-major
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-          umma_bf16(tmem + 256, make_smem_desc(aP + kk * 32, 16, 1024), make_smem_desc(gs + kk * 2048, kHalfTile, 1024), id_t,
-                    (it > 0 || kk > 0) ? 1u : 0u);
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-          umma_bf16(tmem + 256 + HD, make_smem_desc(aS + kk * 32, 16, 1024), make_smem_desc(qs + kk * 2048, kHalfTile, 1024),
-                    id_t, (it > 0 || kk > 0) ? 1u : 0u);
-        umma_commit(&bar[K_QGEMPTY + it % NS]);
-        umma_commit(&bar[K_DSEMPTY]);
-        if (it == nit - 1) umma_commit(&bar[K_DONE]);
-        if (tm) tm[2] = clock64();                       // dV / dK issued
-      }
-      if (!ok && issued) drain_mma(&bar[K_DRAIN]);
-    }
-  } else {
-    const int wg = warp >> 2, rt = tid & 127;          // query half and key row of this thread
-    const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    const unsigned long long offset = M.offset + (M.step_ptr ? __ldg(M.step_ptr) * 65536ull : 0ull);
-    const int key = k0 + rt;
-    bool key_dead = key >= M.Sk;
-    if constexpr (MSK != 0) key_dead = key_dead || (M.kpm && __ldg(M.kpm + (long long)b * M.kpm_ld + key));
-    const bool keys_plain = MSK == 0 && (k0 + kBlk <= M.Sk);
-    bool ok = true;
-    long long* tr = (p.trace && blockIdx.x == 0 && lane == 0 && (warp & 3) == 0) ? p.trace + (warp >> 2) * 128 : nullptr;
-    for (int it = 0; it < nit; ++it) {
-      const int st = it % NS, buf = it & 1;
-      const int qbase = (s_begin + it) * kHalf + wg * 32;      // first query of this thread
-      if (tr && it < 16) tr[it * 8 + 0] = clock64();
-      uint32_t good = mbar_wait(&bar[K_QGFULL + st], (uint32_t)(it / NS) & 1u, abort_flag, status, tmo) ? 1u : 0u;
-      if (tr && it < 16) tr[it * 8 + 1] = clock64();
-      if (good) good = mbar_wait(&bar[K_SDPFULL + buf], (uint32_t)(it >> 1) & 1u, abort_flag, status, tmo) ? 1u : 0u;
-      if (!__all_sync(0xffffffffu, good)) { ok = false; break; }
-      tc_fence_after();
-      if (tr && it < 16) tr[it * 8 + 2] = clock64();
-      float x[32], dp[32];
-      tmem_ld32f(lane_addr + (uint32_t)(buf * 128 + wg * 32), x);
-      tmem_ld32f(lane_addr + (uint32_t)(buf * 128 + 64 + wg * 32), dp);
-      tmem_ld_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bar[K_SDPEMPTY + buf]);
-      if (tr && it < 16) tr[it * 8 + 3] = clock64();
-      // the diagonal crosses the first two sub-blocks of a causal key block
-      const bool plain = keys_plain && !(M.causal && it < 2);
-      const float4* lse4 = reinterpret_cast<const float4*>(sStat + st * 2 * kHalf + wg * 32);
-      const float4* del4 = reinterpret_cast<const float4*>(sStat + st * 2 * kHalf + kHalf + wg * 32);
-      // Dropout bits.  One generator call covers four neighbouring keys, which sit in four neighbouring lanes: each lane
-      // calls it for every fourth query and the four exchange their nibbles (eight calls a thread instead of 32;
-      // 2 x 8 heads of 1024 x 1024, head_dim 64, causal: dK / dV 110 -> 43.3 us).
-      uint32_t kw[4] = {0u, 0u, 0u, 0u};                       // kw[e]: nibble g = keys of the quad, query 4 g + e
-      if constexpr (DRP) {
-        uint32_t mine = 0;
-#pragma unroll
-        for (int g = 0; g < 8; ++g) {
-          const int q = min(qbase + 4 * g + (lane & 3), M.Sq - 1);
-          const unsigned long long idx = ((unsigned long long)bh * M.Sq + q) * (unsigned long long)M.Sk + (key & ~3);
-          const uint4 r = philox4x32(M.seed, offset, idx >> 2);
-          mine |= ((r.x >= M.thresh ? 1u : 0u) | (r.y >= M.thresh ? 2u : 0u) | (r.z >= M.thresh ? 4u : 0u) |
-                   (r.w >= M.thresh ? 8u : 0u)) << (4 * g);
-        }
-#pragma unroll
-        for (int e = 0; e < 4; ++e) kw[e] = __shfl_sync(0xffffffffu, mine, (lane & ~3) + e) >> (lane & 3);
-      }
-#pragma unroll
-      for (int g = 0; g < 8; ++g) {
-        const float4 L4 = lse4[g], D4 = del4[g];
-        const float lse_[4] = {L4.x, L4.y, L4.z, L4.w}, del_[4] = {D4.x, D4.y, D4.z, D4.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int i = 4 * g + e;
-          const int q = qbase + i;
-          float xs = x[i] * M.scale_log2;
-          if (!plain) {
-            if constexpr (MSK == 2) {
-              if (q < M.Sq && key < M.Sk) {
-                const long long mi = (long long)q * M.mask_ld + key;
-                xs += (M.mask_fp32 ? __ldg(reinterpret_cast<const float*>(M.mask) + mi)
-                                   : __bfloat162float(__ldg(reinterpret_cast<const __nv_bfloat16*>(M.mask) + mi))) * kLog2e;
+            for (int i = 0; i < 64; ++i) {
+              const int q = qbase + i;
+              float xs = x[i] * M.scale_log2;
+              if constexpr (MSK == 2) {
+                if (q < M.Sq && key < M.Sk) {
+                  const long long mi = (long long)q * M.mask_ld + key;
+                  xs += (M.mask_fp32 ? __ldg(reinterpret_cast<const float*>(M.mask) + mi)
+                                     : __bfloat162float(__ldg(reinterpret_cast<const __nv_bfloat16*>(M.mask) + mi))) * kLog2e;
+                }
               }
+              x[i] = key_dead || (M.causal && key > q) ? -INFINITY : xs + nl[i];
             }
-            if (key_dead || (M.causal && key > q)) xs = -INFINITY;
           }
-          const float pr = ex2_approx(xs - lse_[e]);
-          bool kp = true;
-          if constexpr (DRP) kp = (kw[e] >> (4 * g)) & 1u;
-          const float d = kp ? dp[i] * M.drop_scale : 0.f;
-          dp[i] = pr * (d - del_[e]);             // dS
-          x[i] = kp ? pr * M.drop_scale : 0.f;    // dropped probability
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            float* e = x + 32 * c;
+#pragma unroll
+            for (int i = 0; i < 32; ++i) e[i] = ex2_approx(e[i]);
+            if constexpr (DRP) {
+              float d[32];
+#pragma unroll
+              for (int i = 0; i < 32; ++i) d[i] = (kw[c][i & 3] >> (i & ~3)) & 1u ? e[i] * M.drop_scale : 0.f;
+              store_bf16x32(aS + (uint32_t)(c * 16), d);
+            } else {
+              store_bf16x32(aS + (uint32_t)(c * 16), e);
+            }
+          }
+          publish_rows(&bar[B_PFULL], lane);
+          if (tr && it < 16) tr[it * 8 + 2] = clock64();
+          if (!wait(B_DPFULL, ndp++ & 1u)) { ok = false; break; }
+          tc_fence_after();
+          if (tr && it < 16) tr[it * 8 + 3] = clock64();
+          float dp[64];
+          tmem_ld32f(aP, dp);
+          tmem_ld32f(aP + 32, dp + 32);
+          tmem_ld_wait();
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+#pragma unroll
+            for (int i = 32 * c; i < 32 * c + 32; i += 4) {
+              const float4 D = *reinterpret_cast<const float4*>(ndel + i);
+              if constexpr (DRP) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) dp[i + e] = (kw[c][e] >> (i - 32 * c)) & 1u ? dp[i + e] * M.drop_scale : 0.f;
+              }
+              const float2 u = mul2(make_float2(x[i], x[i + 1]), add2(make_float2(dp[i], dp[i + 1]), make_float2(D.x, D.y)));
+              const float2 v = mul2(make_float2(x[i + 2], x[i + 3]), add2(make_float2(dp[i + 2], dp[i + 3]), make_float2(D.z, D.w)));
+              x[i] = u.x; x[i + 1] = u.y; x[i + 2] = v.x; x[i + 3] = v.y;
+            }
+            store_bf16x32(aP + (uint32_t)(c * 16), x + 32 * c);
+          }
+          publish_rows(&bar[B_DSFULL], lane);
+          if (tr && it < 16) tr[it * 8 + 4] = clock64();
+        }
+      } else {
+        const int q0 = w.qb * kBlk, nb = M.causal ? min(nkb, w.qb + 1) : nkb;
+        const int row = q0 + rt;
+        const bool live = row < M.Sq;
+        const float nlse = live ? -__ldg(p.lse + (long long)bh * M.Sq + row) : -INFINITY;
+        const float ndel = live ? -__ldg(p.delta + (long long)bh * M.Sq + row) : 0.f;
+        const float2 nl = make_float2(nlse, nlse), nd = make_float2(ndel, ndel);
+        for (int j = 0; j < nb; ++j) {
+          const int col0 = j * kBlk + wg * 64;
+          const uint32_t dead[2] = {dead_keys<MSK>(M, b, col0, lane), dead_keys<MSK>(M, b, col0 + 32, lane)};
+          uint32_t keep[2] = {0xffffffffu, 0xffffffffu};
+          if constexpr (DRP) {
+            keep[0] = keep_bits<32>(M, offset, bh, min(row, M.Sq - 1), col0);
+            keep[1] = keep_bits<32>(M, offset, bh, min(row, M.Sq - 1), col0 + 32);
+          }
+          if (!wait(B_SFULL + (j & 1), (ns >> (j & 1)) & 1u)) { ok = false; break; }
+          ns ^= 1u << (j & 1);
+          tc_fence_after();
+          const uint32_t aS = (j & 1 ? tmem + 384 : tS) + lane_off + (uint32_t)(wg * 64);
+          float x[64];
+          tmem_ld32f(aS, x);
+          tmem_ld32f(aS + 32, x + 32);
+          tmem_ld_wait();
+          const bool plain = MSK != 2 && !(dead[0] | dead[1]) && !(M.causal && j == w.qb) && (j * kBlk + kBlk <= M.Sk);
+          if (plain) {
+#pragma unroll
+            for (int i = 0; i < 64; i += 2) {
+              const float2 u = fma2(make_float2(x[i], x[i + 1]), sc, nl);
+              x[i] = u.x; x[i + 1] = u.y;
+            }
+          } else {
+            score_chunk<32, MSK>(x, row, col0, dead[0], M, false);
+            score_chunk<32, MSK>(x + 32, row, col0 + 32, dead[1], M, false);
+#pragma unroll
+            for (int i = 0; i < 64; ++i) x[i] += nlse;
+          }
+#pragma unroll
+          for (int i = 0; i < 64; ++i) x[i] = ex2_approx(x[i]);
+          if (!wait(B_DPFULL, ndp++ & 1u)) { ok = false; break; }
+          tc_fence_after();
+          float dp[64];
+          tmem_ld32f(aP, dp);
+          tmem_ld32f(aP + 32, dp + 32);
+          tmem_ld_wait();
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+#pragma unroll
+            for (int i = 32 * c; i < 32 * c + 32; i += 2) {
+              if constexpr (DRP) {
+                dp[i] = (keep[c] >> (i & 31)) & 1u ? dp[i] * M.drop_scale : 0.f;
+                dp[i + 1] = (keep[c] >> ((i + 1) & 31)) & 1u ? dp[i + 1] * M.drop_scale : 0.f;
+              }
+              const float2 u = mul2(make_float2(x[i], x[i + 1]), add2(make_float2(dp[i], dp[i + 1]), nd));
+              x[i] = u.x; x[i + 1] = u.y;
+            }
+            store_bf16x32(aP + (uint32_t)(c * 16), x + 32 * c);
+          }
+          publish_rows(&bar[B_DSFULL], lane);
         }
       }
-      if (tr && it < 16) tr[it * 8 + 4] = clock64() + (x[0] == 12345.f ? 1 : 0);
-      if (it > 0) {
-        // the products of the previous sub-block must have read the two tiles
-        good = mbar_wait(&bar[K_DSEMPTY], (uint32_t)(it - 1) & 1u, abort_flag, status, tmo) ? 1u : 0u;
-        if (!__all_sync(0xffffffffu, good)) { ok = false; break; }
-      }
-      if (tr && it < 16) tr[it * 8 + 5] = clock64();
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const uint32_t off = sw128(rt, wg * 4 + c);
-        *reinterpret_cast<uint4*>(sP + off) = pack8f(x + 8 * c);
-        *reinterpret_cast<uint4*>(sS + off) = pack8f(dp + 8 * c);
-      }
-      if (tr && it < 16) tr[it * 8 + 6] = clock64();
-      fence_proxy_async_smem();
-      tc_fence_before();
-      mbar_arrive(&bar[K_DSFULL]);
-      if (tr && it < 16) tr[it * 8 + 7] = clock64();
-    }
-    if (ok && nit > 0) {
-      uint32_t good = mbar_wait(&bar[K_DONE], 0, abort_flag, status, tmo) ? 1u : 0u;
-      if (!__all_sync(0xffffffffu, good)) ok = false;
-    }
-    if (ok) {
+      if (ok) ok = wait(B_ACC, n & 1u);
+      if (!ok) break;
       tc_fence_after();
-      __nv_bfloat16* dvp = key < M.Sk ? row_ptr(p.dv, b, key, h) : nullptr;
-      __nv_bfloat16* dkp = key < M.Sk ? row_ptr(p.dk, b, key, h) : nullptr;
+      const int r0 = (w.kb >= 0 ? w.kb : w.qb) * kBlk + (warp & 3) * 32;      // the warp's first row
+      const int left = (w.kb >= 0 ? M.Sk : M.Sq) - r0;
+      const int nacc = w.kb >= 0 ? 2 : 1;
+      for (int a = 0; a < nacc; ++a) {
+        const DRef& out = w.kb < 0 ? p.dq : a ? p.dk : p.dv;
+        __nv_bfloat16* dst = row_ptr(out, b, r0, h) + wg * (HD / 2);
+        const float mul = w.kb >= 0 && a == 0 ? 1.f : M.sm_scale;
 #pragma unroll
-      for (int cc = 0; cc < HD / 64; ++cc) {
-        const int c = wg * (HD / 64) + cc;
-        float o[32];
-        if (nit > 0) { tmem_ld32f(lane_addr + (uint32_t)(256 + c * 32), o); tmem_ld_wait(); }
-        else {
+        for (int c = 0; c < HD / 64; ++c) {
+          float o[32];
+          tmem_ld32f(tAcc + lane_off + (uint32_t)(a * HD + wg * (HD / 2) + c * 32), o);
+          tmem_ld_wait();
+          if (a + 1 == nacc && c + 1 == HD / 64) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bar[B_ACCREAD]);
+          }
 #pragma unroll
-          for (int i = 0; i < 32; ++i) o[i] = 0.f;
-        }
-        if (dvp) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) *reinterpret_cast<uint4*>(dvp + c * 32 + q * 8) = pack8f(o + 8 * q);
-        }
-        if (nit > 0) { tmem_ld32f(lane_addr + (uint32_t)(256 + HD + c * 32), o); tmem_ld_wait(); }
-#pragma unroll
-        for (int i = 0; i < 32; ++i) o[i] *= M.sm_scale;
-        if (dkp) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) *reinterpret_cast<uint4*>(dkp + c * 32 + q * 8) = pack8f(o + 8 * q);
+          for (int i = 0; i < 32; ++i) o[i] *= mul;
+          store_rows32(dst + c * 32, out.ss, left, o, lane);
         }
       }
     }
@@ -1011,6 +1215,22 @@ __global__ void __launch_bounds__(kThreads, 1) flash_dkv_kernel(const __grid_con
 thread_local std::string g_ferr;
 long long* g_flash_trace = nullptr;
 int ffail(const std::string& s) { g_ferr = s; return -1; }
+
+int device_sms() {
+  static int n[64] = {0};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) dev = 0;
+  if (!n[dev]) cudaDeviceGetAttribute(&n[dev], cudaDevAttrMultiProcessorCount, dev);
+  return n[dev];
+}
+
+// How many heads run side by side: as many as leave what their CTAs read again and again well inside L2.  Over all heads at once,
+// longest blocks first, long sequences came from HBM each time (16 heads of 8192 x 128: backward 870 us, 790 in groups of 4).
+int head_group(long long bytes_per_head, int BH) {
+  const long long g = (32ll << 20) / std::max(bytes_per_head, 1ll);
+  return (int)std::min<long long>(std::max(g, 1ll), BH);
+}
 
 uint32_t thresh_of(float pdrop) {
   if (pdrop <= 0.f) return 0u;
@@ -1080,13 +1300,11 @@ int fill_common(const RtpFlashArgs* a, FlashParams& P) {
   P.q = dref(a->q); P.k = dref(a->k); P.v = dref(a->v); P.o = dref(a->o);
   return 0;
 }
-constexpr int smem_fwd(int hd) { return 1024 + (hd / 64) * kSub * 5 + 2 * kSub + 256 + (int)sizeof(Xchg); }
-constexpr int smem_dq(int hd) { return 1024 + (hd / 64) * (2 * kSub + 2 * kBwdStages * kHalfTile) + kSub + 256; }
-constexpr int smem_dkv(int hd) {
-  return 1024 + (hd / 64) * (2 * kSub + 2 * kBwdStages * kHalfTile) + 2 * kSub + 256 + kBwdStages * 2 * kHalf * 4;
-}
+constexpr int smem_fwd(int hd) { return 1024 + (hd / 64) * kSub * 6 + 256 + 2 * 256 * 4; }
+// backward: seven tiles, control block, statistics of two blocks of queries
+constexpr int smem_bwd(int hd) { return kBwdSlack + (hd / 64) * kSub * 7 + 256 + 2 * 2 * kBlk * 4; }
 static_assert(sizeof(Ctl) <= 256, "control block");
-static_assert(smem_dq(128) <= 232448 && smem_dkv(128) <= 232448 && smem_fwd(128) <= 232448, "shared memory budget");
+static_assert(smem_fwd(128) <= 232448 && smem_bwd(128) <= 232448, "shared memory budget");
 
 template <auto Kern>
 int launch_flash(const FlashParams& P, int grid, int smem, cudaStream_t stream, const char* what) {
@@ -1108,10 +1326,18 @@ int rtp_flash_fwd(const RtpFlashArgs* a, void* stream) {
   static thread_local FlashParams P;
   if (fill_common(a, P)) return -1;
   if (!a->lse) return ffail("flash attention: lse buffer required");
-  const int grid = ((a->Sq + kBlk - 1) / kBlk) * a->B * a->H;
+  // One row tile a CTA, its keys shared out, as long as that is one wave (2 heads of 4096 x 4096 x 128: 49 -> 37 us); two row tiles
+  // a CTA beyond it, where they share the copies of K and V.
+  const int tiles = (a->Sq + kBlk - 1) / kBlk, BH = a->B * a->H;
+  P.split = (long long)tiles * BH <= device_sms();
+  P.group = head_group(4ll * a->Sk * a->head_dim, BH);
+  const int grid = (P.split ? tiles : (tiles + 1) / 2) * BH;
+  const bool more = grid > device_sms();         // 48 heads of 999 x 128: 31 -> 28 us
   cudaStream_t s = (cudaStream_t)stream;
   const bool drp = P.m.thresh != 0;
-#define RTP_FWD(HD, MSK, DRP) launch_flash<flash_fwd_kernel<HD, MSK, DRP>>(P, grid, smem_fwd(HD), s, "flash_fwd")
+#define RTP_FWD(HD, MSK, DRP)                                                                         \
+  (more ? launch_flash<flash_fwd_kernel<HD, MSK, DRP, true>>(P, grid, smem_fwd(HD), s, "flash_fwd")   \
+        : launch_flash<flash_fwd_kernel<HD, MSK, DRP, false>>(P, grid, smem_fwd(HD), s, "flash_fwd"))
 #define RTP_FWD_HD(HD) (a->mask ? (drp ? RTP_FWD(HD, 2, true) : RTP_FWD(HD, 2, false))  \
                         : a->kpm ? (drp ? RTP_FWD(HD, 1, true) : RTP_FWD(HD, 1, false)) \
                                  : (drp ? RTP_FWD(HD, 0, true) : RTP_FWD(HD, 0, false)))
@@ -1128,19 +1354,19 @@ int rtp_flash_bwd(const RtpFlashArgs* a, void* stream) {
       check_ref(a->dv, "dv", a->head_dim))
     return -1;
   if (make_map3(&P.mdo, &P.do_seq1, a->dout, a->B, a->Sq, "dout")) return -1;
-  if (make_map3(&P.mq64, &P.q_seq1, a->q, a->B, a->Sq, "q", 64u)) return -1;
-  if (make_map3(&P.mdo64, &P.do_seq1, a->dout, a->B, a->Sq, "dout", 64u)) return -1;
-  if (make_map3(&P.mk64, &P.k_seq1, a->k, a->B, a->Sk, "k", 64u)) return -1;
-  if (make_map3(&P.mv64, &P.v_seq1, a->v, a->B, a->Sk, "v", 64u)) return -1;
   P.dout = dref(a->dout); P.dq = dref(a->dq); P.dk = dref(a->dk); P.dv = dref(a->dv);
-  const int gq = ((a->Sq + kBlk - 1) / kBlk) * a->B * a->H;
-  const int gk = ((a->Sk + kBlk - 1) / kBlk) * a->B * a->H;
+  const int grid = ((a->Sq + kBlk - 1) / kBlk + (a->Sk + kBlk - 1) / kBlk) * a->B * a->H;
+  const bool more = grid > 2 * device_sms();   // one or two rounds are over sooner without (16 heads of 1024 x 1024: 55 us, 60)
   cudaStream_t s = (cudaStream_t)stream;
   const bool drp = P.m.thresh != 0;
-#define RTP_BWD(HD, MSK, DRP)                                                                              \
-  (launch_flash<flash_dq_kernel<HD, MSK, DRP>>(P, gq, smem_dq(HD), s, "flash_dq")                          \
-       ? -1                                                                                                \
-       : launch_flash<flash_dkv_kernel<HD, MSK, DRP>>(P, gk, smem_dkv(HD), s, "flash_dkv"))
+  P.group = head_group(4ll * (a->Sq + a->Sk) * a->head_dim, a->B * a->H);
+  const long long rows = (long long)a->B * a->Sq * a->H, per = 256 / (a->head_dim / 8);
+  const cudaError_t e = launch_k(a->head_dim == 64 ? flash_delta_kernel<64> : flash_delta_kernel<128>,
+                                 dim3((unsigned)((rows + per - 1) / per)), dim3(256), 0, s, P.o, P.dout, P.delta, a->Sq, a->H, rows);
+  if (e != cudaSuccess) return ffail(std::string("flash_delta: ") + cudaGetErrorString(e));
+#define RTP_BWD(HD, MSK, DRP)                                                                         \
+  (more ? launch_flash<flash_bwd_kernel<HD, MSK, DRP, true>>(P, grid, smem_bwd(HD), s, "flash_bwd")   \
+        : launch_flash<flash_bwd_kernel<HD, MSK, DRP, false>>(P, grid, smem_bwd(HD), s, "flash_bwd"))
 #define RTP_BWD_HD(HD) (a->mask ? (drp ? RTP_BWD(HD, 2, true) : RTP_BWD(HD, 2, false))  \
                         : a->kpm ? (drp ? RTP_BWD(HD, 1, true) : RTP_BWD(HD, 1, false)) \
                                  : (drp ? RTP_BWD(HD, 0, true) : RTP_BWD(HD, 0, false)))
