@@ -107,7 +107,11 @@ __device__ __forceinline__ void add8(float* v, const uint4& u) {
   v[4] += bf16_lo(u.z); v[5] += bf16_hi(u.z); v[6] += bf16_lo(u.w); v[7] += bf16_hi(u.w);
 }
 
-template <bool PAIR, int MAXJ>
+// SRC: a job adds to its output or masks it; FUN: a job has an activation or dropout.  Merely branched over, that code cost every
+// launch: twice the spills, and a fifth of the epilogue's time went into instruction fetch.  With it compiled out and both
+// halves of a row's 64 columns fetched at once (us, before -> now): 256 x 64 -> 256 4.5 -> 3.4, 1024 x 512 -> 512 6.6 -> 5.5,
+// 1024 x 2048 -> 2048 13.4 -> 12.4, 8192 x 8 -> 8192 73 -> 45, 36864 x 64 -> 288 20 -> 13.6; added to its output 25 -> 21.
+template <bool PAIR, int MAXJ, bool SRC, bool FUN>
 __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_constant__ Params<MAXJ> P) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -296,15 +300,18 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
       const Job& J = P.job[find_job(P, t)];
       int tm, tn;
       tile_pos(J, t - J.tile0, tm, tn);
-      const int M = J.M, N = J.N, bn = J.bn, act = J.act, part = J.part;
+      const int M = J.M, N = J.N, bn = J.bn, part = J.part;
+      [[maybe_unused]] const int act = J.act;
       const int row0 = tm * TM + (int)crank * kTM + quad * 32, n0 = tn * bn;
       const __nv_bfloat16* c = reinterpret_cast<const __nv_bfloat16*>(J.c);
       const __nv_bfloat16* mask = reinterpret_cast<const __nv_bfloat16*>(J.mask);
       const __nv_bfloat16* bias = reinterpret_cast<const __nv_bfloat16*>(J.bias);
       __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(J.d);
-      const long long ldd = J.ldd, ldc = J.ldc, ldmask = J.ldmask;
-      const uint32_t thresh = J.drop_thresh;
-      const unsigned long long drop_off = J.offset + (J.step_ptr ? __ldg(J.step_ptr) * 65536ull : 0ull);
+      const long long ldd = J.ldd;
+      [[maybe_unused]] const long long ldc = J.ldc, ldmask = J.ldmask;
+      [[maybe_unused]] const uint32_t thresh = J.drop_thresh;
+      [[maybe_unused]] unsigned long long drop_off = 0;
+      if constexpr (FUN) drop_off = J.offset + (J.step_ptr ? __ldg(J.step_ptr) * 65536ull : 0ull);
       bool waited = false;
       if (J.sum && half == 0) {
         uint32_t good = 1;
@@ -326,22 +333,27 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
         const int col0 = n0 + ch * 64;
         const int ccol = col0 + (lane & 7) * 8;                      // column of this lane in the coalesced view
         // the accumulate source is fetched while the accumulator is still being made
-        uint4 cv[8];
-        const __nv_bfloat16* pre = c ? c : mask;
-        const long long ldpre = c ? ldc : ldmask;
-        if (pre) {
+        [[maybe_unused]] uint4 cv[8];
+        [[maybe_unused]] const __nv_bfloat16* pre = c ? c : mask;
+        if constexpr (SRC) {
+          const long long ldpre = c ? ldc : ldmask;
+          if (pre) {
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const int row = row0 + 4 * k + (lane >> 3);
-            cv[k] = make_uint4(0u, 0u, 0u, 0u);
-            if (row < M && ccol < N) cv[k] = __ldcg(reinterpret_cast<const uint4*>(pre + (long long)row * ldpre + ccol));
+            for (int k = 0; k < 8; ++k) {
+              const int row = row0 + 4 * k + (lane >> 3);
+              cv[k] = make_uint4(0u, 0u, 0u, 0u);
+              if (row < M && ccol < N) cv[k] = __ldcg(reinterpret_cast<const uint4*>(pre + (long long)row * ldpre + ccol));
+            }
           }
         }
-        uint4 bv[8];
-        if (bias) {
+        // so is the bias, where no other source takes the registers (a job with both is rare)
+        [[maybe_unused]] uint4 bv[8];
+        auto bias8 = [&](int q) {
+          return bias && col0 + q * 8 < N ? __ldg(reinterpret_cast<const uint4*>(bias + col0 + q * 8)) : make_uint4(0u, 0u, 0u, 0u);
+        };
+        if constexpr (!SRC) {
 #pragma unroll
-          for (int q = 0; q < 8; ++q)
-            bv[q] = col0 + q * 8 < N ? __ldg(reinterpret_cast<const uint4*>(bias + col0 + q * 8)) : make_uint4(0u, 0u, 0u, 0u);
+          for (int q = 0; q < 8; ++q) bv[q] = bias8(q);
         }
         if (!waited) {
           uint32_t good = 1;
@@ -351,75 +363,98 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
           tc_fence_after();
           waited = true;
         }
-        if (pre) {
-          __syncwarp();
+        uint32_t ra[2][32];                      // 64 columns of this thread's row
+        const uint32_t acc_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * 256 + ch * 64);
+        if constexpr (SRC) {
+          if (pre) {
+            __syncwarp();
 #pragma unroll
-          for (int k = 0; k < 8; ++k) *reinterpret_cast<uint4*>((k & 1 ? coal1 : coal0) + 4 * k * kPitch) = cv[k];
-          __syncwarp();
+            for (int k = 0; k < 8; ++k) *reinterpret_cast<uint4*>((k & 1 ? coal1 : coal0) + 4 * k * kPitch) = cv[k];
+            __syncwarp();
+          }
+        }
+        if (!SRC || part) {
+          tmem_ld_32x32(acc_addr, ra[0]);
+          tmem_ld_32x32(acc_addr + 32, ra[1]);
+          tmem_ld_wait();
+        }
+        if (part) {          // a slice of a contraction: rows of 256 bytes per thread, a few tiles in all
+          if (row0 + lane < M) {
+            float* dp = reinterpret_cast<float*>(J.d) + (long long)(row0 + lane) * ldd + col0;
+#pragma unroll
+            for (int q = 0; q < 16; ++q)
+              if (col0 + 4 * q < N)
+                reinterpret_cast<uint4*>(dp)[q] = make_uint4(ra[q >> 3][4 * (q & 7)], ra[q >> 3][4 * (q & 7) + 1],
+                                                             ra[q >> 3][4 * (q & 7) + 2], ra[q >> 3][4 * (q & 7) + 3]);
+          }
+          continue;
         }
 #pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {         // 32 columns at a time: one TMEM load, half a staged row
-          uint32_t ra[32];
-          tmem_ld_32x32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * 256 + ch * 64 + hh * 32), ra);
-          tmem_ld_wait();
+        for (int hh = 0; hh < 2; ++hh) {
           const int colh = col0 + hh * 32;
-          if (part) {        // a slice of a contraction: rows of 128 bytes per thread, a few tiles in all
-            if (row0 + lane < M) {
-              float* dp = reinterpret_cast<float*>(J.d) + (long long)(row0 + lane) * ldd + colh;
-#pragma unroll
-              for (int q = 0; q < 8; ++q)
-                if (colh + 4 * q < N)
-                  reinterpret_cast<float4*>(dp)[q] = make_float4(__uint_as_float(ra[4 * q]), __uint_as_float(ra[4 * q + 1]),
-                                                                 __uint_as_float(ra[4 * q + 2]), __uint_as_float(ra[4 * q + 3]));
-            }
-            continue;
+          if constexpr (SRC) {
+            tmem_ld_32x32(acc_addr + hh * 32, ra[hh]);
+            tmem_ld_wait();
           }
           float v[32];
 #pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(ra[i]);
-          if (c) {
+          for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(ra[hh][i]);
+          if constexpr (SRC) {
+            if (c) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) add8(v + 8 * q, *reinterpret_cast<const uint4*>(own + (((4 * hh + q) ^ osw) << 4)));
+              for (int q = 0; q < 4; ++q) add8(v + 8 * q, *reinterpret_cast<const uint4*>(own + (((4 * hh + q) ^ osw) << 4)));
+            }
           }
-          if (bias) {
+          if constexpr (SRC) {
+            if (bias) {
+#pragma unroll
+              for (int q = 0; q < 4; ++q) add8(v + 8 * q, bias8(4 * hh + q));
+            }
+          } else {
 #pragma unroll
             for (int q = 0; q < 4; ++q) add8(v + 8 * q, bv[4 * hh + q]);
           }
-          if (act == 1) {
+          if constexpr (FUN) {
+            if (act == 1) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = fmaxf(v[i], 0.f);
-          } else if (act == 2) {
+              for (int i = 0; i < 32; ++i) v[i] = fmaxf(v[i], 0.f);
+            } else if (act == 2) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = 0.5f * v[i] * (1.f + erff(v[i] * 0.70710678118654752f));
+              for (int i = 0; i < 32; ++i) v[i] = 0.5f * v[i] * (1.f + erff(v[i] * 0.70710678118654752f));
+            }
           }
-          if (mask) {
-            const float ms = J.mask_scale;
+          if constexpr (SRC) {
+            if (mask) {
+              const float ms = J.mask_scale;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              uint4 u = make_uint4(0u, 0u, 0u, 0u);
-              if (!c) u = *reinterpret_cast<const uint4*>(own + (((4 * hh + q) ^ osw) << 4));
-              else if (row0 + lane < M && colh + q * 8 < N)     // both at once is rare: not fetched ahead
-                u = __ldcg(reinterpret_cast<const uint4*>(mask + (long long)(row0 + lane) * ldmask + colh + q * 8));
-              const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+              for (int q = 0; q < 4; ++q) {
+                uint4 u = make_uint4(0u, 0u, 0u, 0u);
+                if (!c) u = *reinterpret_cast<const uint4*>(own + (((4 * hh + q) ^ osw) << 4));
+                else if (row0 + lane < M && colh + q * 8 < N)     // both at once is rare: not fetched ahead
+                  u = __ldcg(reinterpret_cast<const uint4*>(mask + (long long)(row0 + lane) * ldmask + colh + q * 8));
+                const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                v[8 * q + 2 * i] = bf16_lo(w[i]) > 0.f ? v[8 * q + 2 * i] * ms : 0.f;
-                v[8 * q + 2 * i + 1] = bf16_hi(w[i]) > 0.f ? v[8 * q + 2 * i + 1] * ms : 0.f;
+                for (int i = 0; i < 4; ++i) {
+                  v[8 * q + 2 * i] = bf16_lo(w[i]) > 0.f ? v[8 * q + 2 * i] * ms : 0.f;
+                  v[8 * q + 2 * i + 1] = bf16_hi(w[i]) > 0.f ? v[8 * q + 2 * i + 1] * ms : 0.f;
+                }
               }
             }
           }
-          if (thresh) {
-            // element index = position in the logical [M, N] output (N and the column are multiples of 4)
-            const unsigned long long e4 = ((unsigned long long)(row0 + lane) * (unsigned long long)N + (unsigned long long)colh) >> 2;
-            const float dsc = J.drop_scale;
-            const unsigned long long sd = J.seed;
+          if constexpr (FUN) {
+            if (thresh) {
+              // element index = position in the logical [M, N] output (N and the column are multiples of 4)
+              const unsigned long long e4 = ((unsigned long long)(row0 + lane) * (unsigned long long)N + (unsigned long long)colh) >> 2;
+              const float dsc = J.drop_scale;
+              const unsigned long long sd = J.seed;
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-              const uint4 rr = philox4x32(sd, drop_off, e4 + q);
-              v[4 * q] = rr.x >= thresh ? v[4 * q] * dsc : 0.f;
-              v[4 * q + 1] = rr.y >= thresh ? v[4 * q + 1] * dsc : 0.f;
-              v[4 * q + 2] = rr.z >= thresh ? v[4 * q + 2] * dsc : 0.f;
-              v[4 * q + 3] = rr.w >= thresh ? v[4 * q + 3] * dsc : 0.f;
+              for (int q = 0; q < 8; ++q) {
+                const uint4 rr = philox4x32(sd, drop_off, e4 + q);
+                v[4 * q] = rr.x >= thresh ? v[4 * q] * dsc : 0.f;
+                v[4 * q + 1] = rr.y >= thresh ? v[4 * q + 1] * dsc : 0.f;
+                v[4 * q + 2] = rr.z >= thresh ? v[4 * q + 2] * dsc : 0.f;
+                v[4 * q + 3] = rr.w >= thresh ? v[4 * q + 3] * dsc : 0.f;
+              }
             }
           }
 #pragma unroll
@@ -428,7 +463,6 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
                 make_uint4(pack_bf16(v[8 * q], v[8 * q + 1]), pack_bf16(v[8 * q + 2], v[8 * q + 3]),
                            pack_bf16(v[8 * q + 4], v[8 * q + 5]), pack_bf16(v[8 * q + 6], v[8 * q + 7]));
         }
-        if (part) continue;
         __syncwarp();
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
@@ -534,14 +568,14 @@ int sms() {
 // {17.3, 14.5, 13.9, 21.1}, its backward {19.1, 23.3, 27.0, 37.8}, forward 1024 x 512 -> 512 {10.0, 8.2, 7.6, 7.2},
 // 8192 x 2048 -> 8192 {185, 252, 257, 454}.
 // A column-sum tile loads 16 KB per k-block and CTA.
-// `drain` is what bounds a tile of few k-blocks: the epilogue's warps empty one accumulator at a time, and a fifth of the
-// k-loop's clocks come on top (8192 x 8192 with K = 8 / 512, us: {72.8, 88.2, 84.6, 146} / {81, 96, 97, 155}); three fifths
+// `drain` is what bounds a tile of few k-blocks: the epilogue's warps empty one accumulator at a time, and two fifths of the
+// k-loop's clocks come on top (8192 x 8192 with K = 8 / 512, us: {45, 59, 58, 90} / {62, 79, 80, 139}); three fifths
 // of `epi` are left to add for the last one.  Without it the weight gradient of a few tokens fell into 64-wide tiles, each
 // as long as a 128-wide one: backward of 8 x 2048 -> 8192 70 to 82 us, now 47 (65 before there was a choice).
 constexpr int kSumClk = 330;
 struct TileShape { bool pair; int bn, clk, epi, drain; };
-constexpr TileShape kShapes[4] = {{true, 256, 650, 4600, 9400}, {true, 128, 545, 1700, 6000},
-                                  {false, 128, 530, 700, 5500}, {false, 64, 480, 0, 4750}};
+constexpr TileShape kShapes[4] = {{true, 256, 650, 4600, 5600}, {true, 128, 545, 1700, 3700},
+                                  {false, 128, 530, 700, 3600}, {false, 64, 480, 0, 3000}};
 constexpr int kTileFixed = 300;       // hand-over between two tiles of a unit
 
 // a GEMM, or the column sums of its A
@@ -554,7 +588,7 @@ Tiles tiles_of(const Item& x, const TileShape& s) {
   const int tm = s.pair ? 256 : 128;
   const long long k = (x.g->K + 63) / 64, rows = (x.g->M + tm - 1) / tm;
   if (x.sum) return Tiles{k * kSumClk + kTileFixed, rows, 0};
-  const long long loop = k * s.clk + kTileFixed, drain = s.drain + loop / 5;
+  const long long loop = k * s.clk + kTileFixed, drain = s.drain + loop * 2 / 5;
   return Tiles{std::max(loop, drain), rows * ((x.g->N + s.bn - 1) / s.bn), loop >= drain ? s.epi : s.epi * 3 / 5};
 }
 // Clocks of the longest unit of a launch in which job i uses tile shape sh[i]; `ord` sorts the jobs by falling tile cost.
@@ -603,9 +637,9 @@ long long makespan(const Item* it, int n, const TileShape* const* sh, int units,
   return best + epi;
 }
 
-template <bool PAIR, int MAXJ>
+template <bool PAIR, int MAXJ, bool SRC, bool FUN>
 int launch_local(const Params<MAXJ>& P, cudaStream_t stream) {
-  if (ensure_smem<local_gemm_kernel<PAIR, MAXJ>>(kSmem) != cudaSuccess) return lfail("cudaFuncSetAttribute failed");
+  if (ensure_smem<local_gemm_kernel<PAIR, MAXJ, SRC, FUN>>(kSmem) != cudaSuccess) return lfail("cudaFuncSetAttribute failed");
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(PAIR ? 2 * P.units : P.units);
   cfg.blockDim = dim3(kThreads);
@@ -625,7 +659,7 @@ int launch_local(const Params<MAXJ>& P, cudaStream_t stream) {
   }
   cfg.attrs = at;
   cfg.numAttrs = nat;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, local_gemm_kernel<PAIR, MAXJ>, P);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, local_gemm_kernel<PAIR, MAXJ, SRC, FUN>, P);
   return e == cudaSuccess ? 0 : lfail(std::string("launch local_gemm_kernel: ") + cudaGetErrorString(e));
 }
 
@@ -674,9 +708,11 @@ int run(const Item* it, int n, int pair_policy, unsigned long long* status, unsi
   memset(static_cast<void*>(&P), 0, sizeof(P));
   const int tm = pair ? 256 : 128;
   int widest = 0, total = 0;
-  bool sums = false;
+  bool sums = false, src = false, fun = false;
   for (int q = 0; q < n; ++q) {
     const LocalGemm& x = *it[best_ord[q]].g;
+    src = src || x.c || x.mask;
+    fun = fun || x.act || x.drop_p > 0.f;
     Job& J = P.job[q];
     J.sum = it[best_ord[q]].sum ? 1 : 0;
     J.part = x.part;
@@ -725,7 +761,9 @@ int run(const Item* it, int n, int pair_policy, unsigned long long* status, unsi
     P.ones_off = pair ? kArea + kStageOut : P.stages * P.stage_bytes;
   }
   P.status = status; P.timeout_ns = 2 * timeout_ns;
-  return pair ? launch_local<true, MAXJ>(P, stream) : launch_local<false, MAXJ>(P, stream);
+#define RTP_LOCAL(SRC, FUN) (pair ? launch_local<true, MAXJ, SRC, FUN>(P, stream) : launch_local<false, MAXJ, SRC, FUN>(P, stream))
+  return src ? (fun ? RTP_LOCAL(true, true) : RTP_LOCAL(true, false)) : (fun ? RTP_LOCAL(false, true) : RTP_LOCAL(false, false));
+#undef RTP_LOCAL
 }
 
 int items_of(const LocalGemm* jobs, int n, Item* it) {
