@@ -1,15 +1,20 @@
 // Short-sequence attention (S = 32 or 64, head_dim 64) on tcgen05 tensor cores.
 //
-// One CTA of 128 threads handles 128 / S (batch, head) pairs at once: their query rows are stacked into one
-// 128-row operand, so that every product is an M = 128 UMMA.  Each head gets its own chain of UMMAs against its own
-// K / V rows and its own TMEM columns; thread t owns stacked row t (TMEM lane t), so the softmax of a row and the
-// dS algebra of the backward pass run entirely in that thread's registers, without shuffles.
+// One CTA of 128 threads handles 128 / S (batch, head) pairs at once: their query rows and their key rows are stacked into
+// 128-row operands, so that every product is one chain of M = 128 UMMAs.  Thread t owns stacked row t (TMEM lane t) and works on
+// the columns of its own head, so the softmax of a row and the dS algebra of the backward pass run entirely in that thread's
+// registers, without shuffles.
 //
-//   forward :  S_q = Q K_q^T  ->  P = dropout(softmax(scale * S))  ->  O_q = P K-compact x V_q
-//   backward:  S_q, dP_q = dO V_q^T  ->  dS  ->  dQ_q = dS x K_q ;  dK = dS^T x Q ;  dV = P_drop^T x dO
+//   forward :  S = Q K^T (all pairs of stacked rows)  ->  P = dropout(softmax(scale * S)) of the own head  ->  O = P V
+//   backward:  S, dP = dO V^T  ->  dS  ->  dQ = dS K ;  dK = dS^T Q ;  dV = P_drop^T dO
 //
-// dS^T and P_drop^T are written to shared memory as block-diagonal [128 x 128] MN-major A operands (row t of the
-// stack writes k-row t, 16-byte stores), so dK and dV of all stacked heads come out of one chain of eight UMMAs each.
+// P and dS are [128 x 128] tiles with zeros between different heads.  Written once, row per thread, the dS tile is read K-major for
+// dQ and MN-major (transposed) for dK.  P takes the place of operands that are no longer needed, and the results take the place
+// of S and dP in TMEM: 48 / 112 KB and 128 / 256 columns, so that two CTAs and more share an SM (one chain a head, with 64 / 144 KB
+// and 256 / 512 columns, had one in backward: 1024 heads of 32 x 64 took two rounds).
+// us, that form -> this: 1024 heads of 32 with dropout, forward 10.2 -> 7.9, backward 21.0 -> 11.0; 32 heads of 32 5.8 -> 5.4 and
+// 9.7 -> 8.2; 1024 heads of 64 17.8 -> 15.7 and 47.4 -> 26.3.
+//
 // Operands are fetched with plain 16-byte loads into 128-byte-swizzled tiles (the strided token order s*B + b of the
 // packed projection needs no tensor map); "fence.proxy.async" publishes them to the tensor core.
 //
@@ -31,6 +36,7 @@ using namespace rtp;
 constexpr int kHd = 64;
 constexpr int kRows = 128;                 // stacked rows per CTA
 constexpr int kTile = kRows * 128;         // one [128 x 64] bf16 operand tile, 128-byte rows: 16 KB
+constexpr int kSlack = 512;                // for the alignment of the tiles, which shared memory starts with anyhow
 
 __device__ unsigned int g_attn_tc_error;        // set when a bounded wait for the CTA's own UMMAs ran out
 __device__ unsigned long long* g_attn_trace;   // tuning aid: timeline of CTA 0 (16 words), null = off
@@ -65,12 +71,39 @@ __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity) {
   }
   return true;
 }
-__device__ __forceinline__ uint32_t pack2(float a, float b) {
-  __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&v);
+// Keep bits of the S_T probabilities that start at element e0 (a multiple of 4): bit c set = kept.
+template <int S_T>
+__device__ __forceinline__ uint64_t keep_row(uint64_t seed, uint64_t offset, uint64_t e0, uint32_t thresh) {
+  uint64_t keep = ~0ull;
+  if (!thresh) return keep;
+  keep = 0;
+#pragma unroll
+  for (int c4 = 0; c4 < S_T / 4; ++c4) {
+    const uint4 rr = philox4x32(seed, offset, (e0 >> 2) + c4);
+    const uint32_t k4 = (rr.x >= thresh ? 1u : 0u) | (rr.y >= thresh ? 2u : 0u) | (rr.z >= thresh ? 4u : 0u) | (rr.w >= thresh ? 8u : 0u);
+    keep |= (uint64_t)k4 << (4 * c4);
+  }
+  return keep;
 }
-__device__ __forceinline__ float lo(uint32_t u) { return __uint_as_float(u << 16); }
-__device__ __forceinline__ float hi(uint32_t u) { return __uint_as_float(u & 0xffff0000u); }
+// Row `row` of a [128 x 128] tile of two [128 x 64] sub-tiles: the S_T values of head q at its columns, zeros elsewhere.
+template <int S_T>
+__device__ __forceinline__ void write_diagonal(uint8_t* tile, int row, int q, const float* v) {
+  constexpr int N = S_T / 8;
+  uint4 w[N];
+#pragma unroll
+  for (int k = 0; k < N; ++k)
+    w[k] = make_uint4(pack_bf16(v[8 * k], v[8 * k + 1]), pack_bf16(v[8 * k + 2], v[8 * k + 3]), pack_bf16(v[8 * k + 4], v[8 * k + 5]),
+                      pack_bf16(v[8 * k + 6], v[8 * k + 7]));
+#pragma unroll
+  for (int g = 0; g < 16 / N; ++g) {
+    const bool own = g == q;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      const int c = g * N + k;
+      *reinterpret_cast<uint4*>(tile + (c >> 3) * kTile + sw128(row, c & 7)) = own ? w[k] : make_uint4(0u, 0u, 0u, 0u);
+    }
+  }
+}
 
 // Stacks rows [q * S_T + s] = token (s, b_q), columns col[q] .. col[q] + 64 of `src` (row pitch ld) into swizzled tiles.
 // A thread's eight 16-byte loads per tile are all issued before the first shared-memory store, so that they overlap
@@ -150,21 +183,25 @@ __global__ void __launch_bounds__(128) attn_tc_fwd_kernel(const __nv_bfloat16* _
                                                           uint64_t seed, uint64_t offset,
                                                           const unsigned long long* __restrict__ step_ptr, int n_bh) {
   constexpr int HPC = kRows / S_T;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  extern __shared__ __align__(1024) uint8_t smem_tiles[];
+  uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_tiles) + 1023) & ~uintptr_t(1023));
+  if (sm - smem_tiles > kSlack) {
+    if (threadIdx.x == 0) atomicExch(&g_attn_tc_error, 1u);
+    return;
+  }
   uint8_t* sQ = sm;
   uint8_t* sK = sm + kTile;
   uint8_t* sV = sm + 2 * kTile;
-  uint8_t* sP = sm + 3 * kTile;
-  Ctl* ctl = reinterpret_cast<Ctl*>(sm + 4 * kTile);
-  const int tid = threadIdx.x, warp = tid >> 5;
+  uint8_t* sP = sm;                         // [128 x 128], over Q and K
+  Ctl* ctl = reinterpret_cast<Ctl*>(sm + 3 * kTile);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int D = heads * kHd;
   ATT_STAMP(0);
-  setup<S_T>(ctl, tid, warp, B, heads, nshard, n_bh, 256);
+  setup<S_T>(ctl, tid, warp, B, heads, nshard, n_bh, 128);
   ATT_STAMP(1);
-  if (step_ptr) offset += __ldg(step_ptr) * 65536ull;
   const uint32_t tmem = ctl->tmem_base;
-
+  const int q = tid / S_T, s = tid % S_T;
+  uint64_t keep;
   {
     HeadRef hq[HPC], hk[HPC], hv[HPC];
 #pragma unroll
@@ -177,6 +214,9 @@ __global__ void __launch_bounds__(128) attn_tc_fwd_kernel(const __nv_bfloat16* _
     fetch_stack<S_T>(va, qkv, 3 * D, B, hq, tid);
     fetch_stack<S_T>(vb, qkv, 3 * D, B, hk, tid);
     fetch_stack<S_T>(vc, qkv, 3 * D, B, hv, tid);
+    // the dropout bits are worked out while the loads are in flight
+    if (step_ptr) offset += __ldg(step_ptr) * 65536ull;
+    keep = keep_row<S_T>(seed, offset, ((uint64_t)(blockIdx.x * HPC + q) * S_T + s) * S_T, thresh);
     store_stack(sQ, va, tid);
     store_stack(sK, vb, tid);
     store_stack(sV, vc, tid);
@@ -186,21 +226,18 @@ __global__ void __launch_bounds__(128) attn_tc_fwd_kernel(const __nv_bfloat16* _
   ATT_STAMP(2);
 
   if (warp == 0 && elect_one()) {
-    const uint32_t idesc = make_idesc_bf16(128, S_T, 0, 0);
+    const uint32_t idesc = make_idesc_bf16(128, 128, 0, 0);
     const uint32_t aq = smem_u32(sQ), bk = smem_u32(sK);
 #pragma unroll
-    for (int q = 0; q < HPC; ++q)
-#pragma unroll
-      for (int kk = 0; kk < kHd / 16; ++kk)
-        umma_bf16(tmem + q * S_T, make_smem_desc(aq + kk * 32, 16, 1024),
-                  make_smem_desc(bk + q * S_T * 128 + kk * 32, 16, 1024), idesc, kk > 0 ? 1u : 0u);
+    for (int kk = 0; kk < kHd / 16; ++kk)
+      umma_bf16(tmem, make_smem_desc(aq + kk * 32, 16, 1024), make_smem_desc(bk + kk * 32, 16, 1024), idesc, kk > 0 ? 1u : 0u);
     umma_commit(&ctl->bar[0]);
   }
   wait_bar(&ctl->bar[0], 0);
+  __syncwarp();
   tc_fence_after();
   ATT_STAMP(3);
 
-  const int q = tid / S_T, s = tid % S_T;
   const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
   {
     float x[S_T];
@@ -217,26 +254,10 @@ __global__ void __launch_bounds__(128) attn_tc_fwd_kernel(const __nv_bfloat16* _
       x[c] = __expf(x[c] - mx);
       sum += x[c];
     }
-    const float inv = 1.f / sum;
-    const int bh = blockIdx.x * HPC + q;
-    const uint64_t e0 = ((uint64_t)bh * S_T + s) * S_T;
+    const float inv = 1.f / sum, kept = thresh ? inv * drop_scale : inv;
 #pragma unroll
-    for (int c4 = 0; c4 < S_T / 4; ++c4) {
-      float m0 = inv, m1 = inv, m2 = inv, m3 = inv;
-      if (thresh) {
-        const uint4 rr = philox4x32(seed, offset, (e0 >> 2) + c4);
-        m0 = rr.x >= thresh ? inv * drop_scale : 0.f;
-        m1 = rr.y >= thresh ? inv * drop_scale : 0.f;
-        m2 = rr.z >= thresh ? inv * drop_scale : 0.f;
-        m3 = rr.w >= thresh ? inv * drop_scale : 0.f;
-      }
-      x[4 * c4] *= m0; x[4 * c4 + 1] *= m1; x[4 * c4 + 2] *= m2; x[4 * c4 + 3] *= m3;
-    }
-#pragma unroll
-    for (int c8 = 0; c8 < S_T / 8; ++c8)
-      *reinterpret_cast<uint4*>(sP + sw128(tid, c8)) =
-          make_uint4(pack2(x[8 * c8], x[8 * c8 + 1]), pack2(x[8 * c8 + 2], x[8 * c8 + 3]),
-                     pack2(x[8 * c8 + 4], x[8 * c8 + 5]), pack2(x[8 * c8 + 6], x[8 * c8 + 7]));
+    for (int c = 0; c < S_T; ++c) x[c] *= (keep >> c) & 1ull ? kept : 0.f;
+    write_diagonal<S_T>(sP, tid, q, x);
   }
   ATT_STAMP(4);
   fence_proxy_async_smem();
@@ -249,33 +270,30 @@ __global__ void __launch_bounds__(128) attn_tc_fwd_kernel(const __nv_bfloat16* _
     const uint32_t idesc = make_idesc_bf16(128, kHd, 0, 1);
     const uint32_t ap = smem_u32(sP), bv = smem_u32(sV);
 #pragma unroll
-    for (int qq = 0; qq < HPC; ++qq)
-#pragma unroll
-      for (int kk = 0; kk < S_T / 16; ++kk)
-        umma_bf16(tmem + qq * kHd, make_smem_desc(ap + kk * 32, 16, 1024),
-                  make_smem_desc(bv + qq * S_T * 128 + kk * 2048, 8192, 1024), idesc, kk > 0 ? 1u : 0u);
+    for (int kk = 0; kk < 8; ++kk)
+      umma_bf16(tmem, make_smem_desc(ap + (kk >> 2) * kTile + (kk & 3) * 32, 16, 1024), make_smem_desc(bv + kk * 2048, 8192, 1024),
+                idesc, kk > 0 ? 1u : 0u);
     umma_commit(&ctl->bar[1]);
   }
   wait_bar(&ctl->bar[1], 0);
+  __syncwarp();
   tc_fence_after();
   ATT_STAMP(6);
   {
+    // a warp's 32 rows belong to one head and to consecutive positions
     float o[kHd];
-    load_row<kHd>(lane_addr + q * kHd, o);
-    if (ctl->valid[q]) {
-      uint4* dst = reinterpret_cast<uint4*>(out + (size_t)(s * B + ctl->b[q]) * D + ctl->h[q] * kHd);
-#pragma unroll
-      for (int c8 = 0; c8 < 8; ++c8)
-        dst[c8] = make_uint4(pack2(o[8 * c8], o[8 * c8 + 1]), pack2(o[8 * c8 + 2], o[8 * c8 + 3]),
-                             pack2(o[8 * c8 + 4], o[8 * c8 + 5]), pack2(o[8 * c8 + 6], o[8 * c8 + 7]));
-    }
+    load_row<kHd>(lane_addr, o);
+    __nv_bfloat16* dst = out + (size_t)((s - lane) * B + ctl->b[q]) * D + ctl->h[q] * kHd;
+    const int rows = ctl->valid[q] ? 32 : 0;
+    store_rows32(dst, (long long)B * D, rows, o, lane);
+    store_rows32(dst + 32, (long long)B * D, rows, o + 32, lane);
   }
   ATT_STAMP(7);
   tc_fence_before();
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
-    tmem_dealloc(tmem, 256);
+    tmem_dealloc(tmem, 128);
   }
   ATT_STAMP(8);
 }
@@ -288,24 +306,27 @@ __global__ void __launch_bounds__(128) attn_tc_bwd_kernel(const __nv_bfloat16* _
                                                           uint64_t seed, uint64_t offset,
                                                           const unsigned long long* __restrict__ step_ptr, int n_bh) {
   constexpr int HPC = kRows / S_T;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  extern __shared__ __align__(1024) uint8_t smem_tiles[];
+  uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_tiles) + 1023) & ~uintptr_t(1023));
+  if (sm - smem_tiles > kSlack) {
+    if (threadIdx.x == 0) atomicExch(&g_attn_tc_error, 1u);
+    return;
+  }
   uint8_t* sQ = sm;
   uint8_t* sK = sm + kTile;
-  uint8_t* sV = sm + 2 * kTile;
-  uint8_t* sG = sm + 3 * kTile;            // dO
-  uint8_t* sS = sm + 4 * kTile;            // dS, compact K-major [128 x S_T]
-  uint8_t* sTS = sm + 5 * kTile;           // dS^T, block-diagonal MN-major A [k = stacked row][m = stacked key]: 32 KB
-  uint8_t* sTP = sm + 7 * kTile;           // P_drop^T, same form: 32 KB
-  Ctl* ctl = reinterpret_cast<Ctl*>(sm + 9 * kTile);
-  const int tid = threadIdx.x, warp = tid >> 5;
+  uint8_t* sG = sm + 2 * kTile;            // dO
+  uint8_t* sV = sm + 3 * kTile;
+  uint8_t* sP = sV;                        // dropped probabilities [128 x 128], over V and the tile behind it
+  uint8_t* sS = sm + 5 * kTile;            // dS [128 x 128]
+  Ctl* ctl = reinterpret_cast<Ctl*>(sm + 7 * kTile);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int D = heads * kHd;
   ATT_STAMP(0);
-  setup<S_T>(ctl, tid, warp, B, heads, nshard, n_bh, 512);
+  setup<S_T>(ctl, tid, warp, B, heads, nshard, n_bh, 256);
   ATT_STAMP(1);
-  if (step_ptr) offset += __ldg(step_ptr) * 65536ull;
   const uint32_t tmem = ctl->tmem_base;
-
+  const int q = tid / S_T, s = tid % S_T;
+  uint64_t keep;
   {
     HeadRef hq[HPC], hk[HPC], hv[HPC], hg[HPC];
 #pragma unroll
@@ -318,42 +339,36 @@ __global__ void __launch_bounds__(128) attn_tc_bwd_kernel(const __nv_bfloat16* _
     uint4 va[8], vb[8], vc[8], vd[8];
     fetch_stack<S_T>(va, qkv, 3 * D, B, hq, tid);
     fetch_stack<S_T>(vb, qkv, 3 * D, B, hk, tid);
-    fetch_stack<S_T>(vc, qkv, 3 * D, B, hv, tid);
-    fetch_stack<S_T>(vd, dout, D, B, hg, tid);
-    // the off-diagonal blocks of the transposed operands stay zero (filled while the loads are in flight)
-#pragma unroll 4
-    for (int i = tid; i < 4 * kTile / 16; i += 128) reinterpret_cast<uint4*>(sTS)[i] = make_uint4(0u, 0u, 0u, 0u);
+    fetch_stack<S_T>(vc, dout, D, B, hg, tid);
+    fetch_stack<S_T>(vd, qkv, 3 * D, B, hv, tid);
+    // the dropout bits are worked out while the loads are in flight
+    if (step_ptr) offset += __ldg(step_ptr) * 65536ull;
+    keep = keep_row<S_T>(seed, offset, ((uint64_t)(blockIdx.x * HPC + q) * S_T + s) * S_T, thresh);
     store_stack(sQ, va, tid);
     store_stack(sK, vb, tid);
-    store_stack(sV, vc, tid);
-    store_stack(sG, vd, tid);
+    store_stack(sG, vc, tid);
+    store_stack(sV, vd, tid);
   }
   fence_proxy_async_smem();
   __syncthreads();
   ATT_STAMP(2);
 
   if (warp == 0 && elect_one()) {
-    const uint32_t idesc = make_idesc_bf16(128, S_T, 0, 0);
+    const uint32_t idesc = make_idesc_bf16(128, 128, 0, 0);
     const uint32_t aq = smem_u32(sQ), bk = smem_u32(sK), ag = smem_u32(sG), bv = smem_u32(sV);
 #pragma unroll
-    for (int qq = 0; qq < HPC; ++qq)
+    for (int kk = 0; kk < kHd / 16; ++kk)
+      umma_bf16(tmem, make_smem_desc(aq + kk * 32, 16, 1024), make_smem_desc(bk + kk * 32, 16, 1024), idesc, kk > 0 ? 1u : 0u);
 #pragma unroll
-      for (int kk = 0; kk < kHd / 16; ++kk)
-        umma_bf16(tmem + qq * S_T, make_smem_desc(aq + kk * 32, 16, 1024),
-                  make_smem_desc(bk + qq * S_T * 128 + kk * 32, 16, 1024), idesc, kk > 0 ? 1u : 0u);
-#pragma unroll
-    for (int qq = 0; qq < HPC; ++qq)
-#pragma unroll
-      for (int kk = 0; kk < kHd / 16; ++kk)
-        umma_bf16(tmem + 128 + qq * S_T, make_smem_desc(ag + kk * 32, 16, 1024),
-                  make_smem_desc(bv + qq * S_T * 128 + kk * 32, 16, 1024), idesc, kk > 0 ? 1u : 0u);
+    for (int kk = 0; kk < kHd / 16; ++kk)
+      umma_bf16(tmem + 128, make_smem_desc(ag + kk * 32, 16, 1024), make_smem_desc(bv + kk * 32, 16, 1024), idesc, kk > 0 ? 1u : 0u);
     umma_commit(&ctl->bar[0]);
   }
   wait_bar(&ctl->bar[0], 0);
+  __syncwarp();
   tc_fence_after();
   ATT_STAMP(3);
 
-  const int q = tid / S_T, s = tid % S_T;
   const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
   {
     float x[S_T], dp[S_T];
@@ -372,125 +387,83 @@ __global__ void __launch_bounds__(128) attn_tc_bwd_kernel(const __nv_bfloat16* _
       sum += x[c];
     }
     const float inv = 1.f / sum;
-    const int bh = blockIdx.x * HPC + q;
-    const uint64_t e0 = ((uint64_t)bh * S_T + s) * S_T;
-    // x <- P, dp <- m * dP (gradient wrt the un-dropped probability); the mask m is kept as a bit set
-    uint64_t keep = ~0ull;
+    // x <- P, dp <- m * dP (gradient wrt the un-dropped probability)
     float dot = 0.f;
 #pragma unroll
-    for (int c4 = 0; c4 < S_T / 4; ++c4) {
-      uint32_t k4 = 0xfu;
-      if (thresh) {
-        const uint4 rr = philox4x32(seed, offset, (e0 >> 2) + c4);
-        k4 = (rr.x >= thresh ? 1u : 0u) | (rr.y >= thresh ? 2u : 0u) | (rr.z >= thresh ? 4u : 0u) |
-             (rr.w >= thresh ? 8u : 0u);
-        keep = (keep & ~(0xfull << (4 * c4))) | ((uint64_t)k4 << (4 * c4));
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int c = 4 * c4 + i;
-        x[c] *= inv;
-        dp[c] = ((k4 >> i) & 1u) ? dp[c] * drop_scale : 0.f;
-        dot += dp[c] * x[c];
-      }
+    for (int c = 0; c < S_T; ++c) {
+      x[c] *= inv;
+      dp[c] = (keep >> c) & 1ull ? dp[c] * drop_scale : 0.f;
+      dot += dp[c] * x[c];
     }
     // dS (into dp) and the dropped probabilities (into x)
 #pragma unroll
     for (int c = 0; c < S_T; ++c) {
       dp[c] = x[c] * (dp[c] - dot);
-      x[c] = ((keep >> c) & 1ull) ? x[c] * drop_scale : 0.f;
+      x[c] = (keep >> c) & 1ull ? x[c] * drop_scale : 0.f;
     }
-    // compact dS row, and row t of both transposed operands (k-row t; columns of this head's keys)
-    const int m0 = q * S_T;
-    uint8_t* ts = sTS + (tid >> 6) * 16384 + (m0 >> 6) * 8192;
-    uint8_t* tp = sTP + (tid >> 6) * 16384 + (m0 >> 6) * 8192;
-    const int kr = tid & 63, cb = (m0 & 63) >> 3;
-#pragma unroll
-    for (int c8 = 0; c8 < S_T / 8; ++c8) {
-      const uint4 vs = make_uint4(pack2(dp[8 * c8], dp[8 * c8 + 1]), pack2(dp[8 * c8 + 2], dp[8 * c8 + 3]),
-                                  pack2(dp[8 * c8 + 4], dp[8 * c8 + 5]), pack2(dp[8 * c8 + 6], dp[8 * c8 + 7]));
-      const uint4 vp = make_uint4(pack2(x[8 * c8], x[8 * c8 + 1]), pack2(x[8 * c8 + 2], x[8 * c8 + 3]),
-                                  pack2(x[8 * c8 + 4], x[8 * c8 + 5]), pack2(x[8 * c8 + 6], x[8 * c8 + 7]));
-      *reinterpret_cast<uint4*>(sS + sw128(tid, c8)) = vs;
-      *reinterpret_cast<uint4*>(ts + sw128(kr, cb + c8)) = vs;
-      *reinterpret_cast<uint4*>(tp + sw128(kr, cb + c8)) = vp;
-    }
+    write_diagonal<S_T>(sS, tid, q, dp);
+    write_diagonal<S_T>(sP, tid, q, x);
   }
   ATT_STAMP(4);
   fence_proxy_async_smem();
   tc_fence_before();
-  __syncthreads();   // S and dP have been read everywhere: their TMEM columns are reused for dQ
+  __syncthreads();   // S and dP have been read everywhere: their TMEM columns are reused for the results
   ATT_STAMP(5);
 
   if (warp == 0 && elect_one()) {
     tc_fence_after();
-    const uint32_t as = smem_u32(sS), bk = smem_u32(sK), bq = smem_u32(sQ), bg = smem_u32(sG);
-    const uint32_t ats = smem_u32(sTS), atp = smem_u32(sTP);
+    const uint32_t as = smem_u32(sS), ap = smem_u32(sP), bk = smem_u32(sK), bq = smem_u32(sQ), bg = smem_u32(sG);
     const uint32_t id_q = make_idesc_bf16(128, kHd, 0, 1), id_t = make_idesc_bf16(128, kHd, 1, 1);
 #pragma unroll
-    for (int qq = 0; qq < HPC; ++qq)
-#pragma unroll
-      for (int kk = 0; kk < S_T / 16; ++kk)
-        umma_bf16(tmem + qq * kHd, make_smem_desc(as + kk * 32, 16, 1024),
-                  make_smem_desc(bk + qq * S_T * 128 + kk * 2048, 8192, 1024), id_q, kk > 0 ? 1u : 0u);
+    for (int j = 0; j < 8; ++j)
+      umma_bf16(tmem, make_smem_desc(as + (j >> 2) * kTile + (j & 3) * 32, 16, 1024), make_smem_desc(bk + j * 2048, 8192, 1024), id_q,
+                j > 0 ? 1u : 0u);
 #pragma unroll
     for (int j = 0; j < 8; ++j)
-      umma_bf16(tmem + 256, make_smem_desc(ats + (j >> 2) * 16384 + (j & 3) * 2048, 8192, 1024),
-                make_smem_desc(bq + j * 2048, 8192, 1024), id_t, j > 0 ? 1u : 0u);
+      umma_bf16(tmem + 64, make_smem_desc(as + j * 2048, kTile, 1024), make_smem_desc(bq + j * 2048, 8192, 1024), id_t,
+                j > 0 ? 1u : 0u);
 #pragma unroll
     for (int j = 0; j < 8; ++j)
-      umma_bf16(tmem + 320, make_smem_desc(atp + (j >> 2) * 16384 + (j & 3) * 2048, 8192, 1024),
-                make_smem_desc(bg + j * 2048, 8192, 1024), id_t, j > 0 ? 1u : 0u);
+      umma_bf16(tmem + 128, make_smem_desc(ap + j * 2048, kTile, 1024), make_smem_desc(bg + j * 2048, 8192, 1024), id_t,
+                j > 0 ? 1u : 0u);
     umma_commit(&ctl->bar[1]);
   }
   wait_bar(&ctl->bar[1], 0);
+  __syncwarp();
   tc_fence_after();
   ATT_STAMP(6);
-  if (ctl->valid[q]) {
-    __nv_bfloat16* rowp = dqkv + (size_t)(s * B + ctl->b[q]) * (3 * D);
-    float o[kHd];
-    load_row<kHd>(lane_addr + q * kHd, o);
-    uint4* dst = reinterpret_cast<uint4*>(rowp + ctl->cq[q]);
+  {
+    // a warp's 32 rows belong to one head and to consecutive positions
+    __nv_bfloat16* rowp = dqkv + (size_t)((s - lane) * B + ctl->b[q]) * (3 * D);
+    const long long pitch = 3ll * B * D;
+    const int rows = ctl->valid[q] ? 32 : 0;
 #pragma unroll
-    for (int c8 = 0; c8 < 8; ++c8)
-      dst[c8] = make_uint4(pack2(o[8 * c8] * sm_scale, o[8 * c8 + 1] * sm_scale),
-                           pack2(o[8 * c8 + 2] * sm_scale, o[8 * c8 + 3] * sm_scale),
-                           pack2(o[8 * c8 + 4] * sm_scale, o[8 * c8 + 5] * sm_scale),
-                           pack2(o[8 * c8 + 6] * sm_scale, o[8 * c8 + 7] * sm_scale));
-    load_row<kHd>(lane_addr + 256, o);
-    dst = reinterpret_cast<uint4*>(rowp + ctl->ck[q]);
+    for (int r = 0; r < 3; ++r) {
+      const int col = r == 0 ? ctl->cq[q] : r == 1 ? ctl->ck[q] : ctl->cv[q];
+      float o[kHd];
+      load_row<kHd>(lane_addr + r * kHd, o);
+      if (r < 2) {
 #pragma unroll
-    for (int c8 = 0; c8 < 8; ++c8)
-      dst[c8] = make_uint4(pack2(o[8 * c8] * sm_scale, o[8 * c8 + 1] * sm_scale),
-                           pack2(o[8 * c8 + 2] * sm_scale, o[8 * c8 + 3] * sm_scale),
-                           pack2(o[8 * c8 + 4] * sm_scale, o[8 * c8 + 5] * sm_scale),
-                           pack2(o[8 * c8 + 6] * sm_scale, o[8 * c8 + 7] * sm_scale));
-    load_row<kHd>(lane_addr + 320, o);
-    dst = reinterpret_cast<uint4*>(rowp + ctl->cv[q]);
-#pragma unroll
-    for (int c8 = 0; c8 < 8; ++c8)
-      dst[c8] = make_uint4(pack2(o[8 * c8], o[8 * c8 + 1]), pack2(o[8 * c8 + 2], o[8 * c8 + 3]),
-                           pack2(o[8 * c8 + 4], o[8 * c8 + 5]), pack2(o[8 * c8 + 6], o[8 * c8 + 7]));
-  } else {
-    // tcgen05.ld is warp-collective: rows without a head still take part
-    float o[kHd];
-    load_row<kHd>(lane_addr + q * kHd, o);
-    load_row<kHd>(lane_addr + 256, o);
-    load_row<kHd>(lane_addr + 320, o);
+        for (int c = 0; c < kHd; ++c) o[c] *= sm_scale;
+      }
+      store_rows32(rowp + col, pitch, rows, o, lane);
+      store_rows32(rowp + col + 32, pitch, rows, o + 32, lane);
+    }
   }
   ATT_STAMP(7);
   tc_fence_before();
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
-    tmem_dealloc(tmem, 512);
+    tmem_dealloc(tmem, 256);
   }
   ATT_STAMP(8);
 }
 
 std::string g_err;
-constexpr int kFwdSmem = 4 * kTile + 1024 + 256;
-constexpr int kBwdSmem = 9 * kTile + 1024 + 256;
+constexpr int kFwdSmem = 3 * kTile + kSlack + 256;
+constexpr int kBwdSmem = 7 * kTile + kSlack + 256;
+static_assert(2 * (kBwdSmem + 1024) <= 233472, "two CTAs of the backward kernel on an SM");
 uint32_t thresh_of(float p) {
   if (p <= 0.f) return 0u;
   double t = (double)p * 4294967296.0;

@@ -134,43 +134,6 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
       : "memory");
 }
 
-// 4 x 4 transpose of 16-byte chunks among four neighbouring lanes: lane i of four has chunks 0..3 of its row and leaves with
-// chunk i of the four rows.
-__device__ __forceinline__ uint4 sel4(bool a, const uint4& x, const uint4& y) {
-  return make_uint4(a ? x.x : y.x, a ? x.y : y.y, a ? x.z : y.z, a ? x.w : y.w);
-}
-__device__ __forceinline__ uint4 shfl4(const uint4& v, int d) {
-  return make_uint4(__shfl_xor_sync(0xffffffffu, v.x, d), __shfl_xor_sync(0xffffffffu, v.y, d), __shfl_xor_sync(0xffffffffu, v.z, d),
-                    __shfl_xor_sync(0xffffffffu, v.w, d));
-}
-__device__ __forceinline__ void transpose4(uint4 (&v)[4], int lane) {
-#pragma unroll
-  for (int d = 1; d < 4; d *= 2) {
-    const bool up = lane & d;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (k & d) continue;
-      const uint4 got = shfl4(sel4(up, v[k], v[k + d]), d);      // what the partner needs of this pair goes to it
-      if (up) v[k] = got; else v[k + d] = got;
-    }
-  }
-}
-// 32 columns of a warp's 32 rows to global memory as bf16: four lanes write 64 consecutive bytes of a row.  One row a thread, 16
-// bytes at a time, the 32 lanes of each store touched 32 lines (with it 288 -> 280 us, backward of 4 x 16 heads of 2048 x 128).  `rows` of the warp's rows are there; dst: row 0.
-__device__ __forceinline__ void store_rows32(__nv_bfloat16* dst, long long pitch, int rows, const float* o, int lane) {
-  uint4 v[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k)
-    v[k] = make_uint4(pack_bf16(o[8 * k], o[8 * k + 1]), pack_bf16(o[8 * k + 2], o[8 * k + 3]), pack_bf16(o[8 * k + 4], o[8 * k + 5]),
-                      pack_bf16(o[8 * k + 6], o[8 * k + 7]));
-  transpose4(v, lane);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int r = (lane & ~3) + k;
-    if (r < rows) *reinterpret_cast<uint4*>(dst + r * pitch + (lane & 3) * 8) = v[k];
-  }
-}
-
 // Loads one [128 rows x 64 * SUB columns] tile of a (batch, head) into SUB swizzled sub-tiles.
 template <int SUB>
 __device__ __forceinline__ void load_tile(uint32_t dst, const CUtensorMap* map, int seq1, int col, int b, int s0,
