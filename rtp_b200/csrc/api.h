@@ -116,6 +116,8 @@ typedef struct {
   const void* x; long long ldx;
   void* y; long long ldy;
   int act;
+  const int* fill;                     // optional, device [n_local * world]: rows of each expert's cap that hold tokens; the
+                                       // others get zeros, or (1-rank ring only: a hint) what the product makes of them
 } RtpExpertFwd;
 int rtp_expert_fwd(const RtpRing* ring, const RtpExpertFwd* op, void* stream);
 typedef struct {
@@ -127,6 +129,7 @@ typedef struct {
   void* grad_home;                     // same layout as home
   const float* dbias_full;             // fp32 [world*n_local, out] per-expert column sums of dy (null: no bias)
   const void* mask; long long ldmask; float mask_scale;   // optional activation backward applied to dx
+  const int* fill;                     // as in RtpExpertFwd; rows of dy beyond it are zero, those of dx become zero
 } RtpExpertBwd;
 int rtp_expert_bwd(const RtpRing* ring, const RtpExpertBwd* op, void* stream);
 // 1 if the launch makes the experts' bias gradients itself when dbias_full is null (1-rank ring, aligned operands).

@@ -1165,6 +1165,7 @@ int local_expert_fwd(const RtpRing& R, const RtpExpertFwd& op, rtp::LocalGemm* j
     j[e].d = reinterpret_cast<__nv_bfloat16*>(op.y) + (long long)e * op.cap * op.ldy; j[e].ldd = op.ldy;
     if (op.bias_off >= 0) j[e].bias = w + op.bias_off;
     j[e].act = op.act;
+    if (op.fill && !op.act) j[e].m_fill = op.fill + e;
   }
   return all_ok(j, op.n_local) ? op.n_local : 0;
 }
@@ -1180,11 +1181,14 @@ int local_expert_bwd(const RtpRing& R, const RtpExpertBwd& op, rtp::LocalGemm* j
     w.M = op.out_features; w.N = op.in_features; w.K = op.cap;
     w.d = g; w.ldd = op.in_features;
     if (op.bias_off >= 0) w.bsum = g + op.bias_off;
+    const int* fill = op.fill && !op.mask ? op.fill + e : nullptr;
+    w.k_fill = fill;
     if (!op.dx) continue;
     rtp::LocalGemm& d = j[n++] = rtp::LocalGemm{};
     d.a = dy; d.lda = op.ldy;
     d.b = reinterpret_cast<const __nv_bfloat16*>(op.home) + e * op.expert_stride; d.ldb = op.in_features; d.b_mn = 1;
     d.M = op.cap; d.N = op.in_features; d.K = op.out_features;
+    d.m_fill = fill;
     d.d = reinterpret_cast<__nv_bfloat16*>(op.dx) + (long long)e * op.cap * op.lddx; d.ldd = op.lddx;
     if (op.mask) {
       d.mask = reinterpret_cast<const __nv_bfloat16*>(op.mask) + (long long)e * op.cap * op.ldmask;

@@ -61,6 +61,7 @@ struct alignas(64) Job {
   int sum;                                       // 1: d[m] = sum_k A[m, k] (+ c[m]); B is the tile of ones, bn = 16
   unsigned long long seed, offset;
   const unsigned long long* step_ptr;
+  const int *m_fill, *k_fill;                    // see LocalGemm
 };
 
 template <int MAXJ>
@@ -107,11 +108,24 @@ __device__ __forceinline__ void add8(float* v, const uint4& u) {
   v[4] += bf16_lo(u.z); v[5] += bf16_hi(u.z); v[6] += bf16_lo(u.w); v[7] += bf16_hi(u.w);
 }
 
+// k-blocks of a tile whose first row is row0; 0: nothing to do but to write zeros
+template <bool FILL>
+__device__ __forceinline__ int tile_kblocks(const Job& J, int row0) {
+  int n = J.kblocks;
+  if constexpr (FILL) {
+    if (J.m_fill && row0 >= __ldg(J.m_fill)) n = 0;
+    if (J.k_fill) n = min(n, (__ldg(J.k_fill) + 63) >> 6);
+  }
+  return n;
+}
+
+// FILL: a job has rows that are not in use (the padded capacity of experts: 8 experts of 2560 rows of which 2048 are filled,
+// 2048 <-> 8192, forward and backward @FILL@).
 // SRC: a job adds to its output or masks it; FUN: a job has an activation or dropout.  Merely branched over, that code cost every
 // launch: twice the spills, and a fifth of the epilogue's time went into instruction fetch.  With it compiled out and both
 // halves of a row's 64 columns fetched at once (us, before -> now): 256 x 64 -> 256 4.5 -> 3.4, 1024 x 512 -> 512 6.6 -> 5.5,
 // 1024 x 2048 -> 2048 13.4 -> 12.4, 8192 x 8 -> 8192 73 -> 45, 36864 x 64 -> 288 20 -> 13.6; added to its output 25 -> 21.
-template <bool PAIR, int MAXJ, bool SRC, bool FUN>
+template <bool PAIR, int MAXJ, bool SRC, bool FUN, bool FILL>
 __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_constant__ Params<MAXJ> P) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -185,7 +199,7 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
         const int nb = b_mn ? bn_cta >> 6 : 1;
         const bool sum = J.sum;                     // B is already in shared memory
         const uint32_t tx = sum ? kABytesL : kABytesL + bn_cta * kKB * 2;
-        const int kblocks = J.kblocks;
+        const int kblocks = tile_kblocks<FILL>(J, tm * TM);
         for (int kb = 0; kb < kblocks; ++kb) {
           if (!mbar_wait_s(empty_s + stage * 8, phase ^ 1, abort_flag, status, tmo)) { ok = false; break; }
           const uint32_t sa = tiles_s + stage * stage_bytes, sb = sa + kABytesL, bar = full_s + stage * 8;
@@ -227,10 +241,17 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
         if (r * units >= total) break;
         if (t >= total) continue;
         const Job& J = P.job[find_job(P, t)];
+        int row0 = 0;
+        if constexpr (FILL) {
+          int tm, tn;
+          tile_pos(J, t - J.tile0, tm, tn);
+          row0 = tm * TM;
+        }
+        const int kblocks = tile_kblocks<FILL>(J, row0);
+        if (FILL && !kblocks) continue;
         const uint32_t idesc = make_idesc_bf16(TM, J.bn, J.a_mn, J.b_mn);
         const uint32_t a_step = J.a_mn ? 128u : 2u, b_step = J.b_mn ? 128u : 2u;    // 16 elements of k, in 16-byte units
         const uint64_t da0 = make_smem_desc(0, J.a_mn ? 8192u : 16u, 1024), db0 = make_smem_desc(0, J.b_mn ? 8192u : 16u, 1024);
-        const int kblocks = J.kblocks;
         const uint32_t ones = J.sum ? (tiles_s + P.ones_off) >> 4 : 0u;
         if (!mbar_wait(&ctl->tmem_empty[acc], acc_phase ^ 1, abort_flag, status, tmo)) { ok = false; break; }
         tc_fence_after();
@@ -273,7 +294,14 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
         const int t = unit_tile(r, unit, units);
         if (r * units >= total) break;
         if (t >= total) continue;
-        const int kblocks = P.job[find_job(P, t)].kblocks;
+        const Job& J = P.job[find_job(P, t)];
+        int row0 = 0;
+        if constexpr (FILL) {
+          int tm, tn;
+          tile_pos(J, t - J.tile0, tm, tn);
+          row0 = tm * TM;
+        }
+        const int kblocks = tile_kblocks<FILL>(J, row0);
         for (int kb = 0; kb < kblocks; ++kb) {
           if (!mbar_wait_s(full_s + stage * 8, phase, abort_flag, status, tmo)) { ok = false; break; }
           mbar_arrive_cluster(lead + stage * 8);
@@ -312,6 +340,21 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
       [[maybe_unused]] const uint32_t thresh = J.drop_thresh;
       [[maybe_unused]] unsigned long long drop_off = 0;
       if constexpr (FUN) drop_off = J.offset + (J.step_ptr ? __ldg(J.step_ptr) * 65536ull : 0ull);
+      if constexpr (FILL) {
+        if (!tile_kblocks<FILL>(J, tm * TM)) {               // no accumulator: zeros
+          if (J.sum) {
+            if (half == 0 && row0 + lane < M) d[row0 + lane] = __float2bfloat16(0.f);
+          } else {
+            for (int ch = half; ch * 64 < bn; ch += 2)
+#pragma unroll
+              for (int k = 0; k < 8; ++k) {
+                const int row = row0 + 4 * k + (lane >> 3), col = n0 + ch * 64 + (lane & 7) * 8;
+                if (row < M && col < N) *reinterpret_cast<uint4*>(d + (long long)row * ldd + col) = make_uint4(0u, 0u, 0u, 0u);
+              }
+          }
+          continue;
+        }
+      }
       bool waited = false;
       if (J.sum && half == 0) {
         uint32_t good = 1;
@@ -637,9 +680,9 @@ long long makespan(const Item* it, int n, const TileShape* const* sh, int units,
   return best + epi;
 }
 
-template <bool PAIR, int MAXJ, bool SRC, bool FUN>
+template <bool PAIR, int MAXJ, bool SRC, bool FUN, bool FILL = false>
 int launch_local(const Params<MAXJ>& P, cudaStream_t stream) {
-  if (ensure_smem<local_gemm_kernel<PAIR, MAXJ, SRC, FUN>>(kSmem) != cudaSuccess) return lfail("cudaFuncSetAttribute failed");
+  if (ensure_smem<local_gemm_kernel<PAIR, MAXJ, SRC, FUN, FILL>>(kSmem) != cudaSuccess) return lfail("cudaFuncSetAttribute failed");
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(PAIR ? 2 * P.units : P.units);
   cfg.blockDim = dim3(kThreads);
@@ -659,7 +702,7 @@ int launch_local(const Params<MAXJ>& P, cudaStream_t stream) {
   }
   cfg.attrs = at;
   cfg.numAttrs = nat;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, local_gemm_kernel<PAIR, MAXJ, SRC, FUN>, P);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, local_gemm_kernel<PAIR, MAXJ, SRC, FUN, FILL>, P);
   return e == cudaSuccess ? 0 : lfail(std::string("launch local_gemm_kernel: ") + cudaGetErrorString(e));
 }
 
@@ -708,11 +751,12 @@ int run(const Item* it, int n, int pair_policy, unsigned long long* status, unsi
   memset(static_cast<void*>(&P), 0, sizeof(P));
   const int tm = pair ? 256 : 128;
   int widest = 0, total = 0;
-  bool sums = false, src = false, fun = false;
+  bool sums = false, src = false, fun = false, fill = false;
   for (int q = 0; q < n; ++q) {
     const LocalGemm& x = *it[best_ord[q]].g;
     src = src || x.c || x.mask;
     fun = fun || x.act || x.drop_p > 0.f;
+    fill = fill || x.m_fill || x.k_fill;
     Job& J = P.job[q];
     J.sum = it[best_ord[q]].sum ? 1 : 0;
     J.part = x.part;
@@ -721,6 +765,8 @@ int run(const Item* it, int n, int pair_policy, unsigned long long* status, unsi
     J.tiles_m = (x.M + tm - 1) / tm;
     J.group = 8;
     J.a_mn = (unsigned char)x.a_mn;
+    J.m_fill = J.sum ? nullptr : x.m_fill;
+    J.k_fill = x.k_fill;
     if (operand_map(&J.ma, &J.a3, x.a, x.M, x.K, x.lda, x.a_mn, 128)) return -1;
     if (J.sum) {
       sums = true;
@@ -761,6 +807,10 @@ int run(const Item* it, int n, int pair_policy, unsigned long long* status, unsi
     P.ones_off = pair ? kArea + kStageOut : P.stages * P.stage_bytes;
   }
   P.status = status; P.timeout_ns = 2 * timeout_ns;
+  if (fill) {
+    if (src || fun) return lfail("local_gemm: rows in use go with plain jobs only");
+    return pair ? launch_local<true, MAXJ, false, false, true>(P, stream) : launch_local<false, MAXJ, false, false, true>(P, stream);
+  }
 #define RTP_LOCAL(SRC, FUN) (pair ? launch_local<true, MAXJ, SRC, FUN>(P, stream) : launch_local<false, MAXJ, SRC, FUN>(P, stream))
   return src ? (fun ? RTP_LOCAL(true, true) : RTP_LOCAL(true, false)) : (fun ? RTP_LOCAL(false, true) : RTP_LOCAL(false, false));
 #undef RTP_LOCAL
@@ -795,6 +845,7 @@ bool local_gemm_ok(const LocalGemm& g) {
   if (!al16(g.d) || g.ldd % 8 || !al16(g.c) || !al16(g.mask) || !al16(g.bias)) return false;
   if ((g.c && g.ldc % 8) || (g.mask && g.ldmask % 8)) return false;
   if (g.part && (g.c || g.bias || g.act || g.mask || g.drop_p > 0.f || g.bsum_add)) return false;
+  if ((g.m_fill || g.k_fill) && (g.c || g.act || g.mask || g.drop_p > 0.f || g.bsum_add || g.part)) return false;
   return !g.bsum || g.a_mn;
 }
 

@@ -26,6 +26,11 @@ struct LocalGemm {
   // 1: d and bsum are fp32 and receive the bare sums (no c, bias, activation, mask or dropout): one slice of a contraction
   // that local_reduce adds up
   int part;
+  // Rows that are in use, known on the device only (expert capacities).  m_fill: output rows from there on get zeros, whatever A
+  // holds; k_fill: elements of the contraction, of which those from there on contribute nothing (A or B is zero there) and up
+  // to the next multiple of 64 are finite.  A launch with one of them has no c, mask, activation or dropout.
+  const int* m_fill;
+  const int* k_fill;
 };
 
 // Whether the local kernels take this job (16-byte aligned rows, N a multiple of 8).

@@ -1350,14 +1350,20 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* g, const __nv_bfloat16* u
 
 // ------------------------------------------------------------------------------------------------
 // MoE token movement by index (top-2): slot[s, k] is the destination row (expert * capacity + position) of choice k
-// of token s, or -1.  One warp per (token, choice).  M % 8 == 0.
+// of token s, or -1.  One warp per (token, choice).  M % 8 == 0.  fill (may be null): for each group of `cap` destination rows
+// one more than its last row that a token went to (zeroed by the caller).
 // ------------------------------------------------------------------------------------------------
 __global__ void moe_scatter_kernel(const __nv_bfloat16* __restrict__ src, const int* __restrict__ slot,
-                                   const float* __restrict__ scale, __nv_bfloat16* __restrict__ dst, int S, int M) {
+                                   const float* __restrict__ scale, __nv_bfloat16* __restrict__ dst, int S, int M,
+                                   int* fill, int cap) {
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (w >= 2 * S) return;
   const int sl = slot[w];
   if (sl < 0) return;
+  if (fill && lane == 0) {
+    const int e = sl / cap, n = sl - e * cap + 1;
+    if (n > *reinterpret_cast<volatile int*>(fill + e)) atomicMax(fill + e, n);      // few get here: slots rise with the tokens
+  }
   const float sc = scale ? scale[w] : 1.f;
   const __nv_bfloat16* a = src + (size_t)(w >> 1) * M;
   __nv_bfloat16* d = dst + (size_t)sl * M;
@@ -1728,13 +1734,15 @@ int rtp_swiglu_bwd(const void* g, const void* u, long long ld, const void* dy, v
   return 0;
 }
 int rtp_moe_scatter(const void* src, const int* slot, const float* scale, void* dst, int S, int M, long long dst_rows,
-                    void* stream) {
+                    int* fill, int cap, void* stream) {
   if (M % 8) { k_err = "moe: M must be a multiple of 8"; return -1; }
+  if (fill && (cap <= 0 || dst_rows % cap)) { k_err = "moe: rows must be whole capacities"; return -1; }
   cudaError_t e = cudaMemsetAsync(dst, 0, (size_t)dst_rows * M * 2, (cudaStream_t)stream);
+  if (e == cudaSuccess && fill) e = cudaMemsetAsync(fill, 0, (size_t)(dst_rows / cap) * sizeof(int), (cudaStream_t)stream);
   if (e != cudaSuccess) return kfail("moe memset", e);
   const long long threads = 2ll * S * 32;
   moe_scatter_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)src, slot, scale, (__nv_bfloat16*)dst, S, M);
+      (const __nv_bfloat16*)src, slot, scale, (__nv_bfloat16*)dst, S, M, fill, cap);
   LAUNCH_CHECK("moe_scatter");
   return 0;
 }

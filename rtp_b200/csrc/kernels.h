@@ -92,7 +92,7 @@ int rtp_swiglu_fwd(const void* g, const void* u, long long ld, void* y, long lon
 int rtp_swiglu_bwd(const void* g, const void* u, long long ld, const void* dy, void* dg, void* du, long long ldo,
                    long long rows, int cols, void* stream);
 int rtp_moe_scatter(const void* src, const int* slot, const float* scale, void* dst, int S, int M, long long dst_rows,
-                    void* stream);
+                    int* fill, int cap, void* stream);
 int rtp_moe_gather(const void* src, const int* slot, const float* scale, void* dst, int S, int M, void* stream);
 int rtp_moe_rowdot(const void* a, const void* b, const int* slot, float* out, int S, int M, void* stream);
 int rtp_add(const void* a, const void* b, void* out, long long n, void* stream);

@@ -101,6 +101,7 @@ class ExpertFwd(C.Structure):
         ("cap", C.c_int), ("n_local", C.c_int), ("in_features", C.c_int), ("out_features", C.c_int),
         ("home", C.c_void_p), ("expert_stride", C.c_longlong), ("bias_off", C.c_longlong), ("shard_bytes", C.c_ulonglong),
         ("x", C.c_void_p), ("ldx", C.c_longlong), ("y", C.c_void_p), ("ldy", C.c_longlong), ("act", C.c_int),
+        ("fill", C.c_void_p),
     ]
 
 
@@ -110,7 +111,7 @@ class ExpertBwd(C.Structure):
         ("home", C.c_void_p), ("expert_stride", C.c_longlong), ("bias_off", C.c_longlong), ("shard_bytes", C.c_ulonglong),
         ("x", C.c_void_p), ("ldx", C.c_longlong), ("dy", C.c_void_p), ("ldy", C.c_longlong),
         ("dx", C.c_void_p), ("lddx", C.c_longlong), ("grad_home", C.c_void_p), ("dbias_full", C.c_void_p),
-        ("mask", C.c_void_p), ("ldmask", C.c_longlong), ("mask_scale", C.c_float),
+        ("mask", C.c_void_p), ("ldmask", C.c_longlong), ("mask_scale", C.c_float), ("fill", C.c_void_p),
     ]
 
 

@@ -44,7 +44,7 @@ def _L():
         L.rtp_col2im.argtypes = [vp, vp] + [i] * 13 + [vp]
         L.rtp_adam.argtypes = [vp, vp, i, i, vp, f, f, f, f, f, i, f, f, vp, vp]
         L.rtp_add.argtypes = [vp, vp, vp, ll, vp]
-        L.rtp_moe_scatter.argtypes = [vp, vp, vp, vp, i, i, ll, vp]
+        L.rtp_moe_scatter.argtypes = [vp, vp, vp, vp, i, i, ll, vp, i, vp]
         L.rtp_moe_gather.argtypes = [vp, vp, vp, vp, i, i, vp]
         L.rtp_moe_rowdot.argtypes = [vp, vp, vp, vp, i, i, vp]
         L.rtp_gelu_fwd.argtypes = [vp, vp, ll, vp]
@@ -282,11 +282,14 @@ def swiglu_packed_bwd(y, dy, nshard):
     return dp
 
 
-def moe_scatter(src, slot, scale, dst_rows):
-    """dst[slot[s, k]] = scale[s, k] * src[s] (rows without a token stay zero). slot: int32 [S, 2], -1 = dropped."""
+def moe_scatter(src, slot, scale, dst_rows, fill=None):
+    """dst[slot[s, k]] = scale[s, k] * src[s] (rows without a token stay zero). slot: int32 [S, 2], -1 = dropped.
+    ``fill``: int32 [E] that receives, for each of E equal groups of rows, the number of rows up to the last one with a token."""
     S, M = src.shape
     dst = torch.empty(dst_rows, M, dtype=src.dtype, device=src.device)
-    _check(_L().rtp_moe_scatter(_p(src), _p(slot), _p(scale), _p(dst), S, M, dst_rows, _lib.stream_ptr()), "moe_scatter")
+    cap = dst_rows // fill.numel() if fill is not None else 0
+    _check(_L().rtp_moe_scatter(_p(src), _p(slot), _p(scale), _p(dst), S, M, dst_rows, _p(fill), cap, _lib.stream_ptr()),
+           "moe_scatter")
     return dst
 
 

@@ -16,14 +16,16 @@ def _slots(idx, loc, valid, capacity):
 
 class _Dispatch(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, slot, rows):
+    def forward(ctx, x, slot, rows, num_experts):
         ctx.save_for_backward(slot)
-        return K.moe_scatter(x.contiguous(), slot, None, rows)
+        fill = torch.empty(num_experts, dtype=torch.int32, device=x.device)
+        ctx.mark_non_differentiable(fill)
+        return K.moe_scatter(x.contiguous(), slot, None, rows, fill), fill
 
     @staticmethod
-    def backward(ctx, g):
+    def backward(ctx, g, _):
         (slot,) = ctx.saved_tensors
-        return K.moe_gather(g.contiguous(), slot, None), None, None
+        return K.moe_gather(g.contiguous(), slot, None), None, None, None
 
 
 class _Combine(torch.autograd.Function):
@@ -45,8 +47,17 @@ class _Combine(torch.autograd.Function):
 
 def dispatch(x, idx, loc, valid, num_experts, capacity):
     slot = _slots(idx, loc, valid, capacity)
-    out = _Dispatch.apply(x, slot, num_experts * capacity)
-    return out.view(num_experts, capacity, x.shape[1])
+    out, fill = _Dispatch.apply(x, slot, num_experts * capacity, num_experts)
+    out = out.view(num_experts, capacity, x.shape[1])
+    out._rtp_fill = (fill, out._version)     # holds as long as nobody writes to the rows (see rows_in_use)
+    return out
+
+
+def rows_in_use(dispatched):
+    """int32 [E]: for each expert of a tensor made by :func:`dispatch` the rows up to the last one with a token (those behind it
+    are zeros), or None where that is not known or the tensor has been written to since."""
+    fill, version = getattr(dispatched, "_rtp_fill", (None, None))
+    return fill if fill is not None and dispatched._version == version else None
 
 
 def combine(expert_output, idx, loc, gate, valid):

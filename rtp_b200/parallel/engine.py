@@ -864,12 +864,13 @@ def _mha_inplace(owner, sub, x, is_causal, attn_mask, key_padding_mask, training
 # --------------------------------------------------------------------------------------------------
 class _FusedExpertLinearFn(torch.autograd.Function):
     """x: [E_total, cap, in] (dispatched tokens, expert-major) -> [E_total, cap, out].  ``spec`` = (ring, flat range,
-    n_local, in_f, out_f, expert_stride, bias_off, places) with places = [(offset, numel, shape)] of the given
-    parameters inside the flat range (order: e0.weight, e0.bias, e1.weight, ...)."""
+    n_local, in_f, out_f, expert_stride, bias_off, places, fill) with places = [(offset, numel, shape)] of the given
+    parameters inside the flat range (order: e0.weight, e0.bias, e1.weight, ...) and fill = None or the rows of each expert
+    that hold tokens: what becomes of the others reaches neither the layer's output nor a gradient."""
 
     @staticmethod
     def forward(ctx, spec, x, *params):
-        ring, flat, L, in_f, out_f, stride, bias_off, places = spec
+        ring, flat, L, in_f, out_f, stride, bias_off, places, fill = spec
         eng = get_engine(ring)
         E, cap, _ = x.shape
         x2 = x.reshape(E * cap, in_f).contiguous()
@@ -879,6 +880,7 @@ class _FusedExpertLinearFn(torch.autograd.Function):
         op.home, op.expert_stride, op.bias_off = flat.data_ptr(), stride, bias_off
         op.shard_bytes = _round_up(flat.numel() * 2, 16)
         op.x, op.ldx, op.y, op.ldy, op.act = x2.data_ptr(), in_f, y.data_ptr(), out_f, 0
+        op.fill = fill.data_ptr() if fill is not None else None
         _lib.check(_lib.lib().rtp_expert_fwd(C.byref(eng.ring), C.byref(op), _lib.stream_ptr()), "rtp_expert_fwd")
         ctx.spec, ctx.eng = spec, eng
         ctx.save_for_backward(x2)
@@ -887,7 +889,7 @@ class _FusedExpertLinearFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        ring, flat, L, in_f, out_f, stride, bias_off, places = ctx.spec
+        ring, flat, L, in_f, out_f, stride, bias_off, places, fill = ctx.spec
         (x2,) = ctx.saved_tensors
         E, cap = ctx.dims
         dy2 = dy.reshape(E * cap, out_f).contiguous()
@@ -902,6 +904,7 @@ class _FusedExpertLinearFn(torch.autograd.Function):
         if dx is not None:
             op.dx, op.lddx = dx.data_ptr(), in_f
         op.grad_home = gflat.data_ptr()
+        op.fill = fill.data_ptr() if fill is not None else None
         if bias_off >= 0 and not _lib.lib().rtp_expert_bwd_folds_bias(C.byref(ctx.eng.ring), C.byref(op)):
             dbias = torch.empty(E, out_f, dtype=torch.float32, device=dy.device)
             for g in range(E):
@@ -916,6 +919,8 @@ def fused_experts(module, dispatched):
     """Both linears of every (rotating) expert on the fused kernels; the activation in between is an elementwise
     kernel.  ``module`` is a ``WeightMOELayer`` whose experts expose ``linear1`` / ``linear2`` / ``activation``."""
     from ..ops import functional as FO
+    from ..ops.moe import rows_in_use
+    fill = rows_in_use(dispatched) if module.ring.world == 1 else None
     lay, flat = module._layout, module._full_param
     L = module.num_local_experts
     experts = list(module.experts)
@@ -934,7 +939,7 @@ def fused_experts(module, dispatched):
                 p = getattr(getattr(experts[e], layer), nm)
                 places.append((lay.offset_of(f"{e}.{layer}.{nm}") - off0, p.numel(), p.shape))
                 params.append(p)
-        return (module.ring, rng, L, in_f, out_f, stride, bias_off, places), params
+        return (module.ring, rng, L, in_f, out_f, stride, bias_off, places, fill), params
 
     s1, p1 = spec_for("linear1")
     s2, p2 = spec_for("linear2")

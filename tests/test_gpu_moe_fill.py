@@ -1,0 +1,62 @@
+"""Experts whose capacity is not full: rows that hold no token are left out of the products (csrc/gemm_local.cu), at numbers of
+tokens around the edges of its tiles and k-blocks, an expert without any and one that is full.
+
+Tolerance: outputs and gradients are compared with the same layer on a copy of the dispatched tensor, which is not known to have
+unused rows: the same sums of the same products, apart from zeros,
+which tiles of another shape may round differently once (2^-7 of the value), and once more on the way through the hidden layer."""
+import pytest
+import torch
+import torch.nn as nn
+
+pytestmark = pytest.mark.gpu
+BF = torch.bfloat16
+
+
+@pytest.mark.parametrize("E,cap,D,H,counts", [(2, 320, 72, 200, (0, 320)), (4, 320, 72, 200, (1, 63, 64, 65)),
+                                              (4, 640, 136, 264, (127, 128, 129, 256)), (8, 1280, 512, 1024, (0, 1, 257, 600, 640, 1000, 1279, 1280))])
+def test_unused_rows(E, cap, D, H, counts):
+    from rtp_b200.module.moe import WeightMOELayer, combine_by_index, dispatch_by_index
+    from rtp_b200.ops.moe import rows_in_use
+    from rtp_b200.parallel.engine import fused_experts
+    torch.manual_seed(cap)
+
+    class Expert(nn.Module):
+        def __init__(self):
+            super().__init__()
+            self.linear1, self.linear2, self.activation = nn.Linear(D, H), nn.Linear(H, D), nn.GELU()
+    layer = WeightMOELayer(nn.Identity(), nn.ModuleList([Expert() for _ in range(E)]), device="cuda", dtype=BF)
+    # tokens in random order, each with one choice (the other is dropped), expert e taking counts[e] of them
+    idx = torch.cat([torch.full((n,), e) for e, n in enumerate(counts)])
+    loc = torch.cat([torch.arange(n) for n in counts])
+    perm = torch.randperm(idx.numel())
+    idx, loc = idx[perm], loc[perm]
+    S = idx.numel()
+    pair = torch.stack([idx, torch.zeros_like(idx)], 1).cuda(), torch.stack([loc, torch.zeros_like(loc)], 1).cuda()
+    valid = torch.tensor([True, False]).expand(S, 2).cuda()
+    gate = torch.rand(S, 2, device="cuda")
+    x = torch.randn(S, D, device="cuda").to(BF).requires_grad_()
+    dy = torch.randn(S, D, device="cuda").to(BF)
+    params = list(layer.experts.parameters())
+    results = []
+    for known in (True, False):
+        d = dispatch_by_index(x, *pair, valid, E, cap)
+        fill = rows_in_use(d)
+        assert fill.tolist() == list(counts)
+        if not known:
+            d = d.clone()
+            assert rows_in_use(d) is None
+        y = combine_by_index(fused_experts(layer, d), *pair, gate, valid)
+        results.append([y.detach(), *torch.autograd.grad(y, [x, *params], dy)])
+    for a, b in zip(*results):
+        assert a.isfinite().all()
+        assert bool(((a.double() - b.double()).abs() <= 2.0 ** -7 * b.double().abs() + 1e-3 * b.double().abs().max()).all())
+
+
+def test_written_rows_count():
+    from rtp_b200.ops.moe import dispatch, rows_in_use
+    x = torch.randn(8, 64, device="cuda").to(BF)
+    idx, loc = torch.zeros(8, 2, dtype=torch.long, device="cuda"), torch.arange(16, device="cuda").view(8, 2)
+    d = dispatch(x, idx, loc, torch.ones(8, 2, dtype=torch.bool, device="cuda"), 2, 32)
+    assert rows_in_use(d).tolist() == [16, 0]
+    d[1, 3] = 1
+    assert rows_in_use(d) is None
