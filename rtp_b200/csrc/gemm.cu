@@ -1122,35 +1122,30 @@ int local_linear_bwd(const RtpRing& R, const RtpLinearBwd& op, rtp::LocalGemm* j
 }
 // A weight gradient of a few tiles whose contraction runs over many tokens (a convolution's: [64, 288] over 36 864
 // positions) keeps a handful of SMs busy for hundreds of k-blocks.  Where its 128 x 128 tiles fill at most an eighth of the
-// SMs and each has 128 k-blocks or more, the contraction falls into eight slices that leave fp32 sums in a workspace.
-// Whole backward, cold L2, unsplit -> split: that convolution 187 -> 78 us (weights alone 165 -> 39), 512 x 512 over 36 864
-// 185 -> 84, 768 x 384 over 8 192 (18 tiles, the most that split) 50 -> 44.  Over 4 096 positions the launches that add up
-// the slices cost more than they save: [64, 288] 27.6 -> 29.7, 768 x 384 28.2 -> 36.9.
-constexpr int kWgradSlices = 8;
-long long part_stride(const rtp::LocalGemm& w) { return (long long)w.M * w.N + (w.bsum ? (w.M + 3) / 4 * 4 : 0); }
-bool splits_wgrad(const rtp::LocalGemm& w) {
-  const long long tiles = (long long)((w.M + 127) / 128) * ((w.N + 127) / 128);
-  return !w.c && !w.bsum_add && tiles * 8 <= sm_count() && w.K >= 128 * 64;
+// SMs and each has 128 k-blocks or more, the contraction falls into slices that leave fp32 sums in a workspace: as many as give
+// every SM one, of eight k-blocks or more, so that the tiles of the input gradient go on in whole rounds behind them.
+// Whole backward, cold L2, unsplit -> eight slices: that convolution 187 -> 78 us, 512 x 512 over 36 864 185 -> 84,
+// 768 x 384 over 8 192 (18 tiles, the most that split) 50 -> 44; eight slices -> this, warm: 54 -> 38, 71 -> 54, 28 -> 22.  Over 4 096 positions the launch that adds up
+// the slices cost more than it saved (eight slices): [64, 288] 27.6 -> 29.7, 768 x 384 28.2 -> 36.9.
+long long part_stride(const rtp::LocalGemm& w) { return ((long long)w.M * w.N + 3) / 4 * 4 + (w.bsum ? (w.M + 3) / 4 * 4 : 0); }
+long long wgrad_tiles(const rtp::LocalGemm& w) { return (long long)((w.M + 127) / 128) * ((w.N + 127) / 128); }
+bool splits_wgrad(const rtp::LocalGemm& w) { return !w.c && !w.bsum_add && wgrad_tiles(w) * 8 <= sm_count() && w.K >= 128 * 64; }
+int wgrad_slices(const rtp::LocalGemm& w) {
+  const int kb = (w.K + 63) / 64, want = (int)std::max(1ll, std::min<long long>(sm_count() / wgrad_tiles(w), kb / 8));
+  const int per = (kb + want - 1) / want;
+  return (kb + per - 1) / per;                   // none without a k-block
 }
-int run_split_bwd(const RtpRing& R, const RtpLinearBwd& op, const rtp::LocalGemm* j, int n, void* stream) {
-  rtp::LocalGemm all[rtp::kLocalMaxJobs];
-  const rtp::LocalGemm& w = j[0];
+int run_split_bwd(const RtpRing& R, const RtpLinearBwd& op, rtp::LocalGemm* j, int n, void* stream) {
+  rtp::LocalGemm& w = j[0];
+  const long long stride = part_stride(w), off = ((long long)w.M * w.N + 3) / 4 * 4;
+  void *d = w.d, *bsum = w.bsum;
   float* part = reinterpret_cast<float*>(op.scratch);
-  const long long stride = part_stride(w);
-  const int per = ((w.K + 63) / 64 + kWgradSlices - 1) / kWgradSlices * 64;      // k of a slice
-  int m = 0, slices = 0;
-  for (int k0 = 0; k0 < w.K; k0 += per, ++slices) {
-    rtp::LocalGemm& x = all[m++] = w;
-    x.a = reinterpret_cast<const __nv_bfloat16*>(w.a) + (long long)k0 * w.lda;
-    x.b = reinterpret_cast<const __nv_bfloat16*>(w.b) + (long long)k0 * w.ldb;
-    x.K = std::min(per, w.K - k0);
-    x.d = part + slices * stride; x.ldd = w.N; x.part = 1;
-    if (w.bsum) x.bsum = part + slices * stride + (long long)w.M * w.N;
-  }
-  for (int i = 1; i < n; ++i) all[m++] = j[i];
-  if (run_local(R, all, m, stream)) return -1;
-  if (rtp::local_reduce(part, slices, stride, w.d, (long long)w.M * w.N, (cudaStream_t)stream) ||
-      (w.bsum && rtp::local_reduce(part + (long long)w.M * w.N, slices, stride, w.bsum, w.M, (cudaStream_t)stream)))
+  w.part = wgrad_slices(w);
+  w.part_stride = stride;
+  w.d = part; w.ldd = w.N;
+  if (bsum) w.bsum = part + off;
+  if (run_local(R, j, n, stream)) return -1;
+  if (rtp::local_reduce(part, w.part, stride, d, (long long)w.M * w.N, off, bsum, bsum ? w.M : 0, (cudaStream_t)stream))
     return fail(rtp::local_gemm_error());
   return 0;
 }
@@ -1603,7 +1598,7 @@ int rtp_linear_bwd(const RtpRing* ring, const RtpLinearBwd* op, void* stream) {
   rtp::LocalGemm jobs[rtp::kLocalMaxJobs];
   if (const int n = local_linear_bwd(*ring, *op, jobs)) {
     if (op->scratch && splits_wgrad(jobs[0]) && (reinterpret_cast<uintptr_t>(op->scratch) & 15) == 0 &&
-        op->scratch_bytes >= (unsigned long long)(kWgradSlices * part_stride(jobs[0]) * 4))
+        op->scratch_bytes >= (unsigned long long)(wgrad_slices(jobs[0]) * part_stride(jobs[0]) * 4))
       return run_split_bwd(*ring, *op, jobs, n, stream);
     return run_local(*ring, jobs, n, stream);
   }
@@ -1619,7 +1614,7 @@ int rtp_linear_bwd(const RtpRing* ring, const RtpLinearBwd* op, void* stream) {
 unsigned long long rtp_linear_bwd_scratch(const RtpRing* ring, const RtpLinearBwd* op) {
   rtp::LocalGemm jobs[rtp::kLocalMaxJobs];
   if (!local_linear_bwd(*ring, *op, jobs) || !splits_wgrad(jobs[0])) return 0;
-  return (unsigned long long)(kWgradSlices * part_stride(jobs[0]) * 4);
+  return (unsigned long long)(wgrad_slices(jobs[0]) * part_stride(jobs[0]) * 4);
 }
 int rtp_linear_bwd_folds_bias(const RtpRing* ring, const RtpLinearBwd* op) {
   rtp::LocalGemm jobs[rtp::kLocalMaxJobs];

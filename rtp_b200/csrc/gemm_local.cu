@@ -57,7 +57,8 @@ struct alignas(64) Job {
   float mask_scale, drop_scale;
   uint32_t drop_thresh;
   int act;
-  int part;                                      // 1: fp32 results, bare sums
+  int kper, slice_tiles;                         // > 0: k-blocks and tiles of a slice (fp32 results, bare sums)
+  long long part_stride;                         // between the results of two slices
   int sum;                                       // 1: d[m] = sum_k A[m, k] (+ c[m]); B is the tile of ones, bn = 16
   unsigned long long seed, offset;
   const unsigned long long* step_ptr;
@@ -108,10 +109,17 @@ __device__ __forceinline__ void add8(float* v, const uint4& u) {
   v[4] += bf16_lo(u.z); v[5] += bf16_hi(u.z); v[6] += bf16_lo(u.w); v[7] += bf16_hi(u.w);
 }
 
-// k-blocks of a tile whose first row is row0; 0: nothing to do but to write zeros
+// The slice that the lt-th tile of a job belongs to (0: the contraction is whole); lt becomes its number in the slice.
+__device__ __forceinline__ int tile_slice(const Job& j, int& lt) {
+  if (!j.kper) return 0;
+  const int s = lt / j.slice_tiles;
+  lt -= s * j.slice_tiles;
+  return s;
+}
+// k-blocks of a tile of slice s whose first row is row0; 0: nothing to do but to write zeros
 template <bool FILL>
-__device__ __forceinline__ int tile_kblocks(const Job& J, int row0) {
-  int n = J.kblocks;
+__device__ __forceinline__ int tile_kblocks(const Job& J, int s, int row0) {
+  int n = J.kper ? min(J.kper, J.kblocks - s * J.kper) : J.kblocks;
   if constexpr (FILL) {
     if (J.m_fill && row0 >= __ldg(J.m_fill)) n = 0;
     if (J.k_fill) n = min(n, (__ldg(J.k_fill) + 63) >> 6);
@@ -189,8 +197,9 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
         if (r * units >= total) break;
         if (t >= total) continue;
         const Job& J = P.job[find_job(P, t)];
-        int tm, tn;
-        tile_pos(J, t - J.tile0, tm, tn);
+        int tm, tn, lt = t - J.tile0;
+        const int slice = tile_slice(J, lt), kb0 = slice * J.kper;
+        tile_pos(J, lt, tm, tn);
         const int bn_cta = PAIR ? J.bn >> 1 : J.bn;
         const int m0 = tm * TM + (int)crank * kTM, n0 = tn * J.bn + (int)crank * bn_cta;
         const unsigned long long ma = reinterpret_cast<unsigned long long>(&J.ma);
@@ -199,13 +208,13 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
         const int nb = b_mn ? bn_cta >> 6 : 1;
         const bool sum = J.sum;                     // B is already in shared memory
         const uint32_t tx = sum ? kABytesL : kABytesL + bn_cta * kKB * 2;
-        const int kblocks = tile_kblocks<FILL>(J, tm * TM);
+        const int kblocks = tile_kblocks<FILL>(J, slice, tm * TM);
         for (int kb = 0; kb < kblocks; ++kb) {
           if (!mbar_wait_s(empty_s + stage * 8, phase ^ 1, abort_flag, status, tmo)) { ok = false; break; }
           const uint32_t sa = tiles_s + stage * stage_bytes, sb = sa + kABytesL, bar = full_s + stage * 8;
           issued |= 1u << stage;
           parity = (parity & ~(1u << stage)) | (phase << stage);
-          const int k0 = kb * kKB;
+          const int k0 = (kb0 + kb) * kKB;
           mbar_arrive_expect_tx_s(bar, tx);
           if (a3) tma_load_3d_s(sa, ma, 0, k0, m0 >> 6, bar);
           else if (a_mn) {
@@ -241,13 +250,14 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
         if (r * units >= total) break;
         if (t >= total) continue;
         const Job& J = P.job[find_job(P, t)];
-        int row0 = 0;
+        int row0 = 0, lt = t - J.tile0;
+        const int slice = tile_slice(J, lt);
         if constexpr (FILL) {
           int tm, tn;
-          tile_pos(J, t - J.tile0, tm, tn);
+          tile_pos(J, lt, tm, tn);
           row0 = tm * TM;
         }
-        const int kblocks = tile_kblocks<FILL>(J, row0);
+        const int kblocks = tile_kblocks<FILL>(J, slice, row0);
         if (FILL && !kblocks) continue;
         const uint32_t idesc = make_idesc_bf16(TM, J.bn, J.a_mn, J.b_mn);
         const uint32_t a_step = J.a_mn ? 128u : 2u, b_step = J.b_mn ? 128u : 2u;    // 16 elements of k, in 16-byte units
@@ -295,13 +305,14 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
         if (r * units >= total) break;
         if (t >= total) continue;
         const Job& J = P.job[find_job(P, t)];
-        int row0 = 0;
+        int row0 = 0, lt = t - J.tile0;
+        const int slice = tile_slice(J, lt);
         if constexpr (FILL) {
           int tm, tn;
-          tile_pos(J, t - J.tile0, tm, tn);
+          tile_pos(J, lt, tm, tn);
           row0 = tm * TM;
         }
-        const int kblocks = tile_kblocks<FILL>(J, row0);
+        const int kblocks = tile_kblocks<FILL>(J, slice, row0);
         for (int kb = 0; kb < kblocks; ++kb) {
           if (!mbar_wait_s(full_s + stage * 8, phase, abort_flag, status, tmo)) { ok = false; break; }
           mbar_arrive_cluster(lead + stage * 8);
@@ -326,9 +337,11 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
       if (r * units >= total) break;
       if (t >= total) continue;
       const Job& J = P.job[find_job(P, t)];
-      int tm, tn;
-      tile_pos(J, t - J.tile0, tm, tn);
-      const int M = J.M, N = J.N, bn = J.bn, part = J.part;
+      int tm, tn, lt = t - J.tile0;
+      const int slice = tile_slice(J, lt);
+      tile_pos(J, lt, tm, tn);
+      const int M = J.M, N = J.N, bn = J.bn, part = J.kper;
+      float* const fd = reinterpret_cast<float*>(J.d) + slice * J.part_stride;      // slices: fp32 results
       [[maybe_unused]] const int act = J.act;
       const int row0 = tm * TM + (int)crank * kTM + quad * 32, n0 = tn * bn;
       const __nv_bfloat16* c = reinterpret_cast<const __nv_bfloat16*>(J.c);
@@ -341,7 +354,7 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
       [[maybe_unused]] unsigned long long drop_off = 0;
       if constexpr (FUN) drop_off = J.offset + (J.step_ptr ? __ldg(J.step_ptr) * 65536ull : 0ull);
       if constexpr (FILL) {
-        if (!tile_kblocks<FILL>(J, tm * TM)) {               // no accumulator: zeros
+        if (!tile_kblocks<FILL>(J, slice, tm * TM)) {               // no accumulator: zeros
           if (J.sum) {
             if (half == 0 && row0 + lane < M) d[row0 + lane] = __float2bfloat16(0.f);
           } else {
@@ -368,7 +381,7 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
         tmem_ld_wait();
         const int m = row0 + lane;
         if (m < M) {
-          if (J.part) reinterpret_cast<float*>(J.d)[m] = __uint_as_float(ra[0]);
+          if (part) fd[m] = __uint_as_float(ra[0]);
           else d[m] = __float2bfloat16(__uint_as_float(ra[0]) + (c ? __bfloat162float(c[m]) : 0.f));
         }
       }
@@ -423,7 +436,7 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
         }
         if (part) {          // a slice of a contraction: rows of 256 bytes per thread, a few tiles in all
           if (row0 + lane < M) {
-            float* dp = reinterpret_cast<float*>(J.d) + (long long)(row0 + lane) * ldd + col0;
+            float* dp = fd + (long long)(row0 + lane) * ldd + col0;
 #pragma unroll
             for (int q = 0; q < 16; ++q)
               if (col0 + 4 * q < N)
@@ -542,15 +555,21 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
   }
 }
 
-// Adds up the slices of a split contraction, four elements a thread, always in the same order.  A few hundred KB that are
-// still in L2: bound by its launch (a few us).
+// Adds up the slices of a split contraction, four elements a thread, always in the same order: two ranges of them (a weight
+// gradient and its bias gradient).  A few MB that are still in L2: bound by its launch and by the latency of its loads.
 __global__ void __launch_bounds__(256) local_reduce_kernel(const float* __restrict__ part, int n, long long stride,
-                                                           __nv_bfloat16* __restrict__ out, long long len) {
+                                                           __nv_bfloat16* __restrict__ out, long long len, long long off2,
+                                                           __nv_bfloat16* __restrict__ out2, long long len2) {
   pdl_prologue();
-  const long long i = (blockIdx.x * 256ll + threadIdx.x) * 4;
+  long long i = (blockIdx.x * 256ll + threadIdx.x) * 4;
+  const long long first = (len + 3) / 4 * 4;
+  if (i >= first) {
+    i -= first;
+    part += off2; out = out2; len = len2;
+  }
   if (i >= len) return;
   float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
+#pragma unroll 8
   for (int k = 0; k < n; ++k) {
     const float4 v = __ldcs(reinterpret_cast<const float4*>(part + k * stride + i));
     s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
@@ -629,7 +648,8 @@ constexpr int kMaxItems = kLocalMaxJobs + kLocalMaxJobs / 2;
 struct Tiles { long long cost, count, epi; };
 Tiles tiles_of(const Item& x, const TileShape& s) {
   const int tm = s.pair ? 256 : 128;
-  const long long k = (x.g->K + 63) / 64, rows = (x.g->M + tm - 1) / tm;
+  const long long kb = (x.g->K + 63) / 64, slices = std::max(x.g->part, 1), k = (kb + slices - 1) / slices;
+  const long long rows = (x.g->M + tm - 1) / tm * slices;
   if (x.sum) return Tiles{k * kSumClk + kTileFixed, rows, 0};
   const long long loop = k * s.clk + kTileFixed, drain = s.drain + loop * 2 / 5;
   return Tiles{std::max(loop, drain), rows * ((x.g->N + s.bn - 1) / s.bn), loop >= drain ? s.epi : s.epi * 3 / 5};
@@ -759,8 +779,9 @@ int run(const Item* it, int n, int pair_policy, unsigned long long* status, unsi
     fill = fill || x.m_fill || x.k_fill;
     Job& J = P.job[q];
     J.sum = it[best_ord[q]].sum ? 1 : 0;
-    J.part = x.part;
     J.M = x.M; J.kblocks = (x.K + 63) / 64;
+    const int slices = std::max(x.part, 1);
+    if (x.part) { J.kper = (J.kblocks + slices - 1) / slices; J.part_stride = x.part_stride; }
     J.tile0 = total;
     J.tiles_m = (x.M + tm - 1) / tm;
     J.group = 8;
@@ -773,7 +794,8 @@ int run(const Item* it, int n, int pair_policy, unsigned long long* status, unsi
       J.bn = J.N = 16; J.tiles_n = 1;
       J.d = x.bsum;
       if (x.bsum_add) J.c = x.bsum;
-      total += J.tiles_m;
+      J.slice_tiles = J.tiles_m;
+      total += J.tiles_m * slices;
       continue;
     }
     J.bn = best_sh[best_ord[q]]->bn;
@@ -786,7 +808,8 @@ int run(const Item* it, int n, int pair_policy, unsigned long long* status, unsi
     // it: forward 4096 x 2048 -> 50304 563 -> 546 us, 8192 rows 1147 -> 1103.  Not for a tall one (weight gradient of 50304 x
     // 2048 over 4096 1238 -> 1298 us) nor a long contraction (8192^3 724 -> 740).
     if (J.tiles_n >= J.tiles_m && 16ll * tm * x.K * 2 <= (32ll << 20)) J.group = 16;
-    total += J.tiles_m * J.tiles_n;
+    J.slice_tiles = J.tiles_m * J.tiles_n;
+    total += J.slice_tiles * slices;
     J.d = x.d; J.ldd = x.ldd; J.c = x.c; J.ldc = x.ldc; J.bias = x.bias; J.act = x.act;
     J.mask = x.mask; J.ldmask = x.ldmask; J.mask_scale = x.mask_scale;
     if (x.drop_p > 0.f) {
@@ -829,10 +852,12 @@ int items_of(const LocalGemm* jobs, int n, Item* it) {
 
 }  // namespace
 
-int local_reduce(const float* part, int n, long long stride, void* out, long long len, cudaStream_t stream) {
-  if (len <= 0) return 0;
-  const cudaError_t e = launch_k(local_reduce_kernel, dim3((unsigned)((len + 1023) / 1024)), dim3(256), 0, stream, part, n, stride,
-                                 reinterpret_cast<__nv_bfloat16*>(out), len);
+int local_reduce(const float* part, int n, long long stride, void* out, long long len, long long off2, void* out2, long long len2,
+                 cudaStream_t stream) {
+  const long long items = (len + 3) / 4 + (len2 + 3) / 4;
+  if (items <= 0) return 0;
+  const cudaError_t e = launch_k(local_reduce_kernel, dim3((unsigned)((items + 255) / 256)), dim3(256), 0, stream, part, n, stride,
+                                 reinterpret_cast<__nv_bfloat16*>(out), len, off2, reinterpret_cast<__nv_bfloat16*>(out2), len2);
   return e == cudaSuccess ? 0 : lfail(std::string("launch local_reduce_kernel: ") + cudaGetErrorString(e));
 }
 
@@ -844,6 +869,8 @@ bool local_gemm_ok(const LocalGemm& g) {
   if (!al16(g.a) || !al16(g.b) || g.lda % 8 || g.ldb % 8) return false;
   if (!al16(g.d) || g.ldd % 8 || !al16(g.c) || !al16(g.mask) || !al16(g.bias)) return false;
   if ((g.c && g.ldc % 8) || (g.mask && g.ldmask % 8)) return false;
+  // every slice has a k-block of its own
+  if (g.part < 0 || (g.part && ((g.K + 63) / 64 + g.part - 1) / g.part * (g.part - 1) >= (g.K + 63) / 64)) return false;
   if (g.part && (g.c || g.bias || g.act || g.mask || g.drop_p > 0.f || g.bsum_add)) return false;
   if ((g.m_fill || g.k_fill) && (g.c || g.act || g.mask || g.drop_p > 0.f || g.bsum_add || g.part)) return false;
   return !g.bsum || g.a_mn;

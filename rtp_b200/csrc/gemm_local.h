@@ -23,9 +23,11 @@ struct LocalGemm {
   const unsigned long long* step_ptr;
   // column sums of A (a_mn = 1 only): bsum[m] (+)= sum_k A[m, k], in bf16
   void* bsum; int bsum_add;
-  // 1: d and bsum are fp32 and receive the bare sums (no c, bias, activation, mask or dropout): one slice of a contraction
-  // that local_reduce adds up
+  // > 0: the contraction falls into this many slices (a multiple of 64 elements each, the last one may be shorter), and d and bsum
+  // are fp32 and receive the bare sums of slice s (no c, bias, activation, mask or dropout) at d + s * part_stride and bsum +
+  // s * part_stride, for local_reduce to add up; d has a pitch of N
   int part;
+  long long part_stride;
   // Rows that are in use, known on the device only (expert capacities).  m_fill: output rows from there on get zeros, whatever A
   // holds; k_fill: elements of the contraction, of which those from there on contribute nothing (A or B is zero there) and up
   // to the next multiple of 64 are finite.  A launch with one of them has no c, mask, activation or dropout.
@@ -40,8 +42,10 @@ bool local_gemm_ok(const LocalGemm& g);
 constexpr int kLocalMaxJobs = 16;
 int local_gemm(const LocalGemm* jobs, int n, int pair_policy, unsigned long long* status, unsigned long long timeout_ns,
                cudaStream_t stream);
-// out[i] = bf16(sum over n parts of part[k * stride + i]), i < len (parts 16-byte aligned, stride a multiple of 4)
-int local_reduce(const float* part, int n, long long stride, void* out, long long len, cudaStream_t stream);
+// out[i] = bf16(sum over n parts of part[k * stride + i]), i < len, and out2[i] the same of part[k * stride + off2 + i], i < len2
+// (parts 16-byte aligned, stride and off2 multiples of 4)
+int local_reduce(const float* part, int n, long long stride, void* out, long long len, long long off2, void* out2, long long len2,
+                 cudaStream_t stream);
 const char* local_gemm_error();
 
 }  // namespace rtp

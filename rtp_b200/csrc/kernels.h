@@ -79,6 +79,7 @@ int rtp_im2col(const void* x, void* cols, int B, int C, int H, int W, int KH, in
                int dh, int dw, int Kp, void* stream);
 int rtp_col2im(const void* dcols, void* dx, int B, int C, int H, int W, int KH, int KW, int sh, int sw, int ph, int pw,
                int dh, int dw, int Kp, void* stream);
+int rtp_nchw_rows(const void* src, void* dst, int B, int C, int P, void* stream);   // [B, C, P] -> [B * P, C]
 int rtp_colsum(const void* x, long long ld, int M, int N, float* out, void* stream);
 int rtp_adam(const RtpAdamTensor* tensors_dev, const int* block_start_dev, int ntensors, int total_blocks,
              const long long* step_dev, float lr, float beta1, float beta2, float eps, float weight_decay, int adamw,

@@ -42,6 +42,7 @@ def _L():
         L.rtp_im2col_last_error.restype = C.c_char_p
         L.rtp_im2col.argtypes = [vp, vp] + [i] * 13 + [vp]
         L.rtp_col2im.argtypes = [vp, vp] + [i] * 13 + [vp]
+        L.rtp_nchw_rows.argtypes = [vp, vp, i, i, i, vp]
         L.rtp_adam.argtypes = [vp, vp, i, i, vp, f, f, f, f, f, i, f, f, vp, vp]
         L.rtp_add.argtypes = [vp, vp, vp, ll, vp]
         L.rtp_moe_scatter.argtypes = [vp, vp, vp, vp, i, i, ll, vp, i, vp]
@@ -502,3 +503,15 @@ def col2im(dcols, x_shape, kernel, stride=1, padding=0, dilation=1):
     if rc != 0:
         raise RuntimeError("col2im: " + _L().rtp_im2col_last_error().decode())
     return dx
+
+
+def nchw_rows(x):
+    """[B, C, H, W] bf16 as rows [B*H*W, C]."""
+    B, Cc, H, W = x.shape
+    if not x.is_contiguous():
+        return x.permute(0, 2, 3, 1).reshape(-1, Cc).contiguous()
+    out = torch.empty(B * H * W, Cc, dtype=x.dtype, device=x.device)
+    rc = _L().rtp_nchw_rows(_p(x), _p(out), B, Cc, H * W, _lib.stream_ptr())
+    if rc != 0:
+        raise RuntimeError("nchw_rows: " + _L().rtp_im2col_last_error().decode())
+    return out

@@ -513,9 +513,8 @@ class _FusedConvFn(torch.autograd.Function):
         owner, conv, spec = ctx.owner, ctx.conv, ctx.spec
         (cols,) = ctx.saved_tensors
         Cout = spec.out_f
-        dy2d = dy.permute(0, 2, 3, 1).reshape(-1, Cout)
-        if not dy2d.is_contiguous():
-            dy2d = dy2d.contiguous()
+        rows = dy.permute(0, 2, 3, 1)
+        dy2d = rows.reshape(-1, Cout) if rows.is_contiguous() else K.nchw_rows(dy)
         dcols, gflat = linear_bwd_raw(ctx.eng, spec.flat, spec.info, cols, dy2d, False, ctx.Kp, Cout,
                                       need_dx=ctx.needs_input_grad[2])
         dx = None
