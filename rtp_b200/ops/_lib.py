@@ -251,7 +251,8 @@ def check(rc: int, what: str):
 
 
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current stream of the current device (0.2 us; a ``torch.cuda.Stream`` object takes 3)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 _status_words = {}

@@ -36,14 +36,11 @@ def next_dropout_offset() -> int:
 
 def _ref4(t):
     """FlashRef of a [B, S, H, hd] view."""
-    B, S, H, hd = t.shape
-    if t.stride(3) != 1:
+    _, _, H, hd = t.shape
+    sb, ss, sh, sd = t.stride()
+    if sd != 1:
         raise ValueError("head_dim must have unit stride")
-    r = _lib.FlashRef()
-    r.ptr, r.sb, r.ss = t.data_ptr(), t.stride(0), t.stride(1)
-    r.col_base, r.hpg, r.gstride, r.hstride = 0, H, 0, t.stride(2)
-    r.width = (H - 1) * t.stride(2) + hd
-    return r
+    return _lib.FlashRef(t.data_ptr(), sb, ss, (H - 1) * sh + hd, 0, H, 0, sh)
 
 
 def _ref_packed(buf, which, B, S, H, hd, nshard, seq_first, row_width):
@@ -61,7 +58,8 @@ def _ref_packed(buf, which, B, S, H, hd, nshard, seq_first, row_width):
     return r
 
 
-def _mask_args(a, attn_mask, key_padding_mask, keep):
+def _mask_args(a, attn_mask, key_padding_mask, keep, converted=False):
+    """``converted``: the key-padding mask is one that an earlier call appended to ``keep``."""
     if attn_mask is not None:
         m = attn_mask
         if m.dtype == torch.bool:
@@ -74,8 +72,8 @@ def _mask_args(a, attn_mask, key_padding_mask, keep):
         a.mask, a.mask_ld, a.mask_fp32 = m.data_ptr(), m.stride(0), int(m.dtype == torch.float32)
     if key_padding_mask is not None:
         k = key_padding_mask
-        k = (k != 0) if k.dtype != torch.bool else k
-        k = k.to(torch.uint8).contiguous()
+        if not converted:                      # a copy of its own: backward reads it again
+            k = (k if k.dtype == torch.bool else k != 0).to(torch.uint8).contiguous()
         keep.append(k)
         a.kpm, a.kpm_ld = k.data_ptr(), k.stride(0)
 
@@ -133,7 +131,7 @@ class _FlashFn(torch.autograd.Function):
         it = iter(keep)
         m = next(it) if has_mask else None
         kp = next(it) if has_kpm else None
-        _mask_args(a, m, kp, [])
+        _mask_args(a, m, kp, [], True)
         _common(a, B, H, Sq, Sk, hd, causal, sm_scale, drop_p, seed, offset, step, q.device)
         _check(_lib.lib().rtp_flash_bwd(C.byref(a), _lib.stream_ptr()), "rtp_flash_bwd")
         return dq, dk, dv, None, None, None, None, None, None, None, None

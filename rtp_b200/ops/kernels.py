@@ -475,31 +475,36 @@ def _pair(v):
     return (v, v) if isinstance(v, int) else tuple(v)
 
 
+def conv_geometry(H, W, kernel, stride, padding, dilation):
+    """(KH, KW, sh, sw, ph, pw, dh, dw, OH, OW)"""
+    (KH, KW), (sh, sw), (ph, pw), (dh, dw) = _pair(kernel), _pair(stride), _pair(padding), _pair(dilation)
+    return (KH, KW, sh, sw, ph, pw, dh, dw, (H + 2 * ph - dh * (KH - 1) - 1) // sh + 1,
+            (W + 2 * pw - dw * (KW - 1) - 1) // sw + 1)
+
+
 def conv_out_size(H, W, kernel, stride, padding, dilation):
-    (KH, KW), (sh, sw), (ph, pw), (dh, dw) = _pair(kernel), _pair(stride), _pair(padding), _pair(dilation)
-    return (H + 2 * ph - dh * (KH - 1) - 1) // sh + 1, (W + 2 * pw - dw * (KW - 1) - 1) // sw + 1
+    return conv_geometry(H, W, kernel, stride, padding, dilation)[8:]
 
 
-def im2col(x, kernel, stride=1, padding=0, dilation=1, Kp=None):
-    """Patch matrix [B*OH*OW, Kp] of a contiguous NCHW bf16 tensor; column (c, kh, kw), zero padded up to Kp."""
+def im2col(x, kernel, stride=1, padding=0, dilation=1, Kp=None, geom=None):
+    """Patch matrix [B*OH*OW, Kp] of a contiguous NCHW bf16 tensor; column (c, kh, kw), zero padded up to Kp.  ``geom``: the
+    :func:`conv_geometry` where the caller has it."""
     B, Cc, H, W = x.shape
-    (KH, KW), (sh, sw), (ph, pw), (dh, dw) = _pair(kernel), _pair(stride), _pair(padding), _pair(dilation)
-    OH, OW = conv_out_size(H, W, kernel, stride, padding, dilation)
-    Kp = Kp or Cc * KH * KW
-    cols = torch.empty(B * OH * OW, Kp, dtype=x.dtype, device=x.device)
-    rc = _L().rtp_im2col(_p(x), _p(cols), B, Cc, H, W, KH, KW, sh, sw, ph, pw, dh, dw, Kp, _lib.stream_ptr())
+    g = geom or conv_geometry(H, W, kernel, stride, padding, dilation)
+    Kp = Kp or Cc * g[0] * g[1]
+    cols = torch.empty(B * g[8] * g[9], Kp, dtype=x.dtype, device=x.device)
+    rc = _L().rtp_im2col(x.data_ptr(), cols.data_ptr(), B, Cc, H, W, *g[:8], Kp, _lib.stream_ptr())
     if rc != 0:
         raise RuntimeError("im2col: " + _L().rtp_im2col_last_error().decode())
     return cols
 
 
-def col2im(dcols, x_shape, kernel, stride=1, padding=0, dilation=1):
+def col2im(dcols, x_shape, kernel, stride=1, padding=0, dilation=1, geom=None):
     """Adjoint of im2col: gradient with respect to the NCHW input."""
     B, Cc, H, W = x_shape
-    (KH, KW), (sh, sw), (ph, pw), (dh, dw) = _pair(kernel), _pair(stride), _pair(padding), _pair(dilation)
+    g = geom or conv_geometry(H, W, kernel, stride, padding, dilation)
     dx = torch.empty(B, Cc, H, W, dtype=dcols.dtype, device=dcols.device)
-    rc = _L().rtp_col2im(_p(dcols), _p(dx), B, Cc, H, W, KH, KW, sh, sw, ph, pw, dh, dw, dcols.shape[1],
-                         _lib.stream_ptr())
+    rc = _L().rtp_col2im(dcols.data_ptr(), dx.data_ptr(), B, Cc, H, W, *g[:8], dcols.shape[1], _lib.stream_ptr())
     if rc != 0:
         raise RuntimeError("col2im: " + _L().rtp_im2col_last_error().decode())
     return dx

@@ -483,7 +483,8 @@ class _FusedConvFn(torch.autograd.Function):
         K_ = conv.in_channels * conv.kernel_size[0] * conv.kernel_size[1]
         Kp = _round_up(K_, 8)
         Os = conv.out_channels                      # the shard module holds Cout / N channels
-        cols = K.im2col(x, conv.kernel_size, conv.stride, conv.padding, conv.dilation, Kp=Kp)
+        geom = K.conv_geometry(x.shape[2], x.shape[3], conv.kernel_size, conv.stride, conv.padding, conv.dilation)
+        cols = K.im2col(x, None, Kp=Kp, geom=geom)
         has_bias = conv.bias is not None
         if Kp == K_:
             lay = owner._layout
@@ -502,11 +503,10 @@ class _FusedConvFn(torch.autograd.Function):
         places = [(0, Os * Kp, (Os, Kp))] + ([(bias_off, Os, (Os,))] if has_bias else [])
         spec = LinSpec(owner.ring, flat, has_bias, bias_off, False, Kp, Os * N, places)
         y2d = linear_fwd_raw(eng, flat, spec.info, cols, False, Kp, Os * N)
-        OH, OW = K.conv_out_size(x.shape[2], x.shape[3], conv.kernel_size, conv.stride, conv.padding, conv.dilation)
         ctx.owner, ctx.conv, ctx.spec, ctx.eng, ctx.K_, ctx.Kp = owner, conv, spec, eng, K_, Kp
-        ctx.x_shape = x.shape
+        ctx.x_shape, ctx.geom = x.shape, geom
         ctx.save_for_backward(cols)
-        return y2d.view(x.shape[0], OH, OW, Os * N).permute(0, 3, 1, 2)
+        return y2d.view(x.shape[0], geom[8], geom[9], Os * N).permute(0, 3, 1, 2)
 
     @staticmethod
     def backward(ctx, dy):
@@ -519,9 +519,10 @@ class _FusedConvFn(torch.autograd.Function):
                                       need_dx=ctx.needs_input_grad[2])
         dx = None
         if dcols is not None:
-            dx = K.col2im(dcols, ctx.x_shape, conv.kernel_size, conv.stride, conv.padding, conv.dilation)
+            dx = K.col2im(dcols, ctx.x_shape, None, geom=ctx.geom)
         Os = Cout // owner.ring.world
-        gw = gflat[:Os * ctx.Kp].view(Os, ctx.Kp)[:, :ctx.K_].reshape(conv.weight.shape)
+        gw = gflat[:Os * ctx.Kp]
+        gw = gw.view(conv.weight.shape) if ctx.Kp == ctx.K_ else gw.view(Os, ctx.Kp)[:, :ctx.K_].reshape(conv.weight.shape)
         grads = [gw]
         if spec.has_bias:
             grads.append(gflat[spec.bias_off:spec.bias_off + Os])
