@@ -222,7 +222,9 @@ __global__ void __launch_bounds__(T, T == 128 ? 7 : NG == 1 ? 4 : 2) norm_fwd_ke
 
 // Backward: dh = d(norm)/dh (+ dres); dx = dh; dsub = dropout_mask * dh.  Per-thread dgamma / dbeta partials stay in
 // registers across the rows of the block and are added to the fp32 outputs with one atomic per column at the end, so there
-// are few blocks, each with many rows.  R rows are in flight at once and share a reduction (two sums a row, one barrier):
+// are few blocks, each with many rows.  With `part_pitch` every block leaves its sums in a row of its own instead
+// (dgamma + block * part_pitch, dbeta's D columns behind), which norm_param_grads_kernel adds up: no buffer has to be zeroed before
+// and converted after.  R rows are in flight at once and share a reduction (two sums a row, one barrier):
 // one row at a time left the block waiting for a load and two barriers per row.  Narrow rows take T < 256 threads and a
 // block works on 256 / T groups of R rows side by side, whose column sums it adds up before the atomics.
 // 256 x 256 6.6 -> 2.9 us, 650 x 768 8.1 -> 4.6, 1024 x 512 8.5 -> 4.8, 1024 x 2048 with dropout 11.0 -> 9.7,
@@ -236,7 +238,7 @@ __global__ void __launch_bounds__(256, 2) norm_bwd_kernel(
     const float* __restrict__ mean_in, const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ dx,
     __nv_bfloat16* __restrict__ dsub, float* __restrict__ dgamma, float* __restrict__ dbeta, int M, int D, int rms,
     uint32_t thresh, float drop_scale, uint64_t seed, uint64_t offset, const __nv_bfloat16* __restrict__ dres,
-    const unsigned long long* __restrict__ step_ptr, int vec_atomics) {
+    const unsigned long long* __restrict__ step_ptr, int vec_atomics, int part_pitch) {
   pdl_prologue();
   constexpr int G = 256 / T;                   // row groups of the block
   __shared__ float red[2 * 8 * 2 * R];
@@ -375,6 +377,17 @@ __global__ void __launch_bounds__(256, 2) norm_bwd_kernel(
   for (int q = 0; q < NG; ++q) {
     const int c = (q * T + tid) * 8;
     if (c < D) {
+      if (part_pitch) {
+        float4* o = reinterpret_cast<float4*>(dgamma + (size_t)blockIdx.x * part_pitch + c);
+        o[0] = make_float4(pg[q][0], pg[q][1], pg[q][2], pg[q][3]);
+        o[1] = make_float4(pg[q][4], pg[q][5], pg[q][6], pg[q][7]);
+        if (dbeta) {
+          o = reinterpret_cast<float4*>(dbeta + (size_t)blockIdx.x * part_pitch + c);
+          o[0] = make_float4(pb[q][0], pb[q][1], pb[q][2], pb[q][3]);
+          o[1] = make_float4(pb[q][4], pb[q][5], pb[q][6], pb[q][7]);
+        }
+        continue;
+      }
       if (!vec_atomics) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -392,6 +405,34 @@ __global__ void __launch_bounds__(256, 2) norm_bwd_kernel(
       }
     }
   }
+}
+
+// out[c] = bf16(sum over n rows of part[r * pitch + y * D + c]): the gradients of gamma (y = 0) and beta (y = 1).  64 columns a
+// block, 16 rows side by side, always in the same order.  Up to a few MB that are still in L2: bound by its launch.
+__global__ void __launch_bounds__(256) norm_param_grads_kernel(const float* __restrict__ part, int n, int pitch, int D,
+                                                               __nv_bfloat16* __restrict__ dgamma, __nv_bfloat16* __restrict__ dbeta) {
+  pdl_prologue();
+  __shared__ float4 sums[16][16];
+  const int x = threadIdx.x & 15, y = threadIdx.x >> 4, c = blockIdx.x * 64 + x * 4;
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (c < D) {
+    const float* p = part + (size_t)blockIdx.y * D + c;
+#pragma unroll 8
+    for (int r = y; r < n; r += 16) {
+      const float4 v = *reinterpret_cast<const float4*>(p + (size_t)r * pitch);
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+  }
+  sums[y][x] = s;
+  __syncthreads();
+  if (y || c >= D) return;
+#pragma unroll
+  for (int k = 1; k < 16; ++k) {
+    const float4 v = sums[k][x];
+    s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+  }
+  __nv_bfloat16* out = (blockIdx.y ? dbeta : dgamma) + c;
+  out[0] = __float2bfloat16(s.x); out[1] = __float2bfloat16(s.y); out[2] = __float2bfloat16(s.z); out[3] = __float2bfloat16(s.w);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1470,22 +1511,24 @@ int rtp_norm_fwd(const void* x, const void* sub, const void* gamma, const void* 
   LAUNCH_CHECK("norm_fwd");
   return 0;
 }
-int rtp_norm_bwd(const void* dy, const void* h, const void* gamma, const float* mean, const float* rstd, void* dx,
-                 void* dsub, float* dgamma, float* dbeta, int M, int D, int rms, float drop_p,
-                 unsigned long long seed, unsigned long long offset, const void* dres,
-                 const unsigned long long* step_ptr, void* stream) {
+// part_pitch and the number of blocks as in norm_bwd_kernel (blocks may be null)
+static int norm_bwd_launch(const void* dy, const void* h, const void* gamma, const float* mean, const float* rstd, void* dx,
+                           void* dsub, float* dgamma, float* dbeta, int M, int D, int rms, float drop_p, unsigned long long seed,
+                           unsigned long long offset, const void* dres, const unsigned long long* step_ptr, int part_pitch,
+                           int* blocks, void* stream) {
   if (D % 8 || D > 8192) { k_err = "norm: D must be a multiple of 8 and at most 8192"; return -1; }
   const float ds = drop_p > 0.f ? 1.f / (1.f - drop_p) : 1.f;
   const int vec_atomics = ((reinterpret_cast<uintptr_t>(dgamma) | reinterpret_cast<uintptr_t>(dbeta)) & 15) == 0;
   // Few blocks: every block ends with one vector atomic per 4 columns of dgamma / dbeta.  Up to 1024 wide rows one block per
   // SM (256 x 2048 256 blocks 10.3 us, 128 with two rows each 7.4; 1024 x 3072 256 blocks 18.3, 148 14.6), else two.
   const int most = M <= 1024 && D > 1024 ? 148 : 296;
+  int grid = 0;
 #define RTP_NORM_BWD(T, NG, R, AHEAD)                                                                                 \
-  rtp::launch_k(norm_bwd_kernel<T, NG, R, AHEAD>, dim3(std::min((M + 256 / T * R - 1) / (256 / T * R), most)),         \
+  rtp::launch_k(norm_bwd_kernel<T, NG, R, AHEAD>, dim3(grid = std::min((M + 256 / T * R - 1) / (256 / T * R), most)),  \
       dim3(256), 0, (cudaStream_t)stream,                                                                             \
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)h, (const __nv_bfloat16*)gamma, mean, rstd, (__nv_bfloat16*)dx, \
       (__nv_bfloat16*)dsub, dgamma, dbeta, M, D, rms, host_thresh(drop_p), ds, seed, offset,                          \
-      (const __nv_bfloat16*)dres, step_ptr, vec_atomics)
+      (const __nv_bfloat16*)dres, step_ptr, vec_atomics, part_pitch)
   // Rows in flight per group: no more than leave every SM a block or two, one where there are fewer rows than SMs
   // (64 x 4096 with dropout, two rows 7.5 us, one 6.9).
   if (D <= 256) { if (M <= 2368) RTP_NORM_BWD(32, 1, 1, false); else RTP_NORM_BWD(32, 1, 4, false); }
@@ -1502,6 +1545,28 @@ int rtp_norm_bwd(const void* dy, const void* h, const void* gamma, const float* 
   else if (D <= 6144) RTP_NORM_BWD(256, 3, 1, false); else RTP_NORM_BWD(256, 4, 1, false);
 #undef RTP_NORM_BWD
   LAUNCH_CHECK("norm_bwd");
+  if (blocks) *blocks = grid;
+  return 0;
+}
+int rtp_norm_bwd(const void* dy, const void* h, const void* gamma, const float* mean, const float* rstd, void* dx,
+                 void* dsub, float* dgamma, float* dbeta, int M, int D, int rms, float drop_p,
+                 unsigned long long seed, unsigned long long offset, const void* dres,
+                 const unsigned long long* step_ptr, void* stream) {
+  return norm_bwd_launch(dy, h, gamma, mean, rstd, dx, dsub, dgamma, dbeta, M, D, rms, drop_p, seed, offset, dres, step_ptr, 0,
+                         nullptr, stream);
+}
+unsigned long long rtp_norm_bwd_scratch(int D) { return 296ull * 2 * D * sizeof(float); }
+int rtp_norm_bwd_params(const void* dy, const void* h, const void* gamma, const float* mean, const float* rstd, void* dx,
+                        void* dgamma, void* dbeta, float* scratch, int M, int D, int rms, const void* dres, void* stream) {
+  if (M <= 0) { k_err = "norm backward: no rows"; return -1; }
+  if (reinterpret_cast<uintptr_t>(scratch) & 15) { k_err = "norm backward: scratch must be 16-byte aligned"; return -1; }
+  int n = 0;
+  if (norm_bwd_launch(dy, h, gamma, mean, rstd, dx, nullptr, scratch, dbeta ? scratch + D : nullptr, M, D, rms, 0.f, 0, 0, dres,
+                      nullptr, 2 * D, &n, stream))
+    return -1;
+  rtp::launch_k(norm_param_grads_kernel, dim3((D + 63) / 64, dbeta ? 2 : 1), dim3(256), 0, (cudaStream_t)stream, (const float*)scratch, n,
+                2 * D, D, (__nv_bfloat16*)dgamma, (__nv_bfloat16*)dbeta);
+  LAUNCH_CHECK("norm_param_grads");
   return 0;
 }
 int rtp_cross_entropy_scaled(void* logits, long long ld, const long long* target, float* loss, int M, int V, float grad_scale,

@@ -23,6 +23,11 @@ int rtp_norm_bwd(const void* dy, const void* h, const void* gamma, const float* 
                  void* dsub, float* dgamma, float* dbeta, int M, int D, int rms, float drop_p,
                  unsigned long long seed, unsigned long long offset, const void* dres,
                  const unsigned long long* step_ptr, void* stream);
+// The same without dropout and second output, with the gradients of gamma and beta (null: RMSNorm) as bf16, written, not added to.
+// scratch: rtp_norm_bwd_scratch(D) bytes.  M > 0.
+unsigned long long rtp_norm_bwd_scratch(int D);
+int rtp_norm_bwd_params(const void* dy, const void* h, const void* gamma, const float* mean, const float* rstd, void* dx,
+                        void* dgamma, void* dbeta, float* scratch, int M, int D, int rms, const void* dres, void* stream);
 // Loss per row of logits (pitch ld) and, with write_grad, the gradient of grad_scale * (*scale_ptr) * sum of the losses: into
 // `grad` (pitch ldg), the logits stay as they are, or over the logits (grad = null).  scale_ptr: a factor on the device, may
 // be null (rows of at most 65536 logits).

@@ -74,6 +74,9 @@ class _NormFn(torch.autograd.Function):
         from . import kernels as K
         x2, weight, mean, rstd = ctx.saved_tensors
         dy2 = dy.reshape(-1, dy.shape[-1]).contiguous()
+        if weight.dtype == torch.bfloat16 and x2.shape[0] > 0:
+            dx, dg, db = K.norm_bwd_params(dy2, x2, weight, mean, rstd, rms=ctx.rms, has_beta=ctx.has_bias)
+            return dx.view(ctx.shape), dg, db, None, None
         dx, _, dg, db = K.norm_bwd(dy2, x2, weight, mean, rstd, rms=ctx.rms, has_beta=ctx.has_bias, want_dsub=False)
         return dx.view(ctx.shape), dg.to(weight.dtype), (db.to(weight.dtype) if ctx.has_bias else None), None, None
 

@@ -23,6 +23,9 @@ def _L():
         L.rtp_kernels_last_error.restype = C.c_char_p
         L.rtp_norm_fwd.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, i, i, f, i, f, ull, ull, vp, vp]
         L.rtp_norm_bwd.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, f, ull, ull, vp, vp, vp]
+        L.rtp_norm_bwd_scratch.argtypes = [i]
+        L.rtp_norm_bwd_scratch.restype = ull
+        L.rtp_norm_bwd_params.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, vp, vp]
         L.rtp_cross_entropy_scaled.argtypes = [vp, ll, vp, vp, i, i, f, vp, ll, i, vp, ll, vp]
         L.rtp_ce_count.argtypes = [vp, i, ll, vp, vp]
         L.rtp_scale_unless_one.argtypes = [vp, vp, ll, vp]
@@ -99,6 +102,19 @@ def norm_bwd(dy, h, gamma, mean, rstd, *, rms=False, has_beta=True, drop_p=0.0, 
                              M, D, int(rms), float(drop_p), seed, offset, _p(dres), _p(step), _lib.stream_ptr()),
            "norm_bwd")
     return dx, dsub, dgamma, dbeta
+
+
+def norm_bwd_params(dy, h, gamma, mean, rstd, *, rms=False, has_beta=True, dres=None):
+    """Returns (dx, dgamma, dbeta), all bf16 (``dbeta`` None without beta): no buffer to zero before and to convert after."""
+    M, D = dy.shape
+    dx = torch.empty_like(dy)
+    grads = torch.empty(2 if has_beta else 1, D, dtype=torch.bfloat16, device=dy.device)
+    dg, db = grads[0], grads[1] if has_beta else None
+    scratch = torch.empty(_L().rtp_norm_bwd_scratch(D), dtype=torch.uint8, device=dy.device)
+    _check(_L().rtp_norm_bwd_params(_p(dy), _p(h), _p(gamma), _p(mean), _p(rstd), _p(dx), _p(dg), _p(db), _p(scratch), M, D,
+                                    int(rms), _p(dres), _lib.stream_ptr()), "norm_bwd_params")
+    _lib.launches += 1
+    return dx, dg, db
 
 
 def _cross_entropy(logits, target, loss, grad_scale, scale, ignore_index, write_grad, grad):

@@ -49,3 +49,27 @@ def test_norm(D, M, rms, residual):
 def test_many_wide_rows(M, D):
     test_norm(D, M, False, True)
     test_norm(D, M, True, False)
+
+
+@pytest.mark.parametrize("D", [8, 72, 264, 520, 1032, 2048, 5120, 8192])
+@pytest.mark.parametrize("M", [1, 5, 297, 4099])
+@pytest.mark.parametrize("rms", [False, True])
+def test_parameter_gradients_in_place(D, M, rms):
+    """Through autograd: gradients of gamma and beta are one rounding to bf16 of the sums, and two calls give the same bits."""
+    from rtp_b200.ops import functional as FO
+    g = torch.Generator(device="cuda").manual_seed(D + M)
+    x, dy = (torch.randn(M, D, generator=g, device="cuda").to(BF) for _ in range(2))
+    w, b = (torch.randn(D, generator=g, device="cuda").to(BF).requires_grad_() for _ in range(2))
+    x.requires_grad_()
+
+    def run():
+        y = FO.rms_norm(x, w) if rms else FO.layer_norm(x, w, b)
+        return torch.autograd.grad(y, (x, w) if rms else (x, w, b), dy)
+    got = run()
+    assert all(torch.equal(p, q) for p, q in zip(got, run()))
+    hd = x.detach().double()
+    mu = 0.0 if rms else hd.mean(-1, keepdim=True)
+    xh = (hd - mu) * torch.rsqrt((hd - mu).pow(2).mean(-1, keepdim=True) + 1e-5)
+    for t, terms in zip(got[1:], (dy.double() * xh, dy.double())):
+        ref = terms.sum(0)
+        assert bool(((t.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 2.0 ** -16 * terms.abs().sum(0)).all())
