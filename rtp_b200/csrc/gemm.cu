@@ -1125,8 +1125,9 @@ int local_linear_bwd(const RtpRing& R, const RtpLinearBwd& op, rtp::LocalGemm* j
 // SMs and each has 128 k-blocks or more, the contraction falls into slices that leave fp32 sums in a workspace: as many as give
 // every SM one, of eight k-blocks or more, so that the tiles of the input gradient go on in whole rounds behind them.
 // Whole backward, cold L2, unsplit -> eight slices: that convolution 187 -> 78 us, 512 x 512 over 36 864 185 -> 84,
-// 768 x 384 over 8 192 (18 tiles, the most that split) 50 -> 44; eight slices -> this, warm: 54 -> 38, 71 -> 54, 28 -> 22.  Over 4 096 positions the launch that adds up
-// the slices cost more than it saved (eight slices): [64, 288] 27.6 -> 29.7, 768 x 384 28.2 -> 36.9.
+// 768 x 384 over 8 192 (18 tiles, the most that split) 50 -> 44; eight slices -> this, warm: 54 -> 38, 71 -> 54, 28 -> 22.
+// Over 4 096 positions the launch that adds up the slices cost more than it saved (eight slices): [64, 288] 27.6 -> 29.7,
+// 768 x 384 28.2 -> 36.9.
 long long part_stride(const rtp::LocalGemm& w) { return ((long long)w.M * w.N + 3) / 4 * 4 + (w.bsum ? (w.M + 3) / 4 * 4 : 0); }
 long long wgrad_tiles(const rtp::LocalGemm& w) { return (long long)((w.M + 127) / 128) * ((w.N + 127) / 128); }
 bool splits_wgrad(const rtp::LocalGemm& w) { return !w.c && !w.bsum_add && wgrad_tiles(w) * 8 <= sm_count() && w.K >= 128 * 64; }
