@@ -444,6 +444,12 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   return *reinterpret_cast<uint32_t*>(&t);
 }
 
+// A maximum that keeps a NaN, as fmaxf does not.
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
 // 4 x 4 transpose of 16-byte chunks among four neighbouring lanes: lane i of four has chunks 0..3 of its row and leaves with
 // chunk i of the four rows.
 __device__ __forceinline__ uint4 sel4(bool a, const uint4& x, const uint4& y) {

@@ -278,9 +278,9 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
       : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
   return d;
 }
-// 2^x of two numbers on the multiply-add pipes, x >= -126 or taken as that: 2^round(x) rides in as an exponent, the rest is a
-// polynomial of degree 6 in [-1/2, 1/2] (least maximum relative error, by Remez exchange).  Relative error up to 1.1e-7 in
-// fp32, not above ex2.approx; twice its instructions, but the special-function unit has only four lanes an SM quarter.
+// 2^x of two numbers that are not NaN on the multiply-add pipes, x >= -126 or taken as that: 2^round(x) rides in as an exponent, the
+// rest is a polynomial of degree 6 in [-1/2, 1/2] (least maximum relative error, by Remez exchange).  Relative error up to 1.1e-7
+// in fp32, not above ex2.approx; twice its instructions, but the special-function unit has only four lanes an SM quarter.
 __device__ __forceinline__ float2 ex2_poly2(float2 t) {
   const float2 magic = make_float2(12582912.f, 12582912.f);       // 1.5 * 2^23: rounds to integers, which stay in the low bits
   t.x = fmaxf(t.x, -126.f);
@@ -298,11 +298,6 @@ __device__ __forceinline__ float2 ex2_poly2(float2 t) {
   return make_float2(__int_as_float(__float_as_int(p.x) + (__float_as_int(r.x) << 23)),
                      __int_as_float(__float_as_int(p.y) + (__float_as_int(r.y) << 23)));
 }
-__device__ __forceinline__ float max3(float a, float b, float c) {
-  float d;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-  return d;
-}
 __device__ __forceinline__ float max64(const float* s) {
   float m0 = s[0], m1 = s[1], m2 = s[2], m3 = s[3];
 #pragma unroll
@@ -310,7 +305,7 @@ __device__ __forceinline__ float max64(const float* s) {
     m0 = max3(m0, s[i], s[i + 1]); m1 = max3(m1, s[i + 2], s[i + 3]);
     m2 = max3(m2, s[i + 4], s[i + 5]); m3 = max3(m3, s[i + 6], s[i + 7]);
   }
-  return fmaxf(max3(max3(m0, m1, m2), m3, s[60]), max3(s[61], s[62], s[63]));
+  return max3(max3(max3(m0, m1, m2), m3, s[60]), s[61], max3(s[61], s[62], s[63]));
 }
 // The CTAs are persistent: when a role is done with one piece of work it goes on with the next, so that copies and products of
 // the next run under the end of the last, and TMEM and barriers are set up once.  A CTA's first work is its own blockIdx.x; from
@@ -619,7 +614,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_kernel(const __grid_con
       tmem_ld32f(aS + 96, s + 96);
       float mx = max64(s);
       tmem_ld_wait();
-      mx = fmaxf(mx, max64(s + 64));
+      mx = max3(mx, mx, max64(s + 64));
       if (plain) mx *= M.scale_log2;      // the scale is positive: the maximum commutes with it
       const float cand = fmaxf(m_used, mx);
       const bool need = cand > m_used + kRescaleGap;
@@ -642,7 +637,9 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_kernel(const __grid_con
       }
       float2 ra = make_float2(0.f, 0.f), rb = ra;
       const float2 mul2 = make_float2(mul, mul), ref2 = make_float2(-mref, -mref);
-      // some: one exponential in four by polynomial (blocks without masked scores, which have to become 0)
+      // some: one exponential in four by polynomial.  That is for blocks without masked scores, which have to become 0, whose rows
+      // all have a finite maximum: a NaN or an infinite score has to reach the output, and a row of -inf alone has no weights;
+      // a -inf below a finite maximum gets 2^-126 beside 2^-8 or more.
       auto exponentials = [&](auto some) {
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
@@ -676,7 +673,8 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_kernel(const __grid_con
         }
       }
       };
-      if (!DRP && plain) exponentials(std::true_type{}); else exponentials(std::false_type{});
+      if (!DRP && plain && __all_sync(0xffffffffu, fabsf(mx) < INFINITY)) exponentials(std::true_type{});
+      else exponentials(std::false_type{});
       m_used = m_new;
       l += (ra.x + ra.y) + (rb.x + rb.y);
       if (tr && ns < 16) tr[ns * 8 + 2] = clock64();
