@@ -594,7 +594,8 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_kernel(const __grid_con
       if (tr && ns < 16) tr[ns * 8 + 1] = clock64();
       // A block that needs more than the scale is put right in TMEM first, 32 columns at a time, so that the loop below is one
       // for all blocks; one that only needs the scale keeps the raw scores: the scale rides in the exponent's multiply-add.
-      const bool plain = MSK != 2 && !(dead[0] | dead[1] | dead[2] | dead[3]) && !(M.causal && c == gt) && (col0 + kBlk <= M.Sk);
+      const bool plain = MSK != 2 && !(dead[0] | dead[1] | dead[2] | dead[3]) && !(M.causal && c == gt) && (col0 + kBlk <= M.Sk) &&
+                         M.scale_log2 >= 0.f;          // the maximum commutes with a positive scale only
       if (!plain) {
 #pragma unroll 1
         for (int q = 0; q < 4; ++q) {
@@ -615,7 +616,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_kernel(const __grid_con
       float mx = max64(s);
       tmem_ld_wait();
       mx = max3(mx, mx, max64(s + 64));
-      if (plain) mx *= M.scale_log2;      // the scale is positive: the maximum commutes with it
+      if (plain) mx *= M.scale_log2;
       const float cand = fmaxf(m_used, mx);
       const bool need = cand > m_used + kRescaleGap;
       const float m_new = need ? cand : m_used;

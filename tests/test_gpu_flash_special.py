@@ -56,3 +56,31 @@ def test_minus_infinity_has_no_weight(B, H, S, hd):
     o = forward(q, k, v)
     assert bool((o[0, :, 0] == 0).all())
     assert ((o[:, :, 1:].double() - ref[:, :, 1:]).norm() <= 2.0 ** -7 * ref[:, :, 1:].norm()).item()
+
+
+@pytest.mark.parametrize("padded", [False, True])
+@pytest.mark.parametrize("B,H,S,hd", SHAPES)
+def test_negative_scale(B, H, S, hd, padded):
+    """Scores far apart, so that a reference other than their maximum overflows."""
+    from rtp_b200.ops.flash import flash_attention
+    q, k, v = (t.requires_grad_() for t in inputs(B, H, S, hd))
+    do = torch.randn_like(q)
+    kpm = None
+    if padded:
+        kpm = torch.zeros(B, S, dtype=torch.bool, device="cuda")
+        kpm[:, 200:] = True
+    o = flash_attention(q, k, v, key_padding_mask=kpm, sm_scale=-8.0)
+    got = [o.detach(), *torch.autograd.grad(o, (q, k, v), do)]
+    x, y, z = (t.detach().double().transpose(1, 2).requires_grad_() for t in (q, k, v))
+    s = x @ y.transpose(-1, -2) * -8.0
+    if padded:
+        s = s.masked_fill(kpm[:, None, None], float("-inf"))
+    r = (torch.softmax(s, -1) @ z).transpose(1, 2)
+    # Scores are sums of hd products in fp32, a few hundred in size: 2^-23 * 2^9 * sqrt(hd) < 2^-10 of a weight, below P's rounding.
+    # Gradients: dS = P (dP - delta), and delta is made of the output as bf16.  Rows with nearly all weight on one key have dP close
+    # to delta there, so that its rounding counts as much as those of dS and of the result: twice the bound.
+    ref = [r, *(t.transpose(1, 2) for t in torch.autograd.grad(r, (x, y, z), do.double()))]
+    for name, a, b in zip(("o", "dq", "dk", "dv"), got, ref):
+        assert a.isfinite().all(), name
+        bound = 2.0 ** -7 if name == "o" else 2.0 ** -6
+        assert ((a.double() - b).norm() <= bound * b.norm()).item(), (name, ((a.double() - b).norm() / b.norm()).item())
