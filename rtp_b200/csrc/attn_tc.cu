@@ -8,10 +8,13 @@
 //   forward :  S = Q K^T (all pairs of stacked rows)  ->  P = dropout(softmax(scale * S)) of the own head  ->  O = P V
 //   backward:  S, dP = dO V^T  ->  dS  ->  dQ = dS K ;  dK = dS^T Q ;  dV = P_drop^T dO
 //
-// P and dS are [128 x 128] tiles with zeros between different heads.  Written once, row per thread, the dS tile is read K-major for
-// dQ and MN-major (transposed) for dK.  P takes the place of operands that are no longer needed, and the results take the place
-// of S and dP in TMEM: 48 / 112 KB and 128 / 256 columns, so that two CTAs and more share an SM (one chain a head, with 64 / 144 KB
-// and 256 / 512 columns, had one in backward: 1024 heads of 32 x 64 took two rounds).
+// P and dS are [128 x 128] tiles with zeros between different heads.  Where V (forward) or Q, K or dO (backward) hold a value that
+// is not finite, these zeros would make NaN of it in the rows of other heads: such a CTA multiplies one head's rows at a time and
+// each head keeps what came of its own.  The look for such values is free, it is taken while the tensor cores make S and dP (at the
+// end, from the results, it took 0.5 us of a backward of 8).  Written once, row per thread, the dS tile is read K-major for dQ and
+// MN-major (transposed) for dK.  P takes the place of operands that are no longer needed, and the results take the place of S and dP
+// in TMEM: 48 / 112 KB and 128 / 256 columns, so that two CTAs and more share an SM (one chain a head, with 64 / 144 KB and 256 /
+// 512 columns, had one in backward: 1024 heads of 32 x 64 took two rounds).
 // us, that form -> this: 1024 heads of 32 with dropout, forward 10.2 -> 7.9, backward 21.0 -> 11.0; 32 heads of 32 5.8 -> 5.4 and
 // 9.7 -> 8.2; 1024 heads of 64 17.8 -> 15.7 and 47.4 -> 26.3.
 //
@@ -25,6 +28,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -176,6 +180,27 @@ __device__ __forceinline__ void load_row(uint32_t taddr, float (&x)[S_T]) {
   }
 }
 
+// 1 if one of these bf16 is an infinity or a NaN
+__device__ __forceinline__ int not_finite(const uint4 (&v)[8]) {
+  uint32_t m = 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    m = __vimax3_u16x2(m, v[i].x & 0x7fff7fffu, v[i].y & 0x7fff7fffu);
+    m = __vimax3_u16x2(m, v[i].z & 0x7fff7fffu, v[i].w & 0x7fff7fffu);
+  }
+  return (m & 0xffffu) >= 0x7f80u || (m >> 16) >= 0x7f80u;
+}
+// The products of a CTA, each over the 128 stacked rows in slices of 16, or over the rows of head g alone.
+template <int S_T, typename... Products>
+__device__ __forceinline__ void each_slice(bool all, int g, Products... products) {
+  auto chain = [](auto product, int j0, auto n) {
+#pragma unroll
+    for (int i = 0; i < decltype(n)::value; ++i) product(j0 + i, i > 0);
+  };
+  if (all) (chain(products, 0, std::integral_constant<int, kRows / 16>{}), ...);
+  else (chain(products, g * (S_T / 16), std::integral_constant<int, S_T / 16>{}), ...);
+}
+
 template <int S_T>
 __global__ void __launch_bounds__(128) attn_tc_fwd_kernel(const __nv_bfloat16* __restrict__ qkv,
                                                           __nv_bfloat16* __restrict__ out, int B, int heads, int nshard,
@@ -202,6 +227,7 @@ __global__ void __launch_bounds__(128) attn_tc_fwd_kernel(const __nv_bfloat16* _
   const uint32_t tmem = ctl->tmem_base;
   const int q = tid / S_T, s = tid % S_T;
   uint64_t keep;
+  uint4 va[8], vb[8], vc[8];
   {
     HeadRef hq[HPC], hk[HPC], hv[HPC];
 #pragma unroll
@@ -210,7 +236,6 @@ __global__ void __launch_bounds__(128) attn_tc_fwd_kernel(const __nv_bfloat16* _
       hk[qq] = {ctl->valid[qq], ctl->b[qq], ctl->ck[qq]};
       hv[qq] = {ctl->valid[qq], ctl->b[qq], ctl->cv[qq]};
     }
-    uint4 va[8], vb[8], vc[8];
     fetch_stack<S_T>(va, qkv, 3 * D, B, hq, tid);
     fetch_stack<S_T>(vb, qkv, 3 * D, B, hk, tid);
     fetch_stack<S_T>(vc, qkv, 3 * D, B, hv, tid);
@@ -233,6 +258,7 @@ __global__ void __launch_bounds__(128) attn_tc_fwd_kernel(const __nv_bfloat16* _
       umma_bf16(tmem, make_smem_desc(aq + kk * 32, 16, 1024), make_smem_desc(bk + kk * 32, 16, 1024), idesc, kk > 0 ? 1u : 0u);
     umma_commit(&ctl->bar[0]);
   }
+  const int odd = not_finite(vc);
   wait_bar(&ctl->bar[0], 0);
   __syncwarp();
   tc_fence_after();
@@ -262,35 +288,39 @@ __global__ void __launch_bounds__(128) attn_tc_fwd_kernel(const __nv_bfloat16* _
   ATT_STAMP(4);
   fence_proxy_async_smem();
   tc_fence_before();
-  __syncthreads();   // every row of S has been read: its TMEM columns are reused for O
+  const int parts = __syncthreads_or(odd) ? HPC : 1;
   ATT_STAMP(5);
 
-  if (warp == 0 && elect_one()) {
+#pragma unroll 1
+  for (int g = 0; g < parts; ++g) {
+    if (warp == 0 && elect_one()) {
+      tc_fence_after();
+      const uint32_t idesc = make_idesc_bf16(128, kHd, 0, 1);
+      const uint32_t ap = smem_u32(sP), bv = smem_u32(sV);
+      auto product = [&](int j, bool add) {        // 16 of the stacked keys
+        umma_bf16(tmem, make_smem_desc(ap + (j >> 2) * kTile + (j & 3) * 32, 16, 1024), make_smem_desc(bv + j * 2048, 8192, 1024), idesc,
+                  add ? 1u : 0u);
+      };
+      each_slice<S_T>(parts == 1, g, product);
+      umma_commit(&ctl->bar[1]);
+    }
+    wait_bar(&ctl->bar[1], g & 1);
+    __syncwarp();
     tc_fence_after();
-    const uint32_t idesc = make_idesc_bf16(128, kHd, 0, 1);
-    const uint32_t ap = smem_u32(sP), bv = smem_u32(sV);
-#pragma unroll
-    for (int kk = 0; kk < 8; ++kk)
-      umma_bf16(tmem, make_smem_desc(ap + (kk >> 2) * kTile + (kk & 3) * 32, 16, 1024), make_smem_desc(bv + kk * 2048, 8192, 1024),
-                idesc, kk > 0 ? 1u : 0u);
-    umma_commit(&ctl->bar[1]);
+    ATT_STAMP(6);
+    if (parts == 1 || g == q) {
+      // a warp's 32 rows belong to one head and to consecutive positions
+      float o[kHd];
+      load_row<kHd>(lane_addr, o);
+      __nv_bfloat16* dst = out + (size_t)((s - lane) * B + ctl->b[q]) * D + ctl->h[q] * kHd;
+      const int rows = ctl->valid[q] ? 32 : 0;
+      store_rows32(dst, (long long)B * D, rows, o, lane);
+      store_rows32(dst + 32, (long long)B * D, rows, o + 32, lane);
+    }
+    ATT_STAMP(7);
+    tc_fence_before();
+    __syncthreads();
   }
-  wait_bar(&ctl->bar[1], 0);
-  __syncwarp();
-  tc_fence_after();
-  ATT_STAMP(6);
-  {
-    // a warp's 32 rows belong to one head and to consecutive positions
-    float o[kHd];
-    load_row<kHd>(lane_addr, o);
-    __nv_bfloat16* dst = out + (size_t)((s - lane) * B + ctl->b[q]) * D + ctl->h[q] * kHd;
-    const int rows = ctl->valid[q] ? 32 : 0;
-    store_rows32(dst, (long long)B * D, rows, o, lane);
-    store_rows32(dst + 32, (long long)B * D, rows, o + 32, lane);
-  }
-  ATT_STAMP(7);
-  tc_fence_before();
-  __syncthreads();
   if (warp == 0) {
     tc_fence_after();
     tmem_dealloc(tmem, 128);
@@ -327,6 +357,7 @@ __global__ void __launch_bounds__(128) attn_tc_bwd_kernel(const __nv_bfloat16* _
   const uint32_t tmem = ctl->tmem_base;
   const int q = tid / S_T, s = tid % S_T;
   uint64_t keep;
+  uint4 va[8], vb[8], vc[8], vd[8];
   {
     HeadRef hq[HPC], hk[HPC], hv[HPC], hg[HPC];
 #pragma unroll
@@ -336,7 +367,6 @@ __global__ void __launch_bounds__(128) attn_tc_bwd_kernel(const __nv_bfloat16* _
       hv[qq] = {ctl->valid[qq], ctl->b[qq], ctl->cv[qq]};
       hg[qq] = {ctl->valid[qq], ctl->b[qq], ctl->h[qq] * kHd};   // dO has [T, D] layout: column of head h is h * 64
     }
-    uint4 va[8], vb[8], vc[8], vd[8];
     fetch_stack<S_T>(va, qkv, 3 * D, B, hq, tid);
     fetch_stack<S_T>(vb, qkv, 3 * D, B, hk, tid);
     fetch_stack<S_T>(vc, dout, D, B, hg, tid);
@@ -364,6 +394,7 @@ __global__ void __launch_bounds__(128) attn_tc_bwd_kernel(const __nv_bfloat16* _
       umma_bf16(tmem + 128, make_smem_desc(ag + kk * 32, 16, 1024), make_smem_desc(bv + kk * 32, 16, 1024), idesc, kk > 0 ? 1u : 0u);
     umma_commit(&ctl->bar[0]);
   }
+  const int odd = not_finite(va) | not_finite(vb) | not_finite(vc);
   wait_bar(&ctl->bar[0], 0);
   __syncwarp();
   tc_fence_after();
@@ -407,52 +438,55 @@ __global__ void __launch_bounds__(128) attn_tc_bwd_kernel(const __nv_bfloat16* _
   ATT_STAMP(4);
   fence_proxy_async_smem();
   tc_fence_before();
-  __syncthreads();   // S and dP have been read everywhere: their TMEM columns are reused for the results
+  const int parts = __syncthreads_or(odd) ? HPC : 1;   // S and dP have been read everywhere: the results take their TMEM columns
   ATT_STAMP(5);
 
-  if (warp == 0 && elect_one()) {
-    tc_fence_after();
-    const uint32_t as = smem_u32(sS), ap = smem_u32(sP), bk = smem_u32(sK), bq = smem_u32(sQ), bg = smem_u32(sG);
-    const uint32_t id_q = make_idesc_bf16(128, kHd, 0, 1), id_t = make_idesc_bf16(128, kHd, 1, 1);
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-      umma_bf16(tmem, make_smem_desc(as + (j >> 2) * kTile + (j & 3) * 32, 16, 1024), make_smem_desc(bk + j * 2048, 8192, 1024), id_q,
-                j > 0 ? 1u : 0u);
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-      umma_bf16(tmem + 64, make_smem_desc(as + j * 2048, kTile, 1024), make_smem_desc(bq + j * 2048, 8192, 1024), id_t,
-                j > 0 ? 1u : 0u);
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-      umma_bf16(tmem + 128, make_smem_desc(ap + j * 2048, kTile, 1024), make_smem_desc(bg + j * 2048, 8192, 1024), id_t,
-                j > 0 ? 1u : 0u);
-    umma_commit(&ctl->bar[1]);
-  }
-  wait_bar(&ctl->bar[1], 0);
-  __syncwarp();
-  tc_fence_after();
-  ATT_STAMP(6);
-  {
-    // a warp's 32 rows belong to one head and to consecutive positions
-    __nv_bfloat16* rowp = dqkv + (size_t)((s - lane) * B + ctl->b[q]) * (3 * D);
-    const long long pitch = 3ll * B * D;
-    const int rows = ctl->valid[q] ? 32 : 0;
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      const int col = r == 0 ? ctl->cq[q] : r == 1 ? ctl->ck[q] : ctl->cv[q];
-      float o[kHd];
-      load_row<kHd>(lane_addr + r * kHd, o);
-      if (r < 2) {
-#pragma unroll
-        for (int c = 0; c < kHd; ++c) o[c] *= sm_scale;
-      }
-      store_rows32(rowp + col, pitch, rows, o, lane);
-      store_rows32(rowp + col + 32, pitch, rows, o + 32, lane);
+#pragma unroll 1
+  for (int g = 0; g < parts; ++g) {
+    if (warp == 0 && elect_one()) {
+      tc_fence_after();
+      const uint32_t as = smem_u32(sS), ap = smem_u32(sP), bk = smem_u32(sK), bq = smem_u32(sQ), bg = smem_u32(sG);
+      const uint32_t id_q = make_idesc_bf16(128, kHd, 0, 1), id_t = make_idesc_bf16(128, kHd, 1, 1);
+      // 16 of the stacked keys (dQ) or queries
+      auto dq = [&](int j, bool add) {
+        umma_bf16(tmem, make_smem_desc(as + (j >> 2) * kTile + (j & 3) * 32, 16, 1024), make_smem_desc(bk + j * 2048, 8192, 1024), id_q,
+                  add ? 1u : 0u);
+      };
+      auto dk = [&](int j, bool add) {
+        umma_bf16(tmem + 64, make_smem_desc(as + j * 2048, kTile, 1024), make_smem_desc(bq + j * 2048, 8192, 1024), id_t, add ? 1u : 0u);
+      };
+      auto dv = [&](int j, bool add) {
+        umma_bf16(tmem + 128, make_smem_desc(ap + j * 2048, kTile, 1024), make_smem_desc(bg + j * 2048, 8192, 1024), id_t, add ? 1u : 0u);
+      };
+      each_slice<S_T>(parts == 1, g, dq, dk, dv);
+      umma_commit(&ctl->bar[1]);
     }
+    wait_bar(&ctl->bar[1], g & 1);
+    __syncwarp();
+    tc_fence_after();
+    ATT_STAMP(6);
+    if (parts == 1 || g == q) {
+      // a warp's 32 rows belong to one head and to consecutive positions
+      __nv_bfloat16* rowp = dqkv + (size_t)((s - lane) * B + ctl->b[q]) * (3 * D);
+      const long long pitch = 3ll * B * D;
+      const int rows = ctl->valid[q] ? 32 : 0;
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        const int col = r == 0 ? ctl->cq[q] : r == 1 ? ctl->ck[q] : ctl->cv[q];
+        float o[kHd];
+        load_row<kHd>(lane_addr + r * kHd, o);
+        if (r < 2) {
+#pragma unroll
+          for (int c = 0; c < kHd; ++c) o[c] *= sm_scale;
+        }
+        store_rows32(rowp + col, pitch, rows, o, lane);
+        store_rows32(rowp + col + 32, pitch, rows, o + 32, lane);
+      }
+    }
+    ATT_STAMP(7);
+    tc_fence_before();
+    __syncthreads();
   }
-  ATT_STAMP(7);
-  tc_fence_before();
-  __syncthreads();
   if (warp == 0) {
     tc_fence_after();
     tmem_dealloc(tmem, 256);
