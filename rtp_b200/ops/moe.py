@@ -49,13 +49,14 @@ def dispatch(x, idx, loc, valid, num_experts, capacity):
     slot = _slots(idx, loc, valid, capacity)
     out, fill = _Dispatch.apply(x, slot, num_experts * capacity, num_experts)
     out = out.view(num_experts, capacity, x.shape[1])
-    out._rtp_fill = (fill, out._version)     # holds as long as nobody writes to the rows (see rows_in_use)
+    if not out.is_inference():                   # an inference tensor does not count its writes
+        out._rtp_fill = (fill, out._version)     # holds as long as nobody writes to the rows (see rows_in_use)
     return out
 
 
 def rows_in_use(dispatched):
     """int32 [E]: for each expert of a tensor made by :func:`dispatch` the rows up to the last one with a token (those behind it
-    are zeros), or None where that is not known or the tensor has been written to since."""
+    are zeros), or None where that is not known (inference mode) or the tensor has been written to since."""
     fill, version = getattr(dispatched, "_rtp_fill", (None, None))
     return fill if fill is not None and dispatched._version == version else None
 

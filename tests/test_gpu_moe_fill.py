@@ -60,3 +60,34 @@ def test_written_rows_count():
     assert rows_in_use(d).tolist() == [16, 0]
     d[1, 3] = 1
     assert rows_in_use(d) is None
+
+
+def layer_of(kind, tokens, D=64, H=128, E=8):
+    from rtp_b200.models.moe_lm import Expert
+    from rtp_b200.module.moe import MOELayer, WeightMOELayer
+    from rtp_b200.module.top2gate import Top2Gate, WeightTop2Gate
+    torch.manual_seed(1)
+    experts = nn.ModuleList([Expert(D, H) for _ in range(E)])
+    if kind == "rotating":
+        layer = WeightMOELayer(WeightTop2Gate(D, E, device="cuda", dtype=BF), experts, device="cuda", dtype=BF)
+    else:
+        layer = MOELayer(Top2Gate(D, E), experts).to("cuda", BF)
+    x = torch.randn(1, tokens, D, device="cuda").to(BF)
+
+    def run():
+        torch.manual_seed(2)                  # the noise of the second choice
+        return layer(x), layer.l_aux
+    return run
+
+
+@pytest.mark.parametrize("kind", ["rotating", "all-to-all"])
+def test_inference_mode(kind):
+    """The same outputs as without gradients (tiles without tokens differ, which reach no output: one rounding, 2^-8, each way)."""
+    run = layer_of(kind, 512)
+    with torch.no_grad():
+        y, aux = run()
+    with torch.inference_mode():
+        z, aux2 = run()
+    assert y.isfinite().all() and y.norm() > 0
+    assert torch.equal(aux, aux2)
+    assert bool(((y.double() - z.double()).abs() <= 2.0 ** -7 * y.double().abs() + 1e-3 * y.double().abs().max()).all())
