@@ -20,7 +20,8 @@ class _Dispatch(torch.autograd.Function):
         ctx.save_for_backward(slot)
         fill = torch.empty(num_experts, dtype=torch.int32, device=x.device)
         ctx.mark_non_differentiable(fill)
-        return K.moe_scatter(x.contiguous(), slot, None, rows, fill), fill
+        # without a capacity there is nothing to count (and no row: every token is dropped)
+        return K.moe_scatter(x.contiguous(), slot, None, rows, fill if rows else None), fill if rows else fill.zero_()
 
     @staticmethod
     def backward(ctx, g, _):

@@ -62,16 +62,16 @@ def test_written_rows_count():
     assert rows_in_use(d) is None
 
 
-def layer_of(kind, tokens, D=64, H=128, E=8):
+def layer_of(kind, tokens, D=64, H=128, E=8, capacity=1.0):
     from rtp_b200.models.moe_lm import Expert
     from rtp_b200.module.moe import MOELayer, WeightMOELayer
     from rtp_b200.module.top2gate import Top2Gate, WeightTop2Gate
     torch.manual_seed(1)
     experts = nn.ModuleList([Expert(D, H) for _ in range(E)])
     if kind == "rotating":
-        layer = WeightMOELayer(WeightTop2Gate(D, E, device="cuda", dtype=BF), experts, device="cuda", dtype=BF)
+        layer = WeightMOELayer(WeightTop2Gate(D, E, device="cuda", dtype=BF, capacity_factor=capacity), experts, device="cuda", dtype=BF)
     else:
-        layer = MOELayer(Top2Gate(D, E), experts).to("cuda", BF)
+        layer = MOELayer(Top2Gate(D, E, capacity), experts).to("cuda", BF)
     x = torch.randn(1, tokens, D, device="cuda").to(BF)
 
     def run():
@@ -91,3 +91,16 @@ def test_inference_mode(kind):
     assert y.isfinite().all() and y.norm() > 0
     assert torch.equal(aux, aux2)
     assert bool(((y.double() - z.double()).abs() <= 2.0 ** -7 * y.double().abs() + 1e-3 * y.double().abs().max()).all())
+
+
+def test_no_capacity():
+    """Fewer places than one an expert: every token is dropped and the layer gives zeros, and so do its gradients."""
+    from rtp_b200.module.moe import dispatch_by_index
+    y, _ = layer_of("all-to-all", 8, capacity=0.25)()
+    assert y.shape == (1, 8, 64) and bool((y == 0).all())
+    x = torch.randn(8, 64, device="cuda").to(BF).requires_grad_()
+    idx, none = torch.zeros(8, 2, dtype=torch.long, device="cuda"), torch.zeros(8, 2, dtype=torch.bool, device="cuda")
+    d = dispatch_by_index(x, idx, idx, none, 4, 0)
+    assert d.shape == (4, 0, 64)
+    (g,) = torch.autograd.grad(d, x, torch.empty_like(d))
+    assert bool((g == 0).all())
