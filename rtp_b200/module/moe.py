@@ -71,12 +71,14 @@ def _combine(combine_weights: Tensor, expert_output: Tensor) -> Tensor:
     return torch.einsum("sec,ecm->sm", combine_weights, expert_output)
 
 
-def dispatch_by_index(x: Tensor, idx: Tensor, loc: Tensor, valid: Tensor, num_experts: int, capacity: int) -> Tensor:
+def dispatch_by_index(x: Tensor, idx: Tensor, loc: Tensor, valid: Tensor, num_experts: int, capacity: int,
+                      count_rows: bool = True) -> Tensor:
     """Index form of ``einsum("sec,sm->ecm", dispatch_mask, x)``: token s goes to slot ``loc[s, k]`` of expert
-    ``idx[s, k]`` for each valid choice k.  O(S*M) instead of O(S*E*C*M)."""
+    ``idx[s, k]`` for each valid choice k.  O(S*M) instead of O(S*E*C*M).  ``count_rows``: on a GPU the result also knows
+    how far each expert's rows are filled, which ``fused_experts`` on a ring of one rank reads."""
     from ..ops import moe as MK
     if MK.use_kernels(x):
-        return MK.dispatch(x, idx, loc, valid, num_experts, capacity)
+        return MK.dispatch(x, idx, loc, valid, num_experts, capacity, count_rows)
     S, M = x.shape
     dummy = num_experts * capacity
     slot = torch.where(valid, idx * capacity + loc, torch.full_like(idx, dummy))
@@ -97,13 +99,13 @@ def combine_by_index(expert_output: Tensor, idx: Tensor, loc: Tensor, gate: Tens
     return (flat[slot] * g.unsqueeze(-1)).sum(dim=1)
 
 
-def _route(gate_module, x):
+def _route(gate_module, x, count_rows):
     """(l_aux, dispatch fn, combine fn) from a gate: index form when the gate offers ``route``, else the dense
-    [S, E, C] tensors of the reference."""
+    [S, E, C] tensors of the reference.  ``count_rows``: see ``dispatch_by_index``."""
     if hasattr(gate_module, "route"):
         l_aux, idx, loc, g, valid, capacity = gate_module.route(x)
         E = getattr(gate_module, "num_experts", None) or gate_module.wg.out_features
-        return (l_aux.to(x.dtype), lambda t: dispatch_by_index(t, idx, loc, valid, E, capacity),
+        return (l_aux.to(x.dtype), lambda t: dispatch_by_index(t, idx, loc, valid, E, capacity, count_rows),
                 lambda eo: combine_by_index(eo, idx, loc, g, valid))
     l_aux, combine_weights, dispatch_mask = gate_module(x)
     return l_aux, (lambda t: _dispatch(dispatch_mask, t)), (lambda eo: _combine(combine_weights, eo))
@@ -128,7 +130,7 @@ class MOELayer(nn.Module):
         assert len(input[0].shape) == 3, "input Tensor must have dimensions: (s)equence, (t)oken, (m)odel"
         d_model = input[0].shape[2]
         reshaped = input[0].reshape(-1, d_model)
-        self.l_aux, dispatch, combine = _route(self.gate, reshaped)
+        self.l_aux, dispatch, combine = _route(self.gate, reshaped, False)
         dispatched = dispatch(reshaped)
         dispatched = _AllToAll.apply(self.ring.group, dispatched)
         dispatched = dispatched.reshape(self.world_size, self.num_local_experts, -1, d_model)
@@ -211,7 +213,7 @@ class WeightMOELayer(RotatedModule):
         d_model = input[0].shape[2]
         _guard_plain_launches(self.world_size, input[0].is_cuda)
         reshaped = input[0].reshape(-1, d_model)
-        self.l_aux, dispatch, combine = _route(self.gate, reshaped)
+        self.l_aux, dispatch, combine = _route(self.gate, reshaped, self.world_size == 1)
         dispatched = dispatch(reshaped)                          # [E, C, M]
         N, L = self.world_size, self.num_local_experts
         experts, names = self.experts, self._pnames

@@ -16,15 +16,12 @@ def _slots(idx, loc, valid, capacity):
 
 class _Dispatch(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, slot, rows, num_experts):
+    def forward(ctx, x, slot, rows, fill):
         ctx.save_for_backward(slot)
-        fill = torch.empty(num_experts, dtype=torch.int32, device=x.device)
-        ctx.mark_non_differentiable(fill)
-        # without a capacity there is nothing to count (and no row: every token is dropped)
-        return K.moe_scatter(x.contiguous(), slot, None, rows, fill if rows else None), fill if rows else fill.zero_()
+        return K.moe_scatter(x.contiguous(), slot, None, rows, fill)
 
     @staticmethod
-    def backward(ctx, g, _):
+    def backward(ctx, g):
         (slot,) = ctx.saved_tensors
         return K.moe_gather(g.contiguous(), slot, None), None, None, None
 
@@ -46,11 +43,15 @@ class _Combine(torch.autograd.Function):
         return d_eo, None, d_gate
 
 
-def dispatch(x, idx, loc, valid, num_experts, capacity):
+def dispatch(x, idx, loc, valid, num_experts, capacity, count_rows=True):
+    """``count_rows``: the result is for :func:`rows_in_use`.  Not done in inference mode (such a tensor does not count its writes)
+    and without a capacity (no row, nothing to count)."""
     slot = _slots(idx, loc, valid, capacity)
-    out, fill = _Dispatch.apply(x, slot, num_experts * capacity, num_experts)
-    out = out.view(num_experts, capacity, x.shape[1])
-    if not out.is_inference():                   # an inference tensor does not count its writes
+    fill = None
+    if count_rows and capacity > 0 and not torch.is_inference_mode_enabled():
+        fill = torch.empty(num_experts, dtype=torch.int32, device=x.device)
+    out = _Dispatch.apply(x, slot, num_experts * capacity, fill).view(num_experts, capacity, x.shape[1])
+    if fill is not None:
         out._rtp_fill = (fill, out._version)     # holds as long as nobody writes to the rows (see rows_in_use)
     return out
 

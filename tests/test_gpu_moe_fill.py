@@ -104,3 +104,13 @@ def test_no_capacity():
     assert d.shape == (4, 0, 64)
     (g,) = torch.autograd.grad(d, x, torch.empty_like(d))
     assert bool((g == 0).all())
+
+
+@pytest.mark.parametrize("kind,counted", [("rotating", True), ("all-to-all", False)])
+def test_rows_are_counted_for_who_reads_them(kind, counted, monkeypatch):
+    from rtp_b200.ops import kernels as K
+    seen, scatter = [], K.moe_scatter
+    monkeypatch.setattr(K, "moe_scatter", lambda src, slot, scale, rows, fill=None: seen.append(fill) or scatter(src, slot, scale, rows, fill))
+    with torch.no_grad():
+        layer_of(kind, 64)()
+    assert len(seen) == 1 and (seen[0] is not None) == counted
