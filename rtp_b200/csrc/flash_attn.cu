@@ -18,7 +18,8 @@
 // What it gives (us, before: one row tile a CTA with two threads a row, P and dS through shared memory, dQ and dK / dV in
 // launches of their own; now), forward and backward: 1 x 16 heads of 8192 x 8192 x 128 causal 338 -> 242 and 1 134 -> 805,
 // 4 x 16 of 2048 causal 126 -> 90 and 400 -> 285, 8 x 20 of 512 x 2048 x 64 121 -> 90 and 433 -> 250, 4 x 8 of 256 x 256 x 64
-// 8.3 -> 10 and 19 -> 13.  Per 128 x 128 block at head_dim 128 (SM clocks): forward 1 700 (tensor work 1 024, exponentials
+// 6.7 -> 6.4 and 20 -> 15, 4 x 8 of 64 x 64 x 64 5.1 -> 5.2.  One that is a little slower: a forward of one key block on more than
+// half of the SMs (8 x 16 of 64 x 64 x 64 5.5 -> 5.9), which cannot start under the one before for want of registers.  Per 128 x 128 block at head_dim 128 (SM clocks): forward 1 700 (tensor work 1 024, exponentials
 // 1 024), dK / dV 3 100 (tensor work 2 048), dQ 2 080 (1 536).  The forward is bound by the exponentials and the hand-overs
 // between row threads and issuer, dK / dV by the chain P -> dV -> S of the next block (TMEM has no room for a second S).
 //
@@ -62,6 +63,7 @@ struct DRef {                          // device copy of an RtpFlashRef
   int col_base, hpg, gstride, hstride;
 };
 __device__ __forceinline__ int head_col(const DRef& r, int h) {
+  if (h < r.hpg) return r.col_base + h * r.hstride;      // one group of heads: no division
   return r.col_base + (h / r.hpg) * r.gstride + (h % r.hpg) * r.hstride;
 }
 __device__ __forceinline__ __nv_bfloat16* row_ptr(const DRef& r, int b, int s, int h) {
@@ -151,6 +153,7 @@ __device__ __forceinline__ void load_tile(uint32_t dst, const CUtensorMap* map, 
 // 2 an additive mask (with or without key padding); `dead`: bit i set = key col0 + i is padding (dead_keys).
 template <int NC, int MSK>
 __device__ __forceinline__ void score_chunk(float* x, int row, int col0, uint32_t dead, const MaskArgs& m, bool plain) {
+  static_assert(NC == 32, "one word of bits");
 #pragma unroll
   for (int i = 0; i < NC; ++i) x[i] *= m.scale_log2;
   if (plain) return;
@@ -186,19 +189,13 @@ __device__ __forceinline__ void score_chunk(float* x, int row, int col0, uint32_
     }
   }
   }
-  if constexpr (MSK) {
-    if (dead) {
+  // bit i: key col0 + i has no weight
+  uint32_t off = MSK ? dead : 0u;
+  if (m.causal && col0 + NC - 1 > row) off |= row < col0 ? 0xffffffffu : 0xffffffffu << (row + 1 - col0);
+  if (col0 + NC > m.Sk) off |= col0 >= m.Sk ? 0xffffffffu : 0xffffffffu << (m.Sk - col0);
+  if (off) {
 #pragma unroll
-      for (int i = 0; i < NC; ++i) if ((dead >> i) & 1u) x[i] = -INFINITY;
-    }
-  }
-  if (m.causal && col0 + NC - 1 > row) {
-#pragma unroll
-    for (int i = 0; i < NC; ++i) if (col0 + i > row) x[i] = -INFINITY;
-  }
-  if (col0 + NC > m.Sk) {
-#pragma unroll
-    for (int i = 0; i < NC; ++i) if (col0 + i >= m.Sk) x[i] = -INFINITY;
+    for (int i = 0; i < NC; ++i) if ((off >> i) & 1u) x[i] = -INFINITY;
   }
 }
 // Padding bits of keys col0 .. col0 + 31, one byte per lane and a ballot (the warp works on one batch entry and one range
@@ -413,19 +410,26 @@ enum { F_QFULL = 0 /* 2 tiles */, F_QEMPTY = 2 /* 2 */, F_KFULL = 4 /* 2 stages 
        F_SFULL = 12 /* 2 tiles */, F_PFULL = 14 /* 2 */, F_PTAIL = 16 /* 2 */, F_OFULL = 18 /* 2 */, F_WFULL = 20, F_TAKEN = 21,
        F_DRAIN = 22 };
 
-// What blockIdx.x stands for: row tiles g0 (and g0 + 1) of a (batch, head), with n0 and n1 steps; nload key blocks in all.
+// What blockIdx.x stands for: row tiles g0 (and g0 + 1) of head h of batch entry b, with n0 and n1 steps; nload key blocks in all.
 struct FwdWork {
-  int g0, bh, n0, n1, nload;
+  int g0, bh, b, h, n0, n1, nload;
 };
 __device__ __forceinline__ FwdWork fwd_work(const FlashParams& p, int blk) {
   const int nqb = (p.m.Sq + kBlk - 1) / kBlk, nkb = (p.m.Sk + kBlk - 1) / kBlk, BH = p.B * p.H;
-  const int per = p.split ? 1 : 2;                                  // row tiles of a piece of work
-  // heaviest (last) query blocks of a group of heads first
-  const int nt = (nqb + per - 1) / per, grp = blk / (p.group * nt) * p.group;
-  const int in_grp = blk - grp * nt, heads = min(p.group, BH - grp);
+  // row tiles of a piece of work: one or two; heaviest (last) query blocks of a group of heads first
+  const int nt = p.split ? nqb : (nqb + 1) >> 1, span = p.group * nt;
+  int grp = 0;
+  if (blk >= span) {
+    const int g = blk / span;
+    grp = g * p.group;
+    blk -= g * span;
+  }
+  const int heads = min(p.group, BH - grp), level = blk / heads;
   FwdWork w;
-  w.g0 = (nt - 1 - in_grp / heads) * per;
-  w.bh = grp + in_grp % heads;
+  w.g0 = (nt - 1 - level) * (p.split ? 1 : 2);
+  w.bh = grp + blk - level * heads;
+  w.b = w.bh / p.H;
+  w.h = w.bh - w.b * p.H;
   const int nb0 = p.m.causal ? min(nkb, w.g0 + 1) : nkb;            // key blocks of the first tile, of the second
   const int nb1 = w.g0 + 1 >= nqb ? 0 : p.m.causal ? min(nkb, w.g0 + 2) : nkb;
   w.n0 = p.split ? (nb0 + 1) >> 1 : nb0;
@@ -452,6 +456,10 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_kernel(const __grid_con
   // counts by barrier index: copies and commits 1 each, P (its first three quarters, its last) 4: one per row warp of the tile,
   // next work 1 and 10 (producer, issuer, eight row warps)
   const int counts[23] = {1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 4, 4, 4, 4, 1, 1, 1, 10, 1};
+  // The first work is looked up before the wait for the previous kernel: its divisions took 1 000 clocks between set-up and the first
+  // copy, of the 12 000 of a launch of one key block (4 x 8 heads of 64 x 64).
+  const FwdWork first = fwd_work(p, (int)blockIdx.x);
+  asm volatile("" ::"r"(first.b), "r"(first.h), "r"(first.g0), "r"(first.nload));
   const uint32_t tmem = setup_cta(ctl, counts, 23, warp, lane);
   volatile uint32_t* abort_flag = &ctl->abort_flag;
   unsigned long long* status = p.status;
@@ -477,8 +485,8 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_kernel(const __grid_con
       auto wait = [&](int i, uint32_t ph) { return mbar_wait(&bar[i], ph, abort_flag, status, tmo); };
       uint32_t n = 0;
       for (int blk = (int)blockIdx.x; blk >= 0 && ok; blk = following(n++, false)) {
-        const FwdWork w = fwd_work(p, blk);
-        const int b = w.bh / p.H, h = w.bh % p.H;
+        const FwdWork w = n == 0 ? first : fwd_work(p, blk);
+        const int b = w.b, h = w.h;
         const int cq = head_col(p.q, h), ck = head_col(p.k, h), cv = head_col(p.v, h);
         auto load_q = [&](int t) {
           const uint32_t ph = nq[t]++ & 1u;
@@ -521,7 +529,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_kernel(const __grid_con
       };
       uint32_t n = 0, kv0 = 0, np[2] = {0, 0}, nq[2] = {0, 0};      // blocks before this work, P tiles and Q tiles so far
       for (int blk = (int)blockIdx.x; blk >= 0 && ok; blk = following(n++, false)) {
-        const FwdWork w = fwd_work(p, blk);
+        const FwdWork w = n == 0 ? first : fwd_work(p, blk);
         const int n0 = w.n0, n1 = w.n1;
         mbar_arrive(&bar[F_TAKEN]);
         ok = wait(F_QFULL, nq[0]++ & 1u) && issue_s(0, kv0, split || n1 == 0, !split && n0 == 1);
@@ -576,9 +584,9 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_kernel(const __grid_con
     // stamps of the two tiles' first warps of CTA 0: [warp 0 | warp 4][step < 16][event < 8]
     long long* tr = (p.trace && blockIdx.x == 0 && lane == 0 && (warp & 3) == 0) ? p.trace + (warp >> 2) * 128 : nullptr;
     for (int blk = (int)blockIdx.x; blk >= 0; blk = following(n++, true)) {
-    const FwdWork w = fwd_work(p, blk);
+    const FwdWork w = n == 0 ? first : fwd_work(p, blk);
     if (lane == 0) mbar_arrive(&bar[F_TAKEN]);
-    const int bh = w.bh, b = bh / p.H, h = bh % p.H, n1 = w.n1;
+    const int bh = w.bh, b = w.b, h = w.h, n1 = w.n1;
     const int nt = t ? n1 : w.n0, gt = w.g0 + (split ? 0 : t);
     const int row = gt * kBlk + rt;
     float m_used = -INFINITY, l = 0.f;
@@ -592,18 +600,24 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_kernel(const __grid_con
       if (!__all_sync(0xffffffffu, good)) { ok = false; break; }
       tc_fence_after();
       if (tr && ns < 16) tr[ns * 8 + 1] = clock64();
-      // A block that needs more than the scale is put right in TMEM first, 32 columns at a time, so that the loop below is one
+      // A block that needs more than the scale is put right in TMEM first, 32 or 64 columns at a time, so that the loop below is one
       // for all blocks; one that only needs the scale keeps the raw scores: the scale rides in the exponent's multiply-add.
       const bool plain = MSK != 2 && !(dead[0] | dead[1] | dead[2] | dead[3]) && !(M.causal && c == gt) && (col0 + kBlk <= M.Sk) &&
                          M.scale_log2 >= 0.f;          // the maximum commutes with a positive scale only
       if (!plain) {
+        constexpr int NQ = MSK == 2 ? 1 : 2;           // chunks at a time: the additive mask's code is long
 #pragma unroll 1
-        for (int q = 0; q < 4; ++q) {
-          float x[32];
-          tmem_ld32f(aS + (uint32_t)(q * 32), x);
+        for (int q = 0; q < 4; q += NQ) {
+          float x[32 * NQ];
+#pragma unroll
+          for (int u = 0; u < NQ; ++u) tmem_ld32f(aS + (uint32_t)((q + u) * 32), x + 32 * u);
           tmem_ld_wait();
-          score_chunk<32, MSK>(x, row, col0 + 32 * q, q == 0 ? dead[0] : q == 1 ? dead[1] : q == 2 ? dead[2] : dead[3], M, false);
-          tmem_st32f(aS + (uint32_t)(q * 32), x);
+#pragma unroll
+          for (int u = 0; u < NQ; ++u) {
+            const uint32_t dd = q + u == 0 ? dead[0] : q + u == 1 ? dead[1] : q + u == 2 ? dead[2] : dead[3];
+            score_chunk<32, MSK>(x + 32 * u, row, col0 + 32 * (q + u), dd, M, false);
+            tmem_st32f(aS + (uint32_t)((q + u) * 32), x + 32 * u);
+          }
         }
         tmem_st_wait();
       }
@@ -622,26 +636,31 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_kernel(const __grid_con
       const float m_new = need ? cand : m_used;
       const float mref = (m_new == -INFINITY) ? 0.f : m_new;
       const float mul = plain ? M.scale_log2 : 1.f;
-      if (i > 0 && __any_sync(0xffffffffu, need)) {
-        // the S that was waited for came after the P V of the tile's previous step: O is complete up to there
-        const float alpha = need ? ex2_approx(m_used - cand) : 1.f;
-#pragma unroll
-        for (int q = 0; q < HD / 32; ++q) {
-          float o[32];
-          tmem_ld32f(aO + (uint32_t)(q * 32), o);
-          tmem_ld_wait();
-#pragma unroll
-          for (int e = 0; e < 32; ++e) o[e] *= alpha;
-          tmem_st32f(aO + (uint32_t)(q * 32), o);
-        }
-        l *= alpha;
-      }
-      float2 ra = make_float2(0.f, 0.f), rb = ra;
-      const float2 mul2 = make_float2(mul, mul), ref2 = make_float2(-mref, -mref);
       // some: one exponential in four by polynomial.  That is for blocks without masked scores, which have to become 0, whose rows
       // all have a finite maximum: a NaN or an infinite score has to reach the output, and a row of -inf alone has no weights;
       // a -inf below a finite maximum gets 2^-126 beside 2^-8 or more.
-      auto exponentials = [&](auto some) {
+      const bool fin = fabsf(mx) < INFINITY;
+      bool some = !DRP && plain;
+      if (__any_sync(0xffffffffu, (i > 0 && need) || !fin)) {
+        if (i > 0 && __any_sync(0xffffffffu, need)) {
+          // the S that was waited for came after the P V of the tile's previous step: O is complete up to there
+          const float alpha = need ? ex2_approx(m_used - cand) : 1.f;
+#pragma unroll
+          for (int q = 0; q < HD / 32; ++q) {
+            float o[32];
+            tmem_ld32f(aO + (uint32_t)(q * 32), o);
+            tmem_ld_wait();
+#pragma unroll
+            for (int e = 0; e < 32; ++e) o[e] *= alpha;
+            tmem_st32f(aO + (uint32_t)(q * 32), o);
+          }
+          l *= alpha;
+        }
+        some = some && __all_sync(0xffffffffu, fin);
+      }
+      float2 ra = make_float2(0.f, 0.f), rb = ra;
+      const float2 mul2 = make_float2(mul, mul), ref2 = make_float2(-mref, -mref);
+      auto exponentials = [&](auto poly) {
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         float* e = s + 32 * q;
@@ -652,7 +671,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_kernel(const __grid_con
         for (int k = 0; k < 32; k += 4) {
           float2 x = fma2(make_float2(e[k], e[k + 1]), mul2, ref2), y = fma2(make_float2(e[k + 2], e[k + 3]), mul2, ref2);
           x = make_float2(ex2_approx(x.x), ex2_approx(x.y));
-          if (decltype(some)::value && (k & 4)) y = ex2_poly2(y);
+          if (decltype(poly)::value && (k & 4)) y = ex2_poly2(y);
           else y = make_float2(ex2_approx(y.x), ex2_approx(y.y));
           ra = add2(ra, x);
           rb = add2(rb, y);
@@ -674,14 +693,26 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_kernel(const __grid_con
         }
       }
       };
-      if (!DRP && plain && __all_sync(0xffffffffu, fabsf(mx) < INFINITY)) exponentials(std::true_type{});
-      else exponentials(std::false_type{});
+      if (some) exponentials(std::true_type{}); else exponentials(std::false_type{});
       m_used = m_new;
       l += (ra.x + ra.y) + (rb.x + rb.y);
       if (tr && ns < 16) tr[ns * 8 + 2] = clock64();
     }
-    if (ok && nt > 0) {
-      const uint32_t good = mbar_wait(&bar[F_OFULL + t], no++ & 1u, abort_flag, status, tmo) ? 1u : 0u;
+    const int r0 = gt * kBlk + (warp & 3) * 32;        // the warp's first row
+    __nv_bfloat16* const dst = row_ptr(p.o, b, r0, h);
+    const bool lone = split && n1 == 0;                // one key block: the tile's second warpgroup takes half of the columns
+    if (lone) {
+      if (t == 0) {
+        sX[rt] = m_used;
+        sX[128 + rt] = l;
+      }
+      asm volatile("bar.sync 1, 256;" ::: "memory");   // under the product P V
+      m_used = sX[rt];
+      l = sX[128 + rt];
+    }
+    const bool stores = nt > 0 || lone;
+    if (ok && stores) {
+      const uint32_t good = mbar_wait(&bar[F_OFULL + (lone ? 0 : t)], no++ & 1u, abort_flag, status, tmo) ? 1u : 0u;
       if (!__all_sync(0xffffffffu, good)) ok = false;
     }
     tc_fence_after();
@@ -712,15 +743,14 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_kernel(const __grid_con
       l = l * a_own + l_o * a_other;
       m_used = m_all;
     }
-    if (ok && nt > 0) {
+    if (ok && stores) {
       const float inv = l > 0.f ? 1.f / l : 0.f;
       const float* xi = reinterpret_cast<const float*>(sK) + (t ^ 1) * (HD / 2) * 128;
-      const int r0 = gt * kBlk + (warp & 3) * 32;      // the warp's first row
-      __nv_bfloat16* dst = row_ptr(p.o, b, r0, h);
-      const int c0 = merge ? t * OC : 0, c1 = merge ? c0 + OC : 2 * OC;
+      const int c0 = split ? t * OC : 0, c1 = split ? c0 + OC : 2 * OC;
+      const uint32_t aR = lone ? lane_addr + 256u : aO;
       for (int q = c0; q < c1; ++q) {
         float o[32];
-        tmem_ld32f(aO + (uint32_t)(q * 32), o);
+        tmem_ld32f(aR + (uint32_t)(q * 32), o);
         tmem_ld_wait();
         if (merge) {
 #pragma unroll
@@ -730,7 +760,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_fwd_kernel(const __grid_con
         for (int e = 0; e < 32; ++e) o[e] *= inv;
         store_rows32(dst + q * 32, p.o.ss, M.Sq - r0, o, lane);
       }
-      if (row < M.Sq && p.lse && !(merge && t)) {
+      if (row < M.Sq && p.lse && !(split && t)) {
         const float mref = (m_used == -INFINITY) ? 0.f : m_used;
         p.lse[(long long)bh * M.Sq + row] = l > 0.f ? mref + log2f(l) : INFINITY;
       }
@@ -1288,8 +1318,9 @@ int rtp_flash_fwd(const RtpFlashArgs* a, void* stream) {
   static thread_local FlashParams P;
   if (fill_common(a, P)) return -1;
   if (!a->lse) return ffail("flash attention: lse buffer required");
-  // One row tile a CTA, its keys shared out, as long as that is one wave (2 heads of 4096 x 4096 x 128: 49 -> 37 us); two row tiles
-  // a CTA beyond it, where they share the copies of K and V.
+  // One row tile a CTA, its keys shared out, as long as that is one wave; two row tiles a CTA beyond it, where they share the copies
+  // of K and V.  Two tiles -> shared out, us: 2 heads of 4096 x 4096 x 128 49 -> 37, 32 of 1024 keys x 128 17.7 -> 13.9, 32 of
+  // 256 x 256 x 64 9.2 -> 7.2, 4 of 384 x 384 x 64 9.5 -> 7.6; one key block the same either way.
   const int tiles = (a->Sq + kBlk - 1) / kBlk, BH = a->B * a->H;
   P.split = (long long)tiles * BH <= device_sms();
   P.group = head_group(4ll * a->Sk * a->head_dim, BH);
