@@ -7,8 +7,9 @@
 // Patches overlap, so im2col reads its input from shared memory and col2im keeps the patches of a few output rows there: each
 // reads global memory once (or a little more) in whole lines and is bound by the patch matrix.  One thread per patch of a
 // channel, every element from global memory, is what is left for inputs whose rows do not fit.  us, that form -> this
-// (64 x 32 x 26 x 26, 3 x 3; 64 x 1 x 28 x 28, 3 x 3; 32 x 64 x 32 x 32, 5 x 5, padding 1): im2col 36, 6.2, 314 -> 13.5, 2.5, 58,
-// col2im 49, 6.2, 181 -> 23, 3.3, 120.
+// (64 x 32 x 26 x 26, 3 x 3; 64 x 1 x 28 x 28, 3 x 3; 32 x 64 x 32 x 32, 5 x 5, padding 1): im2col 36, 6.2, 314 -> 14.5, 2.6, 57,
+// col2im 49, 6.2, 181 -> 23, 3.1, 120.  The patches of one row of 26 positions and 8 channels do not fit from 7 x 7 on: col2im of
+// 64 x 32 x 26 x 26, 7 x 7 stays at 195.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -92,6 +93,8 @@ constexpr int kSmemConv = 96 * 1024;        // two blocks an SM
 struct RowTile {
   int R, rows, Wp;                          // output rows of a block, input rows that they read, row pitch
 };
+// U loads of a thread in flight.
+template <int U>
 __global__ void __launch_bounds__(256) im2col_rows_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ cols,
                                                           ConvGeom g, RowTile t) {
   extern __shared__ __align__(16) uint8_t smem[];
@@ -109,12 +112,23 @@ __global__ void __launch_bounds__(256) im2col_rows_kernel(const __nv_bfloat16* _
   int w = threadIdx.x % t.Wp, r = threadIdx.x / t.Wp % t.rows, c = threadIdx.x / t.Wp / t.rows;
   pdl_prologue();
   const __nv_bfloat16* src = x + (size_t)b * g.C * g.H * g.W;
-  for (int i = threadIdx.x; i < zero_at; i += 256) {
-    const int h = h0 + r, v = w - g.pw;
-    tile[i] = h >= 0 && h < g.H && v >= 0 && v < g.W ? src[((size_t)c * g.H + h) * g.W + v] : __float2bfloat16(0.f);
-    w += dw; r += dr; c += dc;
-    if (w >= t.Wp) { w -= t.Wp; ++r; }
-    if (r >= t.rows) { r -= t.rows; ++c; }
+  const unsigned short* src16 = reinterpret_cast<const unsigned short*>(src);
+  unsigned short* tile16 = reinterpret_cast<unsigned short*>(tile);
+  for (int i = threadIdx.x; i < zero_at; i += U * 256) {
+    uint32_t e[U];
+    bool in[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int h = h0 + r, v = w - g.pw;
+      in[u] = i + u * 256 < zero_at && h >= 0 && h < g.H && v >= 0 && v < g.W;
+      e[u] = __ldg(src16 + (in[u] ? (c * g.H + h) * g.W + v : 0));      // an image has fewer than 2^31 elements
+      w += dw; r += dr; c += dc;
+      if (w >= t.Wp) { w -= t.Wp; ++r; }
+      if (r >= t.rows) { r -= t.rows; ++c; }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i + u * 256 < zero_at) tile16[i + u * 256] = in[u] ? (unsigned short)e[u] : (unsigned short)0;
   }
   __syncthreads();
   const int chunks = g.Kp / 8, total = nrow * g.OW * chunks;
@@ -136,7 +150,7 @@ __global__ void __launch_bounds__(256) im2col_rows_kernel(const __nv_bfloat16* _
 // col2im through shared memory.  Block: R input rows and CG channels of one image.  The patches of the output rows that touch them
 // lie in shared memory, the CG channels of a position side by side, positions an odd number of words apart: neighbouring threads
 // sum neighbouring input columns, which read neighbouring positions (stride 1) without bank conflicts.
-// KT, ST > 0: kernel and stride known, dilation 1, and the loops over a patch are unrolled.
+// ST > 0: stride known and dilation 1, no divisions; KT > 0: kernel known too, and the loops over a patch are unrolled.
 struct FoldTile {
   int R, CG, nout, pitch;                   // input rows and channels of a block, output rows held at most, elements per position
 };
@@ -226,6 +240,15 @@ int launch_geom(ConvGeom& g, int B, int C, int H, int W, int KH, int KW, int sh,
   return 0;
 }
 
+int device_sms() {
+  static int n[64] = {0};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) dev = 0;
+  if (!n[dev]) cudaDeviceGetAttribute(&n[dev], cudaDevAttrMultiProcessorCount, dev);
+  return n[dev];
+}
+
 template <int KT, int ST>
 cudaError_t launch_fold(const ConvGeom& g, const FoldTile& t, unsigned blocks, size_t bytes, const void* dcols, void* dx, cudaStream_t stream) {
   const cudaError_t e = ensure_smem<col2im_rows_kernel<KT, ST>>(kSmemConv);
@@ -247,16 +270,21 @@ int rtp_im2col(const void* x, void* cols, int B, int C, int H, int W, int KH, in
   RowTile t;
   t.Wp = std::max((g.OW - 1) * sw + (KW - 1) * dw + 1, 1);
   auto bytes = [&](int R) { return (long long)Kp * 4 + (long long)C * ((R - 1) * sh + (KH - 1) * dh + 1) * t.Wp * 2; };
-  if (Kp % 8 == 0 && (reinterpret_cast<uintptr_t>(cols) & 15) == 0 && bytes(1) <= kSmemConv) {
+  if (Kp % 8 == 0 && (reinterpret_cast<uintptr_t>(cols) & 15) == 0 && bytes(1) <= kSmemConv && (long long)C * H * W <= 0x7fffffff) {
     t.R = 1;
-    while (t.R < 8 && t.R < g.OH && bytes(2 * t.R) <= kSmemConv && (long long)B * ((g.OH + 2 * t.R - 1) / (2 * t.R)) >= 2 * 148) t.R *= 2;
+    while (t.R < 8 && t.R < g.OH && bytes(2 * t.R) <= kSmemConv && (long long)B * ((g.OH + 2 * t.R - 1) / (2 * t.R)) >= 2 * device_sms())
+      t.R *= 2;
     t.rows = (t.R - 1) * sh + (KH - 1) * dh + 1;
     const long long blocks = (long long)B * ((g.OH + t.R - 1) / t.R);
     if (blocks <= 0x7fffffff) {
-      cudaError_t e = rtp::ensure_smem<im2col_rows_kernel>(kSmemConv);
+      // Loads in flight pay for tiles of 16 loads a thread and more at stride 1.  us, one in flight and four: 64 x 32 x 26 x 26, 3 x 3 16.1
+      // and 14.5, 8 x 512 x 14 x 14, 3 x 3 31.8 and 31.0; 64 x 32 x 26 x 26, 2 x 2 by 2 6.0 and 7.4, 32 x 64 x 32 x 32, 3 x 3 by 2 9.5
+      // and 12.4, 64 x 1 x 28 x 28, 3 x 3 2.6 and 2.9.
+      const bool four = sh == 1 && (long long)C * t.rows * t.Wp >= 16 * 256;
+      cudaError_t e = four ? rtp::ensure_smem<im2col_rows_kernel<4>>(kSmemConv) : rtp::ensure_smem<im2col_rows_kernel<1>>(kSmemConv);
       if (e == cudaSuccess)
-        e = rtp::launch_k(im2col_rows_kernel, dim3((unsigned)blocks), dim3(256), (size_t)bytes(t.R), (cudaStream_t)stream,
-                          (const __nv_bfloat16*)x, (__nv_bfloat16*)cols, g, t);
+        e = rtp::launch_k(four ? im2col_rows_kernel<4> : im2col_rows_kernel<1>, dim3((unsigned)blocks), dim3(256), (size_t)bytes(t.R),
+                          (cudaStream_t)stream, (const __nv_bfloat16*)x, (__nv_bfloat16*)cols, g, t);
       if (e != cudaSuccess) { g_err = std::string("im2col: ") + cudaGetErrorString(e); return -1; }
       return 0;
     }
@@ -282,24 +310,25 @@ int rtp_col2im(const void* dcols, void* dx, int B, int C, int H, int W, int KH, 
     return (long long)t.nout * g.OW * t.pitch * 2;
   };
   if (Kp % 8 == 0 && (reinterpret_cast<uintptr_t>(dcols) & 15) == 0) {
-    // Small blocks, many to an SM: all channels if a row of them takes 48 KB at most, else groups of a multiple of 8; more rows as
-    // long as they fit 32 KB and every SM has two blocks (64 x 32 x 26 x 26: up to 96 KB a block 30 us, 48 KB 23, this 20).
+    // Small blocks, many to an SM: all channels if a row of them takes 48 KB at most and the rows are blocks enough for two an SM, else
+    // groups of a multiple of 8; more rows as long as they fit 32 KB and every SM has two blocks (64 x 32 x 26 x 26: up to 96 KB a
+    // block 30 us, 48 KB 23, this 20; 8 x 256 x 14 x 14, 1 x 1, all channels 8.1 us, groups 4.6).
     int CG = C;
-    while (CG > 8 && held(1, CG) > 48 * 1024) CG = (CG / 2 + 7) / 8 * 8;
+    while (CG > 8 && (held(1, CG) > 48 * 1024 || (long long)B * H * ((C + CG - 1) / CG) < 2 * device_sms())) CG = (CG / 2 + 7) / 8 * 8;
     if (held(1, CG) <= kSmemConv) {
       const long long groups = (C + CG - 1) / CG;
       int R = 1;
-      while (R < 16 && R < H && held(2 * R, CG) <= 32 * 1024 && B * groups * ((H + 2 * R - 1) / (2 * R)) >= 2 * 148) R *= 2;
+      while (R < 16 && R < H && held(2 * R, CG) <= 32 * 1024 && B * groups * ((H + 2 * R - 1) / (2 * R)) >= 2 * device_sms()) R *= 2;
       const size_t bytes = (size_t)held(R, CG);
       const long long blocks = B * groups * ((H + R - 1) / R);
       if (blocks <= 0x7fffffff) {
-        const bool plain = KH == KW && sh == sw && dh == 1 && dw == 1;
-        cudaStream_t st = (cudaStream_t)stream;
-        const cudaError_t e = plain && KH == 3 && sh == 1   ? launch_fold<3, 1>(g, t, (unsigned)blocks, bytes, dcols, dx, st)
-                              : plain && KH == 3 && sh == 2 ? launch_fold<3, 2>(g, t, (unsigned)blocks, bytes, dcols, dx, st)
-                              : plain && KH == 5 && sh == 1 ? launch_fold<5, 1>(g, t, (unsigned)blocks, bytes, dcols, dx, st)
-                              : plain && KH == 5 && sh == 2 ? launch_fold<5, 2>(g, t, (unsigned)blocks, bytes, dcols, dx, st)
-                                                            : launch_fold<0, 0>(g, t, (unsigned)blocks, bytes, dcols, dx, st);
+        // A stride that is not known costs two divisions for each entry of a patch.  us, neither known, stride, both: 64 x 32 x 26 x 26,
+        // 3 x 3 44, 28, 23; 32 x 64 x 32 x 32, 5 x 5 153, 157, 120, by 2 73, 46, 45; 64 x 32 x 26 x 26, 2 x 2 by 2 33, 18, 1 x 1 17, 11.
+        const int st = sh == sw && dh == 1 && dw == 1 && sh <= 2 ? sh : 0, kt = st && KH == KW && (KH == 3 || KH == 5) ? KH : 0;
+        const auto launch = kt == 3 ? (st == 1 ? launch_fold<3, 1> : launch_fold<3, 2>)
+                            : kt == 5 ? (st == 1 ? launch_fold<5, 1> : launch_fold<5, 2>)
+                            : st == 1 ? launch_fold<0, 1> : st == 2 ? launch_fold<0, 2> : launch_fold<0, 0>;
+        const cudaError_t e = launch(g, t, (unsigned)blocks, bytes, dcols, dx, (cudaStream_t)stream);
         if (e != cudaSuccess) { g_err = std::string("col2im: ") + cudaGetErrorString(e); return -1; }
         return 0;
       }

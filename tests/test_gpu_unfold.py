@@ -13,6 +13,7 @@ BF = torch.bfloat16
 @pytest.mark.parametrize("B,C,H,W,k,s,p,d", [
     (1, 1, 3, 3, (3, 3), 1, 0, 1), (64, 32, 26, 26, (3, 3), 1, 0, 1), (3, 5, 9, 13, (3, 2), (2, 1), (1, 0), 1),
     (2, 64, 32, 32, (5, 5), 1, 2, 1), (2, 17, 23, 12, (3, 3), 3, 1, 2), (300, 3, 12, 12, (5, 5), 2, 1, 1),
+    (8, 256, 14, 14, (1, 1), 1, 0, 1), (2, 24, 27, 26, (2, 2), 2, 0, 1), (3, 20, 15, 17, (7, 7), 1, 3, 1), (2, 9, 21, 20, (7, 3), 2, 3, 1),
     (1, 130, 40, 56, (5, 5), 1, 1, 1), (1, 600, 20, 60, (5, 5), 1, 0, 1), (2, 8, 30, 2000, (1, 1), 4, 0, 1), (1, 9, 7, 3000, (7, 3), 1, 3, 1)])
 def test_unfold_and_fold(B, C, H, W, k, s, p, d):
     from rtp_b200.ops import kernels as K
