@@ -1511,41 +1511,52 @@ int rtp_norm_fwd(const void* x, const void* sub, const void* gamma, const void* 
   LAUNCH_CHECK("norm_fwd");
   return 0;
 }
-// part_pitch and the number of blocks as in norm_bwd_kernel (blocks may be null)
+// Threads a row and rows in flight per group of a backward launch: no more rows than leave every SM a block or two, one where there
+// are fewer rows than SMs (64 x 4096 with dropout, two rows 7.5 us, one 6.9).
+struct NormBwdShape { int T, R; };
+static NormBwdShape norm_bwd_shape(int M, int D) {
+  if (D <= 256) return {32, M <= 2368 ? 1 : 4};
+  if (D <= 512) return {64, M <= 148 ? 1 : M <= 1184 ? 2 : 4};
+  if (D <= 1024) return {128, M <= 148 ? 1 : M <= 592 ? 2 : 4};
+  if (D <= 2048) return {256, M <= 1024 || M >= 4096 ? 2 : 4};
+  if (D <= 4096) return {256, M <= 148 ? 1 : 2};
+  return {256, 1};
+}
+// Few blocks: every block ends with one vector atomic per 4 columns of dgamma / dbeta.  Up to 1024 wide rows one block per
+// SM (256 x 2048 256 blocks 10.3 us, 128 with two rows each 7.4; 1024 x 3072 256 blocks 18.3, 148 14.6), else two.
+static int norm_bwd_blocks(int M, int D) {
+  const NormBwdShape s = norm_bwd_shape(M, D);
+  const int rows = 256 / s.T * s.R;
+  return std::min((M + rows - 1) / rows, M <= 1024 && D > 1024 ? 148 : 296);
+}
+// part_pitch as in norm_bwd_kernel
 static int norm_bwd_launch(const void* dy, const void* h, const void* gamma, const float* mean, const float* rstd, void* dx,
                            void* dsub, float* dgamma, float* dbeta, int M, int D, int rms, float drop_p, unsigned long long seed,
                            unsigned long long offset, const void* dres, const unsigned long long* step_ptr, int part_pitch,
-                           int* blocks, void* stream) {
+                           void* stream) {
   if (D % 8 || D > 8192) { k_err = "norm: D must be a multiple of 8 and at most 8192"; return -1; }
   const float ds = drop_p > 0.f ? 1.f / (1.f - drop_p) : 1.f;
   const int vec_atomics = ((reinterpret_cast<uintptr_t>(dgamma) | reinterpret_cast<uintptr_t>(dbeta)) & 15) == 0;
-  // Few blocks: every block ends with one vector atomic per 4 columns of dgamma / dbeta.  Up to 1024 wide rows one block per
-  // SM (256 x 2048 256 blocks 10.3 us, 128 with two rows each 7.4; 1024 x 3072 256 blocks 18.3, 148 14.6), else two.
-  const int most = M <= 1024 && D > 1024 ? 148 : 296;
-  int grid = 0;
+  const int R = norm_bwd_shape(M, D).R;
 #define RTP_NORM_BWD(T, NG, R, AHEAD)                                                                                 \
-  rtp::launch_k(norm_bwd_kernel<T, NG, R, AHEAD>, dim3(grid = std::min((M + 256 / T * R - 1) / (256 / T * R), most)),  \
-      dim3(256), 0, (cudaStream_t)stream,                                                                             \
+  rtp::launch_k(norm_bwd_kernel<T, NG, R, AHEAD>, dim3(norm_bwd_blocks(M, D)), dim3(256), 0, (cudaStream_t)stream,     \
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)h, (const __nv_bfloat16*)gamma, mean, rstd, (__nv_bfloat16*)dx, \
       (__nv_bfloat16*)dsub, dgamma, dbeta, M, D, rms, host_thresh(drop_p), ds, seed, offset,                          \
       (const __nv_bfloat16*)dres, step_ptr, vec_atomics, part_pitch)
-  // Rows in flight per group: no more than leave every SM a block or two, one where there are fewer rows than SMs
-  // (64 x 4096 with dropout, two rows 7.5 us, one 6.9).
-  if (D <= 256) { if (M <= 2368) RTP_NORM_BWD(32, 1, 1, false); else RTP_NORM_BWD(32, 1, 4, false); }
+  if (D <= 256) { if (R == 1) RTP_NORM_BWD(32, 1, 1, false); else RTP_NORM_BWD(32, 1, 4, false); }
   else if (D <= 512) {
-    if (M <= 148) RTP_NORM_BWD(64, 1, 1, false); else if (M <= 1184) RTP_NORM_BWD(64, 1, 2, false);
+    if (R == 1) RTP_NORM_BWD(64, 1, 1, false); else if (R == 2) RTP_NORM_BWD(64, 1, 2, false);
     else RTP_NORM_BWD(64, 1, 4, false);
   } else if (D <= 1024) {
-    if (M <= 148) RTP_NORM_BWD(128, 1, 1, false); else if (M <= 592) RTP_NORM_BWD(128, 1, 2, false);
+    if (R == 1) RTP_NORM_BWD(128, 1, 1, false); else if (R == 2) RTP_NORM_BWD(128, 1, 2, false);
     else RTP_NORM_BWD(128, 1, 4, false);
   } else if (D <= 2048) {
-    if (M <= 1024) RTP_NORM_BWD(256, 1, 2, false); else if (M < 4096) RTP_NORM_BWD(256, 1, 4, false);
+    if (M <= 1024) RTP_NORM_BWD(256, 1, 2, false); else if (R == 4) RTP_NORM_BWD(256, 1, 4, false);
     else RTP_NORM_BWD(256, 1, 2, true);
-  } else if (D <= 4096) { if (M <= 148) RTP_NORM_BWD(256, 2, 1, false); else RTP_NORM_BWD(256, 2, 2, false); }
+  } else if (D <= 4096) { if (R == 1) RTP_NORM_BWD(256, 2, 1, false); else RTP_NORM_BWD(256, 2, 2, false); }
   else if (D <= 6144) RTP_NORM_BWD(256, 3, 1, false); else RTP_NORM_BWD(256, 4, 1, false);
 #undef RTP_NORM_BWD
   LAUNCH_CHECK("norm_bwd");
-  if (blocks) *blocks = grid;
   return 0;
 }
 int rtp_norm_bwd(const void* dy, const void* h, const void* gamma, const float* mean, const float* rstd, void* dx,
@@ -1553,19 +1564,21 @@ int rtp_norm_bwd(const void* dy, const void* h, const void* gamma, const float* 
                  unsigned long long seed, unsigned long long offset, const void* dres,
                  const unsigned long long* step_ptr, void* stream) {
   return norm_bwd_launch(dy, h, gamma, mean, rstd, dx, dsub, dgamma, dbeta, M, D, rms, drop_p, seed, offset, dres, step_ptr, 0,
-                         nullptr, stream);
+                         stream);
 }
-unsigned long long rtp_norm_bwd_scratch(int D) { return 296ull * 2 * D * sizeof(float); }
+unsigned long long rtp_norm_bwd_scratch(int M, int D, int has_beta) {
+  return (unsigned long long)norm_bwd_blocks(M, D) * (has_beta ? 2 : 1) * D * sizeof(float);
+}
 int rtp_norm_bwd_params(const void* dy, const void* h, const void* gamma, const float* mean, const float* rstd, void* dx,
                         void* dgamma, void* dbeta, float* scratch, int M, int D, int rms, const void* dres, void* stream) {
   if (M <= 0) { k_err = "norm backward: no rows"; return -1; }
   if (reinterpret_cast<uintptr_t>(scratch) & 15) { k_err = "norm backward: scratch must be 16-byte aligned"; return -1; }
-  int n = 0;
+  const int pitch = dbeta ? 2 * D : D;
   if (norm_bwd_launch(dy, h, gamma, mean, rstd, dx, nullptr, scratch, dbeta ? scratch + D : nullptr, M, D, rms, 0.f, 0, 0, dres,
-                      nullptr, 2 * D, &n, stream))
+                      nullptr, pitch, stream))
     return -1;
-  rtp::launch_k(norm_param_grads_kernel, dim3((D + 63) / 64, dbeta ? 2 : 1), dim3(256), 0, (cudaStream_t)stream, (const float*)scratch, n,
-                2 * D, D, (__nv_bfloat16*)dgamma, (__nv_bfloat16*)dbeta);
+  rtp::launch_k(norm_param_grads_kernel, dim3((D + 63) / 64, dbeta ? 2 : 1), dim3(256), 0, (cudaStream_t)stream, (const float*)scratch,
+                norm_bwd_blocks(M, D), pitch, D, (__nv_bfloat16*)dgamma, (__nv_bfloat16*)dbeta);
   LAUNCH_CHECK("norm_param_grads");
   return 0;
 }

@@ -24,8 +24,8 @@ int rtp_norm_bwd(const void* dy, const void* h, const void* gamma, const float* 
                  unsigned long long seed, unsigned long long offset, const void* dres,
                  const unsigned long long* step_ptr, void* stream);
 // The same without dropout and second output, with the gradients of gamma and beta (null: RMSNorm) as bf16, written, not added to.
-// scratch: rtp_norm_bwd_scratch(D) bytes.  M > 0.
-unsigned long long rtp_norm_bwd_scratch(int D);
+// scratch: rtp_norm_bwd_scratch(M, D, dbeta != null) bytes, a row for each block of the launch.  M > 0.
+unsigned long long rtp_norm_bwd_scratch(int M, int D, int has_beta);
 int rtp_norm_bwd_params(const void* dy, const void* h, const void* gamma, const float* mean, const float* rstd, void* dx,
                         void* dgamma, void* dbeta, float* scratch, int M, int D, int rms, const void* dres, void* stream);
 // Loss per row of logits (pitch ld) and, with write_grad, the gradient of grad_scale * (*scale_ptr) * sum of the losses: into

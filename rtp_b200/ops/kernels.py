@@ -23,7 +23,7 @@ def _L():
         L.rtp_kernels_last_error.restype = C.c_char_p
         L.rtp_norm_fwd.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, i, i, f, i, f, ull, ull, vp, vp]
         L.rtp_norm_bwd.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, f, ull, ull, vp, vp, vp]
-        L.rtp_norm_bwd_scratch.argtypes = [i]
+        L.rtp_norm_bwd_scratch.argtypes = [i, i, i]
         L.rtp_norm_bwd_scratch.restype = ull
         L.rtp_norm_bwd_params.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, vp, vp]
         L.rtp_cross_entropy_scaled.argtypes = [vp, ll, vp, vp, i, i, f, vp, ll, i, vp, ll, vp]
@@ -110,7 +110,7 @@ def norm_bwd_params(dy, h, gamma, mean, rstd, *, rms=False, has_beta=True, dres=
     dx = torch.empty_like(dy)
     grads = torch.empty(2 if has_beta else 1, D, dtype=torch.bfloat16, device=dy.device)
     dg, db = grads[0], grads[1] if has_beta else None
-    scratch = torch.empty(_L().rtp_norm_bwd_scratch(D), dtype=torch.uint8, device=dy.device)
+    scratch = torch.empty(_L().rtp_norm_bwd_scratch(M, D, int(has_beta)), dtype=torch.uint8, device=dy.device)
     _check(_L().rtp_norm_bwd_params(_p(dy), _p(h), _p(gamma), _p(mean), _p(rstd), _p(dx), _p(dg), _p(db), _p(scratch), M, D,
                                     int(rms), _p(dres), _lib.stream_ptr()), "norm_bwd_params")
     _lib.launches += 1

@@ -73,3 +73,22 @@ def test_parameter_gradients_in_place(D, M, rms):
     for t, terms in zip(got[1:], (dy.double() * xh, dy.double())):
         ref = terms.sum(0)
         assert bool(((t.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 2.0 ** -16 * terms.abs().sum(0)).all())
+
+
+@pytest.mark.parametrize("M,D", [(1, 264), (5, 8192), (300, 520), (1024, 2048), (5000, 1032), (4099, 8192)])
+@pytest.mark.parametrize("rms", [False, True])
+def test_parameter_gradients_workspace(M, D, rms):
+    """The workspace is as large as the launch needs: all of it is written, nothing behind it, and it grows with neither the rows
+    beyond two blocks an SM nor a beta that is not there."""
+    from rtp_b200.ops import _lib
+    from rtp_b200.ops import kernels as K
+    L = K._L()
+    n = L.rtp_norm_bwd_scratch(M, D, int(not rms))
+    assert n % (D * 4 * (1 if rms else 2)) == 0 and n <= min(M, 296) * D * 4 * (1 if rms else 2)
+    buf = torch.full((n // 4 + 64,), float("inf"), device="cuda")
+    x, dy = (torch.randn(M, D, device="cuda").to(BF) for _ in range(2))
+    w, out, dx = torch.ones(D, device="cuda", dtype=BF), torch.empty(2, D, device="cuda", dtype=BF), torch.empty_like(dy)
+    mean, rstd = torch.zeros(M, device="cuda"), torch.ones(M, device="cuda")
+    K._check(L.rtp_norm_bwd_params(K._p(dy), K._p(x), K._p(w), None if rms else K._p(mean), K._p(rstd), K._p(dx), K._p(out[0]),
+                                   None if rms else K._p(out[1]), K._p(buf), M, D, int(rms), None, _lib.stream_ptr()), "norm_bwd_params")
+    assert buf[:n // 4].isfinite().all() and bool((buf[n // 4:] == float("inf")).all())
