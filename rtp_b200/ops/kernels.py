@@ -108,8 +108,8 @@ def norm_bwd_params(dy, h, gamma, mean, rstd, *, rms=False, has_beta=True, dres=
     """Returns (dx, dgamma, dbeta), all bf16 (``dbeta`` None without beta): no buffer to zero before and to convert after."""
     M, D = dy.shape
     dx = torch.empty_like(dy)
-    grads = torch.empty(2 if has_beta else 1, D, dtype=torch.bfloat16, device=dy.device)
-    dg, db = grads[0], grads[1] if has_beta else None
+    dg = torch.empty(D, dtype=torch.bfloat16, device=dy.device)          # they become .grad of two parameters: no views of one tensor
+    db = torch.empty_like(dg) if has_beta else None
     scratch = torch.empty(_L().rtp_norm_bwd_scratch(M, D, int(has_beta)), dtype=torch.uint8, device=dy.device)
     _check(_L().rtp_norm_bwd_params(_p(dy), _p(h), _p(gamma), _p(mean), _p(rstd), _p(dx), _p(dg), _p(db), _p(scratch), M, D,
                                     int(rms), _p(dres), _lib.stream_ptr()), "norm_bwd_params")

@@ -92,3 +92,13 @@ def test_parameter_gradients_workspace(M, D, rms):
     K._check(L.rtp_norm_bwd_params(K._p(dy), K._p(x), K._p(w), None if rms else K._p(mean), K._p(rstd), K._p(dx), K._p(out[0]),
                                    None if rms else K._p(out[1]), K._p(buf), M, D, int(rms), None, _lib.stream_ptr()), "norm_bwd_params")
     assert buf[:n // 4].isfinite().all() and bool((buf[n // 4:] == float("inf")).all())
+
+
+def test_parameter_gradients_are_tensors_of_their_own():
+    from rtp_b200.ops import functional as FO
+    x = torch.randn(7, 64, device="cuda").to(BF)
+    w, b = (torch.ones(64, device="cuda", dtype=BF, requires_grad=True) for _ in range(2))
+    FO.layer_norm(x, w, b).sum().backward()
+    assert w.grad.untyped_storage().data_ptr() != b.grad.untyped_storage().data_ptr()
+    w.grad.detach_()
+    b.grad.detach_()
