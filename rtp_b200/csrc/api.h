@@ -116,8 +116,9 @@ typedef struct {
   const void* x; long long ldx;
   void* y; long long ldy;
   int act;
-  const int* fill;                     // optional, device [n_local * world]: rows of each expert's cap that hold tokens; the
-                                       // others get zeros, or (1-rank ring only: a hint) what the product makes of them
+  const int* fill;                     // optional, device [n_local * world]: rows of each expert's cap that hold tokens.  A hint, which
+                                       // rings, activations and unaligned operands ignore: the other rows of x are zero, and those of
+                                       // y get zeros or what the product and the bias make of them
 } RtpExpertFwd;
 int rtp_expert_fwd(const RtpRing* ring, const RtpExpertFwd* op, void* stream);
 typedef struct {
@@ -129,7 +130,7 @@ typedef struct {
   void* grad_home;                     // same layout as home
   const float* dbias_full;             // fp32 [world*n_local, out] per-expert column sums of dy (null: no bias)
   const void* mask; long long ldmask; float mask_scale;   // optional activation backward applied to dx
-  const int* fill;                     // as in RtpExpertFwd; rows of dy beyond it are zero, those of dx become zero
+  const int* fill;                     // as in RtpExpertFwd; the other rows of dy are zero, and those of dx become zero
 } RtpExpertBwd;
 int rtp_expert_bwd(const RtpRing* ring, const RtpExpertBwd* op, void* stream);
 // 1 if the launch makes the experts' bias gradients itself when dbias_full is null (1-rank ring, aligned operands).

@@ -472,7 +472,8 @@ __device__ __forceinline__ void transpose4(uint4 (&v)[4], int lane) {
   }
 }
 // 32 columns of a warp's 32 rows to global memory as bf16: four lanes write 64 consecutive bytes of a row.  One row a thread, 16
-// bytes at a time, the 32 lanes of each store touched 32 lines (with it 288 -> 280 us, backward of 4 x 16 heads of 2048 x 128).  `rows` of the warp's rows are there; dst: row 0.
+// bytes at a time, the 32 lanes of each store touched 32 lines (with it 288 -> 280 us, backward of 4 x 16 heads of 2048 x 128).
+// `rows` of the warp's rows are there; dst: row 0.
 __device__ __forceinline__ void store_rows32(__nv_bfloat16* dst, long long pitch, int rows, const float* o, int lane) {
   uint4 v[4];
 #pragma unroll

@@ -371,10 +371,11 @@ __device__ __forceinline__ void publish_rows(uint64_t* bar, int lane) {
   __syncwarp();
   if (lane == 0) mbar_arrive(bar);
 }
-// Waits of all lanes of a warp; false for all if one ran out.
+// Waits of all lanes of a warp; false for all if one ran out.  Not polled as the issuer's are: forward and backward of 16 heads of
+// 8192 x 8192 x 128 took 1 036 us polled, 1 028 suspended, shorter ones the same either way.
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, unsigned long long* status,
                                           unsigned long long tmo) {
-  const uint32_t good = mbar_spin(bar, parity, abort_flag, status, tmo) ? 1u : 0u;
+  const uint32_t good = mbar_wait(bar, parity, abort_flag, status, tmo) ? 1u : 0u;
   return __all_sync(0xffffffffu, good);
 }
 // D[128 x 128] = A B^T of two [128 x HD] K-major tiles
@@ -1232,7 +1233,7 @@ uint32_t thresh_of(float pdrop) {
 }
 
 // 3-D map {width columns, dim1, dim2} over a [batch, seq, width] view; the dimension with the smaller stride comes first.
-int make_map3(CUtensorMap* m, int* seq1, const RtpFlashRef& r, int B, int S, const char* what, unsigned rows = 128u) {
+int make_map3(CUtensorMap* m, int* seq1, const RtpFlashRef& r, int B, int S, const char* what) {
   EncodeTiledFn enc = get_encode_tiled();
   if (!enc) return ffail("cuTensorMapEncodeTiled entry point not found");
   if ((reinterpret_cast<uintptr_t>(r.ptr) & 15) != 0) return ffail(std::string(what) + ": base is not 16-byte aligned");
@@ -1243,7 +1244,7 @@ int make_map3(CUtensorMap* m, int* seq1, const RtpFlashRef& r, int B, int S, con
   cuuint64_t dims[3] = {(cuuint64_t)r.width, (cuuint64_t)(s_first ? S : B), (cuuint64_t)(s_first ? B : S)};
   cuuint64_t strides[2] = {(cuuint64_t)(s_first ? r.ss : r.sb) * 2, (cuuint64_t)(s_first ? r.sb : r.ss) * 2};
   if (B == 1) strides[1] = strides[0] * (cuuint64_t)S;   // a single batch: any legal pitch
-  cuuint32_t box[3] = {64u, s_first ? rows : 1u, s_first ? 1u : rows};
+  cuuint32_t box[3] = {64u, s_first ? (cuuint32_t)kBlk : 1u, s_first ? 1u : (cuuint32_t)kBlk};
   cuuint32_t estr[3] = {1u, 1u, 1u};
   CUresult rc = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, r.ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);

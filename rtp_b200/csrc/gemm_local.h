@@ -28,9 +28,10 @@ struct LocalGemm {
   // s * part_stride, for local_reduce to add up; d has a pitch of N
   int part;
   long long part_stride;
-  // Rows that are in use, known on the device only (expert capacities).  m_fill: output rows from there on get zeros, whatever A
-  // holds; k_fill: elements of the contraction, of which those from there on contribute nothing (A or B is zero there) and up
-  // to the next multiple of 64 are finite.  A launch with one of them has no c, mask, activation or dropout.
+  // Rows that are in use, known on the device only (expert capacities); a hint.  m_fill: output rows from there on may be anything:
+  // a tile of rows behind it gets zeros, the rest of the tile that it lies in what the product and the bias make of A.  k_fill: elements
+  // of the contraction, of which those from there on contribute nothing (A or B is zero there, A if there is a bsum) and up to the next
+  // multiple of 64 are finite.  A launch with one of them has no c, mask, activation or dropout.
   const int* m_fill;
   const int* k_fill;
 };
