@@ -12,6 +12,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_DIR = os.path.join(os.path.dirname(HERE), "lib")
 LIB_PATH = os.path.join(LIB_DIR, "librtp_b200.so")
 SOURCES = ["gemm.cu", "gemm_local.cu", "kernels.cu", "attn_tc.cu", "flash_attn.cu", "ring_shift.cu", "gate_rope.cu", "im2col.cu", "noalloc.cu"]
+# sources with many variants of a kernel, compiled in parts side by side: the macro that names a part, their number
+PARTS = {"flash_attn.cu": ("RTP_FLASH_PART", 4)}
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "--use_fast_math", "-Xcompiler", "-fPIC", "-Xcompiler", "-O3",
@@ -46,13 +48,15 @@ def build(force=False, verbose=False):
     objs = []
     procs = []
     for src in sources():
-        obj = os.path.join(LIB_DIR, os.path.basename(src) + ".o")
-        cmd = [nvcc, *NVCC_FLAGS, "-c", src, "-o", obj]
-        if verbose:
-            cmd.insert(1, "-Xptxas")
-            cmd.insert(2, "-v")
-        procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
-        objs.append(obj)
+        name = os.path.basename(src)
+        macro, parts = PARTS.get(name, (None, 1))
+        for part in range(parts):
+            obj = os.path.join(LIB_DIR, f"{name}.{part}.o" if macro else name + ".o")
+            cmd = [nvcc, *NVCC_FLAGS, *([f"-D{macro}={part}", "-diag-suppress", "177"] if macro else []), "-c", src, "-o", obj]
+            if verbose:
+                cmd[1:1] = ["-Xptxas", "-v"]
+            procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
+            objs.append(obj)
     for src, p in procs:
         out, _ = p.communicate()
         if verbose or p.returncode:

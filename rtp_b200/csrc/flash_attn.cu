@@ -1204,6 +1204,64 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_kernel(const __grid_con
   teardown_cta(tmem, warp);
 }
 
+// =====================================================================================================  parts
+// Twelve variants for each direction and head_dim take 17 s of compilation; the build makes an object of each of the four side by side
+// (RTP_FLASH_PART 0 to 3; undefined: all in one).  Part 0 has the entry points.
+#ifdef RTP_FLASH_PART
+#define RTP_FLASH_HAS(k) (RTP_FLASH_PART == k)
+#else
+#define RTP_FLASH_HAS(k) 1
+#endif
+
+constexpr int smem_fwd(int hd) { return 1024 + (hd / 64) * kSub * 6 + 256 + 2 * 256 * 4; }
+// backward: seven tiles, control block, statistics of two blocks of queries
+constexpr int smem_bwd(int hd) { return kBwdSlack + (hd / 64) * kSub * 7 + 256 + 2 * 2 * kBlk * 4; }
+static_assert(sizeof(Ctl) <= 256, "control block");
+static_assert(smem_fwd(128) <= 232448 && smem_bwd(128) <= 232448, "shared memory budget");
+
+template <auto Kern>
+cudaError_t launch_flash(const FlashParams& P, int grid, int smem, cudaStream_t stream) {
+  const cudaError_t e = ensure_smem<Kern>(smem);
+  return e != cudaSuccess ? e : launch_k(Kern, dim3(grid), dim3(kThreads), smem, stream, P);
+}
+// mask: none, key padding, additive
+#define RTP_FLASH(KERNEL, SMEM, HD, MSK, DRP)                                                 \
+  (more ? launch_flash<KERNEL<HD, MSK, DRP, true>>(P, grid, SMEM(HD), (cudaStream_t)stream)   \
+        : launch_flash<KERNEL<HD, MSK, DRP, false>>(P, grid, SMEM(HD), (cudaStream_t)stream))
+#define RTP_FLASH_PART_FN(NAME, KERNEL, SMEM, HD)                                                                          \
+  extern "C" int NAME(const void* params, int mask, int drp, int more, int grid, void* stream) {                           \
+    const FlashParams& P = *reinterpret_cast<const FlashParams*>(params);                                                  \
+    return (int)(mask == 2   ? (drp ? RTP_FLASH(KERNEL, SMEM, HD, 2, true) : RTP_FLASH(KERNEL, SMEM, HD, 2, false))        \
+                 : mask == 1 ? (drp ? RTP_FLASH(KERNEL, SMEM, HD, 1, true) : RTP_FLASH(KERNEL, SMEM, HD, 1, false))        \
+                             : (drp ? RTP_FLASH(KERNEL, SMEM, HD, 0, true) : RTP_FLASH(KERNEL, SMEM, HD, 0, false)));      \
+  }
+
+
+}  // namespace
+
+// Launches a variant with the FlashParams at `params`; returns a cudaError_t.
+typedef int FlashPart(const void* params, int mask, int drp, int more, int grid, void* stream);
+extern "C" {
+FlashPart rtp_flash_part_fwd64;
+FlashPart rtp_flash_part_fwd128;
+FlashPart rtp_flash_part_bwd64;
+FlashPart rtp_flash_part_bwd128;
+}
+#if RTP_FLASH_HAS(0)
+RTP_FLASH_PART_FN(rtp_flash_part_fwd64, flash_fwd_kernel, smem_fwd, 64)
+#endif
+#if RTP_FLASH_HAS(1)
+RTP_FLASH_PART_FN(rtp_flash_part_fwd128, flash_fwd_kernel, smem_fwd, 128)
+#endif
+#if RTP_FLASH_HAS(2)
+RTP_FLASH_PART_FN(rtp_flash_part_bwd64, flash_bwd_kernel, smem_bwd, 64)
+#endif
+#if RTP_FLASH_HAS(3)
+RTP_FLASH_PART_FN(rtp_flash_part_bwd128, flash_bwd_kernel, smem_bwd, 128)
+#endif
+
+#if RTP_FLASH_HAS(0)
+namespace {
 // =====================================================================================================  host
 thread_local std::string g_ferr;
 long long* g_flash_trace = nullptr;
@@ -1293,20 +1351,8 @@ int fill_common(const RtpFlashArgs* a, FlashParams& P) {
   P.q = dref(a->q); P.k = dref(a->k); P.v = dref(a->v); P.o = dref(a->o);
   return 0;
 }
-constexpr int smem_fwd(int hd) { return 1024 + (hd / 64) * kSub * 6 + 256 + 2 * 256 * 4; }
-// backward: seven tiles, control block, statistics of two blocks of queries
-constexpr int smem_bwd(int hd) { return kBwdSlack + (hd / 64) * kSub * 7 + 256 + 2 * 2 * kBlk * 4; }
-static_assert(sizeof(Ctl) <= 256, "control block");
-static_assert(smem_fwd(128) <= 232448 && smem_bwd(128) <= 232448, "shared memory budget");
-
-template <auto Kern>
-int launch_flash(const FlashParams& P, int grid, int smem, cudaStream_t stream, const char* what) {
-  cudaError_t e = ensure_smem<Kern>(smem);
-  if (e != cudaSuccess) return ffail(std::string(what) + ": cudaFuncSetAttribute: " + cudaGetErrorString(e));
-  e = launch_k(Kern, dim3(grid), dim3(kThreads), smem, stream, P);
-  if (e != cudaSuccess) return ffail(std::string(what) + ": " + cudaGetErrorString(e));
-  return 0;
-}
+int mask_kind(const RtpFlashArgs* a) { return a->mask ? 2 : a->kpm ? 1 : 0; }
+int launched(int e, const char* what) { return e == (int)cudaSuccess ? 0 : ffail(std::string(what) + ": " + cudaGetErrorString((cudaError_t)e)); }
 
 }  // namespace
 
@@ -1327,17 +1373,8 @@ int rtp_flash_fwd(const RtpFlashArgs* a, void* stream) {
   P.group = head_group(4ll * a->Sk * a->head_dim, BH);
   const int grid = (P.split ? tiles : (tiles + 1) / 2) * BH;
   const bool more = grid > device_sms();         // 48 heads of 999 x 128: 31 -> 28 us
-  cudaStream_t s = (cudaStream_t)stream;
-  const bool drp = P.m.thresh != 0;
-#define RTP_FWD(HD, MSK, DRP)                                                                         \
-  (more ? launch_flash<flash_fwd_kernel<HD, MSK, DRP, true>>(P, grid, smem_fwd(HD), s, "flash_fwd")   \
-        : launch_flash<flash_fwd_kernel<HD, MSK, DRP, false>>(P, grid, smem_fwd(HD), s, "flash_fwd"))
-#define RTP_FWD_HD(HD) (a->mask ? (drp ? RTP_FWD(HD, 2, true) : RTP_FWD(HD, 2, false))  \
-                        : a->kpm ? (drp ? RTP_FWD(HD, 1, true) : RTP_FWD(HD, 1, false)) \
-                                 : (drp ? RTP_FWD(HD, 0, true) : RTP_FWD(HD, 0, false)))
-  return a->head_dim == 64 ? RTP_FWD_HD(64) : RTP_FWD_HD(128);
-#undef RTP_FWD_HD
-#undef RTP_FWD
+  return launched((a->head_dim == 64 ? rtp_flash_part_fwd64 : rtp_flash_part_fwd128)(&P, mask_kind(a), P.m.thresh != 0, more, grid, stream),
+                  "flash_fwd");
 }
 
 int rtp_flash_bwd(const RtpFlashArgs* a, void* stream) {
@@ -1352,21 +1389,14 @@ int rtp_flash_bwd(const RtpFlashArgs* a, void* stream) {
   const int grid = ((a->Sq + kBlk - 1) / kBlk + (a->Sk + kBlk - 1) / kBlk) * a->B * a->H;
   const bool more = grid > 2 * device_sms();   // one or two rounds are over sooner without (16 heads of 1024 x 1024: 55 us, 60)
   cudaStream_t s = (cudaStream_t)stream;
-  const bool drp = P.m.thresh != 0;
   P.group = head_group(4ll * (a->Sq + a->Sk) * a->head_dim, a->B * a->H);
   const long long rows = (long long)a->B * a->Sq * a->H, per = 256 / (a->head_dim / 8);
   const cudaError_t e = launch_k(a->head_dim == 64 ? flash_delta_kernel<64> : flash_delta_kernel<128>,
                                  dim3((unsigned)((rows + per - 1) / per)), dim3(256), 0, s, P.o, P.dout, P.delta, a->Sq, a->H, rows);
   if (e != cudaSuccess) return ffail(std::string("flash_delta: ") + cudaGetErrorString(e));
-#define RTP_BWD(HD, MSK, DRP)                                                                         \
-  (more ? launch_flash<flash_bwd_kernel<HD, MSK, DRP, true>>(P, grid, smem_bwd(HD), s, "flash_bwd")   \
-        : launch_flash<flash_bwd_kernel<HD, MSK, DRP, false>>(P, grid, smem_bwd(HD), s, "flash_bwd"))
-#define RTP_BWD_HD(HD) (a->mask ? (drp ? RTP_BWD(HD, 2, true) : RTP_BWD(HD, 2, false))  \
-                        : a->kpm ? (drp ? RTP_BWD(HD, 1, true) : RTP_BWD(HD, 1, false)) \
-                                 : (drp ? RTP_BWD(HD, 0, true) : RTP_BWD(HD, 0, false)))
-  return a->head_dim == 64 ? RTP_BWD_HD(64) : RTP_BWD_HD(128);
-#undef RTP_BWD_HD
-#undef RTP_BWD
+  return launched((a->head_dim == 64 ? rtp_flash_part_bwd64 : rtp_flash_part_bwd128)(&P, mask_kind(a), P.m.thresh != 0, more, grid, stream),
+                  "flash_bwd");
 }
 
 }  // extern "C"
+#endif  // part 0

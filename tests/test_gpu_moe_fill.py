@@ -114,3 +114,41 @@ def test_rows_are_counted_for_who_reads_them(kind, counted, monkeypatch):
     with torch.no_grad():
         layer_of(kind, 64)()
     assert len(seen) == 1 and (seen[0] is not None) == counted
+
+
+@pytest.mark.parametrize("E,cap,D,H,counts", [(4, 320, 72, 200, (1, 63, 64, 65)), (4, 640, 136, 264, (127, 0, 129, 640))])
+def test_against_float64(E, cap, D, H, counts):
+    """Four tensors on the way to the output are rounded to bf16 (2^-9 of the value each, at random), eight on the way to a
+    gradient: norms of the errors within 2^-7 and 2^-6 of those of the results, expert by expert."""
+    from rtp_b200.models.moe_lm import Expert
+    from rtp_b200.module.moe import WeightMOELayer, combine_by_index, dispatch_by_index
+    from rtp_b200.ops.moe import rows_in_use
+    from rtp_b200.parallel.engine import fused_experts
+    torch.manual_seed(cap)
+    layer = WeightMOELayer(nn.Identity(), nn.ModuleList([Expert(D, H) for _ in range(E)]), device="cuda", dtype=BF)
+    idx = torch.cat([torch.full((n,), e) for e, n in enumerate(counts)]).cuda()
+    loc = torch.cat([torch.arange(n) for n in counts]).cuda()
+    S = idx.numel()
+    pair = torch.stack([idx, torch.zeros_like(idx)], 1), torch.stack([loc, torch.zeros_like(loc)], 1)
+    valid = torch.tensor([True, False]).expand(S, 2).cuda()
+    gate = torch.rand(S, 2, device="cuda")
+    x, dy = torch.randn(S, D, device="cuda").to(BF).requires_grad_(), torch.randn(S, D, device="cuda").to(BF)
+    params = list(layer.experts.parameters())
+    d = dispatch_by_index(x, *pair, valid, E, cap)
+    assert rows_in_use(d).tolist() == list(counts)
+    y = combine_by_index(fused_experts(layer, d), *pair, gate, valid)
+    got = [y.detach(), *torch.autograd.grad(y, [x, *params], dy)]
+    xs, ps = x.detach().double().requires_grad_(), [p.detach().double().requires_grad_() for p in params]
+    out = torch.zeros(S, D, dtype=torch.float64, device="cuda")
+    for e in range(E):
+        w1, b1, w2, b2 = ps[4 * e:4 * e + 4]
+        rows = (idx == e).nonzero()[:, 0]
+        h = torch.nn.functional.gelu(xs[rows] @ w1.t() + b1) @ w2.t() + b2
+        out = out.index_add(0, rows, h * gate[rows, :1].double())
+    ref = [out.detach(), *torch.autograd.grad(out, [xs, *ps], dy.double())]
+    for i, (a, b) in enumerate(zip(got, ref)):
+        assert ((a.double() - b).norm() <= (2.0 ** -6 if i else 2.0 ** -7) * b.norm()).item(), (i, ((a.double() - b).norm() / b.norm()).item())
+        if i < 2:
+            for e in range(E):
+                u, v = a[idx == e].double(), b[idx == e]
+                assert ((u - v).norm() <= 2.0 ** -6 * v.norm()).item(), (i, e)
