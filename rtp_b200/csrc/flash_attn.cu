@@ -817,22 +817,27 @@ __global__ void __launch_bounds__(256) flash_delta_kernel(DRef o, DRef g, float*
 enum { B_FULL = 0, B_EMPTY = 7, B_STAT = 14 /* 2 */, B_SFULL = 16 /* 2 */, B_PFULL = 18, B_DPFULL = 19, B_DSFULL = 20, B_ACC = 21,
        B_ACCREAD = 22, B_WFULL = 23, B_TAKEN = 24, B_DRAIN = 25 };
 
-// What blockIdx.x stands for: the key block kb, or (kb < 0) the query block qb, of a (batch, head).
+// What blockIdx.x stands for: the key block kb, or (kb < 0) the query block qb, of head h of batch entry b.
 struct BwdWork {
-  int kb, qb, bh;
+  int kb, qb, bh, b, h;
 };
 __device__ __forceinline__ BwdWork bwd_work(const FlashParams& p, int blk) {
-  const int nq = (p.m.Sq + kBlk - 1) / kBlk, nk = (p.m.Sk + kBlk - 1) / kBlk, BH = p.B * p.H, both = min(nq, nk);
-  // a group of heads: levels of a key block and a query block of each, the longest first (causal: first keys, last queries), then
+  const int nq = (p.m.Sq + kBlk - 1) / kBlk, nk = (p.m.Sk + kBlk - 1) / kBlk, BH = p.B * p.H, both = min(nq, nk), span = p.group * (nq + nk);
+  // a group of heads: a key block of each, a query block of each and so on, the longest first (causal: first keys, last queries), then
   // what one kind has more
-  const int grp = blk / (p.group * (nq + nk)) * p.group, heads = min(p.group, BH - grp);
-  const int r = blk - grp * (nq + nk), level = r / (2 * heads);
-  BwdWork w = {-1, -1, grp + r % heads};
-  if (level < both) { if (r % (2 * heads) < heads) w.kb = level; else w.qb = nq - 1 - level; }
-  else {
-    const int i = (r - 2 * heads * both) / heads;
-    if (nk > nq) w.kb = both + i; else w.qb = nq - 1 - both - i;
+  int grp = 0;
+  if (blk >= span) {
+    const int g = blk / span;
+    grp = g * p.group;
+    blk -= g * span;
   }
+  const int heads = min(p.group, BH - grp), row = blk / heads;
+  BwdWork w = {-1, -1, grp + blk - row * heads, 0, 0};
+  if (row < 2 * both) { if (row & 1) w.qb = nq - 1 - (row >> 1); else w.kb = row >> 1; }
+  else if (nk > nq) w.kb = row - both;
+  else w.qb = nq - 1 + both - row;
+  w.b = w.bh / p.H;
+  w.h = w.bh - w.b * p.H;
   return w;
 }
 
@@ -855,6 +860,8 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_kernel(const __grid_con
   // counts by barrier index: copies and commits 1; statistics 32 (lanes); P and dS, accumulators read 8 (one per row warp); next work
   // 1 and 10 (producer, issuer, eight row warps)
   const int counts[26] = {1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 32, 32, 1, 1, 8, 1, 8, 1, 8, 1, 10, 1};
+  const BwdWork first = bwd_work(p, (int)blockIdx.x);       // before the wait for the previous kernel, as in forward
+  asm volatile("" ::"r"(first.b), "r"(first.h), "r"(first.kb), "r"(first.qb));
   const uint32_t tmem = setup_cta(ctl, counts, 26, warp, lane);
   volatile uint32_t* abort_flag = &ctl->abort_flag;
   unsigned long long* status = p.status;
@@ -884,8 +891,8 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_kernel(const __grid_con
       return true;
     };
     for (int blk = (int)blockIdx.x; blk >= 0 && ok; blk = following(n++, true)) {
-      const BwdWork w = bwd_work(p, blk);
-      const int b = w.bh / p.H, h = w.bh % p.H;
+      const BwdWork w = n == 0 ? first : bwd_work(p, blk);
+      const int b = w.b, h = w.h;
       const int cq = head_col(p.q, h), ck = head_col(p.k, h), cv = head_col(p.v, h), cg = head_col(p.dout, h);
       if (w.kb >= 0) {
         const long long base = (long long)w.bh * M.Sq;
@@ -946,7 +953,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_kernel(const __grid_con
         return true;
       };
       for (int blk = (int)blockIdx.x; blk >= 0 && ok; blk = following(n++, false)) {
-        const BwdWork w = bwd_work(p, blk);
+        const BwdWork w = n == 0 ? first : bwd_work(p, blk);
         mbar_arrive(&bar[B_TAKEN]);
         const uint32_t read = (n & 1u) ^ 1u;            // the accumulators of the work before have been read out
         if (w.kb >= 0) {
@@ -1004,9 +1011,9 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_kernel(const __grid_con
     auto wait = [&](int i, uint32_t ph) { return warp_wait(&bar[i], ph, abort_flag, status, tmo); };
     long long* tr = (p.trace && blockIdx.x == 0 && lane == 0 && (warp & 3) == 0) ? p.trace + (warp >> 2) * 128 : nullptr;
     for (int blk = (int)blockIdx.x; blk >= 0 && ok; blk = following(n++, true)) {
-      const BwdWork w = bwd_work(p, blk);
+      const BwdWork w = n == 0 ? first : bwd_work(p, blk);
       if (lane == 0) mbar_arrive(&bar[B_TAKEN]);
-      const int bh = w.bh, b = bh / p.H, h = bh % p.H;
+      const int bh = w.bh, b = w.b, h = w.h;
       if (w.kb >= 0) {
         const int k0 = w.kb * kBlk, i0 = M.causal ? w.kb : 0, nit = nqb - i0;
         const uint32_t aS = tS + lane_off + (uint32_t)(wg * 64);
