@@ -15,8 +15,8 @@
 // MN-major (transposed) for dK.  P takes the place of operands that are no longer needed, and the results take the place of S and dP
 // in TMEM: 48 / 112 KB and 128 / 256 columns, so that two CTAs and more share an SM (one chain a head, with 64 / 144 KB and 256 /
 // 512 columns, had one in backward: 1024 heads of 32 x 64 took two rounds).
-// us, that form -> this: 1024 heads of 32 with dropout, forward 10.2 -> 7.9, backward 21.0 -> 11.0; 32 heads of 32 5.8 -> 5.4 and
-// 9.7 -> 8.2; 1024 heads of 64 17.8 -> 15.7 and 47.4 -> 26.3.
+// us, that form -> this: 1024 heads of 32 with dropout, forward 10.4 -> 8.1, backward 20.0 -> 10.9; 32 heads of 32 5.8 -> 5.2 and
+// 10.9 -> 7.9; 1024 heads of 64 17.8 -> 12.8 and 47.4 -> 25.2.
 //
 // Operands are fetched with plain 16-byte loads into 128-byte-swizzled tiles (the strided token order s*B + b of the
 // packed projection needs no tensor map); "fence.proxy.async" publishes them to the tensor core.

@@ -16,12 +16,14 @@
 // comes from a kernel of its own, dQ of a block of queries and dK / dV of a block of keys are pieces of work of one launch.
 //
 // What it gives (us, before: one row tile a CTA with two threads a row, P and dS through shared memory, dQ and dK / dV in
-// launches of their own; now), forward and backward: 1 x 16 heads of 8192 x 8192 x 128 causal 338 -> 242 and 1 134 -> 805,
-// 4 x 16 of 2048 causal 126 -> 90 and 400 -> 285, 8 x 20 of 512 x 2048 x 64 121 -> 90 and 433 -> 250, 4 x 8 of 256 x 256 x 64
-// 6.7 -> 6.4 and 20 -> 15, 4 x 8 of 64 x 64 x 64 5.1 -> 5.2.  One that is a little slower: a forward of one key block on more than
-// half of the SMs (8 x 16 of 64 x 64 x 64 5.5 -> 5.9), which cannot start under the one before for want of registers.  Per 128 x 128 block at head_dim 128 (SM clocks): forward 1 700 (tensor work 1 024, exponentials
-// 1 024), dK / dV 3 100 (tensor work 2 048), dQ 2 080 (1 536).  The forward is bound by the exponentials and the hand-overs
-// between row threads and issuer, dK / dV by the chain P -> dV -> S of the next block (TMEM has no room for a second S).
+// launches of their own; now), forward and backward: 1 x 16 heads of 8192 x 8192 x 128 causal 337 -> 237 and 1 131 -> 788,
+// 4 x 16 of 2048 causal 123 -> 90 and 401 -> 280, 8 x 20 of 512 x 2048 x 64 118 -> 88 and 433 -> 251, 4 x 8 of 256 x 256 x 64
+// 6.4 -> 6.2 and 20 -> 14, 4 x 8 of 64 x 64 x 64 4.9 -> 4.9 and 10.6 -> 9.3.  Heads of one key block that fill more than half of the
+// SMs are slower: 8 x 16 of 64 x 64 x 64 5.3 -> 5.6 and 11.8 -> 16.3 (two pieces of work a head are two rounds of CTAs, which
+// registers keep from overlapping; two pieces a CTA took 17.7).  Per 128 x 128 block at head_dim 128 (SM clocks): forward 1 700 (tensor
+// work 1 024, exponentials 1 024), dK / dV 3 100 (tensor work 2 048), dQ 2 080 (1 536).  The forward is bound by the exponentials and
+// the hand-overs between row threads and issuer, dK / dV by the chain P -> dV -> S of the next block (TMEM has no room for a
+// second S).
 //
 // Each kernel is compiled in variants (no mask, key padding only, additive mask; dropout yes or no; more work than SMs or not):
 // the mask and Philox code unrolled over a row's registers is several times larger than the plain softmax and, when merely
