@@ -16,16 +16,16 @@
 // comes from a kernel of its own, dQ of a block of queries and dK / dV of a block of keys are pieces of work of one launch.
 //
 // What it gives (us, before: one row tile a CTA with two threads a row, P and dS through shared memory, dQ and dK / dV in
-// launches of their own; now), forward and backward: 1 x 16 heads of 8192 x 8192 x 128 causal 337 -> 237 and 1 131 -> 788,
-// 4 x 16 of 2048 causal 123 -> 90 and 401 -> 280, 8 x 20 of 512 x 2048 x 64 118 -> 88 and 433 -> 251, 4 x 8 of 256 x 256 x 64
-// 6.4 -> 6.2 and 20 -> 14, 4 x 8 of 64 x 64 x 64 4.9 -> 4.9 and 10.6 -> 9.3.  Heads of one key block that fill more than half of the
-// SMs are slower: 8 x 16 of 64 x 64 x 64 5.3 -> 5.6 and 11.8 -> 16.3 (two pieces of work a head are two rounds of CTAs, which
-// registers keep from overlapping; two pieces a CTA took 17.7).  Per 128 x 128 block at head_dim 128 (SM clocks): forward 1 700 (tensor
-// work 1 024, exponentials 1 024), dK / dV 3 100 (tensor work 2 048), dQ 2 080 (1 536).  The forward is bound by the exponentials and
-// the hand-overs between row threads and issuer, dK / dV by the chain P -> dV -> S of the next block (TMEM has no room for a
-// second S).
+// launches of their own; now), forward and backward: 1 x 16 heads of 8192 x 8192 x 128 causal 337 -> 237 and 1 131 -> 795,
+// 4 x 16 of 2048 causal 123 -> 91 and 401 -> 280, 8 x 20 of 512 x 2048 x 64 118 -> 88 and 433 -> 244, 4 x 8 of 256 x 256 x 64
+// 6.4 -> 6.2 and 20 -> 14, 4 x 8 of 64 x 64 x 64 4.9 -> 4.9 and 10.7 -> 9.4.  Heads of one key block that fill more than half of
+// the SMs are a little slower: 8 x 16 of 64 x 64 x 64 5.3 -> 5.6 and 11.8 -> 12.8.  Per 128 x 128 block at head_dim 128 (SM
+// clocks): forward 1 700 (tensor work 1 024, exponentials 1 024), dK / dV 3 100 (tensor work 2 048), dQ 2 080 (1 536).  The
+// forward is bound by the exponentials and the hand-overs between row threads and issuer, dK / dV by the chain P -> dV -> S of
+// the next block (TMEM has no room for a second S).
 //
-// Each kernel is compiled in variants (no mask, key padding only, additive mask; dropout yes or no; more work than SMs or not):
+// Each kernel is compiled in variants (no mask, key padding only, additive mask; dropout yes or no; more work than SMs or not; backward:
+// one head a CTA):
 // the mask and Philox code unrolled over a row's registers is several times larger than the plain softmax and, when merely
 // branched over, slowed the row threads down through instruction fetch alone.
 // Every mbarrier wait is bounded; on expiry the CTA records a status code, drains its copies and UMMAs, frees its TMEM
@@ -810,6 +810,8 @@ __global__ void __launch_bounds__(256) flash_delta_kernel(DRef o, DRef g, float*
 // V, S double-buffered:
 //   S = Q K^T, dP = dO V^T  ->  dS = P (dP - delta)  ->  dQ += dS K
 //
+// ONE: heads of one key block and one query block, a CTA a head: dS^T goes to shared memory too, where dQ reads it transposed.
+//
 // Shared memory is seven tiles, each with a "full" and an "empty" barrier of its own, whatever it holds: what follows is copied
 // into a tile as soon as its last product is done, also across pieces of work.
 //   dK / dV:  0 K   1 V   2, 3 Q   4, 5 dO            dQ:  0 Q   1 dO   2, 3, 4 K   5, 6 V
@@ -845,7 +847,7 @@ __device__ __forceinline__ BwdWork bwd_work(const FlashParams& p, int blk) {
 
 constexpr int kBwdSlack = 768;          // all that a CTA's shared memory leaves for the alignment of the tiles (its base has it)
 
-template <int HD, int MSK, bool DRP, bool MORE>
+template <int HD, int MSK, bool DRP, bool MORE, bool ONE = false>
 __global__ void __launch_bounds__(kThreads, 1) flash_bwd_kernel(const __grid_constant__ FlashParams p) {
   constexpr int TILE = (HD / 64) * kSub;
   extern __shared__ __align__(1024) uint8_t smem_tiles[];
@@ -932,6 +934,7 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_kernel(const __grid_con
     // ---------------------------------------------------------------------------------- UMMA issuer
     if (elect_one()) {
       const uint32_t id_s = make_idesc_bf16(128, 128, 0, 0), id_t = make_idesc_bf16(128, HD, 0, 1);
+      [[maybe_unused]] const uint32_t id_q = make_idesc_bf16(128, HD, 1, 1);
       const uint32_t a0 = smem_u32(sm);
       bool ok = true, issued = false;
       uint32_t uses = 0, np = 0, nds = 0, n = 0;        // per tile: parity of its next use; P, dS and pieces of work so far
@@ -973,6 +976,12 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_kernel(const __grid_con
             if (!wait(B_DSFULL, nds++ & 1u)) { ok = false; break; }
             tc_fence_after();
             umma_rows(tAcc + HD, tP, at(2 + st), id_t, it > 0);
+            if constexpr (ONE) {                         // dQ from dS^T in shared memory, into the columns of S
+#pragma unroll
+              for (int kk = 0; kk < 8; ++kk)
+                umma_bf16(tS, make_smem_desc(at(5) + kk * 2048, kSub, 1024), make_smem_desc(at(0) + kk * 2048, kSub, 1024), id_q,
+                          kk > 0 ? 1u : 0u);
+            }
             done_with(2 + st);
             if (more) ok = product(tP, 1, 4 + ot, B_DPFULL, end, false);
             else umma_commit(&bar[B_ACC]);
@@ -1119,7 +1128,16 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_kernel(const __grid_con
               x[i] = u.x; x[i + 1] = u.y; x[i + 2] = v.x; x[i + 3] = v.y;
             }
             store_bf16x32(aP + (uint32_t)(c * 16), x + 32 * c);
+            if constexpr (ONE) {                         // the same row in shared memory: A of dQ, read MN-major
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                const float* e = x + 32 * c + 8 * k;
+                *reinterpret_cast<uint4*>(sm + 5 * TILE + wg * kSub + rt * 128 + (((4 * c + k) ^ (rt & 7)) << 4)) =
+                    make_uint4(pack_bf16(e[0], e[1]), pack_bf16(e[2], e[3]), pack_bf16(e[4], e[5]), pack_bf16(e[6], e[7]));
+              }
+            }
           }
+          if constexpr (ONE) fence_proxy_async_smem();
           publish_rows(&bar[B_DSFULL], lane);
           if (tr && it < 16) tr[it * 8 + 4] = clock64();
         }
@@ -1187,16 +1205,18 @@ __global__ void __launch_bounds__(kThreads, 1) flash_bwd_kernel(const __grid_con
       if (!ok) break;
       tc_fence_after();
       const int r0 = (w.kb >= 0 ? w.kb : w.qb) * kBlk + (warp & 3) * 32;      // the warp's first row
-      const int left = (w.kb >= 0 ? M.Sk : M.Sq) - r0;
-      const int nacc = w.kb >= 0 ? 2 : 1;
+      const int nacc = ONE ? 3 : w.kb >= 0 ? 2 : 1;
       for (int a = 0; a < nacc; ++a) {
-        const DRef& out = w.kb < 0 ? p.dq : a ? p.dk : p.dv;
+        const bool is_q = w.kb < 0 || (ONE && a == 2);
+        const DRef& out = is_q ? p.dq : a ? p.dk : p.dv;
+        const int left = (is_q ? M.Sq : M.Sk) - r0;
         __nv_bfloat16* dst = row_ptr(out, b, r0, h) + wg * (HD / 2);
-        const float mul = w.kb >= 0 && a == 0 ? 1.f : M.sm_scale;
+        const float mul = !is_q && a == 0 ? 1.f : M.sm_scale;
+        const uint32_t acc = ONE && a == 2 ? tS : tAcc + (uint32_t)(a * HD);
 #pragma unroll
         for (int c = 0; c < HD / 64; ++c) {
           float o[32];
-          tmem_ld32f(tAcc + lane_off + (uint32_t)(a * HD + wg * (HD / 2) + c * 32), o);
+          tmem_ld32f(acc + lane_off + (uint32_t)(wg * (HD / 2) + c * 32), o);
           tmem_ld_wait();
           if (a + 1 == nacc && c + 1 == HD / 64) {
             tc_fence_before();
@@ -1233,23 +1253,26 @@ cudaError_t launch_flash(const FlashParams& P, int grid, int smem, cudaStream_t 
   const cudaError_t e = ensure_smem<Kern>(smem);
   return e != cudaSuccess ? e : launch_k(Kern, dim3(grid), dim3(kThreads), smem, stream, P);
 }
-// mask: none, key padding, additive
-#define RTP_FLASH(KERNEL, SMEM, HD, MSK, DRP)                                                 \
-  (more ? launch_flash<KERNEL<HD, MSK, DRP, true>>(P, grid, SMEM(HD), (cudaStream_t)stream)   \
-        : launch_flash<KERNEL<HD, MSK, DRP, false>>(P, grid, SMEM(HD), (cudaStream_t)stream))
-#define RTP_FLASH_PART_FN(NAME, KERNEL, SMEM, HD)                                                                          \
-  extern "C" int NAME(const void* params, int mask, int drp, int more, int grid, void* stream) {                           \
-    const FlashParams& P = *reinterpret_cast<const FlashParams*>(params);                                                  \
-    return (int)(mask == 2   ? (drp ? RTP_FLASH(KERNEL, SMEM, HD, 2, true) : RTP_FLASH(KERNEL, SMEM, HD, 2, false))        \
-                 : mask == 1 ? (drp ? RTP_FLASH(KERNEL, SMEM, HD, 1, true) : RTP_FLASH(KERNEL, SMEM, HD, 1, false))        \
-                             : (drp ? RTP_FLASH(KERNEL, SMEM, HD, 0, true) : RTP_FLASH(KERNEL, SMEM, HD, 0, false)));      \
+// kind: 0 one piece of work a CTA, 1 persistent, 2 (backward) one head a CTA; mask: none, key padding, additive
+#define RTP_FLASH_FWD(HD, MSK, DRP)                                                                                     \
+  (kind == 1 ? launch_flash<flash_fwd_kernel<HD, MSK, DRP, true>>(P, grid, smem_fwd(HD), (cudaStream_t)stream)          \
+             : launch_flash<flash_fwd_kernel<HD, MSK, DRP, false>>(P, grid, smem_fwd(HD), (cudaStream_t)stream))
+#define RTP_FLASH_BWD(HD, MSK, DRP)                                                                                     \
+  (kind == 2   ? launch_flash<flash_bwd_kernel<HD, MSK, DRP, false, true>>(P, grid, smem_bwd(HD), (cudaStream_t)stream) \
+   : kind == 1 ? launch_flash<flash_bwd_kernel<HD, MSK, DRP, true>>(P, grid, smem_bwd(HD), (cudaStream_t)stream)        \
+               : launch_flash<flash_bwd_kernel<HD, MSK, DRP, false>>(P, grid, smem_bwd(HD), (cudaStream_t)stream))
+#define RTP_FLASH_PART_FN(NAME, LAUNCH, HD)                                                              \
+  extern "C" int NAME(const void* params, int mask, int drp, int kind, int grid, void* stream) {         \
+    const FlashParams& P = *reinterpret_cast<const FlashParams*>(params);                                \
+    return (int)(mask == 2   ? (drp ? LAUNCH(HD, 2, true) : LAUNCH(HD, 2, false))                        \
+                 : mask == 1 ? (drp ? LAUNCH(HD, 1, true) : LAUNCH(HD, 1, false))                        \
+                             : (drp ? LAUNCH(HD, 0, true) : LAUNCH(HD, 0, false)));                      \
   }
-
 
 }  // namespace
 
 // Launches a variant with the FlashParams at `params`; returns a cudaError_t.
-typedef int FlashPart(const void* params, int mask, int drp, int more, int grid, void* stream);
+typedef int FlashPart(const void* params, int mask, int drp, int kind, int grid, void* stream);
 extern "C" {
 FlashPart rtp_flash_part_fwd64;
 FlashPart rtp_flash_part_fwd128;
@@ -1257,16 +1280,16 @@ FlashPart rtp_flash_part_bwd64;
 FlashPart rtp_flash_part_bwd128;
 }
 #if RTP_FLASH_HAS(0)
-RTP_FLASH_PART_FN(rtp_flash_part_fwd64, flash_fwd_kernel, smem_fwd, 64)
+RTP_FLASH_PART_FN(rtp_flash_part_fwd64, RTP_FLASH_FWD, 64)
 #endif
 #if RTP_FLASH_HAS(1)
-RTP_FLASH_PART_FN(rtp_flash_part_fwd128, flash_fwd_kernel, smem_fwd, 128)
+RTP_FLASH_PART_FN(rtp_flash_part_fwd128, RTP_FLASH_FWD, 128)
 #endif
 #if RTP_FLASH_HAS(2)
-RTP_FLASH_PART_FN(rtp_flash_part_bwd64, flash_bwd_kernel, smem_bwd, 64)
+RTP_FLASH_PART_FN(rtp_flash_part_bwd64, RTP_FLASH_BWD, 64)
 #endif
 #if RTP_FLASH_HAS(3)
-RTP_FLASH_PART_FN(rtp_flash_part_bwd128, flash_bwd_kernel, smem_bwd, 128)
+RTP_FLASH_PART_FN(rtp_flash_part_bwd128, RTP_FLASH_BWD, 128)
 #endif
 
 #if RTP_FLASH_HAS(0)
@@ -1395,15 +1418,19 @@ int rtp_flash_bwd(const RtpFlashArgs* a, void* stream) {
     return -1;
   if (make_map3(&P.mdo, &P.do_seq1, a->dout, a->B, a->Sq, "dout")) return -1;
   P.dout = dref(a->dout); P.dq = dref(a->dq); P.dk = dref(a->dk); P.dv = dref(a->dv);
-  const int grid = ((a->Sq + kBlk - 1) / kBlk + (a->Sk + kBlk - 1) / kBlk) * a->B * a->H;
-  const bool more = grid > 2 * device_sms();   // one or two rounds are over sooner without (16 heads of 1024 x 1024: 55 us, 60)
+  const int BH = a->B * a->H;
+  // Heads of one block of keys and of queries are a CTA each where two would be two rounds.  us, two -> one: 128 heads of 64 x 64 x 64
+  // 16.2 -> 12.8, of 128 x 128 x 128 20.8 -> 15.8; 64 heads, one round either way, 11.2 -> 11.5 and (64 x 64 x 128) 13.7 -> 16.2.
+  const bool one = a->Sq <= kBlk && a->Sk <= kBlk && BH <= device_sms() && 2 * BH > device_sms();
+  const int grid = one ? BH : ((a->Sq + kBlk - 1) / kBlk + (a->Sk + kBlk - 1) / kBlk) * BH;
+  const int kind = one ? 2 : grid > 2 * device_sms();   // one or two rounds are over sooner without (16 heads of 1024 x 1024: 55 us, 60)
   cudaStream_t s = (cudaStream_t)stream;
-  P.group = head_group(4ll * (a->Sq + a->Sk) * a->head_dim, a->B * a->H);
+  P.group = one ? BH : head_group(4ll * (a->Sq + a->Sk) * a->head_dim, BH);
   const long long rows = (long long)a->B * a->Sq * a->H, per = 256 / (a->head_dim / 8);
   const cudaError_t e = launch_k(a->head_dim == 64 ? flash_delta_kernel<64> : flash_delta_kernel<128>,
                                  dim3((unsigned)((rows + per - 1) / per)), dim3(256), 0, s, P.o, P.dout, P.delta, a->Sq, a->H, rows);
   if (e != cudaSuccess) return ffail(std::string("flash_delta: ") + cudaGetErrorString(e));
-  return launched((a->head_dim == 64 ? rtp_flash_part_bwd64 : rtp_flash_part_bwd128)(&P, mask_kind(a), P.m.thresh != 0, more, grid, stream),
+  return launched((a->head_dim == 64 ? rtp_flash_part_bwd64 : rtp_flash_part_bwd128)(&P, mask_kind(a), P.m.thresh != 0, kind, grid, stream),
                   "flash_bwd");
 }
 

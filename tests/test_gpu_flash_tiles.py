@@ -67,3 +67,46 @@ def test_repeats_are_equal(B, H, S):
         o = flash_attention(q, k, v, causal=True)
         runs.append([o.detach(), *torch.autograd.grad(o, (q, k, v), do)])
     assert all(torch.equal(a, b) for a, b in zip(*runs))
+
+
+@pytest.mark.parametrize("B,H,Sq,Sk,hd,causal,pad", [
+    (10, 8, 64, 64, 64, True, False), (10, 8, 1, 128, 64, False, False), (37, 4, 128, 128, 128, True, False),
+    (25, 3, 127, 65, 64, False, True), (9, 16, 65, 127, 128, False, True), (8, 16, 100, 100, 128, True, False)])
+def test_one_head_a_cta(B, H, Sq, Sk, hd, causal, pad):
+    """Heads of one block of keys and of queries, more than half as many as SMs and no more than SMs.  Padding leaves every batch entry
+    half of its keys: with a single one dS is 0 and what is left of it the rounding of two fp32 sums, which no norm measures."""
+    from rtp_b200.ops import _lib
+    from rtp_b200.ops.flash import flash_attention
+    g = torch.Generator(device="cuda").manual_seed(B * 1000 + Sq)
+    q, do = (torch.randn(B, Sq, H, hd, generator=g, device="cuda").to(BF) for _ in range(2))
+    k, v = (torch.randn(B, Sk, H, hd, generator=g, device="cuda").to(BF) for _ in range(2))
+    kpm = torch.arange(Sk, device="cuda")[None] >= torch.randint(Sk // 2, Sk + 1, (B, 1), generator=g, device="cuda") if pad else None
+    for t in (q, k, v):
+        t.requires_grad_()
+    o = flash_attention(q, k, v, causal=causal, key_padding_mask=kpm)
+    got = [o.detach(), *torch.autograd.grad(o, (q, k, v), do)]
+    _lib.check_status()
+    for name, x, r in zip(("o", "dq", "dk", "dv"), got, exact(q.detach(), k.detach(), v.detach(), do, causal, kpm)):
+        assert x.isfinite().all(), name
+        assert ((x.double() - r).norm() <= 2.0 ** -7 * r.norm()).item(), (name, ((x.double() - r).norm() / r.norm()).item())
+        e, n = (x.double() - r).norm(dim=(1, 3)), r.norm(dim=(1, 3))          # head by head
+        assert bool((e <= 2.0 ** -6 * n).all()), (name, (e / n).max().item())
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("masked", [False, True])
+def test_one_head_a_cta_with_dropout(hd, masked):
+    """The same heads in a launch of few, which takes two CTAs a head: the same dropout bits, the same results (P and dS are rounded to
+    bf16 from sums in another orientation: 2^-7 of the norm)."""
+    from rtp_b200.ops.flash import flash_attention
+    g = torch.Generator(device="cuda").manual_seed(hd)
+    q, k, v, do = (torch.randn(10, 100, 8, hd, generator=g, device="cuda").to(BF) for _ in range(4))
+    mask = torch.randn(100, 100, generator=g, device="cuda") if masked else None
+
+    def run(n):
+        x, y, z = (t[:n].clone().requires_grad_() for t in (q, k, v))
+        o = flash_attention(x, y, z, attn_mask=mask, causal=not masked, dropout_p=0.2, seed=3, offset=9)
+        return [o.detach(), *torch.autograd.grad(o, (x, y, z), do[:n])]
+    for a, b in zip(run(10), run(4)):
+        a, b = a[:4].double(), b.double()
+        assert b.norm() > 0 and ((a - b).norm() <= 2.0 ** -7 * b.norm()).item()
